@@ -1053,10 +1053,10 @@ static int capture(abm_ctx* c, void (*fn)(abm_ctx*), cudaGraphExec_t* exec)
 }
 
 // division body (after the flag count): ranks, room checks on a fresh cell list,
-// the ten tries, commit, then the neighbor rebuild the reference does after any
+// up to ten tries, commit, then the neighbor rebuild the reference does after any
 // division (simulation.hpp:1654-1660)
-// the body up to the room checks (before the tries)
-static void enqueue_division_setup(abm_ctx* c)
+// the body up to the first try; use_cond: `cond` is set when further tries are needed
+static void enqueue_division_setup(abm_ctx* c, unsigned long long cond, int use_cond)
 {
     cudaStream_t st = c->st;
     launch_scan(c->div_flags, &c->ctrl->n, c->div_rank, c->scan_sums, c->cap, st);
@@ -1066,8 +1066,16 @@ static void enqueue_division_setup(abm_ctx* c)
     launch_bin_count(c->geom, c->ctrl, c->grid, c->bin_count, c->key, c->slot, c->cap, st);
     launch_scan(c->bin_count, &c->grid->nbins, c->bin_start, c->scan_sums, c->cap_bins, st);
     launch_bin_scatter(c->geom, c->ctrl, c->bin_start, c->key, c->slot, c->sorted_cell, c->sorted_geom, c->cap, st);
-    launch_div_check(c->geom, c->ctrl, c->dp, c->grid, c->bin_start, c->sorted_cell, c->sorted_geom, c->div_flags,
-                     c->mothers, c->div_check, c->div_sat, st);
+    launch_div_first(c->geom, c->phys, c->ctrl, c->dp, c->grid, c->bin_start, c->sorted_cell, c->sorted_geom,
+                     c->div_flags, c->mothers, c->div_check, c->div_sat, c->d1, c->d2, c->dlen, c->dgrowth,
+                     c->div_ok, cond, use_cond, st);
+}
+
+static void enqueue_division_try(abm_ctx* c, int tr, unsigned long long cond, int use_cond)
+{
+    launch_div_try_round(c->geom, c->phys, c->ctrl, c->dp, c->grid, c->bin_start, c->sorted_cell, c->sorted_geom,
+                         c->div_flags, c->mothers, c->div_check, c->div_sat, c->d1, c->d2, c->dlen, c->dgrowth,
+                         c->div_ok, tr, cond, use_cond, c->st);
 }
 
 static void enqueue_division_commit(abm_ctx* c)
@@ -1080,10 +1088,8 @@ static void enqueue_division_commit(abm_ctx* c)
 // criterion holds for every dividing cell): the paths without conditional nodes
 static void enqueue_division_body(abm_ctx* c)
 {
-    enqueue_division_setup(c);
-    launch_div_tries(c->geom, c->phys, c->ctrl, c->dp, c->grid, c->bin_start, c->sorted_cell, c->sorted_geom,
-                     c->div_flags, c->mothers, c->div_check, c->div_sat, c->d1, c->d2, c->dlen, c->dgrowth,
-                     c->div_ok, c->st);
+    enqueue_division_setup(c, 0, 0);
+    for (int tr = 1; tr < max_division_tries(); ++tr) enqueue_division_try(c, tr, 0, 0);
     enqueue_division_commit(c);
 }
 
@@ -1123,25 +1129,21 @@ static int add_conditional(abm_ctx* c, cudaGraph_t graph, std::vector<cudaGraphN
     return ABM_OK;
 }
 
-// the body in a graph: the tries as a WHILE node that runs them until the distance
-// criterion holds for every dividing cell or ten have run (growth.hpp:252), then the
-// commit and the neighbor rebuild
+// the body in a graph: the first try, then a WHILE node that runs further ones until the
+// distance criterion holds for every dividing cell or ten have run (growth.hpp:252), then
+// the commit and the neighbor rebuild
 static int capture_division_body(abm_ctx* c, cudaGraph_t body)
 {
     std::vector<cudaGraphNode_t> bd;
-    int rc = capture_into(c, body, bd, [&]() { enqueue_division_setup(c); });
-    if (rc) return rc;
     cudaGraphConditionalHandle h_try = 0;
-    CK(cudaGraphConditionalHandleCreate(&h_try, body, 1, cudaGraphCondAssignDefault));   // the first try always runs
+    CK(cudaGraphConditionalHandleCreate(&h_try, body, 0, cudaGraphCondAssignDefault));
+    int rc = capture_into(c, body, bd, [&]() { enqueue_division_setup(c, h_try, 1); });
+    if (rc) return rc;
     cudaGraph_t tries;
     rc = add_conditional(c, body, bd, h_try, cudaGraphCondTypeWhile, &tries);
     if (rc) return rc;
     std::vector<cudaGraphNode_t> tb;
-    rc = capture_into(c, tries, tb, [&]() {
-        launch_div_try_round(c->geom, c->phys, c->ctrl, c->dp, c->grid, c->bin_start, c->sorted_cell,
-                             c->sorted_geom, c->div_flags, c->mothers, c->div_check, c->div_sat, c->d1, c->d2,
-                             c->dlen, c->dgrowth, c->div_ok, h_try, c->st);
-    });
+    rc = capture_into(c, tries, tb, [&]() { enqueue_division_try(c, -1, h_try, 1); });
     if (rc) return rc;
     return capture_into(c, body, bd, [&]() { enqueue_division_commit(c); enqueue_rebuild(c); });
 }

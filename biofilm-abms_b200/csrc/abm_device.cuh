@@ -71,6 +71,15 @@ __device__ __forceinline__ bool may_touch(const Geom& a, const Geom& b, double l
     return !(gap > limit + 1e-9);
 }
 
+// How far a segment reaches from its centre, in FP32: every computed distance vector joins
+// points r1 + s n1 and r2 + t n2 with |s| <= h1, |t| <= h2, so |d| >= |r2 - r1| less both
+// reaches, up to rounding.
+__device__ __forceinline__ float segment_reach(double h, double nx, double ny, double nz)
+{
+    const float n2 = (float)(nx * nx + ny * ny + nz * nz);
+    return (float)h * fmaxf(1.f, n2 * 1.000001f);
+}
+
 // ---------------------------------------------------------------------------
 // Exact-rounding vector arithmetic.  The neighbor decision |d| < threshold
 // must come out identically on the GPU and in the CPU restatement, so the

@@ -451,12 +451,6 @@ struct PbShared {
     int q_own[PB_WARPS][64], q_pos[PB_WARPS][64];
 };
 
-__device__ __forceinline__ float pb_reach(double h, double nx, double ny, double nz)
-{
-    const float n2 = (float)(nx * nx + ny * ny + nz * nz);
-    return (float)h * fmaxf(1.f, n2 * 1.000001f);
-}
-
 // exact tests for one queued (own, candidate) product
 __device__ __forceinline__ void pb_exact(const Geom* __restrict__ sorted_geom, const int* __restrict__ sorted_cell,
                                          int base, int own, int pos, const BuildParams& bp, PbShared& sh,
@@ -506,7 +500,7 @@ __global__ void __launch_bounds__(PB_T) k_pair_build(const Grid* grid, const int
             {
                 const Geom x = sorted_geom[base + q];
                 sh.rx[q] = x.rx; sh.ry[q] = x.ry; sh.rz[q] = x.rz;
-                sh.reach[q] = pb_reach(x.h, x.nx, x.ny, x.nz);
+                sh.reach[q] = segment_reach(x.h, x.nx, x.ny, x.nz);
                 sh.cnt[q] = 0;
             }
             __syncthreads();
@@ -556,7 +550,7 @@ __global__ void __launch_bounds__(PB_T) k_pair_build(const Grid* grid, const int
                                     const float fy = (float)(cy - sh.ry[own]);
                                     const float fz = (float)(cz - sh.rz[own]);
                                     const float L = thr + sh.reach[own]
-                                                    + pb_reach(__ldg(&c.h), __ldg(&c.nx), __ldg(&c.ny), __ldg(&c.nz));
+                                                    + segment_reach(__ldg(&c.h), __ldg(&c.nx), __ldg(&c.ny), __ldg(&c.nz));
                                     pass = !(fx * fx + fy * fy + fz * fz > L * L);
                                 }
                             }

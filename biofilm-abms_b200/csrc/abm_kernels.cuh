@@ -318,17 +318,16 @@ void launch_div_count(const Phys* phys, Ctrl* ctrl, const DivideParams& dp, int*
                       unsigned long long cond, int use_cond, cudaStream_t st);
 void launch_div_body_pre(Ctrl* ctrl, const int* flags, const int* rank, int* mothers, int cap_cells,
                          cudaStream_t st);
-void launch_div_check(const Geom* geom, Ctrl* ctrl, const DivideParams& dp, const Grid* grid,
+// room checks and the first try; use_cond: `cond` is set while a further try is needed
+void launch_div_first(const Geom* geom, const Phys* phys, Ctrl* ctrl, const DivideParams& dp, const Grid* grid,
                       const int* bin_start, const int* sorted_cell, const Geom* sorted_geom, const int* flags,
-                      const int* mothers, int* check, int* sat, cudaStream_t st);
-void launch_div_tries(const Geom* geom, const Phys* phys, Ctrl* ctrl, const DivideParams& dp, const Grid* grid,
-                      const int* bin_start, const int* sorted_cell, const Geom* sorted_geom, const int* flags,
-                      const int* mothers, const int* check, int* sat, Geom* d1, Geom* d2, double* dlen,
-                      double* dgrowth, int* ok, cudaStream_t st);
+                      const int* mothers, int* check, int* sat, Geom* d1, Geom* d2, double* dlen, double* dgrowth,
+                      int* ok, unsigned long long cond, int use_cond, cudaStream_t st);
 void launch_div_try_round(const Geom* geom, const Phys* phys, Ctrl* ctrl, const DivideParams& dp, const Grid* grid,
                           const int* bin_start, const int* sorted_cell, const Geom* sorted_geom, const int* flags,
                           const int* mothers, const int* check, int* sat, Geom* d1, Geom* d2, double* dlen,
-                          double* dgrowth, int* ok, unsigned long long cond, cudaStream_t st);
+                          double* dgrowth, int* ok, int tr, unsigned long long cond, int use_cond, cudaStream_t st);
+int max_division_tries();
 void launch_div_commit(Geom* geom, Vel* vel, Phys* phys, Ctrl* ctrl, const DivideParams& dp, const int* mothers,
                        const Geom* d1, const Geom* d2, const double* dlen, const double* dgrowth, int* parents,
                        cudaStream_t st);
