@@ -41,6 +41,11 @@ struct abm_ctx {
     int *lower_end = nullptr, *rev = nullptr;
     int4* pairs = nullptr;                                           // screened pair pass
     int *pair_start = nullptr, *surv = nullptr;
+    int4* act = nullptr;                                             // active pairs (ActiveList)
+    int* n_act = nullptr;
+    unsigned char* keep_entry = nullptr;
+    Geom* gref = nullptr;
+    GridBar* bar = nullptr;
     double4* jbuf = nullptr;
     int* scan_sums = nullptr;
     double *jkr_delta = nullptr, *jkr_radius = nullptr;
@@ -199,7 +204,8 @@ static void free_all(abm_ctx* c)
     if (c->g_rebuild) cudaGraphExecDestroy(c->g_rebuild);
     void* ptrs[] = {c->geom, c->vel, c->phys, c->fcc, c->geom_c, c->vel_c, c->gen_tmp, c->k0buf, c->ctrl, c->grid,
                     c->bbox_acc, c->bbox_counter, c->bin_count, c->bin_start, c->key, c->slot,
-                    c->sorted_cell, c->sorted_geom, c->scratch, c->nbr_count, c->row_ptr, c->col, c->lower_end, c->rev, c->pairs, c->pair_start, c->surv, c->jbuf,
+                    c->sorted_cell, c->sorted_geom, c->scratch, c->nbr_count, c->row_ptr, c->col, c->lower_end, c->rev, c->pairs, c->pair_start, c->surv,
+                    c->act, c->n_act, c->keep_entry, c->gref, c->bar,c->jbuf,
                     c->scan_sums, c->jkr_delta, c->jkr_radius, c->jkr_gam, c->jkr_rad2, c->staging, c->div_flags, c->div_rank,
                     c->mothers, c->div_check, c->div_sat, c->div_ok, c->parents_dev, c->d1, c->d2, c->dlen,
                     c->dgrowth, c->mlp_w, c->log_buf, c->adhere, c->stat_part, c->order, c->order_flag,
@@ -344,6 +350,12 @@ int abm_create(const abm_params* q, abm_ctx** out)
     CK(cudaMalloc(&c->rev, cap * c->cap_nbr * sizeof(int)));
     CK(cudaMalloc(&c->pairs, cap * c->cap_nbr / 2 * sizeof(int4) + sizeof(int4)));
     CK(cudaMalloc(&c->surv, cap * c->cap_nbr / 2 * sizeof(int) + sizeof(int)));
+    CK(cudaMalloc(&c->act, cap * c->cap_nbr / 2 * sizeof(int4) + sizeof(int4)));
+    CK(cudaMalloc(&c->n_act, cap * sizeof(int)));
+    CK(cudaMalloc(&c->keep_entry, cap * c->cap_nbr));
+    CK(cudaMalloc(&c->gref, cap * sizeof(Geom)));
+    CK(cudaMalloc(&c->bar, sizeof(GridBar)));
+    CK(cudaMemset(c->bar, 0, sizeof(GridBar)));
     CK(cudaMalloc(&c->pair_start, (cap + 1) * sizeof(int)));
     CK(cudaMalloc(&c->jbuf, cap * c->cap_nbr * sizeof(double4)));
     CK(cudaMemset(c->lower_end, 0, cap * sizeof(int)));
@@ -374,6 +386,7 @@ int abm_create(const abm_params* q, abm_ctx** out)
     // parameters of the kernels
     MechParams mp;
     mp.R = p.R; mp.Rcell = p.Rcell; mp.E0 = p.E0; mp.Ecell = p.Ecell; mp.sqrtR = std::sqrt(p.R);
+    mp.invR = 1.0 / p.R;
     mp.nz_threshold = p.nz_threshold; mp.coulomb = p.cell_surface_coulomb_coeff; mp.no_surface = p.no_surface;
     StepParams& sp = c->sp;
     sp.mp = mp;
@@ -530,6 +543,7 @@ static int check_status(abm_ctx* c)
     if (h.status & ST_NBR_OVERFLOW) return fail(c, ABM_ERR_CAPACITY, "neighbors per cell exceed cap_neighbors_per_cell");
     if (h.status & ST_BIN_OVERFLOW) return fail(c, ABM_ERR_CAPACITY, "cell-list grid exceeds the bin capacity");
     if (h.status & ST_CELL_OVERFLOW) return fail(c, ABM_ERR_CAPACITY, "division exceeds cap_cells");
+    if (h.status & ST_BARRIER) return fail(c, ABM_ERR_CUDA, "the blocks of a cooperative launch lost one another");
     return ABM_OK;
 }
 
@@ -962,10 +976,11 @@ static void enqueue_rebuild(abm_ctx* c)
 // step-size features (and, learned, the proposed dt)
 static void enqueue_pair_force(abm_ctx* c, int with_gather, bool in_loop = false)
 {
-    launch_pair_screened(c->geom, c->row_ptr, c->lower_end, c->col, c->rev, c->ctrl, c->fp,
-                         c->jkr_delta, c->jkr_radius, c->fcc, c->jbuf, c->p.precision == ABM_PRECISION_MIXED,
-                         c->cap * c->cap_nbr, c->cap, c->num_sms, c->st, with_gather, c->dims, c->p.pair_tile,
-                         c->p.pair_blocks_per_sm, c->pairs, c->surv, in_loop ? &c->sp : nullptr, c->mlp_w);
+    ActiveList al = {c->act, c->n_act, c->keep_entry, c->gref, c->row_ptr, c->bar};
+    launch_pair_screened(c->geom, c->ctrl, c->fp, c->jkr_delta, c->jkr_radius, c->fcc, c->jbuf,
+                         c->p.precision == ABM_PRECISION_MIXED, c->cap * c->cap_nbr, c->cap, c->num_sms, c->st,
+                         with_gather, c->dims, c->p.pair_tile, c->p.pair_blocks_per_sm, c->pairs, c->surv, al,
+                         in_loop ? &c->sp : nullptr, c->mlp_w);
 }
 
 // pair_sum 1 (default): the first attempt sums each cell's shares itself; 2: a
@@ -976,24 +991,26 @@ static bool sum_in_attempt(abm_ctx* c) { return c->p.pair_sum != 2; }
 // makes them, and the step-size proposal
 static void enqueue_loop_pair_force(abm_ctx* c) { enqueue_pair_force(c, sum_in_attempt(c) ? 0 : 1, true); }
 
-// where the attempts of one iteration find the pair force
-static PairGather loop_gather(abm_ctx* c)
+// the attempts of one iteration: the state, and where they find the pair force
+static AttemptArgs loop_attempt(abm_ctx* c)
 {
     const bool f32 = c->p.precision == ABM_PRECISION_MIXED && c->dims == 3;
-    PairGather pg = {sum_in_attempt(c) ? (f32 ? 3 : 2) : 0, c->row_ptr, c->lower_end, c->jbuf, c->fcc,
-                     c->fbuf, c->fmask, c->ystage, c->cap};
-    return pg;
+    AttemptArgs a{};
+    a.geom = c->geom; a.vel = c->vel; a.phys = c->phys; a.fcc = c->fcc; a.ctrl = c->ctrl; a.sp = &c->sp;
+    a.geom_c = c->geom_c; a.vel_c = c->vel_c; a.k0buf = c->k0buf; a.cap_cells = c->cap;
+    a.pg = {sum_in_attempt(c) ? (f32 ? 3 : 2) : 0, c->row_ptr, c->n_act, c->jbuf, c->fcc, c->gref,
+            c->fbuf, c->fmask, c->ystage, c->cap};
+    return a;
 }
 
-// friction with a surface: the trial passes and decision checks that precede an attempt
-// of kind `kind` (no candidates without a surface)
-static void enqueue_friction_rounds(abm_ctx* c, int kind, PairGather pg, double eval_dt = 0.0, int eval_attempt = 0)
+// an attempt of kind `kind`, preceded (friction with a surface) by the trial passes and
+// decision checks that settle its planar contacts (no candidates without a surface)
+static void enqueue_attempt(abm_ctx* c, int kind, const AttemptArgs& a)
 {
-    if (!c->sp.fric || !c->fp.surface || c->verlet) return;
-    launch_friction_rounds(kind, c->geom, c->vel, c->phys, c->fcc, c->ctrl, c->sp, c->geom_c, c->vel_c, c->k0buf,
-                           eval_dt, eval_attempt, c->cap, c->st, pg, c->pairs, c->fr_list, c->fmask, c->p.R);
+    if (c->sp.fric && c->fp.surface && !c->verlet)
+        launch_friction_rounds(kind, a, c->act, c->fr_list, c->fmask, c->p.R, c->st);
+    launch_attempt(kind, a, c->dims, c->st);
 }
-
 
 // one velocity-Verlet step (integration mode 0) at the context's dt, growth included
 static void enqueue_verlet_step(abm_ctx* c)
@@ -1005,20 +1022,10 @@ static void enqueue_verlet_step(abm_ctx* c)
 
 static void enqueue_attempts(abm_ctx* c)
 {
-    cudaStream_t st = c->st;
-    PairGather pg = loop_gather(c);
-    enqueue_friction_rounds(c, MODE_TRIAL, pg);
-    launch_attempt(MODE_TRIAL, c->geom, c->vel, c->phys, c->fcc, c->ctrl, c->sp, c->geom_c, c->vel_c, nullptr,
-                   c->k0buf, 0.0, 0, c->cap, st, 0, 0, pg, c->dims);
-    for (int r = 0; r < c->p.max_tries_update_stepsize; ++r)
-    {
-        enqueue_friction_rounds(c, MODE_RETRY, pg);
-        launch_attempt(MODE_RETRY, c->geom, c->vel, c->phys, c->fcc, c->ctrl, c->sp, c->geom_c, c->vel_c, nullptr,
-                       c->k0buf, 0.0, 0, c->cap, st, 0, 0, pg, c->dims);
-    }
-    enqueue_friction_rounds(c, MODE_FINAL, pg);
-    launch_attempt(MODE_FINAL, c->geom, c->vel, c->phys, c->fcc, c->ctrl, c->sp, c->geom_c, c->vel_c, nullptr,
-                   c->k0buf, 0.0, 0, c->cap, st, 0, 0, pg, c->dims);
+    const AttemptArgs a = loop_attempt(c);
+    enqueue_attempt(c, MODE_TRIAL, a);
+    for (int r = 0; r < c->p.max_tries_update_stepsize; ++r) enqueue_attempt(c, MODE_RETRY, a);
+    enqueue_attempt(c, MODE_FINAL, a);
 }
 
 // the snapshot of a frame marked by this iteration's accepted step (frames enabled)
@@ -1264,25 +1271,22 @@ static int append_iteration(abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode
         if (c->frame_slots > 0) return capture_into(c, G, deps, [&]() { enqueue_frame_snapshot(c); });
         return ABM_OK;
     }
-    PairGather pg = loop_gather(c);
+    AttemptArgs trial = loop_attempt(c);
+    trial.cond = h_retry;
+    trial.use_cond = (retries ? 1 : 0) | (branch ? 2 : 0);
+    trial.cond_run = h_run;
     rc = capture_into(c, G, deps, [&]() {
         enqueue_loop_pair_force(c);
-        enqueue_friction_rounds(c, MODE_TRIAL, pg);
-        launch_attempt(MODE_TRIAL, c->geom, c->vel, c->phys, c->fcc, c->ctrl, c->sp, c->geom_c, c->vel_c, nullptr,
-                       c->k0buf, 0.0, 0, c->cap, c->st, h_retry, (retries ? 1 : 0) | (branch ? 2 : 0), pg, c->dims,
-                       h_run);
+        enqueue_attempt(c, MODE_TRIAL, trial);
     });
     if (rc) return rc;
     auto retry_attempt = [&](int use_cond) {
-        enqueue_friction_rounds(c, MODE_RETRY, pg);
-        launch_attempt(MODE_RETRY, c->geom, c->vel, c->phys, c->fcc, c->ctrl, c->sp, c->geom_c, c->vel_c,
-                       nullptr, c->k0buf, 0.0, 0, c->cap, c->st, h_retry, use_cond, pg, c->dims);
+        AttemptArgs a = loop_attempt(c);
+        a.cond = h_retry;
+        a.use_cond = use_cond;
+        enqueue_attempt(c, MODE_RETRY, a);
     };
-    auto final_attempt = [&]() {
-        enqueue_friction_rounds(c, MODE_FINAL, pg);
-        launch_attempt(MODE_FINAL, c->geom, c->vel, c->phys, c->fcc, c->ctrl, c->sp, c->geom_c, c->vel_c, nullptr,
-                       c->k0buf, 0.0, 0, c->cap, c->st, 0, 0, pg, c->dims);
-    };
+    auto final_attempt = [&]() { enqueue_attempt(c, MODE_FINAL, loop_attempt(c)); };
     if (branch)
     {
         cudaGraph_t body;
@@ -1685,10 +1689,12 @@ int abm_rk_attempt(abm_ctx* c, double dt, int attempt, double* cells_out, double
     if (!c->nbrs_valid) return fail(c, ABM_ERR_STATE, "neighbors not built");
     enqueue_pair_force(c, 1);
     k_clear_eval<<<1, 1, 0, c->st>>>(c->ctrl);
-    PairGather pg = {0, c->row_ptr, c->lower_end, c->jbuf, nullptr, c->fbuf, c->fmask, c->ystage, c->cap};
-    enqueue_friction_rounds(c, 3, pg, dt, attempt);
-    launch_attempt(3, c->geom, c->vel, c->phys, c->fcc, c->ctrl, c->sp, c->geom_c, c->vel_c, c->gen_tmp,
-                   c->k0buf, dt, attempt, c->cap, c->st, 0, 0, pg, c->dims);
+    AttemptArgs a = loop_attempt(c);
+    a.pg.fused = 0;
+    a.err_out = c->gen_tmp;
+    a.eval_dt = dt;
+    a.eval_attempt = attempt;
+    enqueue_attempt(c, 3, a);
     CK(cudaGetLastError());
     const int n = c->n_host;
     if (cells_out && n > 0)
@@ -1944,6 +1950,8 @@ int abm_set_adhesion_flags(abm_ctx* c, const int* flags, int m)
     std::vector<unsigned char> a((size_t)e.back() + 1, 0);
     for (int r = 0; r < m; ++r) a[e[r]] = flags[r] ? 1 : 0;
     CK(cudaMemcpy(c->adhere, a.data(), a.size(), cudaMemcpyHostToDevice));
+    k_screen_stale<<<1, 1, 0, c->st>>>(c->ctrl);       // the active pairs carry the flags
+    CK(cudaGetLastError());
     return ABM_OK;
 }
 

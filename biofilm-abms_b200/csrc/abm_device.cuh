@@ -39,7 +39,8 @@ __device__ __forceinline__ Geom load_geom(const Geom* __restrict__ g, int i)
 }
 
 // Rigorous lower bound test on the distance of two segments: false only when the
-// gap between their projections on the single-precision closest-point direction a,
+// gap between their projections on the unit vector a along the single-precision
+// closest-point direction,
 //     a . (c_b - c_a) - h_a |a . n_a| - h_b |a . n_b|   (FP64),
 // exceeds limit + 1e-9.  For any unit a that gap bounds the distance from below,
 // and the reference's distance (CGAL's minimiser, or the near-parallel branch's
@@ -65,10 +66,10 @@ __device__ __forceinline__ bool may_touch(const Geom& a, const Geom& b, double l
     const double dz = wz + (double)t * b.nz - (double)s * a.nz;
     const double dn = sqrt(dx * dx + dy * dy + dz * dz);
     if (!(dn > 1e-6)) return true;
-    const double ux = dx / dn, uy = dy / dn, uz = dz / dn;
-    const double gap = (ux * wx + uy * wy + uz * wz) - a.h * fabs(ux * a.nx + uy * a.ny + uz * a.nz)
-                       - b.h * fabs(ux * b.nx + uy * b.ny + uz * b.nz);
-    return !(gap > limit + 1e-9);
+    // the gap times dn, so that the direction needs no division
+    const double gap = (dx * wx + dy * wy + dz * wz) - a.h * fabs(dx * a.nx + dy * a.ny + dz * a.nz)
+                       - b.h * fabs(dx * b.nx + dy * b.ny + dz * b.nz);
+    return !(gap > (limit + 1e-9) * dn);
 }
 
 // How far a segment reaches from its centre, in FP32: every computed distance vector joins
@@ -217,9 +218,25 @@ __device__ __forceinline__ Dist dist_geom(const Geom& a, const Geom& b)
                               x3(b.rx, b.ry, b.rz), x3(b.nx, b.ny, b.nz), b.h);
 }
 
+// a . b in FP32 with its roundings fixed: the first two products in the order given
+__device__ __forceinline__ float dot3f(float a0, float b0, float a1, float b1, float a2, float b2)
+{
+    return __fmaf_rn(a2, b2, __fmaf_rn(a0, b0, __fmul_rn(a1, b1)));
+}
+
 // Mixed-precision variant: the generic (skew) branch in FP32, the
-// near-parallel branch (|cos| >= 0.9999, ill-conditioned s, t) in FP64.
-__device__ __forceinline__ Dist dist_geom_mixed(const Geom& a, const Geom& b)
+// near-parallel branch (|cos| >= 0.9999, ill-conditioned s, t) in FP64.  The FP32 products
+// and sums are written with their roundings, so that the result does not depend on where the
+// function is inlined: the learned controller rounds its features to BF16, and a last FP32
+// bit can change the steps it takes.  There are three roundings, equally accurate, one for
+// each kind of pass, as the compiler once contracted them there:
+enum MixedRounding {
+    ROUND_LIST,     // a pass over the active pairs
+    ROUND_STALE,    // such a pass after a stale list (see Ctrl::path): the projections of w
+                    // start from the y product
+    ROUND_ROW,      // the row walk of k_pair_force: h1 n1 rounded before it enters w
+};
+__device__ __forceinline__ Dist dist_geom_mixed(const Geom& a, const Geom& b, int rounding)
 {
     float n1x = (float)a.nx, n1y = (float)a.ny, n1z = (float)a.nz;
     float n2x = (float)b.nx, n2y = (float)b.ny, n2z = (float)b.nz;
@@ -233,24 +250,38 @@ __device__ __forceinline__ Dist dist_geom_mixed(const Geom& a, const Geom& b)
     float rx = (float)(b.rx - a.rx), ry = (float)(b.ry - a.ry), rz = (float)(b.rz - a.rz);
     float h1 = (float)a.h, h2 = (float)b.h;
     // segment 1: -h1 n1 .. +h1 n1 (origin at r1); segment 2: r - h2 n2 .. r + h2 n2
-    float d1x = 2.f * h1 * n1x, d1y = 2.f * h1 * n1y, d1z = 2.f * h1 * n1z;
-    float d2x = 2.f * h2 * n2x, d2y = 2.f * h2 * n2y, d2z = 2.f * h2 * n2z;
-    float p2x = rx - h2 * n2x, p2y = ry - h2 * n2y, p2z = rz - h2 * n2z;
-    float wx = -h1 * n1x - p2x, wy = -h1 * n1y - p2y, wz = -h1 * n1z - p2z;   // p1 - p2
-    float aa = d1x * d1x + d1y * d1y + d1z * d1z;
-    float e = d2x * d2x + d2y * d2y + d2z * d2z;
-    float f = d2x * wx + d2y * wy + d2z * wz;
-    float c = d1x * wx + d1y * wy + d1z * wz;
-    float bb = d1x * d2x + d1y * d2y + d1z * d2z;
+    const float h1d = 2.f * h1, h2d = 2.f * h2;
+    float d1x = __fmul_rn(h1d, n1x), d1y = __fmul_rn(h1d, n1y), d1z = __fmul_rn(h1d, n1z);
+    float d2x = __fmul_rn(h2d, n2x), d2y = __fmul_rn(h2d, n2y), d2z = __fmul_rn(h2d, n2z);
+    float p2x = __fmaf_rn(-h2, n2x, rx), p2y = __fmaf_rn(-h2, n2y, ry), p2z = __fmaf_rn(-h2, n2z, rz);
+    // w = p1 - p2
+    float wx, wy, wz;
+    if (rounding == ROUND_ROW)
+    {
+        wx = __fsub_rn(-__fmul_rn(h1, n1x), p2x);
+        wy = __fsub_rn(-__fmul_rn(h1, n1y), p2y);
+        wz = __fsub_rn(-__fmul_rn(h1, n1z), p2z);
+    }
+    else
+    {
+        wx = __fmaf_rn(-h1, n1x, -p2x); wy = __fmaf_rn(-h1, n1y, -p2y); wz = __fmaf_rn(-h1, n1z, -p2z);
+    }
+    float aa = dot3f(d1x, d1x, d1y, d1y, d1z, d1z);
+    float e = dot3f(d2x, d2x, d2y, d2y, d2z, d2z);
+    float bb = dot3f(d1x, d2x, d1y, d2y, d1z, d2z);
+    const bool swapped = rounding == ROUND_STALE;
+    float f = swapped ? dot3f(d2y, wy, d2x, wx, d2z, wz) : dot3f(d2x, wx, d2y, wy, d2z, wz);
+    float c = swapped ? dot3f(d1y, wy, d1x, wx, d1z, wz) : dot3f(d1x, wx, d1y, wy, d1z, wz);
     float x, y;
     if (aa <= 0.f && e <= 0.f) { x = 0.f; y = 0.f; }
     else if (aa <= 0.f) { x = 0.f; y = fminf(fmaxf(f / e, 0.f), 1.f); }
     else if (e <= 0.f) { y = 0.f; x = fminf(fmaxf(-c / aa, 0.f), 1.f); }
     else
     {
-        float denom = aa * e - bb * bb;
-        float s = denom != 0.f ? fminf(fmaxf((bb * f - c * e) / denom, 0.f), 1.f) : 0.f;
-        float t = (bb * s + f) / e;
+        float denom = __fmaf_rn(aa, e, -__fmul_rn(bb, bb));
+        float num = __fmaf_rn(bb, f, -__fmul_rn(c, e));
+        float s = denom != 0.f ? fminf(fmaxf(num / denom, 0.f), 1.f) : 0.f;
+        float t = __fmaf_rn(bb, s, f) / e;
         if (t < 0.f) { t = 0.f; s = fminf(fmaxf(-c / aa, 0.f), 1.f); }
         else if (t > 1.f) { t = 1.f; s = fminf(fmaxf((bb - c) / aa, 0.f), 1.f); }
         x = s; y = t;
@@ -414,6 +445,7 @@ __device__ __forceinline__ EndPow end_pows(double rz, double nz, double R, doubl
 struct MechParams {
     double R, Rcell, E0, Ecell;
     double sqrtR;
+    double invR;
     double nz_threshold;
     double coulomb;          // cell_surface_coulomb_coeff
     int no_surface;
@@ -430,54 +462,6 @@ __device__ __forceinline__ void surface_dEdq_flat(const MechParams& P, double rz
         rep2 = -(2 * P.E0) * ph * l;
         adh2 = sigma0 * (P.sqrtR / 2) * l / sqrt(ph);
     }
-}
-
-// Cell-surface repulsion + adhesion dE/dq components 2 and 5
-// (mechanics.hpp:673-780 and 800-910, include_constraint = false).
-__device__ __forceinline__ void surface_dEdq(const MechParams& P, bool assume_2d, double rz, double nz,
-                                             double l, double h, double sigma0, double ss,
-                                             const EndPow& w, double& rep2, double& rep5,
-                                             double& adh2, double& adh5)
-{
-    const double R = P.R, E0 = P.E0;
-    rep2 = rep5 = adh2 = adh5 = 0.0;
-    if (assume_2d)
-    {
-        surface_dEdq_flat(P, rz, l, sigma0, rep2, adh2);
-        return;
-    }
-    const double pf0 = 2 * E0, pf1 = (8. / 3.) * E0 * P.sqrtR, pf2 = 2 * E0 * P.sqrtR;
-    double nz2 = nz * nz;
-    const double inz = 1.0 / nz;
-    double int1 = integral1(w, inz, h, 4, ss);   // delta
-    double int2 = integral1(w, inz, h, 3, ss);   // sqrt(delta)
-    rep2 = -pf0 * ((1.0 - nz2) * int1 + P.sqrtR * nz2 * int2);
-    double int3 = integral1(w, inz, h, 6, ss);   // delta^2
-    double int4 = integral2(w, inz, h, 4, ss);   // s delta
-    double int5 = integral1(w, inz, h, 5, ss);   // delta^1.5
-    double int6 = integral2(w, inz, h, 3, ss);   // s sqrt(delta)
-    double d5 = 0.0;
-    d5 -= pf0 * nz * int3;
-    d5 -= pf0 * (1 - nz2) * int4;
-    d5 += pf1 * nz * int5;
-    d5 -= pf2 * nz2 * int6;
-    rep5 = d5;
-    // adhesion
-    const double a0 = P.sqrtR / 2, a1 = 2 * M_PI * R, a2 = 2 * P.sqrtR;
-    double i1 = integral1(w, inz, h, 1, ss);     // delta^-1/2
-    bool partial = fabs(ss) < h;
-    double term2 = partial ? (a1 / 2) * nz : 0.0;
-    adh2 = (a0 * (1 - nz2) * i1 + term2) * sigma0;
-    double i2 = integral1(w, inz, h, 3, ss);     // delta^1/2
-    double i3 = integral2(w, inz, h, 1, ss);     // s delta^-1/2
-    double i4 = (ss > h) ? 2 * h : ((ss > -h) ? ss + h : 0.0);   // integral4
-    double term4 = partial ? (a1 / 2) * (R - rz) : 0.0;
-    double e5 = 0.0;
-    e5 += a2 * nz * i2;
-    e5 += a0 * (1 - nz2) * i3;
-    e5 -= a1 * nz * i4;
-    e5 += term4;
-    adh5 = e5 * sigma0;
 }
 
 // integrals.hpp:400-463 (areaIntegrals)
@@ -510,6 +494,57 @@ __device__ __forceinline__ bool surface_contact(const MechParams& P, bool assume
 {
     if (!assume_2d) return (y[2] - h * y[5] < P.R) || (y[2] + h * y[5] < P.R);
     return y[2] < P.R;
+}
+
+// x / b for a divisor b used many times, from its reciprocal r = 1.0 / b: with r correctly
+// rounded, q0 = x r and one correction by the exact remainder give the correctly rounded
+// quotient (Markstein, IBM J. Res. Dev. 34 (1990) 111, theorem 8; finite b != 0, no
+// underflow), so the result is the bits of x / b at three operations instead of a division.
+__device__ __forceinline__ double div_by(double x, double b, double r)
+{
+    const double q = x * r;
+    return fma(fma(-q, b, x), r, q);
+}
+
+// What a cell's velocity needs at every stage of an attempt and that no stage changes: its
+// ambient drags K = eta0 l and L = K l^2 / 12 with their reciprocals, so that a stage
+// multiplies, and |dr_xy|, |dn_xy| of the stored velocity (Coulomb truncation), read on the
+// first stage in surface contact (negative: not yet read).
+struct CellDrag {
+    double K, L, iK, iL;
+    double drxy, dnxy;
+};
+
+__device__ __forceinline__ CellDrag cell_drag(double l, double eta0)
+{
+    CellDrag d;
+    d.K = eta0 * l;
+    d.L = d.K * l * l / 12;
+    d.iK = 1.0 / d.K;
+    d.iL = 1.0 / d.L;
+    d.drxy = d.dnxy = -1.0;
+    return d;
+}
+
+__device__ __forceinline__ void stored_speeds(CellDrag& d, const Vel* __restrict__ drp)
+{
+    if (d.drxy >= 0.0) return;
+    const double2 d01 = __ldg(reinterpret_cast<const double2*>(drp->v));
+    const double2 d23 = __ldg(reinterpret_cast<const double2*>(drp->v) + 1);
+    const double2 d45 = __ldg(reinterpret_cast<const double2*>(drp->v) + 2);
+    d.drxy = sqrt(d01.x * d01.x + d01.y * d01.y);
+    d.dnxy = sqrt(d23.y * d23.y + d45.x * d45.x);
+}
+
+// A cell clear of the surface (first branch of getVelocities, mechanics.hpp:2011-2100)
+__device__ __forceinline__ void velocity_free(const double y[6], const CellDrag& d, const double f[6], double v[6])
+{
+    const double nx = y[3], ny = y[4], nz = y[5];
+    const double mult = -((nx * f[3] + ny * f[4]) + nz * f[5]);
+    v[0] = div_by(f[0], d.K, d.iK); v[1] = div_by(f[1], d.K, d.iK); v[2] = div_by(f[2], d.K, d.iK);
+    v[3] = div_by(f[3] + mult * nx, d.L, d.iL);
+    v[4] = div_by(f[4] + mult * ny, d.L, d.iL);
+    v[5] = div_by(f[5] + mult * nz, d.L, d.iL);
 }
 
 // The first two branches of getVelocities (mechanics.hpp:2011-2189): a cell clear of
@@ -561,60 +596,115 @@ __device__ __forceinline__ void velocity_free_or_flat(const MechParams& P, bool 
     }
 }
 
-// Velocity of one cell from its generalised force (mechanics.hpp:2011-2347,
-// the three branches: no surface contact, horizontal contact, full 3-D contact).
-// dr, dn: stored velocities of the previous accepted step (Coulomb truncation).
-__device__ __forceinline__ void velocity_solve(const MechParams& P, bool assume_2d, const double y[6],
-                                               double l, double h, double eta0, double eta1_in,
-                                               double ss, const EndPow& w, const Vel* __restrict__ drp,
-                                               const double f[6], double v[6])
+// A tilted cell at or near the surface: cell-surface repulsion and adhesion
+// (mechanics.hpp:673-780 and 800-910, include_constraint = false), the area integrals
+// (integrals.hpp:400-463) and the third branch of getVelocities (mechanics.hpp:2191-2309).
+//
+// A serial chain of FP64 operations per cell bounds the attempts (2600 instructions per
+// warp at 10 cycles each on 2000 cells, no unit busy), so the form is chosen for few
+// operations and few dependent divisions.  With the overlap powers of an end that is clear
+// of the surface set to zero, the three cases of integrals.hpp (both ends in contact, the
+// lower one, none) are one formula: with P_e = p^(e/2), Q_e = q^(e/2),
+//   D_e = int phi^(e/2 - 1) ds   = (P_e - Q_e) / (nz e / 2)
+//   M_e = int s phi^(e/2 - 1) ds = (D_{e+2} - h (P_e + Q_e)) / (nz e / 2)
+// each evaluated once for the forces, the friction and the areas (integral1, integral2).
+// The solve divides by c1 and by the determinant c1 c3 - c5^2 side by side instead of by
+// c1, then c3 - c5^2 / c1.
+// f0: -dE/dq of the pair forces plus noise.
+__device__ __forceinline__ void velocity_tilted(const MechParams& P, const double y[6], double l, double h,
+                                                double eta0, double eta1_in, double sigma0, CellDrag& d,
+                                                const Vel* __restrict__ drp, const double f0[6], double v[6])
 {
-    const double R = P.R, E0 = P.E0, coul = P.coulomb;
-    const double nx = y[3], ny = y[4], nz = y[5];
-    const bool contacting = surface_contact(P, assume_2d, y, h);
-    if (P.no_surface || !contacting || assume_2d)
-        velocity_free_or_flat(P, contacting, y, l, eta0, eta1_in, drp, f, v);
-    else
+    const double R = P.R, E0 = P.E0;
+    const double rz = y[2], nx = y[3], ny = y[4], nz = y[5];
+    const double Rmrz = R - rz;
+    const double inz = 1.0 / nz, ss = Rmrz / nz;
+    const bool both = ss > h, any = ss > -h, partial = fabs(ss) < h;
+    const double p = any ? Rmrz + h * nz : 0.0, q = both ? Rmrz - h * nz : 0.0;
+    const double P1 = sqrt(p), Q1 = sqrt(q);
+    const double P3 = P1 * p, Q3 = Q1 * q, P4 = p * p, Q4 = q * q;
+    const double P5 = P3 * p, Q5 = Q3 * q, P6 = P4 * p, Q6 = Q4 * q, P7 = P5 * p, Q7 = Q5 * q;
+    const double D1 = (P1 - Q1) * inz * 2.0;
+    const double D3 = (P3 - Q3) * inz * (2.0 / 3.0);
+    const double D4 = (P4 - Q4) * inz * 0.5;
+    const double D5 = (P5 - Q5) * inz * (2.0 / 5.0);
+    const double D6 = (P6 - Q6) * inz * (2.0 / 6.0);
+    const double D7 = (P7 - Q7) * inz * (2.0 / 7.0);
+    const double M1 = (D3 - h * (P1 + Q1)) * inz * 2.0;
+    const double M3 = (D5 - h * (P3 + Q3)) * inz * (2.0 / 3.0);
+    const double M4 = (D6 - h * (P4 + Q4)) * inz * 0.5;
+    const double M5 = (D7 - h * (P5 + Q5)) * inz * (2.0 / 5.0);
+    const double nz2 = nz * nz, onz = 1.0 - nz2;
+    const double i4 = both ? 2 * h : (any ? ss + h : 0.0);             // integral4
+    // repulsion and adhesion, components 2 and 5
+    const double pf0 = 2 * E0, pf1 = (8. / 3.) * E0 * P.sqrtR, pf2 = 2 * E0 * P.sqrtR;
+    const double rep_n = onz * D4 + P.sqrtR * nz2 * D3;
+    const double rep2 = -pf0 * rep_n;
+    const double rep5 = pf1 * nz * D5 - pf0 * (nz * D6 + onz * M4) - pf2 * nz2 * M3;
+    const double a0 = P.sqrtR / 2, a1 = 2 * M_PI * R, a2 = 2 * P.sqrtR;
+    const double adh2 = (a0 * onz * D1 + (partial ? (a1 / 2) * nz : 0.0)) * sigma0;
+    const double adh5 = (a2 * nz * D3 + a0 * onz * M1 - a1 * nz * i4 + (partial ? (a1 / 2) * Rmrz : 0.0)) * sigma0;
+    double f[6];
+#pragma unroll
+    for (int c = 0; c < 6; ++c) f[c] = f0[c];
+    f[2] = (f[2] - rep2) - adh2;
+    f[5] = (f[5] - rep5) - adh5;
+    // mechanics.hpp:2080-2090
+    if (!((rz - h * nz < R) || (rz + h * nz < R))) { velocity_free(y, d, f, v); return; }
+    // area integrals
+    const double i5 = (any && !both) ? (ss * ss - h * h) / 2.0 : 0.0;
+    const double i6 = both ? 2 * h * h * h / 3.0 : (any ? (ss * ss * ss + h * h * h) / 3.0 : 0.0);
+    const double piRnz2 = M_PI * R * nz2;
+    const double A1 = P.sqrtR * onz * D3 + piRnz2 * i4;
+    const double A2 = P.sqrtR * onz * M3 + piRnz2 * i5;
+    const double A3 = P.sqrtR * onz * ((2 * M5 + h * h * (P3 - Q3)) * inz * (2.0 / 3.0)) + piRnz2 * i6;
+    double eta1 = eta1_in;
+    if (P.coulomb > 0)
     {
-        double eta1 = eta1_in;
-        double A1, A2, A3;
-        area_integrals(P, nz, h, ss, w, A1, A2, A3);
-        if (coul > 0)
-        {
-            const double2 d01 = __ldg(reinterpret_cast<const double2*>(drp->v));
-            const double2 d23 = __ldg(reinterpret_cast<const double2*>(drp->v) + 1);
-            const double2 d45 = __ldg(reinterpret_cast<const double2*>(drp->v) + 2);
-            double drxy = sqrt(d01.x * d01.x + d01.y * d01.y);
-            double dnxy = sqrt(d23.y * d23.y + d45.x * d45.x);
-            double friction_norm = (A1 * drxy + A2 * dnxy) * (eta1 / R);
-            const double inz = 1.0 / nz;
-            double max_norm = (1 - nz * nz) * integral1(w, inz, h, 4, ss)
-                            + P.sqrtR * nz * nz * integral1(w, inz, h, 3, ss);
-            max_norm *= (2 * E0 * coul);
-            if (friction_norm > max_norm) eta1 = max_norm * R / (A1 * drxy + A2 * dnxy);
-        }
-        const double c1 = eta0 * l + (eta1 / R) * A1;
-        const double c2 = eta0 * l;
-        const double c4 = c2 * l * l / 12;
-        const double c3 = c4 + (eta1 / R) * A3;
-        const double c5 = (eta1 / R) * A2;
-        const double ic1 = 1.0 / c1, ic4 = 1.0 / c4;
-        const double c5c1 = c5 * ic1;
-        const double term1 = c3 - c5 * c5c1;
-        const double it1 = 1.0 / term1;
-        const double w4 = f[3] - f[0] * c5c1;
-        const double w5 = f[4] - f[1] * c5c1;
-        const double nx2 = nx * it1, ny2 = ny * it1, nz2 = nz * ic4;
-        const double alpha = 2 * ((nx * nx2 + ny * ny2) + nz * nz2);
-        const double beta = -((w4 * nx2 + w5 * ny2) + f[5] * nz2);
-        const double lambda = beta / alpha;
-        v[5] = (f[5] + 2 * nz * lambda) * ic4;
-        v[4] = (w5 + 2 * ny * lambda) * it1;
-        v[3] = (w4 + 2 * nx * lambda) * it1;
-        v[2] = f[2] / c2;
-        v[1] = (f[1] - c5 * v[4]) * ic1;
-        v[0] = (f[0] - c5 * v[3]) * ic1;
+        stored_speeds(d, drp);
+        const double slide = A1 * d.drxy + A2 * d.dnxy;
+        const double max_norm = rep_n * (2 * E0 * P.coulomb);
+        if (slide * (eta1 * P.invR) > max_norm) eta1 = max_norm * R / slide;
     }
+    const double eR = eta1 * P.invR;
+    const double c1 = d.K + eR * A1;
+    const double c3 = d.L + eR * A3;
+    const double c5 = eR * A2;
+    const double ic1 = 1.0 / c1, it1 = c1 / (c1 * c3 - c5 * c5);
+    const double c5c1 = c5 * ic1;
+    const double w4 = f[3] - f[0] * c5c1, w5 = f[4] - f[1] * c5c1;
+    // twice the Lagrange multiplier of |n| = 1
+    const double lam = -((w4 * nx + w5 * ny) * it1 + f[5] * nz * d.iL) / ((nx * nx + ny * ny) * it1 + nz2 * d.iL);
+    v[5] = (f[5] + nz * lam) * d.iL;
+    v[4] = (w5 + ny * lam) * it1;
+    v[3] = (w4 + nx * lam) * it1;
+    v[2] = f[2] * d.iK;
+    v[1] = (f[1] - c5 * v[4]) * ic1;
+    v[0] = (f[0] - c5 * v[3]) * ic1;
+}
+
+// getVelocities (mechanics.hpp:2011-2347) of one cell at state y, from f0 = -dE/dq of the
+// pair forces plus noise.  A cell whose lower end is clear of the surface has no surface
+// force and takes the free branch at once; the margin leaves every cell whose contact
+// tests could round either way to velocity_tilted, which makes them.
+__device__ __forceinline__ void cell_velocity_fp64(const MechParams& P, bool a2, const double y[6], double l,
+                                                   double h, double eta0, double eta1, double sigma0, CellDrag& d,
+                                                   const Vel* __restrict__ drp, const double f0[6], double v[6])
+{
+    if (!P.no_surface && a2)
+    {
+        double f[6], rep2 = 0, adh2 = 0;
+        surface_dEdq_flat(P, y[2], l, sigma0, rep2, adh2);
+#pragma unroll
+        for (int c = 0; c < 6; ++c) f[c] = f0[c];
+        f[2] = (f[2] - rep2) - adh2;
+        if (y[2] < P.R) velocity_free_or_flat(P, true, y, l, eta0, eta1, drp, f, v);
+        else velocity_free(y, d, f, v);
+        return;
+    }
+    const bool clear = P.no_surface || y[2] - h * fabs(y[5]) > P.R + 1e-6 * (1.0 + fabs(y[2]));
+    if (clear) velocity_free(y, d, f0, v);
+    else velocity_tilted(P, y, l, h, eta0, eta1, sigma0, d, drp, f0, v);
 }
 
 // ---------------------------------------------------------------------------

@@ -10,14 +10,12 @@
 //                  against an active list with a skin, both shares per pair; the last
 //                  block makes the step-size proposal of the learned controller)
 //                  k_pair_force<G> serves the no-alloc entry point (G lanes per cell)
-//   RK attempt     k_attempt<S, KIND>                                   (stepRungeKuttaAdaptive,
-//                  mechanics.hpp:2406-2612; all stages of a cell in registers, the error
-//                  norm reduced in the same kernel, the step-size controller of
-//                  simulation.hpp:1690-1769 run by the last block to finish)
+//   RK attempt     abm_attempt.cuh
 #include <cstdio>
-#include "abm_kernels.cuh"
+#include "abm_grid.cuh"
 #include "abm_pair.cuh"
 #include "abm_propose.cuh"
+#include "abm_step.cuh"
 
 namespace abm {
 
@@ -152,12 +150,6 @@ void launch_gen6_to_colmajor(const Gen6* g, int n, double* cm, cudaStream_t st)
 // ---------------------------------------------------------------------------
 // Block reductions
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double warp_max(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
 __device__ __forceinline__ double warp_min(double v)
 {
 #pragma unroll
@@ -647,11 +639,11 @@ void launch_csr_fill(const Ctrl* ctrl, const int* row_ptr, const int* scratch, i
 // FP32 variant: segment distance (FP64 near-parallel branch kept), overlap,
 // Hertz / JKR magnitude and direction in single precision
 __device__ __forceinline__ PairOut pair_force_fp32(const Geom& gi, const Geom& gj, const ForceParams& fp,
-                                                   const double* td, const double* tr)
+                                                   const double* td, const double* tr, int rounding)
 {
     PairOut out;
     out.touch = false;
-    Dist d = dist_geom_mixed(gi, gj);
+    Dist d = dist_geom_mixed(gi, gj, rounding);
     // the overlap from the FP64 distance vector, then the force law in FP32
     const double distd = sqrt((d.dx * d.dx + d.dy * d.dy) + d.dz * d.dz);
     const double overlap_d = 2 * fp.R - distd;
@@ -745,7 +737,7 @@ __global__ void __launch_bounds__(PF_T) k_pair_force(const Geom* __restrict__ ge
             const Geom go = load_geom(geom, o);
             PairOut p;
             if (DIM == 2) p = pair_force_2d(gc, go, fp, fp.adhere[k] != 0);
-            else p = MIXED ? pair_force_fp32(gc, go, fp, td, tr) : pair_force_fp64(gc, go, fp, td, tr);
+            else p = MIXED ? pair_force_fp32(gc, go, fp, td, tr, ROUND_ROW) : pair_force_fp64(gc, go, fp, td, tr);
             double4 js = make_double4(0.0, 0.0, 0.0, 0.0);
             if (p.touch)
             {
@@ -878,38 +870,27 @@ void launch_csr_rev(const Ctrl* ctrl, const int* row_ptr, const int* col, int* l
 // ---------------------------------------------------------------------------
 const int PS_T = 256, PS_TILE_MAX = 2048;
 
-template <bool MIXED>
-__device__ __forceinline__ void zero_shares(double4* jbuf, int k, int r)
-{
-    if (MIXED)
-    {
-        float4* fb = reinterpret_cast<float4*>(jbuf);
-        fb[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-        fb[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    else
-    {
-        jbuf[k] = make_double4(0.0, 0.0, 0.0, 0.0);
-        jbuf[r] = make_double4(0.0, 0.0, 0.0, 0.0);
-    }
-}
-
-// One pass per iteration over the pair records.  A refresh iteration (the active
-// list is stale: after a rebuild, an upload or a division, or once the cells may
-// have moved by half the skin since the last refresh, 2 * drift >= skin) screens
-// every pair with the rigorous bound of may_touch, zeroes the shares of the pairs
-// beyond 2R + skin, computes the others and lists them as the new active pairs;
-// the other iterations compute the active pairs only.  A pair left out stays
-// beyond 2R until the next refresh (its distance can fall by at most
-// 2 * drift < skin), so its force is exactly zero in every force law of the
-// reference (all need overlap > 0).  Every share slot is written by exactly one
-// pair, so the order of the active list changes no result.  The last block
-// installs a new list and clears the drift.
+// One pass per iteration.  A refresh iteration (the active list is stale: after a rebuild,
+// an upload or a division, or once some cell has moved by half the skin since the last
+// refresh, 2 * drift >= skin) screens every pair with the rigorous bound of may_touch and
+// lists those that pass as the new active pairs; then, behind a barrier over the pass's
+// blocks, each active pair takes its two share slots (the active entries of a row, in
+// column order, at the row's start) and is computed.  The other iterations compute the
+// active pairs only.  A pair left out stays beyond 2R until the next refresh (its distance
+// can fall by at most 2 * drift < skin), so its force is exactly zero in every force law of
+// the reference (all need overlap > 0), and a row sum over the active entries adds the same
+// terms in the same order.  Every slot is written by exactly one pair, so the order of the
+// active list changes no result.  The last block installs a new list.
+//
+// drift is the largest motion of a cell's segment from where it lay at the refresh, not
+// the sum over the steps of the largest motion in each: in a relaxing 200,000-cell state,
+// where some cell moves 0.05 um in almost every step, the sum refreshed in 20-40 % of the
+// steps (92 us a pass instead of 36).
 // the friction part of a touching pair's shares (FP64): v -= the force on i under the
 // decision at the attempt's positions; a candidate also records the change of v when the
 // decision flips, and is listed for the stage checks
 __device__ __forceinline__ void friction_shares(const Geom& gi, const Geom& gj, const int4& pr, const ForceParams& fp,
-                                                const Dist& d, double dist, double4& own, double4& other)
+                                                const Dist& d, double dist, double4& v)
 {
     const int i = pr.x, j = pr.y;
     const X3 dv = x3(d.dx, d.dy, d.dz);
@@ -927,15 +908,14 @@ __device__ __forceinline__ void friction_shares(const Geom& gi, const Geom& gj, 
     }
     double f[3];
     friction_force(dv, dist, flat0, rv, eta, fp, f);
-    own.x -= f[0]; own.y -= f[1]; own.z -= f[2];
-    other.x -= f[0]; other.y -= f[1]; other.z -= f[2];
+    v.x -= f[0]; v.y -= f[1]; v.z -= f[2];
     if (cand)
     {
         double g[3];
         friction_force(dv, dist, !flat0, rv, eta, fp, g);
         const double4 delta = make_double4(-(g[0] - f[0]), -(g[1] - f[1]), -(g[2] - f[2]), 0.0);
         fp.fbuf[pr.z] = delta;
-        fp.fbuf[pr.w] = delta;
+        fp.fbuf[pr.w] = make_double4(-delta.x, -delta.y, -delta.z, 0.0);
         const int m = FR_CAND | (flat0 ? FR_D0 : 0);
         fp.fmask[pr.z] = m;
         fp.fmask[pr.w] = m;
@@ -947,15 +927,18 @@ __device__ __forceinline__ void friction_shares(const Geom& gi, const Geom& gj, 
     }
 }
 
+// One active pair (pr: i, j, i's slot, j's slot): both shares, the partner's with the minus
+// sign of its force, so that a cell adds all its shares alike.
 template <bool MIXED, int DIM>
-__device__ __forceinline__ void pair_shares(const Geom& gi, const Geom& gj, const int4& pr, const ForceParams& fp,
-                                            const double* __restrict__ td, const double* __restrict__ tr,
-                                            double4* __restrict__ jbuf, double& ovl_max, bool* fr_cand = nullptr)
+__device__ __forceinline__ void pair_shares(const Geom& gi, const Geom& gj, const int4& pr, bool adhere,
+                                            const ForceParams& fp, const double* __restrict__ td,
+                                            const double* __restrict__ tr, double4* __restrict__ jbuf, double& ovl_max,
+                                            bool& fr_cand, int rounding)
 {
     const int k = pr.z, r = pr.w;
     PairOut p;
-    if (DIM == 2) p = pair_force_2d(gi, gj, fp, fp.adhere[k] != 0);
-    else p = MIXED ? pair_force_fp32(gi, gj, fp, td, tr) : pair_force_fp64(gi, gj, fp, td, tr);
+    if (DIM == 2) p = pair_force_2d(gi, gj, fp, adhere);
+    else p = MIXED ? pair_force_fp32(gi, gj, fp, td, tr, rounding) : pair_force_fp64(gi, gj, fp, td, tr);
     if (MIXED)
     {
         // mixed precision: the shares are single-precision forces, stored as such
@@ -964,7 +947,7 @@ __device__ __forceinline__ void pair_shares(const Geom& gi, const Geom& gj, cons
         if (p.touch)
         {
             own = make_float4((float)p.vx, (float)p.vy, (float)p.vz, (float)p.s);
-            other = make_float4((float)p.vx, (float)p.vy, (float)p.vz, (float)p.t);
+            other = make_float4(-own.x, -own.y, -own.z, (float)p.t);
             ovl_max = fmax(ovl_max, p.ovl);
         }
         fb[k] = own;
@@ -972,17 +955,18 @@ __device__ __forceinline__ void pair_shares(const Geom& gi, const Geom& gj, cons
     }
     else
     {
-        double4 own = make_double4(0.0, 0.0, 0.0, 0.0), other = own;
+        double4 own = make_double4(0.0, 0.0, 0.0, 0.0);
+        double t = 0.0;
         if (p.touch)
         {
             own = make_double4(p.vx, p.vy, p.vz, p.s);
-            other = make_double4(p.vx, p.vy, p.vz, p.t);
+            t = p.t;
             ovl_max = fmax(ovl_max, p.ovl);
             if (DIM == 3 && fp.fric)
             {
                 const Dist d = {p.dx, p.dy, p.dz, p.s, p.t};
-                friction_shares(gi, gj, pr, fp, d, p.dist, own, other);
-                if (fr_cand) *fr_cand = (fp.fmask[k] & FR_CAND) != 0;
+                friction_shares(gi, gj, pr, fp, d, p.dist, own);
+                fr_cand = (fp.fmask[k] & FR_CAND) != 0;
             }
         }
         else if (DIM == 3 && fp.fric)
@@ -991,7 +975,7 @@ __device__ __forceinline__ void pair_shares(const Geom& gi, const Geom& gj, cons
             fp.fmask[r] = 0;
         }
         jbuf[k] = own;
-        jbuf[r] = other;
+        jbuf[r] = make_double4(-own.x, -own.y, -own.z, t);
     }
 }
 
@@ -1009,7 +993,7 @@ template <bool MIXED, int DIM, bool PROPOSE>
 __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ geom, const int4* __restrict__ pairs,
                                                       Ctrl* ctrl, ForceParams fp, const double* __restrict__ td,
                                                       const double* __restrict__ tr, double4* __restrict__ jbuf,
-                                                      int* __restrict__ surv, StepParams sp,
+                                                      int* surv, ActiveList al, StepParams sp,
                                                       const float* __restrict__ mlp_w)
 {
     __shared__ bool last;
@@ -1017,7 +1001,9 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
     const bool split = PROPOSE && gridDim.x > 1;
     const bool proposer = split && blockIdx.x == gridDim.x - 1;
     const int work_blocks = split ? gridDim.x - 1 : gridDim.x;
-    const bool refresh = !ctrl->screen_valid || !(2.0 * ctrl->drift * (1.0 + 1e-6) + 1e-9 < fp.skin);
+    auto stale = [&](double moved) { return !ctrl->screen_valid || !(2.0 * moved * (1.0 + 1e-6) + 1e-9 < fp.skin); };
+    const bool refresh = stale(ctrl->drift);
+    const int rounding = MIXED && stale(ctrl->path) ? ROUND_STALE : ROUND_LIST;
     const int lane = threadIdx.x & 31;
     const int stride = work_blocks * blockDim.x;
     double ovl_max = 0.0;
@@ -1025,39 +1011,53 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
         mlp_propose_block(ctrl, sp, mlp_w);
     else if (refresh)
     {
-        const int n_pairs = ctrl->n_dir >> 1;
+        const int n_pairs = ctrl->n_dir >> 1, n = ctrl->n;
         const double limit = 2 * fp.R + fp.skin;
         // warp-uniform rounds, so that every ballot covers all 32 lanes
         for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n_pairs; base += stride)
         {
             const int p = base + lane;
             bool keep = false;
-            int4 pr = make_int4(0, 0, 0, 0);
-            Geom gi, gj;
             if (p < n_pairs)
             {
-                pr = pairs[p];                      // (i, j, lower entry k, partner entry)
-                gi = load_geom(geom, pr.x);
-                gj = load_geom(geom, pr.y);
-                keep = may_touch(gi, gj, limit);
-                if (!keep)
-                {
-                    zero_shares<MIXED>(jbuf, pr.z, pr.w);
-                    if (!MIXED && DIM == 3 && fp.fric) { fp.fmask[pr.z] = 0; fp.fmask[pr.w] = 0; }
-                }
+                const int4 pr = pairs[p];           // (i, j, lower entry k, partner entry)
+                keep = may_touch(load_geom(geom, pr.x), load_geom(geom, pr.y), limit);
+                al.keep[pr.z] = keep;
+                al.keep[pr.w] = keep;
             }
             // warp-aggregated append of the active pairs
             const unsigned mask = __ballot_sync(0xffffffffu, keep);
             int pos = 0;
             if (lane == 0 && mask) pos = atomicAdd(&ctrl->n_surv_next, __popc(mask));
             pos = __shfl_sync(0xffffffffu, pos, 0);
-            if (keep)
+            if (keep) surv[pos + __popc(mask & ((1u << lane) - 1u))] = p;
+        }
+        if (!grid_barrier(al.bar, work_blocks, ctrl)) return;
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+        {
+            int cnt = 0;
+            for (int e = al.row_ptr[i]; e < al.row_ptr[i + 1]; ++e) cnt += al.keep[e];
+            al.n_act[i] = cnt;
+            al.gref[i] = load_geom(geom, i);
+        }
+        const int m = __ldcg(&ctrl->n_surv_next);
+        for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += stride)
+        {
+            const int4 pr = pairs[surv[q]];
+            int4 rec = make_int4(pr.x, pr.y, al.row_ptr[pr.x], al.row_ptr[pr.y]);
             {
-                surv[pos + __popc(mask & ((1u << lane) - 1u))] = p;
-                bool cand = false;
-                pair_shares<MIXED, DIM>(gi, gj, pr, fp, td, tr, jbuf, ovl_max, &cand);
-                if (cand) fp.fr_list[atomicAdd(&ctrl->fr_ncand_next, 1)] = p;
+                int a = 0, b = 0;
+                for (int e = rec.z; e < pr.z; ++e) a += al.keep[e];
+                for (int e = rec.w; e < pr.w; ++e) b += al.keep[e];
+                rec.z += a;
+                rec.w += b;
             }
+            const bool adhere = DIM == 2 && fp.adhere[pr.z] != 0;
+            al.act[q] = make_int4(rec.x, adhere ? rec.y | ACT_ADHERE : rec.y, rec.z, rec.w);
+            bool cand = false;
+            pair_shares<MIXED, DIM>(load_geom(geom, rec.x), load_geom(geom, rec.y), rec, adhere, fp, td, tr, jbuf,
+                                    ovl_max, cand, rounding);
+            if (cand) fp.fr_list[atomicAdd(&ctrl->fr_ncand_next, 1)] = q;
         }
     }
     else
@@ -1065,11 +1065,13 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
         const int m = ctrl->n_surv;
         for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += stride)
         {
-            const int p = surv[q];
-            const int4 pr = pairs[p];
+            int4 rec = al.act[q];
+            const bool adhere = DIM == 2 && rec.y < 0;
+            if (DIM == 2) rec.y &= ~ACT_ADHERE;
             bool cand = false;
-            pair_shares<MIXED, DIM>(load_geom(geom, pr.x), load_geom(geom, pr.y), pr, fp, td, tr, jbuf, ovl_max, &cand);
-            if (cand) fp.fr_list[atomicAdd(&ctrl->fr_ncand_next, 1)] = p;
+            pair_shares<MIXED, DIM>(load_geom(geom, rec.x), load_geom(geom, rec.y), rec, adhere, fp, td, tr, jbuf,
+                                    ovl_max, cand, rounding);
+            if (cand) fp.fr_list[atomicAdd(&ctrl->fr_ncand_next, 1)] = q;
         }
     }
     if (fp.stats && !proposer)
@@ -1096,6 +1098,7 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
             ctrl->screen_valid = 1;
             ctrl->drift = 0.0;
         }
+        if (MIXED && rounding == ROUND_STALE) ctrl->path = 0.0;
         if (fp.fric)
         {
             // the candidates of this pass; no stage has a changed decision yet
@@ -1153,16 +1156,21 @@ void launch_pair_list(const Ctrl* ctrl, const int* row_ptr, const int* lower_end
                                              pairs);
 }
 
-// total dE/dq of each cell from the two shares of every pair (the API paths;
-// the loop's first attempt does the same sum itself)
-__global__ void k_pair_sum_rows(const int* __restrict__ row_ptr, const int* __restrict__ lower_end, const Ctrl* ctrl,
-                                const double4* __restrict__ jbuf, Gen6* fcc, int f32);
+// total dE/dq of each cell from its active shares (the API paths; the loop's first attempt
+// does the same sum itself)
+__global__ void k_pair_sum_rows(const int* __restrict__ row_ptr, const int* __restrict__ n_act, const Ctrl* ctrl,
+                                const double4* __restrict__ jbuf, Gen6* fcc, int f32)
+{
+    const int n = ctrl->n;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        fcc[i] = f32 ? sum_active_shares(reinterpret_cast<const float4*>(jbuf) + row_ptr[i], n_act[i])
+                     : sum_active_shares(jbuf + row_ptr[i], n_act[i]);
+}
 
-void launch_pair_screened(const Geom* geom, const int* row_ptr, const int* lower_end, const int* col,
-                          const int* rev, Ctrl* ctrl, ForceParams fp, const double* jkr_delta,
+void launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, const double* jkr_delta,
                           const double* jkr_radius, Gen6* fcc, double4* jbuf, int mixed, int max_entries,
                           int cap_cells, int num_sms, cudaStream_t st, int with_sum, int dims, int tile,
-                          int blocks_per_sm, const int4* pairs, int* surv, const StepParams* sp,
+                          int blocks_per_sm, const int4* pairs, int* surv, ActiveList al, const StepParams* sp,
                           const float* mlp_w)
 {
     // sp (the loop's pass): the last block also runs the step-size proposal
@@ -1170,44 +1178,26 @@ void launch_pair_screened(const Geom* geom, const int* row_ptr, const int* lower
     if (sp) spv = *sp;
     const int propose = (sp && sp->stats_on) ? 1 : 0;
     // grid: at least `tile` pairs per block, at most the blocks that are resident at
-    // once (blocks_per_sm caps them per SM); the blocks stride over the pairs
+    // once (blocks_per_sm caps them per SM); the blocks stride over the pairs.  The launch
+    // is cooperative: the blocks of a refresh wait for one another.
     tile = tile <= 0 ? 1024 : min(tile, PS_TILE_MAX);
     const int max_pairs = max(max_entries / 2, 1);
     const bool f32 = mixed && dims != 2;
-    auto grid = [&](const void* fn, int& occ_cache) {
-        if (occ_cache == 0)
-        {
-            int occ = 0;
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, PS_T, 0);
-            occ_cache = max(occ, 1);
-        }
-        const int per_sm = blocks_per_sm > 0 ? min(blocks_per_sm, occ_cache) : occ_cache;
-        return max(1, min(cdiv(max_pairs, tile), num_sms * per_sm));
-    };
-    // resident blocks per SM of each instantiation (without, with the proposal)
-    static int occ2[2] = {0, 0}, occ3m[2] = {0, 0}, occ3[2] = {0, 0};
-#define PX_ARGS geom, pairs, ctrl, fp, jkr_delta, jkr_radius, jbuf, surv, spv, mlp_w
-#define PX_LAUNCH(M, D, P, occ) \
-    k_pair_pass<M, D, P><<<grid((const void*)k_pair_pass<M, D, P>, occ[P ? 1 : 0]), PS_T, 0, st>>>(PX_ARGS)
-    if (dims == 2)
-    {
-        if (propose) PX_LAUNCH(false, 2, true, occ2);
-        else PX_LAUNCH(false, 2, false, occ2);
-    }
-    else if (f32)
-    {
-        if (propose) PX_LAUNCH(true, 3, true, occ3m);
-        else PX_LAUNCH(true, 3, false, occ3m);
-    }
-    else
-    {
-        if (propose) PX_LAUNCH(false, 3, true, occ3);
-        else PX_LAUNCH(false, 3, false, occ3);
-    }
-#undef PX_LAUNCH
-#undef PX_ARGS
+    const int p = propose ? 1 : 0;
+    const void* const fn2[2] = {(const void*)k_pair_pass<false, 2, false>, (const void*)k_pair_pass<false, 2, true>};
+    const void* const fn3m[2] = {(const void*)k_pair_pass<true, 3, false>, (const void*)k_pair_pass<true, 3, true>};
+    const void* const fn3[2] = {(const void*)k_pair_pass<false, 3, false>, (const void*)k_pair_pass<false, 3, true>};
+    const void* fn = dims == 2 ? fn2[p] : f32 ? fn3m[p] : fn3[p];
+    int occ = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, PS_T, 0);
+    occ = max(occ, 1);
+    const int per_sm = blocks_per_sm > 0 ? min(blocks_per_sm, occ) : occ;
+    const int grid = max(1, min(cdiv(max_pairs, tile), num_sms * per_sm));
+    void* args[] = {(void*)&geom, (void*)&pairs, (void*)&ctrl, (void*)&fp, (void*)&jkr_delta, (void*)&jkr_radius,
+                    (void*)&jbuf, (void*)&surv, (void*)&al, (void*)&spv, (void*)&mlp_w};
+    cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(PS_T), args, 0, st);
     if (with_sum)
-        k_pair_sum_rows<<<max(cdiv(cap_cells, 128), 1), 128, 0, st>>>(row_ptr, lower_end, ctrl, jbuf, fcc, f32);
+        k_pair_sum_rows<<<max(cdiv(cap_cells, 128), 1), 128, 0, st>>>(al.row_ptr, al.n_act, ctrl, jbuf, fcc, f32);
 }
 
 // to_adhere (2D/include/simulation.hpp:242-258, one group in the adhesion map):
@@ -1262,708 +1252,6 @@ void launch_pair_dEdq_2d(const Geom* geom, const Gen6* fcc, const Ctrl* ctrl, do
                          cudaStream_t st)
 {
     k_pair_dEdq_2d<<<max(cdiv(cap_cells, 256), 1), 256, 0, st>>>(geom, fcc, ctrl, cm);
-}
-
-// ---------------------------------------------------------------------------
-// RK attempt: one thread per cell runs every stage of stepRungeKuttaAdaptive
-// (mechanics.hpp:2406-2612) in registers.  3-D pair forces are stage-invariant
-// (the table is not refreshed between stages and include_constraint = false,
-// mechanics.hpp:2064), so each stage needs only the cell's own state, its
-// precomputed pair force and the surface terms.
-// ---------------------------------------------------------------------------
-const int AT_T = 128;
-
-__device__ __forceinline__ void normalize_n(double y[6])
-{
-    double nrm = sqrt((y[3] * y[3] + y[4] * y[4]) + y[5] * y[5]);
-    y[3] /= nrm; y[4] /= nrm; y[5] /= nrm;
-    if (y[5] < 0) { y[3] = -y[3]; y[4] = -y[4]; y[5] = -y[5]; }
-}
-
-// getVelocities (mechanics.hpp:2011-2347) of one cell at state y; f0 = -dE/dq of
-// the (stage-invariant) pair forces plus noise
-__device__ __forceinline__ void cell_velocity(const StepParams& sp, bool a2, const double y[6],
-                                              double l, double h, double eta0, double eta1, double sigma0,
-                                              const Vel* __restrict__ drp, const double f0[6], double v[6])
-{
-    const MechParams& P = sp.mp;
-    double ss = a2 ? __longlong_as_double(0x7ff8000000000000ll) : (P.R - y[2]) / y[5];
-    EndPow w;
-    w.p = w.q = w.sp = w.sq = 0.0;
-    if (!a2) w = end_pows(y[2], y[5], P.R, h, ss);
-    double rep2 = 0, rep5 = 0, adh2 = 0, adh5 = 0;
-    if (!P.no_surface) surface_dEdq(P, a2, y[2], y[5], l, h, sigma0, ss, w, rep2, rep5, adh2, adh5);
-    double f[6];
-#pragma unroll
-    for (int c = 0; c < 6; ++c) f[c] = f0[c];
-    f[2] = (f[2] - rep2) - adh2;
-    f[5] = (f[5] - rep5) - adh5;
-    velocity_solve(P, a2, y, l, h, eta0, eta1, ss, w, drp, f, v);
-}
-
-// Mixed precision: a cell in surface contact (and not lying on the substrate) takes the
-// FP32 contact branch (velocity_contact_f32); the others keep the FP64 branches (i) and
-// (ii), whose surface forces are zero off the surface and the horizontal shortcut on it
-__device__ __forceinline__ void cell_velocity_f32(const StepParams& sp, bool a2, const double y[6],
-                                                  double l, double h, double eta0, double eta1, double sigma0,
-                                                  const Vel* __restrict__ drp, const double f0[6], double v[6])
-{
-    const MechParams& P = sp.mp;
-    const bool contacting = surface_contact(P, a2, y, h);
-    if (!P.no_surface && contacting && !a2)
-    {
-        velocity_contact_f32(P, y, l, h, eta0, eta1, sigma0, drp, f0, v);
-        return;
-    }
-    double f[6];
-#pragma unroll
-    for (int c = 0; c < 6; ++c) f[c] = f0[c];
-    if (!P.no_surface && a2)
-    {
-        double rep2 = 0, adh2 = 0;
-        surface_dEdq_flat(P, y[2], l, sigma0, rep2, adh2);
-        f[2] = (f[2] - rep2) - adh2;
-    }
-    velocity_free_or_flat(P, contacting, y, l, eta0, eta1, drp, f, v);
-}
-
-template <bool F32>
-__device__ __forceinline__ void cell_velocity_p(const StepParams& sp, bool a2, const double y[6], double l,
-                                                double h, double eta0, double eta1, double sigma0,
-                                                const Vel* __restrict__ drp, const double f0[6], double v[6])
-{
-    if constexpr (F32) cell_velocity_f32(sp, a2, y, l, h, eta0, eta1, sigma0, drp, f0, v);
-    else cell_velocity(sp, a2, y, l, h, eta0, eta1, sigma0, drp, f0, v);
-}
-
-// -dE/dq of the pair forces (getConservativeForces, mechanics.hpp:1768) plus the
-// attempt's noise (mechanics.hpp:2489-2510, forces += noise at :2066)
-template <bool NOISE>
-__device__ __forceinline__ void base_force(const StepParams& sp, const Gen6& cc, int iter, int attempt, int i,
-                                           double f0[6])
-{
-#pragma unroll
-    for (int c = 0; c < 6; ++c) f0[c] = -cc.f[c];
-    if (NOISE)
-    {
-        for (int k = 0; k < 3; ++k)
-        {
-            uint32_t x[4] = {(uint32_t)iter, (uint32_t)attempt, (uint32_t)i, (uint32_t)k};
-            philox4x32_10(x, (uint32_t)sp.seed, (uint32_t)(sp.seed >> 32) ^ RNG_PURPOSE_NOISE);
-            double u0 = philox_u01(x[0], x[1]), u1 = philox_u01(x[2], x[3]);
-            f0[2 * k] += -sp.noise_max[2 * k] + 2 * sp.noise_max[2 * k] * u0;
-            f0[2 * k + 1] += -sp.noise_max[2 * k + 1] + 2 * sp.noise_max[2 * k + 1] * u1;
-        }
-    }
-}
-
-// 2-D noise of one attempt (2D/include/mechanics.hpp:1760-1771): uniform on
-// [-max, max] for (rx, ry, nx, ny), from the 3-D counter slots 0, 1, 3, 4
-__device__ __forceinline__ void noise_2d(const StepParams& sp, int iter, int attempt, int i, double nz[4])
-{
-    double u[6];
-    for (int k = 0; k < 3; ++k)
-    {
-        uint32_t x[4] = {(uint32_t)iter, (uint32_t)attempt, (uint32_t)i, (uint32_t)k};
-        philox4x32_10(x, (uint32_t)sp.seed, (uint32_t)(sp.seed >> 32) ^ RNG_PURPOSE_NOISE);
-        u[2 * k] = philox_u01(x[0], x[1]);
-        u[2 * k + 1] = philox_u01(x[2], x[3]);
-    }
-    const double m = sp.max_noise_2d;
-    nz[0] = -m + 2 * m * u[0]; nz[1] = -m + 2 * m * u[1];
-    nz[2] = -m + 2 * m * u[3]; nz[3] = -m + 2 * m * u[4];
-}
-
-// 2-D getVelocities (2D/include/mechanics.hpp:1503-1667) at stage orientation (y3, y4):
-// dE/dq = (F, S - (n . S) n) + noise from the pair sums cc = (F, S); v = -dE/dq / (K, L)
-// with K = l (eta0 + eta1 rho_c / R), L = l^3 (...) / 12 (:264-279)
-__device__ __forceinline__ void velocity_2d(const StepParams& sp, const double y[6], double l, double eta0,
-                                            double eta1, const Gen6& cc, const double nz[4], double v[6])
-{
-    const double drag = eta0 + eta1 * sp.rho_c / sp.mp.R;
-    const double K = l * drag, L = l * l * l * drag / 12;
-    const double w = y[3] * cc.f[3] + y[4] * cc.f[4];
-    const double d0 = cc.f[0] + nz[0], d1 = cc.f[1] + nz[1];
-    const double d2 = (cc.f[3] - w * y[3]) + nz[2], d3 = (cc.f[4] - w * y[4]) + nz[3];
-    v[0] = -d0 / K; v[1] = -d1 / K; v[2] = 0.0;
-    v[3] = -d2 / L; v[4] = -d3 / L; v[5] = 0.0;
-}
-
-__device__ __forceinline__ Gen6 load_gen6(const Gen6* __restrict__ g, int i)
-{
-    const double2* p = reinterpret_cast<const double2*>(g + i);
-    double2 a = __ldg(p), b = __ldg(p + 1), c = __ldg(p + 2);
-    Gen6 o;
-    o.f[0] = a.x; o.f[1] = a.y; o.f[2] = b.x; o.f[3] = b.y; o.f[4] = c.x; o.f[5] = c.y;
-    return o;
-}
-
-// dE/dq of cell i: the share of its lower neighbors (written by k_pair_force) plus
-// the shares its higher-index neighbors left in the upper part of its row
-__device__ __forceinline__ Gen6 gather_pair_force(const Gen6* fcc, const int* __restrict__ row_ptr,
-                                                  const int* __restrict__ lower_end,
-                                                  const double4* __restrict__ jbuf, int i)
-{
-    Gen6 f = fcc[i];
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    for (int k = lower_end[i]; k < row_ptr[i + 1]; ++k)
-    {
-        double4 js = jbuf[k];
-        acc[0] -= js.x; acc[1] -= js.y; acc[2] -= js.z;
-        acc[3] -= js.w * js.x; acc[4] -= js.w * js.y; acc[5] -= js.w * js.z;
-    }
-    for (int c = 0; c < 6; ++c) f.f[c] += acc[c];
-    return f;
-}
-
-__device__ __forceinline__ double4 widen(const double4& v) { return v; }
-__device__ __forceinline__ double4 widen(const float4& v)
-{
-    return make_double4((double)v.x, (double)v.y, (double)v.z, (double)v.w);
-}
-
-// dE/dq of cell i from both shares of every pair in its row: (v, s v) from its lower
-// entries, (-v, -t v) from the partners' entries, in CSR order.  Shares are stored
-// as double4, or as float4 (mixed precision), summed in FP64 either way.
-template <class SHARE>
-__device__ __forceinline__ Gen6 sum_row_shares(const int* __restrict__ row_ptr, const int* __restrict__ lower_end,
-                                               const SHARE* __restrict__ jbuf, int i)
-{
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    const int le = lower_end[i], r1 = row_ptr[i + 1];
-    for (int k = row_ptr[i]; k < le; ++k)
-    {
-        const double4 js = widen(jbuf[k]);
-        acc[0] += js.x; acc[1] += js.y; acc[2] += js.z;
-        acc[3] += js.w * js.x; acc[4] += js.w * js.y; acc[5] += js.w * js.z;
-    }
-    for (int k = le; k < r1; ++k)
-    {
-        const double4 js = widen(jbuf[k]);
-        acc[0] -= js.x; acc[1] -= js.y; acc[2] -= js.z;
-        acc[3] -= js.w * js.x; acc[4] -= js.w * js.y; acc[5] -= js.w * js.z;
-    }
-    Gen6 f;
-    for (int c = 0; c < 6; ++c) f.f[c] = acc[c];
-    return f;
-}
-
-__global__ void k_pair_sum_rows(const int* __restrict__ row_ptr, const int* __restrict__ lower_end, const Ctrl* ctrl,
-                                const double4* __restrict__ jbuf, Gen6* fcc, int f32)
-{
-    const int n = ctrl->n;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        fcc[i] = f32 ? sum_row_shares(row_ptr, lower_end, reinterpret_cast<const float4*>(jbuf), i)
-                     : sum_row_shares(row_ptr, lower_end, jbuf, i);
-}
-
-// Step-size controller, run once per attempt by the last block
-// (simulation.hpp:1690-1769; the final re-run is accepted unconditionally).
-// commit: the final step copies an accepted proposal (no RK evaluation of its own)
-__device__ void controller_finish(Ctrl* c, const StepParams& sp, int kind, double E, bool commit = false)
-{
-    if (!commit) c->attempts += 1;
-    if (kind == MODE_TRIAL)
-    {
-        c->last_trial_error = E;
-        bool exceeded = E > 1.0;
-        c->first_passed = !exceeded;
-        if (exceeded) c->rejected += 1;
-        if (sp.log_cap > 0)
-        {
-            // complete the feature row of this iteration: the log ratio of the largest
-            // dt the error model accepts, and of this attempt's dt, to the last accepted dt
-            float* row = sp.log_buf + (size_t)(c->log_rows % sp.log_cap) * MLP_LOG_COLS;
-            row[32] = (float)(-sp.inv_q1 * log(E));
-            row[33] = (float)log(c->dt / c->dt_prev);
-            row[34] = (float)log10(E);
-            row[35] = exceeded ? 0.f : 1.f;
-            c->log_rows += 1;
-        }
-        if (sp.propose && !exceeded)
-        {
-            // the proposal passed the error test: accept its candidate state as is
-            c->mode = MODE_COMMIT;
-            c->tries = 0;
-            c->attempt = 1;
-            return;
-        }
-        double factor = 0.9 * pow(1.0 / E, sp.inv_q1);
-        if (factor >= 10) factor = 10;
-        else if (factor < 0.2) factor = 0.2;
-        c->factor = factor;
-        c->tries = 0;
-        c->attempt = 1;
-        if (exceeded && 0 < sp.max_tries) { c->mode = MODE_RETRY; c->dt_try = c->dt * factor; return; }
-    }
-    else if (kind == MODE_RETRY)
-    {
-        c->retries += 1;
-        c->attempt += 1;
-        bool exceeded = E > 1.0;
-        double factor = c->factor * (0.9 * pow(1.0 / E, sp.inv_q1));
-        bool brk = false;
-        if (factor >= 10) { factor = 10; brk = true; }
-        else if (factor < 0.2) { factor = 0.2; brk = true; }
-        c->factor = factor;
-        if (!brk)
-        {
-            c->tries += 1;
-            if (exceeded && c->tries < sp.max_tries) { c->mode = MODE_RETRY; c->dt_try = c->dt * factor; return; }
-        }
-    }
-    else   // MODE_FINAL (or a committed proposal): accepted
-    {
-        c->last_max_error = E;
-        const int h = c->hist_pos;
-        // error of the accepted step before this one (1 before any)
-        const int hp = (h + HIST - 1) % HIST;
-        const double e_prev = c->hist_dt[hp] > 0 ? c->hist_err[hp] : 1.0;
-        const double dt_accepted = c->dt;
-        c->hist_dt[h] = c->dt;
-        c->hist_err[h] = E;
-        c->hist_acc[h] = c->first_passed;
-        c->hist_pos = (h + 1) % HIST;
-        c->since_div = c->n_divide > 0 ? 0 : c->since_div + 1;
-        c->cell_steps += c->n;
-        c->t += c->dt;
-        c->iter += 1;
-        c->iterations += 1;
-        // a frame is due when the time has just passed a multiple of dt_write
-        // (simulation.hpp:2025-2028)
-        if (c->dt_write > 0)
-        {
-            const double t_old_factor = fmod(c->t - c->dt + 1e-12, c->dt_write);
-            const double t_new_factor = fmod(c->t + 1e-12, c->dt_write);
-            if (t_old_factor > t_new_factor) c->frame_due = 1;
-        }
-        if (sp.pi)
-        {
-            // the PI proposal for the next step: dt 0.9 E^(-0.7/k) E_prev^(0.4/k), k the error
-            // order + 1 (Gustafsson's PI rule with the parameters of Hairer & Wanner, Solving
-            // ODEs II, sec. IV.2), the factor held to [0.2, 10], dt to [min, max] step size
-            double f = 0.9 * pow(1.0 / E, 0.7 * sp.inv_q1) * pow(e_prev, 0.4 * sp.inv_q1);
-            if (f >= 10) f = 10;
-            else if (f < 0.2) f = 0.2;
-            double next = dt_accepted * f;
-            if (next < sp.min_stepsize) next = sp.min_stepsize;
-            else if (next > sp.max_stepsize) next = sp.max_stepsize;
-            c->dt = next;
-        }
-        c->mode = MODE_TRIAL;
-        c->tries = 0;
-        c->attempt = 0;
-        return;
-    }
-    // clamp and schedule the final re-run (simulation.hpp:1752-1760)
-    double factor = c->factor;
-    if (c->dt * factor < sp.min_stepsize) factor = sp.min_stepsize / c->dt;
-    else if (c->dt * factor > sp.max_stepsize) factor = sp.max_stepsize / c->dt;
-    c->dt *= factor;
-    c->dt_try = c->dt;
-    c->mode = MODE_FINAL;
-}
-
-// friction: the force of cell i at stage st, f0 minus the change of the dE/dq shares of its
-// candidate contacts whose planar decision at this stage differs from the one at y0; each
-// share enters as the pair sum does, (v, s v) from a lower entry, (-v, -t v) from a partner's
-__device__ __forceinline__ void friction_stage_force(const PairGather& pg, int i, int st, const double f0[6],
-                                                     double fs[6])
-{
-    double acc[6] = {0, 0, 0, 0, 0, 0};
-    const int le = pg.lower_end[i], r1 = pg.row_ptr[i + 1];
-    for (int e = pg.row_ptr[i]; e < r1; ++e)
-    {
-        if (!((pg.fmask[e] >> st) & 1)) continue;
-        const double4 dv = pg.fbuf[e];
-        const double w = pg.jbuf[e].w;
-        const double sg = e < le ? 1.0 : -1.0;
-        acc[0] += sg * dv.x; acc[1] += sg * dv.y; acc[2] += sg * dv.z;
-        acc[3] += sg * w * dv.x; acc[4] += sg * w * dv.y; acc[5] += sg * w * dv.z;
-    }
-#pragma unroll
-    for (int c = 0; c < 6; ++c) fs[c] = f0[c] - acc[c];
-}
-
-// KIND: MODE_TRIAL / MODE_RETRY / MODE_FINAL inside the loop, 3 = API evaluation.
-// Without noise the stage-0 velocity k0 = f(y0) is the same for every attempt of an
-// iteration (y0 and the pair forces do not change), so the trial stores it in k0buf
-// and the retries and the final attempt read it back.
-// Learned controller: the trial (the network's proposal) writes its state in place
-// and first copies y0 (with l in the gamma slot) and the stored velocity to
-// geom_c / vel_c; a proposal that passes the error test closes the step in the
-// trial's last block, one that fails continues with retries and a final attempt
-// that read y0 back from that copy.
-// use_cond bit 0: `cond` is the retry WHILE node's handle; bit 1: `cond_run` is the
-// handle of the IF node around the final attempt (0 after a committed proposal).
-// Launch bounds: six blocks per SM (85 registers) for the 2- and 4-stage tableaux, the
-// fastest measured for the 100k-cell step (three for their friction trial pass, which
-// would spill at six); no bound for the 6- and 7-stage ones, which spill below ~130.
-// V: 0 FP64; 1 mixed precision; 2 FP64 with cell-cell friction, whose candidate contacts
-// add, at each stage whose planar decision differs from the one at y0, the recorded change
-// of their shares; 3 the friction trial pass, which runs only the stages of the cells with
-// candidate contacts and records their stage states (z, n_z) for the decision check, with
-// no other effect.
-template <int S, int KIND, bool NOISE, int DIM, int V>
-__global__ void __launch_bounds__(AT_T, (S <= 4 ? (V == 3 ? 3 : 6) : 1)) k_attempt(Geom* geom, Vel* vel, Phys* phys, const Gen6* fcc,
-                                                 Ctrl* ctrl, StepParams sp, Geom* geom_c, Vel* vel_c,
-                                                 Gen6* err_out, Gen6* k0buf, double eval_dt, int eval_attempt,
-                                                 unsigned long long cond, int use_cond, PairGather pg,
-                                                 unsigned long long cond_run)
-{
-    constexpr bool F32 = V == 1, FRIC = V >= 2, DRY = V == 3;
-    __shared__ double sh_max[AT_T / 32], sh_drift[AT_T / 32];
-    __shared__ double4 sh_stat[AT_T / 32];
-    __shared__ bool last;
-    if (DRY && (!ctrl->fr_pending || (KIND != 3 && ctrl->halted))) return;
-    if (KIND != 3 && ctrl->halted)
-    {
-        // a halted context takes no step: stop an enclosing WHILE node
-        if ((use_cond & 1) && (KIND == MODE_TRIAL || KIND == MODE_RETRY) && blockIdx.x == 0 && threadIdx.x == 0)
-            cudaGraphSetConditional((cudaGraphConditionalHandle)cond, 0u);
-        if ((use_cond & 2) && KIND == MODE_TRIAL && blockIdx.x == 0 && threadIdx.x == 0)
-            cudaGraphSetConditional((cudaGraphConditionalHandle)cond_run, 0u);
-        return;
-    }
-    const int n = ctrl->n;
-    const int n_order = (KIND != 3 && sp.order) ? ctrl->n_order : 0;
-    const int mode = ctrl->mode;
-    const int iter = ctrl->iter;
-    // the learned and PI controllers propose (and test) a step every iteration
-    const bool trial_ran = sp.propose || (iter % sp.iter_update_stepsize == 0);
-    // k0 is shared across attempts only under the reference controller: a passing
-    // proposal needs no second attempt, so it does not store k0 or the total pair force
-    const bool share_k0 = !NOISE && !sp.propose;
-    double dt;
-    int attempt;
-    bool load_k0 = false, store_k0 = false;
-    if (KIND == MODE_TRIAL)
-    {
-        if (!trial_ran) return;   // no step-size update this iteration: FINAL runs at dt
-        dt = ctrl->dt; attempt = 0; store_k0 = share_k0;
-    }
-    else if (KIND == MODE_RETRY)
-    {
-        if (mode != MODE_RETRY)
-        {
-            // no retry pending: make sure an enclosing WHILE node stops
-            if ((use_cond & 1) && blockIdx.x == 0 && threadIdx.x == 0)
-                cudaGraphSetConditional((cudaGraphConditionalHandle)cond, 0u);
-            return;
-        }
-        dt = ctrl->dt_try; attempt = ctrl->attempt; load_k0 = share_k0;
-    }
-    else if (KIND == MODE_FINAL)
-    {
-        dt = (mode == MODE_FINAL) ? ctrl->dt_try : ctrl->dt;
-        attempt = (mode == MODE_FINAL) ? ctrl->attempt : 0;
-        load_k0 = share_k0 && trial_ran;
-    }
-    else { dt = eval_dt; attempt = eval_attempt; }
-    // the step was closed by a proposal that passed the error test
-    if (KIND == MODE_FINAL && mode == MODE_COMMIT) return;
-    const bool commit = false;
-    // a proposal (learned or PI) advances the state in place; the attempts after a failed
-    // proposal start from the copy of y0 it kept
-    const bool in_place = !DRY && (KIND == MODE_TRIAL) && sp.propose;
-    const bool from_backup = (KIND == MODE_RETRY || KIND == MODE_FINAL) && sp.propose;
-    if (DRY) store_k0 = false;
-    // friction: stages whose planar decisions differ from those at y0 somewhere
-    const bool flips = FRIC && ctrl->fr_nflip > 0;
-
-    // the first attempt of an iteration sums the cell's pair shares (pg.fused); under
-    // the reference controller the trial writes the total back for the rest, under the
-    // proposing ones every attempt sums them
-    const bool do_gather = pg.fused && !commit &&
-                           (KIND == MODE_TRIAL || (KIND == MODE_FINAL && !trial_ran) || sp.propose);
-    double local_max = 0.0;
-    bool bad = false;
-    double st_vmax = 0.0, st_v2 = 0.0, st_g = 0.0, st_near = 0.0;
-    // motion bound of each new segment: |dr| + h' |dn| + |dh| (a Hausdorff bound)
-    double local_drift = 0.0;
-    // one cell per thread: the grid covers the capacity (attempt_blocks); thread t takes
-    // the t-th cell of the attempt order (cells appended after the order was made, in
-    // index order).  The body is a do-while(false) block so that `continue` leaves it.
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < n) do
-    {
-        const int i = t < n_order ? sp.order[t] : t;
-        if (DRY)
-        {
-            // only cells with a candidate contact have stage states to report
-            bool any = false;
-            for (int e = pg.row_ptr[i]; e < pg.row_ptr[i + 1] && !any; ++e) any = (pg.fmask[e] & FR_CAND) != 0;
-            if (!any) continue;
-        }
-        const Geom g = load_geom(from_backup ? geom_c : geom, i);
-        const Vel* vprev = (from_backup ? vel_c : vel) + i;
-        const double y0[6] = {g.rx, g.ry, g.rz, g.nx, g.ny, g.nz};
-        // non-finite coordinates (the reference's DEBUG_CHECK_CELL_COORDINATES_NAN,
-        // simulation.hpp:1803-1821): a position alone enters no velocity, so its error
-        // norm would stay finite
-#pragma unroll
-        for (int c = 0; c < 6; ++c) if (!isfinite(y0[c])) bad = true;
-        const double l = from_backup ? g.gamma : phys[i].l;
-        const double eta0 = phys[i].eta0, eta1 = phys[i].eta1, sigma0 = phys[i].sigma0;
-        if (in_place)
-        {
-            Geom b = g;
-            b.gamma = l;
-            geom_c[i] = b;
-            vel_c[i] = vel[i];
-        }
-        const bool a2 = y0[5] < sp.mp.nz_threshold;
-        Gen6 cc;
-        if (do_gather)
-        {
-            cc = pg.fused == 3 ? sum_row_shares(pg.row_ptr, pg.lower_end, reinterpret_cast<const float4*>(pg.jbuf), i)
-               : pg.fused == 2 ? sum_row_shares(pg.row_ptr, pg.lower_end, pg.jbuf, i)
-                               : gather_pair_force(fcc, pg.row_ptr, pg.lower_end, pg.jbuf, i);
-            if (KIND == MODE_TRIAL && !sp.propose && !DRY) pg.fcc_w[i] = cc;
-        }
-        else cc = (KIND == MODE_TRIAL) ? fcc[i] : load_gen6(fcc, i);
-        double f0[6];
-        double nz2[4] = {0.0, 0.0, 0.0, 0.0};
-        if constexpr (DIM == 2)
-        {
-            if (NOISE) noise_2d(sp, iter, attempt, i, nz2);
-        }
-        else base_force<NOISE>(sp, cc, iter, attempt, i, f0);
-        double k[S][6];
-        if (load_k0)
-        {
-            const double2* kp = reinterpret_cast<const double2*>(k0buf + i);
-            double2 a = kp[0], b = kp[1], c = kp[2];
-            k[0][0] = a.x; k[0][1] = a.y; k[0][2] = b.x; k[0][3] = b.y; k[0][4] = c.x; k[0][5] = c.y;
-        }
-        else
-        {
-            if constexpr (DIM == 2) velocity_2d(sp, y0, l, eta0, eta1, cc, nz2, k[0]);
-            else cell_velocity_p<F32>(sp, a2, y0, l, g.h, eta0, eta1, sigma0, vprev, f0, k[0]);
-            if (store_k0)
-            {
-                double2* kp = reinterpret_cast<double2*>(k0buf + i);
-                kp[0] = make_double2(k[0][0], k[0][1]);
-                kp[1] = make_double2(k[0][2], k[0][3]);
-                kp[2] = make_double2(k[0][4], k[0][5]);
-            }
-        }
-#pragma unroll
-        for (int st = 1; st < S; ++st)
-        {
-            double y[6];
-#pragma unroll
-            for (int c = 0; c < 6; ++c)
-            {
-                double m = 0.0;
-#pragma unroll
-                for (int j = 0; j < st; ++j) m += k[j][c] * sp.A[st][j];
-                y[c] = y0[c] + m * dt;
-            }
-            normalize_n(y);
-            if constexpr (DIM == 2) velocity_2d(sp, y, l, eta0, eta1, cc, nz2, k[st]);
-            else if constexpr (FRIC)
-            {
-                if (DRY) pg.ystage[(size_t)st * pg.ystage_ld + i] = make_double2(y[2], y[5]);
-                if (flips)
-                {
-                    double fs[6];
-                    friction_stage_force(pg, i, st, f0, fs);
-                    cell_velocity_p<false>(sp, a2, y, l, g.h, eta0, eta1, sigma0, vprev, fs, k[st]);
-                }
-                else cell_velocity_p<false>(sp, a2, y, l, g.h, eta0, eta1, sigma0, vprev, f0, k[st]);
-            }
-            else cell_velocity_p<F32>(sp, a2, y, l, g.h, eta0, eta1, sigma0, vprev, f0, k[st]);
-        }
-        if (DRY)
-        {
-            pg.ystage[i] = make_double2(y0[2], y0[5]);
-            continue;
-        }
-        double vf1[6], d1[6];
-#pragma unroll
-        for (int c = 0; c < 6; ++c)
-        {
-            double s1 = 0.0, s2 = 0.0;
-#pragma unroll
-            for (int st = 0; st < S; ++st) { s1 += k[st][c] * sp.b[st]; s2 += k[st][c] * sp.bs[st]; }
-            vf1[c] = s1;
-            d1[c] = s1 * dt;
-            double err = d1[c] - s2 * dt;
-            double scaled = err / (sp.tol * (1.0 + fabs(y0[c])));
-            if (isnan(scaled) || isinf(scaled)) bad = true;
-            local_max = fmax(local_max, scaled);
-            if (KIND == 3 && err_out) err_out[i].f[c] = err;
-        }
-        if (KIND == MODE_FINAL || KIND == 3 || in_place)
-        {
-            double y1[6];
-#pragma unroll
-            for (int c = 0; c < 6; ++c) y1[c] = y0[c] + d1[c];
-            normalize_n(y1);
-            Geom go = g;
-            go.rx = y1[0]; go.ry = y1[1]; go.rz = y1[2]; go.nx = y1[3]; go.ny = y1[4]; go.nz = y1[5];
-            Vel vo;
-#pragma unroll
-            for (int c = 0; c < 6; ++c) vo.v[c] = vf1[c];
-            if (KIND == MODE_FINAL || in_place)
-            {
-                // growCells (growth.hpp:51-57) fused with the accepted step
-                const double g_rate = phys[i].growth;
-                double lg = l + g_rate * (4 * sp.mp.R / 3 + l) * dt;
-                go.h = lg / 2;
-                {
-                    const double ax = go.rx - g.rx, ay = go.ry - g.ry, az = go.rz - g.rz;
-                    const double bx = go.nx - g.nx, by = go.ny - g.ny, bz = go.nz - g.nz;
-                    local_drift = fmax(local_drift, sqrt(ax * ax + ay * ay + az * az)
-                                                        + go.h * sqrt(bx * bx + by * by + bz * bz)
-                                                        + fabs(go.h - g.h));
-                }
-                if (from_backup) go.gamma = geom[i].gamma;   // the copy holds l in that slot
-                phys[i].l = lg;
-                geom[i] = go;
-                vel[i] = vo;
-                if (sp.stats_on)
-                {
-                    const double v2 = vf1[0] * vf1[0] + vf1[1] * vf1[1] + vf1[2] * vf1[2];
-                    st_vmax = fmax(st_vmax, sqrt(v2));
-                    st_v2 += v2;
-                    st_g += g_rate;
-                    st_near += (lg > sp.near_div_length) ? 1.0 : 0.0;
-                }
-            }
-            else
-            {
-                geom_c[i] = go;
-                vel_c[i] = vo;
-            }
-        }
-    } while (false);
-    if (DRY) return;
-    if ((KIND == MODE_FINAL || in_place) && sp.stats_on)
-    {
-        // per-block partials of the step-size features, summed in block order later
-        st_vmax = warp_max(st_vmax);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1)
-        {
-            st_v2 += __shfl_xor_sync(0xffffffffu, st_v2, off);
-            st_g += __shfl_xor_sync(0xffffffffu, st_g, off);
-            st_near += __shfl_xor_sync(0xffffffffu, st_near, off);
-        }
-        if ((threadIdx.x & 31) == 0) sh_stat[threadIdx.x >> 5] = make_double4(st_vmax, st_v2, st_g, st_near);
-        __syncthreads();
-        if (threadIdx.x == 0)
-        {
-            double4 a = sh_stat[0];
-            for (int w = 1; w < AT_T / 32; ++w)
-            {
-                const double4 b = sh_stat[w];
-                a.x = fmax(a.x, b.x); a.y += b.y; a.z += b.z; a.w += b.w;
-            }
-            // the last block sums the partials in block order (no contended atomics)
-            sp.stat_part[blockIdx.x] = a;
-        }
-    }
-    if (KIND == MODE_FINAL || in_place)
-    {
-        local_drift = warp_max(local_drift);
-        if ((threadIdx.x & 31) == 0) sh_drift[threadIdx.x >> 5] = local_drift;
-    }
-    // block max of the scaled error, floored at min_error (simulation.hpp:1703)
-    local_max = fmax(local_max, sp.min_error);
-    if (bad) local_max = __longlong_as_double(0x7ff0000000000000ll);
-    local_max = warp_max(local_max);
-    if ((threadIdx.x & 31) == 0) sh_max[threadIdx.x >> 5] = local_max;
-    // any thread of the block that met a non-finite value reports it
-    const int block_bad = __syncthreads_or(bad ? 1 : 0);
-    if (threadIdx.x == 0)
-    {
-        double m = sh_max[0];
-        for (int w = 1; w < AT_T / 32; ++w) m = fmax(m, sh_max[w]);
-        unsigned long long bits = (unsigned long long)__double_as_longlong(m);
-        if (block_bad) atomicOr(&ctrl->status, (int)ST_NAN);
-        if (KIND == MODE_FINAL || in_place)
-        {
-            double dm = sh_drift[0];
-            for (int w = 1; w < AT_T / 32; ++w) dm = fmax(dm, sh_drift[w]);
-            if (dm > 0) atomicMax(&ctrl->drift_bits, (unsigned long long)__double_as_longlong(dm));
-        }
-        if (KIND == 3) { atomicMax(&ctrl->eval_err_bits, bits); last = false; }
-        else
-        {
-            atomicMax(&ctrl->err_bits, bits);
-            __threadfence();
-            unsigned int done = atomicAdd(&ctrl->blocks_done, 1u);
-            last = (done == gridDim.x - 1);
-        }
-    }
-    __syncthreads();
-    if ((KIND == MODE_FINAL || in_place) && sp.stats_on && last)
-    {
-        // step-size features of the accepted step (a failed proposal's are replaced
-        // by the final attempt's): every block's partial, in block order
-        __threadfence();
-        double4 a = make_double4(0.0, 0.0, 0.0, 0.0);
-        for (int b = threadIdx.x; b < gridDim.x; b += AT_T)
-        {
-            const double2* q = reinterpret_cast<const double2*>(sp.stat_part + b);
-            const double2 p0 = __ldcg(q), p1 = __ldcg(q + 1);
-            a.x = fmax(a.x, p0.x); a.y += p0.y; a.z += p1.x; a.w += p1.y;
-        }
-        a.x = warp_max(a.x);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1)
-        {
-            a.y += __shfl_xor_sync(0xffffffffu, a.y, off);
-            a.z += __shfl_xor_sync(0xffffffffu, a.z, off);
-            a.w += __shfl_xor_sync(0xffffffffu, a.w, off);
-        }
-        __syncthreads();
-        if ((threadIdx.x & 31) == 0) sh_stat[threadIdx.x >> 5] = a;
-        __syncthreads();
-        if (threadIdx.x == 0)
-        {
-            double4 t = sh_stat[0];
-            for (int w = 1; w < AT_T / 32; ++w)
-            {
-                const double4 b = sh_stat[w];
-                t.x = fmax(t.x, b.x); t.y += b.y; t.z += b.z; t.w += b.w;
-            }
-            ctrl->st_vmax_bits = (unsigned long long)__double_as_longlong(t.x);
-            ctrl->st_v2_fx = (unsigned long long)llrint(ldexp(t.y, STAT_V2_SHIFT));
-            ctrl->st_g_fx = (unsigned long long)llrint(ldexp(fmax(t.z, 0.0), STAT_G_SHIFT));
-            ctrl->st_near_div = (unsigned long long)t.w;
-        }
-    }
-    if (KIND != 3 && last && threadIdx.x == 0)
-    {
-        __threadfence();
-        double E = __longlong_as_double((long long)atomicAdd(&ctrl->err_bits, 0ull));
-        E = fmax(E, sp.min_error);
-        if (commit) E = ctrl->last_trial_error;
-        // motion of the new state, counted once the step is accepted
-        const double dm = __longlong_as_double((long long)atomicAdd(&ctrl->drift_bits, 0ull));
-        if (KIND == MODE_FINAL) ctrl->drift += dm;
-        ctrl->drift_bits = 0ull;
-        ctrl->err_bits = 0ull;
-        ctrl->blocks_done = 0u;
-        controller_finish(ctrl, sp, KIND, E, commit);
-        if (in_place && ctrl->mode == MODE_COMMIT)
-        {
-            // the proposal passed: its state is in place; close the step and leave
-            // MODE_COMMIT so that this iteration's final attempt exits at once
-            ctrl->drift += dm;
-            controller_finish(ctrl, sp, MODE_FINAL, E, true);
-            ctrl->mode = MODE_COMMIT;
-        }
-        // another retry?  (bounded: the controller schedules at most max_tries of them)
-        if ((use_cond & 1) && (KIND == MODE_TRIAL || KIND == MODE_RETRY))
-            cudaGraphSetConditional((cudaGraphConditionalHandle)cond,
-                                    (ctrl->mode == MODE_RETRY && ctrl->tries < sp.max_tries) ? 1u : 0u);
-        if ((use_cond & 2) && KIND == MODE_TRIAL)
-            cudaGraphSetConditional((cudaGraphConditionalHandle)cond_run, ctrl->mode != MODE_COMMIT ? 1u : 0u);
-    }
 }
 
 // Frame snapshot, at the end of an iteration: when the accepted step marked a frame,
@@ -2055,152 +1343,31 @@ void launch_attempt_order(const Geom* geom, Ctrl* ctrl, const MechParams& P, int
     k_attempt_order<<<blocks, 256, 0, st>>>(ctrl, flag, pos, order);
 }
 
-template <int S, bool NOISE, int DIM, int V>
-static void launch_attempt_s(int kind, int blocks, Geom* geom, Vel* vel, Phys* phys, const Gen6* fcc,
-                             Ctrl* ctrl, const StepParams& sp, Geom* geom_c, Vel* vel_c, Gen6* err_out,
-                             Gen6* k0buf, double eval_dt, int eval_attempt, cudaStream_t st,
-                             unsigned long long cond, int use_cond, PairGather pg, unsigned long long cond_run)
-{
-#define AT_ARGS geom, vel, phys, fcc, ctrl, sp, geom_c, vel_c, err_out, k0buf, eval_dt, eval_attempt, cond, use_cond, pg, cond_run
-#define AT_LAUNCH(K) k_attempt<S, K, NOISE, DIM, V><<<blocks, AT_T, 0, st>>>(AT_ARGS);
-    switch (kind)
-    {
-        case MODE_TRIAL: AT_LAUNCH(MODE_TRIAL) break;
-        case MODE_RETRY: AT_LAUNCH(MODE_RETRY) break;
-        case MODE_FINAL: AT_LAUNCH(MODE_FINAL) break;
-        default: AT_LAUNCH(3) break;
-    }
-#undef AT_LAUNCH
-#undef AT_ARGS
-}
-
 int attempt_blocks(int cap_cells) { return max(cdiv(cap_cells, AT_T), 1); }
 
-void launch_attempt(int kind, Geom* geom, Vel* vel, Phys* phys, const Gen6* fcc, Ctrl* ctrl,
-                    const StepParams& sp, Geom* geom_c, Vel* vel_c, Gen6* err_out, Gen6* k0buf,
-                    double eval_dt, int eval_attempt, int cap_cells, cudaStream_t st,
-                    unsigned long long cond, int use_cond, PairGather pg, int dims, unsigned long long cond_run)
+void launch_attempt(int kind, const AttemptArgs& a, int dims, cudaStream_t st)
 {
-    int blocks = attempt_blocks(cap_cells);
-#define AT_CALL(S, NZ, D, F) launch_attempt_s<S, NZ, D, F>(kind, blocks, geom, vel, phys, fcc, ctrl, sp, geom_c, vel_c, err_out, k0buf, eval_dt, eval_attempt, st, cond, use_cond, pg, cond_run)
-#define AT_CASE(S, D) case S: \
-        if (D == 3 && sp.mixed) { if (sp.noise_on) AT_CALL(S, true, D, (D == 3 ? 1 : 0)); else AT_CALL(S, false, D, (D == 3 ? 1 : 0)); } \
-        else if (D == 3 && sp.fric) { if (sp.noise_on) AT_CALL(S, true, D, (D == 3 ? 2 : 0)); else AT_CALL(S, false, D, (D == 3 ? 2 : 0)); } \
-        else if (sp.noise_on) AT_CALL(S, true, D, 0); \
-        else AT_CALL(S, false, D, 0); \
-        break;
-    if (dims == 2)
+    switch (a.sp->s)
     {
-        // the 2-D driver integrates with Bogacki-Shampine 3(2) (2D/include/simulation.hpp:217-228);
-        // Heun-Euler is kept for comparison runs
-        switch (sp.s)
-        {
-            AT_CASE(2, 2) AT_CASE(4, 2)
-            default: break;
-        }
-        return;
-    }
-    switch (sp.s)
-    {
-        AT_CASE(2, 3) AT_CASE(4, 3) AT_CASE(6, 3) AT_CASE(7, 3)
+        case 2: launch_attempt_2(kind, a, dims, st); break;
+        case 4: launch_attempt_4(kind, a, dims, st); break;
+        case 6: launch_attempt_6(kind, a, dims, st); break;
+        case 7: launch_attempt_7(kind, a, dims, st); break;
         default: break;
     }
-#undef AT_CASE
-#undef AT_CALL
 }
 
-// Friction decision check over the candidate pairs of the last pair pass: the planar
-// decision of each stage from the two cells' stage states (the contact points
-// r + s n of both cells below 1.01 R, mechanics.hpp:1090-1110), compared with the one at
-// y0; a pair whose set of differing stages changed is updated in both entries.  The last
-// block schedules another trial pass when any pair changed.
-__global__ void k_fr_check(Ctrl* ctrl, const int4* __restrict__ pairs, const int* __restrict__ fr_list,
-                           const double4* __restrict__ jbuf, const double2* __restrict__ ystage, int ld, int S,
-                           int* fmask, double R)
+void launch_friction_rounds(int kind, const AttemptArgs& a, const int4* act, const int* fr_list, int* fmask, double R,
+                            cudaStream_t st)
 {
-    __shared__ bool last;
-    if (!ctrl->fr_pending) return;
-    const int m = ctrl->fr_ncand;
-    const double lim = 1.01 * R;
-    int changed = 0, nflip = 0;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < m; q += gridDim.x * blockDim.x)
+    switch (a.sp->s)
     {
-        const int4 pr = pairs[fr_list[q]];
-        const double s = jbuf[pr.z].w, t = jbuf[pr.w].w;
-        const int mk = fmask[pr.z];
-        const bool d0 = (mk & FR_D0) != 0;
-        int fl = 0;
-        for (int st = 1; st < S; ++st)
-        {
-            const double2 a = ystage[(size_t)st * ld + pr.x], b = ystage[(size_t)st * ld + pr.y];
-            const bool flat = __dadd_rn(a.x, __dmul_rn(s, a.y)) < lim && __dadd_rn(b.x, __dmul_rn(t, b.y)) < lim;
-            if (flat != d0) fl |= 1 << st;
-        }
-        if (fl != (mk & FR_FLIPS))
-        {
-            fmask[pr.z] = (mk & ~FR_FLIPS) | fl;
-            fmask[pr.w] = (fmask[pr.w] & ~FR_FLIPS) | fl;
-            changed = 1;
-        }
-        nflip += fl != 0;
-    }
-    changed = __syncthreads_or(changed);
-    if (nflip) atomicAdd(&ctrl->fr_nflip_next, nflip);
-    if (threadIdx.x == 0)
-    {
-        if (changed) atomicOr(&ctrl->fr_changed, 1);
-        __threadfence();
-        last = atomicAdd(&ctrl->fr_blocks, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (last && threadIdx.x == 0)
-    {
-        __threadfence();
-        ctrl->fr_nflip = atomicAdd(&ctrl->fr_nflip_next, 0);
-        ctrl->fr_nflip_next = 0;
-        ctrl->fr_pending = atomicAdd(&ctrl->fr_changed, 0);
-        ctrl->fr_changed = 0;
-        ctrl->fr_blocks = 0u;
-    }
-}
-
-__global__ void k_fr_arm(Ctrl* ctrl) { ctrl->fr_pending = ctrl->fr_ncand > 0 && !ctrl->halted; }
-
-template <int S, int KIND, bool NOISE>
-static void launch_fr_rounds_s(Geom* geom, Vel* vel, Phys* phys, const Gen6* fcc, Ctrl* ctrl, const StepParams& sp,
-                               Geom* geom_c, Vel* vel_c, Gen6* k0buf, double eval_dt, int eval_attempt, int blocks,
-                               cudaStream_t st, PairGather pg, const int4* pairs, const int* fr_list, int* fmask,
-                               double R, int check_blocks)
-{
-    k_fr_arm<<<1, 1, 0, st>>>(ctrl);
-    for (int r = 1; r < S; ++r)
-    {
-        k_attempt<S, KIND, NOISE, 3, 3><<<blocks, AT_T, 0, st>>>(geom, vel, phys, fcc, ctrl, sp, geom_c, vel_c, nullptr, k0buf, eval_dt,
-                                 eval_attempt, 0ull, 0, pg, 0ull);
-        k_fr_check<<<check_blocks, 256, 0, st>>>(ctrl, pairs, fr_list, pg.jbuf, pg.ystage, pg.ystage_ld, S, fmask, R);
-    }
-}
-
-void launch_friction_rounds(int kind, Geom* geom, Vel* vel, Phys* phys, const Gen6* fcc, Ctrl* ctrl,
-                            const StepParams& sp, Geom* geom_c, Vel* vel_c, Gen6* k0buf, double eval_dt,
-                            int eval_attempt, int cap_cells, cudaStream_t st, PairGather pg, const int4* pairs,
-                            const int* fr_list, int* fmask, double R)
-{
-    const int blocks = attempt_blocks(cap_cells);
-    const int cb = 148 * 2;
-#define FR_K(S, K) { if (sp.noise_on) launch_fr_rounds_s<S, K, true>(geom, vel, phys, fcc, ctrl, sp, geom_c, vel_c, k0buf, eval_dt, eval_attempt, blocks, st, pg, pairs, fr_list, fmask, R, cb); \
-                     else launch_fr_rounds_s<S, K, false>(geom, vel, phys, fcc, ctrl, sp, geom_c, vel_c, k0buf, eval_dt, eval_attempt, blocks, st, pg, pairs, fr_list, fmask, R, cb); }
-#define FR_S(S) case S: \
-        switch (kind) { case MODE_TRIAL: FR_K(S, MODE_TRIAL) break; case MODE_RETRY: FR_K(S, MODE_RETRY) break; \
-                        case MODE_FINAL: FR_K(S, MODE_FINAL) break; default: FR_K(S, 3) break; } \
-        break;
-    switch (sp.s)
-    {
-        FR_S(2) FR_S(4) FR_S(6) FR_S(7)
+        case 2: launch_friction_rounds_2(kind, a, act, fr_list, fmask, R, st); break;
+        case 4: launch_friction_rounds_4(kind, a, act, fr_list, fmask, R, st); break;
+        case 6: launch_friction_rounds_6(kind, a, act, fr_list, fmask, R, st); break;
+        case 7: launch_friction_rounds_7(kind, a, act, fr_list, fmask, R, st); break;
         default: break;
     }
-#undef FR_S
-#undef FR_K
 }
 
 __global__ void k_velocities_2d(const Geom* __restrict__ geom, const Phys* __restrict__ phys,
@@ -2214,7 +1381,7 @@ __global__ void k_velocities_2d(const Geom* __restrict__ geom, const Phys* __res
         const double y[6] = {g.rx, g.ry, g.rz, g.nx, g.ny, g.nz};
         const Phys ph = phys[i];
         Gen6 out;
-        velocity_2d(sp, y, ph.l, ph.eta0, ph.eta1, load_gen6(fcc, i), nz, out.f);
+        velocity_2d(y, cell_drag_2d(sp, ph.l, ph.eta0, ph.eta1), load_gen6(fcc, i), nz, out.f);
         v_out[i] = out;
     }
 }
@@ -2233,8 +1400,11 @@ __global__ void k_velocities(const Geom* __restrict__ geom, const Vel* __restric
         base_force<false>(sp, load_gen6(fcc, i), 0, 0, i, f0);
         Gen6 out;
         const Phys ph = phys[i];
-        if (sp.mixed) cell_velocity_f32(sp, a2, y, ph.l, g.h, ph.eta0, ph.eta1, ph.sigma0, vel + i, f0, out.f);
-        else cell_velocity(sp, a2, y, ph.l, g.h, ph.eta0, ph.eta1, ph.sigma0, vel + i, f0, out.f);
+        CellDrag d = cell_drag(ph.l, ph.eta0);
+        if (sp.mixed)
+            cell_velocity<true>(sp.mp, a2, y, ph.l, g.h, ph.eta0, ph.eta1, ph.sigma0, d, vel + i, f0, out.f);
+        else
+            cell_velocity<false>(sp.mp, a2, y, ph.l, g.h, ph.eta0, ph.eta1, ph.sigma0, d, vel + i, f0, out.f);
         v_out[i] = out;
     }
 }

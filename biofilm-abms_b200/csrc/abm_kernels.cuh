@@ -30,6 +30,12 @@ enum StatusBits {
     ST_NBR_OVERFLOW = 2,   // more neighbors than cap_neighbors_per_cell
     ST_BIN_OVERFLOW = 4,   // grid needs more bins than allocated
     ST_CELL_OVERFLOW = 8,  // division would exceed cap_cells
+    ST_BARRIER = 16,       // a grid barrier's bounded wait ran out
+};
+
+// Record of a barrier over the blocks of a cooperative launch (abm_grid.cuh)
+struct GridBar {
+    unsigned int count, gen;
 };
 
 // Device-resident clock, controller and population state.
@@ -98,8 +104,13 @@ struct Ctrl {
     // basal-only compaction: cells kept by the last test, cells dropped so far
     int n_keep;
     long long basal_dropped;
-    double drift;                       // sum over accepted steps of the max segment motion
+    double drift;                       // max over cells of the segment's motion since the last refresh
     unsigned long long drift_bits;      // block maxima of the running attempt (ordered bits)
+    // mixed precision: the sum over the accepted steps of the largest motion in each.  A pass
+    // whose list would be stale by this sum takes ROUND_STALE (dist_geom_mixed), whether or not
+    // the list is stale by `drift`: the rule keeps mixed-precision trajectories bit for bit.
+    double path;
+    unsigned long long path_bits;
 };
 
 struct Grid {
@@ -163,9 +174,9 @@ struct ForceParams {
     double coulomb_cc;              // Coulomb cap coefficient (not positive: no cap)
     const Vel* vel;                 // stored velocities of the cells (dr, dn)
     const double* feta;             // friction coefficient of each cell
-    double4* fbuf;                  // per CSR entry: share change when the contact is planar
-    int* fmask;                     // per CSR entry: FR_* bits
-    int* fr_list;                   // pairs with a planar-contact candidate, this pass
+    double4* fbuf;                  // per active share: its change when the planar decision flips
+    int* fmask;                     // per active share: FR_* bits
+    int* fr_list;                   // active pairs with a planar-contact candidate, this pass
 };
 
 // Friction: a contact with |dz / d| < 1e-3 whose two contact points lie below 1.01 R is taken
@@ -181,17 +192,29 @@ struct BuildParams {
     int cap_per_cell;
 };
 
+// The active pairs: those within 2R + skin at the last refresh.  Each cell's active shares
+// lie at the start of its row's slots in `jbuf`, in the row's column order.
+struct ActiveList {
+    int4* act;                  // (i, j, slot of i's share, slot of j's share); j's sign bit: to_adhere (2-D)
+    int* n_act;                 // active shares of each cell
+    unsigned char* keep;        // per CSR entry: active (made and read by a refresh)
+    Geom* gref;                 // the cells at the last refresh
+    const int* row_ptr;
+    GridBar* bar;
+};
+const int ACT_ADHERE = (int)0x80000000;
+
 // Where an attempt finds the pair force when it completes the sum itself:
-// fused = 1: fcc holds the lower-neighbor share, jbuf the partners' shares;
-// fused = 2: jbuf holds both shares of every pair (screened pass), as double4;
+// fused = 2: jbuf holds both shares of every active pair, as double4;
 // fused = 3: the same as float4 (mixed precision);
 // fused = 0: fcc already holds the total.
 struct PairGather {
     int fused;
     const int* row_ptr;
-    const int* lower_end;
+    const int* n_act;
     const double4* jbuf;
     Gen6* fcc_w;
+    const Geom* gref;
     // friction: the planar-contact corrections of each stage, and the stage states of the
     // cells with candidate contacts (z and n_z per stage, written by the trial passes)
     const double4* fbuf;
@@ -243,13 +266,13 @@ void launch_pair_force(const Geom* geom, const int* row_ptr, const int* lower_en
                        int with_gather = 1, int dims = 3);
 void launch_csr_rev(const Ctrl* ctrl, const int* row_ptr, const int* col, int* lower_end, int* rev,
                     int cap_cells, cudaStream_t st);
-// screened pass over every unordered pair (both shares into jbuf); with_sum also
-// writes each cell's total into fcc.
-void launch_pair_screened(const Geom* geom, const int* row_ptr, const int* lower_end, const int* col, const int* rev, Ctrl* ctrl, ForceParams fp, const double* jkr_delta,
+// pass over the active pairs (both shares into jbuf), refreshing the active list when it is
+// stale; with_sum also writes each cell's total into fcc.
+void launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, const double* jkr_delta,
                           const double* jkr_radius, Gen6* fcc, double4* jbuf, int mixed, int max_entries,
                           int cap_cells, int num_sms, cudaStream_t st, int with_sum, int dims, int tile,
-                          int blocks_per_sm, const int4* pairs, int* surv, const StepParams* sp = nullptr,
-                          const float* mlp_w = nullptr);
+                          int blocks_per_sm, const int4* pairs, int* surv, ActiveList al,
+                          const StepParams* sp = nullptr, const float* mlp_w = nullptr);
 // the list of unordered pairs (i, j < i, lower entry k, partner entry rev[k]) after
 // k_csr_rev, cells in `order` (null: index order): counts -> scan -> fill; uses
 // `count` and `start` (cap_cells + 1) as scratch
@@ -261,11 +284,33 @@ void launch_pair_list(const Ctrl* ctrl, const int* row_ptr, const int* lower_end
 // (writes candidates and errors without touching the controller)
 // cond / use_cond: WHILE-node handle that the trial and retry attempts set to 1
 // when the controller asks for another retry (only inside a CUDA graph)
-void launch_attempt(int kind, Geom* geom, Vel* vel, Phys* phys, const Gen6* fcc, Ctrl* ctrl,
-                    const StepParams& sp, Geom* geom_c, Vel* vel_c, Gen6* err_out, Gen6* k0buf,
-                    double eval_dt, int eval_attempt, int cap_cells, cudaStream_t st,
-                    unsigned long long cond = 0, int use_cond = 0, PairGather pg = PairGather{0, 0, 0, 0, 0},
-                    int dims = 3, unsigned long long cond_run = 0);
+struct AttemptArgs {
+    Geom* geom;
+    Vel* vel;
+    Phys* phys;
+    const Gen6* fcc;
+    Ctrl* ctrl;
+    const StepParams* sp;
+    Geom* geom_c;
+    Vel* vel_c;
+    Gen6* k0buf;
+    int cap_cells;
+    PairGather pg;
+    // the API's evaluation
+    Gen6* err_out;
+    double eval_dt;
+    int eval_attempt;
+    // graph conditions
+    unsigned long long cond;
+    int use_cond;
+    unsigned long long cond_run;
+};
+void launch_attempt(int kind, const AttemptArgs& a, int dims, cudaStream_t st);
+// one translation unit per stage count (abm_attempt.cuh)
+void launch_attempt_2(int kind, const AttemptArgs& a, int dims, cudaStream_t st);
+void launch_attempt_4(int kind, const AttemptArgs& a, int dims, cudaStream_t st);
+void launch_attempt_6(int kind, const AttemptArgs& a, int dims, cudaStream_t st);
+void launch_attempt_7(int kind, const AttemptArgs& a, int dims, cudaStream_t st);
 // accepted proposal of the learned controller: candidate -> state (no-op otherwise)
 // the attempt order of the cells (3-D): full surface solve first (made at every rebuild)
 // one frame of the ring: the state after the accepted step that marked it
@@ -297,6 +342,7 @@ void launch_mlp_grad(const float* master, const float* X, const float* T, int n,
 void launch_mlp_train(float* master, float* m1, float* m2, float* G, const float* X, const float* T, int n,
                       int epochs, float lr, unsigned seed, float* loss_out, cudaStream_t st);
 // features of the running iteration -> log row; with sp.network also the dt of the first attempt
+const int AT_T = 128;           // threads of an attempt block, one cell each
 int attempt_blocks(int cap_cells);
 
 // division (growth.hpp:66-426), abm_divide.cu
@@ -375,12 +421,18 @@ void launch_verlet_step(Geom* geom, Vel* vel, Phys* phys, Geom* geom_c, Vel* vel
                         const int4* pairs, const int* row_ptr, const int* lower_end, double4* jbuf, double4* pbuf,
                         double rho, int cap_cells, int cap_pairs, cudaStream_t st);
 
-// friction (abm_kernels.cu): before an attempt, trial passes that run the stages of the cells
-// with candidate contacts and checks that recompute the candidates' planar decisions from
+// friction: before an attempt, trial passes that run the stages of the cells with
+// candidate contacts and checks that recompute the candidates' planar decisions from
 // the stage states, until the decisions agree with the states (at most stages - 1 rounds)
-void launch_friction_rounds(int kind, Geom* geom, Vel* vel, Phys* phys, const Gen6* fcc, Ctrl* ctrl,
-                            const StepParams& sp, Geom* geom_c, Vel* vel_c, Gen6* k0buf, double eval_dt,
-                            int eval_attempt, int cap_cells, cudaStream_t st, PairGather pg, const int4* pairs,
-                            const int* fr_list, int* fmask, double R);
+void launch_friction_rounds(int kind, const AttemptArgs& a, const int4* act, const int* fr_list, int* fmask, double R,
+                            cudaStream_t st);
+void launch_friction_rounds_2(int kind, const AttemptArgs& a, const int4* act, const int* fr_list, int* fmask,
+                              double R, cudaStream_t st);
+void launch_friction_rounds_4(int kind, const AttemptArgs& a, const int4* act, const int* fr_list, int* fmask,
+                              double R, cudaStream_t st);
+void launch_friction_rounds_6(int kind, const AttemptArgs& a, const int4* act, const int* fr_list, int* fmask,
+                              double R, cudaStream_t st);
+void launch_friction_rounds_7(int kind, const AttemptArgs& a, const int4* act, const int* fr_list, int* fmask,
+                              double R, cudaStream_t st);
 
 }   // namespace abm
