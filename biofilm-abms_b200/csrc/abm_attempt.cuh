@@ -28,7 +28,7 @@ __global__ void __launch_bounds__(AT_T, (S <= 4 ? (V == 3 ? 3 : 6) : 1)) k_attem
                                                  Ctrl* ctrl, StepParams sp, Geom* geom_c, Vel* vel_c,
                                                  Gen6* err_out, Gen6* k0buf, double eval_dt, int eval_attempt,
                                                  unsigned long long cond, int use_cond, PairGather pg,
-                                                 unsigned long long cond_run)
+                                                 unsigned long long cond_run, int flow)
 {
     constexpr bool F32 = V == 1, FRIC = V >= 2, DRY = V == 3;
     __shared__ double sh_max[AT_T / 32], sh_drift[AT_T / 32], sh_path[AT_T / 32];
@@ -42,6 +42,19 @@ __global__ void __launch_bounds__(AT_T, (S <= 4 ? (V == 3 ? 3 : 6) : 1)) k_attem
             cudaGraphSetConditional((cudaGraphConditionalHandle)cond, 0u);
         if ((use_cond & 2) && KIND == MODE_TRIAL && blockIdx.x == 0 && threadIdx.x == 0)
             cudaGraphSetConditional((cudaGraphConditionalHandle)cond_run, 0u);
+        return;
+    }
+    if (KIND != 3 && !DRY && loop_idle(ctrl, flow, KIND == MODE_TRIAL))
+    {
+        // a slow iteration that resumes after a failed first attempt goes on with the retries
+        if (flow == FLOW_SLOW && KIND == MODE_TRIAL && blockIdx.x == 0 && threadIdx.x == 0)
+        {
+            if (use_cond & 1)
+                cudaGraphSetConditional((cudaGraphConditionalHandle)cond,
+                                        (ctrl->todo > 0 && ctrl->mode == MODE_RETRY && ctrl->tries < sp.max_tries) ? 1u : 0u);
+            if (use_cond & 2)
+                cudaGraphSetConditional((cudaGraphConditionalHandle)cond_run, ctrl->todo > 0 ? 1u : 0u);
+        }
         return;
     }
     const int n = ctrl->n;
@@ -99,7 +112,7 @@ __global__ void __launch_bounds__(AT_T, (S <= 4 ? (V == 3 ? 3 : 6) : 1)) k_attem
     const bool do_gather = pg.fused && !commit &&
                            (KIND == MODE_TRIAL || (KIND == MODE_FINAL && !trial_ran) || sp.propose);
     double local_max = 0.0;
-    bool bad = false;
+    bool bad = false, longer = false;
     double st_vmax = 0.0, st_v2 = 0.0, st_g = 0.0, st_near = 0.0;
     // motion of each new segment since the last refresh of the active pairs:
     // |dr| + h' |dn| + |dh| (a Hausdorff bound)
@@ -241,6 +254,7 @@ __global__ void __launch_bounds__(AT_T, (S <= 4 ? (V == 3 ? 3 : 6) : 1)) k_attem
                 const double g_rate = phys[i].growth;
                 double lg = l + g_rate * (4 * sp.mp.R / 3 + l) * dt;
                 go.h = lg / 2;
+                longer = sp.div_on && lg > sp.Ldiv;       // divideMaxLength, growth.hpp:66-71
                 {
                     const Geom q = load_geom(pg.gref, i);
                     const double ax = go.rx - q.rx, ay = go.ry - q.ry, az = go.rz - q.rz;
@@ -305,6 +319,7 @@ __global__ void __launch_bounds__(AT_T, (S <= 4 ? (V == 3 ? 3 : 6) : 1)) k_attem
     }
     if (KIND == MODE_FINAL || in_place)
     {
+        if (longer) atomicOr(&ctrl->div_any, 1);
         local_drift = warp_max(local_drift);
         if ((threadIdx.x & 31) == 0) sh_drift[threadIdx.x >> 5] = local_drift;
         if (F32)
@@ -399,16 +414,19 @@ __global__ void __launch_bounds__(AT_T, (S <= 4 ? (V == 3 ? 3 : 6) : 1)) k_attem
         ctrl->path_bits = 0ull;
         ctrl->err_bits = 0ull;
         ctrl->blocks_done = 0u;
-        controller_finish(ctrl, sp, KIND, E, commit);
+        const bool grown = atomicExch(&ctrl->div_any, 0) != 0;
+        controller_finish(ctrl, sp, KIND, E, grown, commit);
         if (in_place && ctrl->mode == MODE_COMMIT)
         {
             // the proposal passed: its state is in place; close the step and leave
             // MODE_COMMIT so that this iteration's final attempt exits at once
             ctrl->drift = dm;
             ctrl->path += pm;
-            controller_finish(ctrl, sp, MODE_FINAL, E, true);
+            controller_finish(ctrl, sp, MODE_FINAL, E, grown, true);
             ctrl->mode = MODE_COMMIT;
         }
+        else if (flow == FLOW_FAST && KIND == MODE_TRIAL && (sp.propose || ctrl->mode == MODE_RETRY))
+            ctrl->hold = HOLD_RETRY;       // the slow iteration goes on from here
         // another retry?  (bounded: the controller schedules at most max_tries of them)
         if ((use_cond & 1) && (KIND == MODE_TRIAL || KIND == MODE_RETRY))
             cudaGraphSetConditional((cudaGraphConditionalHandle)cond,
@@ -475,14 +493,17 @@ __global__ void k_fr_check(Ctrl* ctrl, const int4* __restrict__ act, const int* 
 }
 
 template <int S>
-__global__ void k_fr_arm(Ctrl* ctrl) { ctrl->fr_pending = ctrl->fr_ncand > 0 && !ctrl->halted; }
+__global__ void k_fr_arm(Ctrl* ctrl, int flow, bool first)
+{
+    ctrl->fr_pending = ctrl->fr_ncand > 0 && !ctrl->halted && !loop_idle(ctrl, flow, first);
+}
 
 template <int KIND, bool NOISE, int DIM, int V>
 static void launch_one(const AttemptArgs& a, cudaStream_t st)
 {
     k_attempt<ABM_STAGES, KIND, NOISE, DIM, V><<<attempt_blocks(a.cap_cells), AT_T, 0, st>>>(
         a.geom, a.vel, a.phys, a.fcc, a.ctrl, *a.sp, a.geom_c, a.vel_c, a.err_out, a.k0buf, a.eval_dt, a.eval_attempt,
-        a.cond, a.use_cond, a.pg, a.cond_run);
+        a.cond, a.use_cond, a.pg, a.cond_run, a.flow);
 }
 
 template <bool NOISE, int DIM, int V>
@@ -525,7 +546,7 @@ void ABM_CAT(launch_attempt_, ABM_STAGES)(int kind, const AttemptArgs& a, int di
 void ABM_CAT(launch_friction_rounds_, ABM_STAGES)(int kind, const AttemptArgs& a, const int4* act, const int* fr_list,
                                                   int* fmask, double R, cudaStream_t st)
 {
-    k_fr_arm<ABM_STAGES><<<1, 1, 0, st>>>(a.ctrl);
+    k_fr_arm<ABM_STAGES><<<1, 1, 0, st>>>(a.ctrl, a.flow, kind == MODE_TRIAL);
     for (int r = 1; r < ABM_STAGES; ++r)
     {
         launch_noise<3, 3>(kind, a, st);

@@ -97,7 +97,8 @@ struct abm_ctx {
     ForceParams fp; StepParams sp; BuildParams bp;
     // graphs
     cudaGraphExec_t g_iter = nullptr, g_rebuild = nullptr;
-    cudaGraphExec_t g_iter_k = nullptr;   // iter_k iterations in one graph (long loops)
+    cudaGraphExec_t g_loop = nullptr;     // many Runge-Kutta iterations (append_loop)
+    cudaGraphExec_t g_iter_k = nullptr;   // iter_k iterations in one graph (Verlet, post-step kernels)
     int iter_k = 1;
     bool graph_fallback = false;     // conditional nodes could not be built
     std::string graph_note;
@@ -201,6 +202,7 @@ static void free_all(abm_ctx* c)
 {
     if (c->g_iter) cudaGraphExecDestroy(c->g_iter);
     if (c->g_iter_k) cudaGraphExecDestroy(c->g_iter_k);
+    if (c->g_loop) cudaGraphExecDestroy(c->g_loop);
     if (c->g_rebuild) cudaGraphExecDestroy(c->g_rebuild);
     void* ptrs[] = {c->geom, c->vel, c->phys, c->fcc, c->geom_c, c->vel_c, c->gen_tmp, c->k0buf, c->ctrl, c->grid,
                     c->bbox_acc, c->bbox_counter, c->bin_count, c->bin_start, c->key, c->slot,
@@ -222,6 +224,7 @@ static void drop_iteration_graphs(abm_ctx* c)
 {
     if (c->g_iter) { cudaGraphExecDestroy(c->g_iter); c->g_iter = nullptr; }
     if (c->g_iter_k) { cudaGraphExecDestroy(c->g_iter_k); c->g_iter_k = nullptr; }
+    if (c->g_loop) { cudaGraphExecDestroy(c->g_loop); c->g_loop = nullptr; }
 }
 
 static void fill_tableau(StepParams& sp, int mode, bool& ok)
@@ -974,13 +977,13 @@ static void enqueue_rebuild(abm_ctx* c)
 // per cell into fcc (the API paths; the loop's first attempt sums them itself)
 // in_loop: the pass of a loop iteration, one of whose blocks also makes the iteration's
 // step-size features (and, learned, the proposed dt)
-static void enqueue_pair_force(abm_ctx* c, int with_gather, bool in_loop = false)
+static void enqueue_pair_force(abm_ctx* c, int with_gather, bool in_loop = false, int flow = FLOW_STEP)
 {
     ActiveList al = {c->act, c->n_act, c->keep_entry, c->gref, c->row_ptr, c->bar};
     launch_pair_screened(c->geom, c->ctrl, c->fp, c->jkr_delta, c->jkr_radius, c->fcc, c->jbuf,
                          c->p.precision == ABM_PRECISION_MIXED, c->cap * c->cap_nbr, c->cap, c->num_sms, c->st,
                          with_gather, c->dims, c->p.pair_tile, c->p.pair_blocks_per_sm, c->pairs, c->surv, al,
-                         in_loop ? &c->sp : nullptr, c->mlp_w);
+                         in_loop ? &c->sp : nullptr, c->mlp_w, flow);
 }
 
 // pair_sum 1 (default): the first attempt sums each cell's shares itself; 2: a
@@ -989,13 +992,19 @@ static bool sum_in_attempt(abm_ctx* c) { return c->p.pair_sum != 2; }
 
 // the loop's pair pass: the shares, plus their per-cell sums unless the first attempt
 // makes them, and the step-size proposal
-static void enqueue_loop_pair_force(abm_ctx* c) { enqueue_pair_force(c, sum_in_attempt(c) ? 0 : 1, true); }
+static void enqueue_loop_pair_force(abm_ctx* c, int flow = FLOW_STEP)
+{
+    enqueue_pair_force(c, sum_in_attempt(c) ? 0 : 1, true, flow);
+}
 
 // the attempts of one iteration: the state, and where they find the pair force
-static AttemptArgs loop_attempt(abm_ctx* c)
+static AttemptArgs loop_attempt(abm_ctx* c, int flow = FLOW_STEP)
 {
     const bool f32 = c->p.precision == ABM_PRECISION_MIXED && c->dims == 3;
     AttemptArgs a{};
+    a.flow = flow;
+    c->sp.div_on = c->div_enabled;
+    c->sp.Ldiv = c->p.Ldiv;
     a.geom = c->geom; a.vel = c->vel; a.phys = c->phys; a.fcc = c->fcc; a.ctrl = c->ctrl; a.sp = &c->sp;
     a.geom_c = c->geom_c; a.vel_c = c->vel_c; a.k0buf = c->k0buf; a.cap_cells = c->cap;
     a.pg = {sum_in_attempt(c) ? (f32 ? 3 : 2) : 0, c->row_ptr, c->n_act, c->jbuf, c->fcc, c->gref,
@@ -1239,7 +1248,7 @@ static int append_post_step(abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode
 // the rest runs only after a failed one:
 //   ... -> trial -> IF(proposal failed){retry x max_tries (each exits at once when
 //   no retry is pending) -> final}
-static int append_iteration(abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode_t>& deps)
+static int append_iteration(abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode_t>& deps, int flow = FLOW_STEP)
 {
     // every handle must belong to a conditional node of this graph, or instantiation fails
     cudaGraphConditionalHandle h_div = 0, h_retry = 0, h_run = 0;
@@ -1251,7 +1260,7 @@ static int append_iteration(abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode
     if (c->div_enabled)
     {
         CK(cudaGraphConditionalHandleCreate(&h_div, G, 0, cudaGraphCondAssignDefault));
-        rc = capture_into(c, G, deps, [&]() { launch_div_count(c->phys, c->ctrl, c->dp, c->div_flags, h_div, 1, c->st); });
+        rc = capture_into(c, G, deps, [&]() { launch_div_count(c->phys, c->ctrl, c->dp, c->div_flags, h_div, 1, c->st, flow); });
         if (rc) return rc;
         cudaGraph_t body;
         rc = add_conditional(c, G, deps, h_div, cudaGraphCondTypeIf, &body);
@@ -1271,22 +1280,22 @@ static int append_iteration(abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode
         if (c->frame_slots > 0) return capture_into(c, G, deps, [&]() { enqueue_frame_snapshot(c); });
         return ABM_OK;
     }
-    AttemptArgs trial = loop_attempt(c);
+    AttemptArgs trial = loop_attempt(c, flow);
     trial.cond = h_retry;
     trial.use_cond = (retries ? 1 : 0) | (branch ? 2 : 0);
     trial.cond_run = h_run;
     rc = capture_into(c, G, deps, [&]() {
-        enqueue_loop_pair_force(c);
+        enqueue_loop_pair_force(c, flow);
         enqueue_attempt(c, MODE_TRIAL, trial);
     });
     if (rc) return rc;
     auto retry_attempt = [&](int use_cond) {
-        AttemptArgs a = loop_attempt(c);
+        AttemptArgs a = loop_attempt(c, flow);
         a.cond = h_retry;
         a.use_cond = use_cond;
         enqueue_attempt(c, MODE_RETRY, a);
     };
-    auto final_attempt = [&]() { enqueue_attempt(c, MODE_FINAL, loop_attempt(c)); };
+    auto final_attempt = [&]() { enqueue_attempt(c, MODE_FINAL, loop_attempt(c, flow)); };
     if (branch)
     {
         cudaGraph_t body;
@@ -1339,7 +1348,76 @@ static int instantiate_iterations(abm_ctx* c, int k, cudaGraphExec_t* exec)
     return ABM_OK;
 }
 
-// One iteration per graph, and (for long loops) iter_k iterations per graph, iter_k
+// The loop graph, appended to G after `deps`: Ctrl::todo iterations.
+//   WHILE(iterations left){ LOOP_FAST x (pair pass -> trial [-> final])
+//                           -> IF(Ctrl::hold){one iteration with everything} }
+// A conditional node costs 6-8 us between two kernels here (the kernels of a small colony take
+// 6 to 20), and an iteration of its own has two of them (divisions, retries), which most
+// iterations do not need.  In a fast iteration the kernels follow each other; a trial whose
+// error test asks for a retry, or a step that leaves a cell longer than Ldiv, sets
+// Ctrl::hold, the rest of the round's kernels leave at once (2 us each), and the slow
+// iteration after the round goes on from there.  64-cell colony 45 -> 28 us an iteration.
+// LOOP_FAST trades the round's own two nodes against those idle kernels.
+const int LOOP_FAST = 8;
+
+static int append_loop(abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode_t>& deps)
+{
+    cudaGraphConditionalHandle h_loop = 0, h_slow = 0;
+    CK(cudaGraphConditionalHandleCreate(&h_loop, G, 1, cudaGraphCondAssignDefault));
+    cudaGraph_t round;
+    int rc = add_conditional(c, G, deps, h_loop, cudaGraphCondTypeWhile, &round);
+    if (rc) return rc;
+    CK(cudaGraphConditionalHandleCreate(&h_slow, round, 0, cudaGraphCondAssignDefault));
+    std::vector<cudaGraphNode_t> rd;
+    rc = capture_into(c, round, rd, [&]() {
+        const AttemptArgs a = loop_attempt(c, FLOW_FAST);
+        for (int k = 0; k < LOOP_FAST; ++k)
+        {
+            enqueue_loop_pair_force(c, FLOW_FAST);
+            enqueue_attempt(c, MODE_TRIAL, a);
+            // under the learned and PI controllers a passing trial closes the step
+            if (!c->sp.propose) enqueue_attempt(c, MODE_FINAL, a);
+            if (c->frame_slots > 0) enqueue_frame_snapshot(c);
+        }
+        launch_loop_round(c->ctrl, h_slow, h_loop, c->st);
+    });
+    if (rc) return rc;
+    cudaGraph_t slow;
+    rc = add_conditional(c, round, rd, h_slow, cudaGraphCondTypeIf, &slow);
+    if (rc) return rc;
+    std::vector<cudaGraphNode_t> sd;
+    return append_iteration(c, slow, sd, FLOW_SLOW);
+}
+
+static int build_loop_graph(abm_ctx* c)
+{
+    cudaGraph_t G;
+    CK(cudaGraphCreate(&G, 0));
+    std::vector<cudaGraphNode_t> deps;
+    int rc = append_loop(c, G, deps);
+    cudaError_t inst = cudaSuccess;
+    if (!rc) inst = cudaGraphInstantiate(&c->g_loop, G, 0);
+    cudaGraphDestroy(G);
+    if (rc) return rc;
+    CK(inst);
+    return ABM_OK;
+}
+
+// Do the iterations of this context run as the loop graph?  The velocity-Verlet step has no
+// conditional node, and the post-step kernels bring the periodic rebuild into the iteration.
+static bool has_loop(const abm_ctx* c) { return !c->verlet && !c->post_on; }
+
+// `step` iterations by the loop graph (no periodic rebuild among them)
+static int launch_loop(abm_ctx* c, int step)
+{
+    launch_loop_begin(c->ctrl, step, c->st);
+    if (c->div_enabled) launch_div_count(c->phys, c->ctrl, c->dp, c->div_flags, 0, 0, c->st, FLOW_BEGIN);
+    CK(cudaGraphLaunch(c->g_loop, c->st));
+    return ABM_OK;
+}
+
+// One iteration per graph, and (for long loops of the contexts without the loop graph) iter_k
+// iterations per graph, iter_k
 // the largest of 10, 5, 4, 2 that divides iter_update_neighbors, so that a K-graph
 // launched at a multiple of iter_k never straddles a periodic rebuild.  The fixed
 // cost of a graph launch (host submission, the conditional nodes' scheduling) is
@@ -1348,9 +1426,7 @@ static int build_iteration_graph(abm_ctx* c)
 {
     int rc = instantiate_iterations(c, 1, &c->g_iter);
     if (rc) return rc;
-    c->iter_k = 1;
-    for (int k : {10, 5, 4, 2})
-        if (c->p.iter_update_neighbors % k == 0) { c->iter_k = k; break; }
+    if (has_loop(c)) return ABM_OK;
     if (c->iter_k > 1) return instantiate_iterations(c, c->iter_k, &c->g_iter_k);
     return ABM_OK;
 }
@@ -1748,7 +1824,7 @@ int abm_divide(abm_ctx* c, int* n_divided)
 const char* abm_graph_info(const abm_ctx* c)
 {
     if (!c) return "";
-    if (!c->g_iter) return "no iteration graph yet";
+    if (!c->g_iter && !c->g_loop) return "no iteration graph yet";
     return c->graph_fallback ? c->graph_note.c_str() : "conditional";
 }
 
@@ -1788,11 +1864,15 @@ int abm_iterate(abm_ctx* c, int n_iters, int n_cells_stop, abm_stats* stats)
         enqueue_rebuild(c);
         c->nbrs_valid = true;
     }
+    c->iter_k = 1;
+    for (int k : {10, 5, 4, 2})
+        if (c->p.iter_update_neighbors % k == 0) { c->iter_k = k; break; }
     if (c->p.use_graphs)
     {
-        if (!c->g_iter && !c->graph_fallback)
+        const bool loop = has_loop(c) && n_iters >= LOOP_FAST / 2;
+        if (!(loop ? c->g_loop : c->g_iter) && !c->graph_fallback)
         {
-            rc = build_iteration_graph(c);
+            rc = loop ? build_loop_graph(c) : build_iteration_graph(c);
             if (rc)
             {
                 // conditional nodes unavailable: keep the error for abm_graph_info and fall back to
@@ -1819,12 +1899,38 @@ int abm_iterate(abm_ctx* c, int n_iters, int n_cells_stop, abm_stats* stats)
         int step = 1;
         if (c->p.use_graphs && !c->graph_fallback)
         {
-            if (c->g_iter_k && c->host_iter % c->iter_k == 0 && n_iters - k >= c->iter_k)
+            // up to the next periodic rebuild or look at the cell count; a few iterations
+            // left over run one by one
+            int run = std::min(n_iters - k, c->p.iter_update_neighbors - c->host_iter % c->p.iter_update_neighbors);
+            if (n_cells_stop > 0 && c->div_enabled)
+            {
+                // the count is looked at where iter_k iterations at a time (single ones off
+                // that grid) first reach next_check
+                int kk = k, hh = c->host_iter;
+                while (kk < next_check && kk < n_iters)
+                {
+                    const int by = (hh % c->iter_k == 0 && n_iters - kk >= c->iter_k) ? c->iter_k : 1;
+                    kk += by;
+                    hh += by;
+                }
+                run = std::min(run, kk - k);
+            }
+            if (has_loop(c) && run >= LOOP_FAST / 2 && c->g_loop)
+            {
+                rc = launch_loop(c, run);
+                if (rc) return rc;
+                step = run;
+            }
+            else if (c->g_iter_k && c->host_iter % c->iter_k == 0 && n_iters - k >= c->iter_k)
             {
                 CK(cudaGraphLaunch(c->g_iter_k, c->st));
                 step = c->iter_k;
             }
-            else CK(cudaGraphLaunch(c->g_iter, c->st));
+            else
+            {
+                if (!c->g_iter) { rc = build_iteration_graph(c); if (rc) return rc; }
+                CK(cudaGraphLaunch(c->g_iter, c->st));
+            }
         }
         else
         {
@@ -2025,6 +2131,8 @@ struct abm_batch {
     std::vector<abm_ctx*> ctxs;
     cudaStream_t st = nullptr;
     cudaGraphExec_t g_iter = nullptr, g_rebuild = nullptr;
+    cudaGraphExec_t g_loop = nullptr;    // the loop graphs of all contexts, or null
+    Ctrl** ctrls = nullptr;              // their control records (device array)
     int k_rebuild = 100;
     std::vector<cudaEvent_t> ev;
     cudaEvent_t done = nullptr;
@@ -2047,10 +2155,65 @@ int batch_fail(abm_batch* b, int code, const std::string& msg)
 void batch_free(abm_batch* b)
 {
     if (b->g_iter) cudaGraphExecDestroy(b->g_iter);
+    if (b->g_loop) cudaGraphExecDestroy(b->g_loop);
+    if (b->ctrls) cudaFree(b->ctrls);
     if (b->g_rebuild) cudaGraphExecDestroy(b->g_rebuild);
     for (cudaEvent_t e : b->ev) cudaEventDestroy(e);
     if (b->done) cudaEventDestroy(b->done);
     if (b->st) cudaStreamDestroy(b->st);
+}
+
+// one graph: every context's next iteration as an independent branch
+int batch_iteration_graph(abm_batch* b)
+{
+    cudaGraph_t G = nullptr;
+    BK(cudaGraphCreate(&G, 0));
+    int rc = ABM_OK;
+    for (abm_ctx* c : b->ctxs)
+    {
+        std::vector<cudaGraphNode_t> deps;
+        rc = append_iteration(c, G, deps);
+        if (rc) { rc = batch_fail(b, rc, "iteration graph of a context: " + c->err); break; }
+    }
+    cudaError_t inst = cudaSuccess;
+    if (!rc) inst = cudaGraphInstantiate(&b->g_iter, G, 0);
+    cudaGraphDestroy(G);
+    if (rc) return rc;
+    BK(inst);
+    return ABM_OK;
+}
+
+// one graph: every context's loop as an independent branch, each at its own pace up to the
+// joint rebuild
+int batch_loop_graph(abm_batch* b)
+{
+    std::vector<Ctrl*> ctrls;
+    for (abm_ctx* c : b->ctxs)
+    {
+        if (!has_loop(c)) return ABM_OK;
+        ctrls.push_back(c->ctrl);
+    }
+    BK(cudaMalloc(&b->ctrls, ctrls.size() * sizeof(Ctrl*)));
+    BK(cudaMemcpy(b->ctrls, ctrls.data(), ctrls.size() * sizeof(Ctrl*), cudaMemcpyHostToDevice));
+    cudaGraph_t G = nullptr;
+    BK(cudaGraphCreate(&G, 0));
+    int rc = ABM_OK;
+    for (abm_ctx* c : b->ctxs)
+    {
+        std::vector<cudaGraphNode_t> deps;
+        if (c->div_enabled)
+            rc = capture_into(c, G, deps, [&]() {
+                launch_div_count(c->phys, c->ctrl, c->dp, c->div_flags, 0, 0, c->st, FLOW_BEGIN);
+            });
+        if (!rc) rc = append_loop(c, G, deps);
+        if (rc) { rc = batch_fail(b, rc, "loop graph of a context: " + c->err); break; }
+    }
+    cudaError_t inst = cudaSuccess;
+    if (!rc) inst = cudaGraphInstantiate(&b->g_loop, G, 0);
+    cudaGraphDestroy(G);
+    if (rc) return rc;
+    BK(inst);
+    return ABM_OK;
 }
 }   // namespace
 
@@ -2084,7 +2247,7 @@ int abm_batch_create(abm_ctx* const* ctxs, int n, abm_batch** out)
         if (!c->nbrs_valid) { enqueue_rebuild(c); c->nbrs_valid = true; }
     }
     int rc = ABM_OK;
-    cudaGraph_t G = nullptr, GR = nullptr;
+    cudaGraph_t GR = nullptr;
     do {
         if (cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming) != cudaSuccess)
@@ -2094,33 +2257,29 @@ int abm_batch_create(abm_ctx* const* ctxs, int n, abm_batch** out)
             if (cudaEventCreateWithFlags(&b->ev[k], cudaEventDisableTiming) != cudaSuccess)
                 rc = batch_fail(b, ABM_ERR_CUDA, "event creation failed");
         if (rc) break;
-        // one graph: every context's iteration as an independent branch
-        if (cudaGraphCreate(&G, 0) != cudaSuccess || cudaGraphCreate(&GR, 0) != cudaSuccess)
+        if (cudaGraphCreate(&GR, 0) != cudaSuccess)
         { rc = batch_fail(b, ABM_ERR_CUDA, "graph creation failed"); break; }
         for (abm_ctx* c : b->ctxs)
         {
-            std::vector<cudaGraphNode_t> deps;
-            rc = append_iteration(c, G, deps);
-            if (rc) { rc = batch_fail(b, rc, "iteration graph of a context: " + c->err); break; }
             std::vector<cudaGraphNode_t> rdeps;
             rc = capture_into(c, GR, rdeps, [&]() { enqueue_rebuild(c); });
             if (rc) { rc = batch_fail(b, rc, "rebuild graph of a context: " + c->err); break; }
         }
         if (rc) break;
-        if (cudaGraphInstantiate(&b->g_iter, G, 0) != cudaSuccess ||
-            cudaGraphInstantiate(&b->g_rebuild, GR, 0) != cudaSuccess)
+        if (cudaGraphInstantiate(&b->g_rebuild, GR, 0) != cudaSuccess)
         { rc = batch_fail(b, ABM_ERR_CUDA, "graph instantiation failed"); break; }
+        rc = batch_loop_graph(b);
+        if (!rc && !b->g_loop) rc = batch_iteration_graph(b);
     } while (0);
-    if (G) cudaGraphDestroy(G);
     if (GR) cudaGraphDestroy(GR);
     if (rc) { batch_free(b); delete b; return rc; }
     *out = b;
     return ABM_OK;
 }
 
-// n_iters iterations of every context: one graph launch per iteration, the joint
-// neighbor rebuild every iter_update_neighbors iterations (all contexts take their
-// steps in lockstep, so their cadences coincide).  Work already queued on the
+// n_iters iterations of every context: one graph launch up to the next joint neighbor
+// rebuild, every iter_update_neighbors iterations (a few iterations left over: one launch
+// each).  Work already queued on the
 // contexts' streams runs first; their streams wait for the batch at the end.
 int abm_batch_iterate(abm_batch* b, int n_iters)
 {
@@ -2131,13 +2290,25 @@ int abm_batch_iterate(abm_batch* b, int n_iters)
         BK(cudaEventRecord(b->ev[k], b->ctxs[k]->st));
         BK(cudaStreamWaitEvent(b->st, b->ev[k], 0));
     }
-    for (int it = 0; it < n_iters; ++it)
+    for (int it = 0; it < n_iters;)
     {
-        BK(cudaGraphLaunch(b->g_iter, b->st));
+        int run = std::min(n_iters - it, b->k_rebuild - b->ctxs[0]->host_iter % b->k_rebuild);
+        if (b->g_loop && run >= LOOP_FAST / 2)
+        {
+            launch_loop_begin_all(b->ctrls, n, run, b->st);
+            BK(cudaGraphLaunch(b->g_loop, b->st));
+        }
+        else
+        {
+            run = 1;
+            if (!b->g_iter) { int rc = batch_iteration_graph(b); if (rc) return rc; }
+            BK(cudaGraphLaunch(b->g_iter, b->st));
+        }
+        it += run;
         bool rebuild = false;
         for (abm_ctx* c : b->ctxs)
         {
-            c->host_iter += 1;
+            c->host_iter += run;
             rebuild = (c->host_iter % b->k_rebuild == 0);
         }
         if (rebuild) BK(cudaGraphLaunch(b->g_rebuild, b->st));

@@ -32,11 +32,19 @@ static inline int cdiv_d(long long a, long long b) { return (int)((a + b - 1) / 
 const int DV_T = 128;
 const int DIV_TRIES = 10;
 
+// FLOW_BEGIN (before the first round of the loop graph): mothers or the cell limit make the
+// first iteration a slow one
 __global__ void k_div_count(const Phys* __restrict__ phys, Ctrl* ctrl, DivideParams dp, int* flags,
-                            unsigned long long cond, int use_cond)
+                            unsigned long long cond, int use_cond, int flow)
 {
     __shared__ int sh_cnt;
     __shared__ bool last;
+    if (flow == FLOW_SLOW && loop_idle(ctrl, flow, true))
+    {
+        if (use_cond && blockIdx.x == 0 && threadIdx.x == 0)
+            cudaGraphSetConditional((cudaGraphConditionalHandle)cond, 0u);
+        return;
+    }
     if (threadIdx.x == 0) sh_cnt = 0;
     __syncthreads();
     const int n = ctrl->n;
@@ -74,6 +82,11 @@ __global__ void k_div_count(const Phys* __restrict__ phys, Ctrl* ctrl, DividePar
         ctrl->div_done = (total == 0);
         ctrl->div_tries = 0;
         if (use_cond) cudaGraphSetConditional((cudaGraphConditionalHandle)cond, total > 0 ? 1u : 0u);
+        if (flow == FLOW_BEGIN)
+        {
+            ctrl->hold = (total > 0 || halt) ? HOLD_START : HOLD_NONE;
+            ctrl->n_divide = 0;            // counted again by the slow iteration
+        }
     }
 }
 
@@ -411,10 +424,10 @@ __global__ void k_div_commit(Geom* geom, Vel* vel, Phys* phys, Ctrl* ctrl, Divid
 }
 
 void launch_div_count(const Phys* phys, Ctrl* ctrl, const DivideParams& dp, int* flags,
-                      unsigned long long cond, int use_cond, cudaStream_t st)
+                      unsigned long long cond, int use_cond, cudaStream_t st, int flow)
 {
     int blocks = max(min(cdiv_d(dp.cap_cells, 256), 296), 1);
-    k_div_count<<<blocks, 256, 0, st>>>(phys, ctrl, dp, flags, cond, use_cond);
+    k_div_count<<<blocks, 256, 0, st>>>(phys, ctrl, dp, flags, cond, use_cond, flow);
 }
 
 void launch_div_body_pre(Ctrl* ctrl, const int* flags, const int* rank, int* mothers, int cap_cells,

@@ -994,10 +994,10 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
                                                       Ctrl* ctrl, ForceParams fp, const double* __restrict__ td,
                                                       const double* __restrict__ tr, double4* __restrict__ jbuf,
                                                       int* surv, ActiveList al, StepParams sp,
-                                                      const float* __restrict__ mlp_w)
+                                                      const float* __restrict__ mlp_w, int flow)
 {
     __shared__ bool last;
-    if (ctrl->halted) return;
+    if (ctrl->halted || loop_idle(ctrl, flow, true)) return;
     const bool split = PROPOSE && gridDim.x > 1;
     const bool proposer = split && blockIdx.x == gridDim.x - 1;
     const int work_blocks = split ? gridDim.x - 1 : gridDim.x;
@@ -1171,7 +1171,7 @@ void launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, const do
                           const double* jkr_radius, Gen6* fcc, double4* jbuf, int mixed, int max_entries,
                           int cap_cells, int num_sms, cudaStream_t st, int with_sum, int dims, int tile,
                           int blocks_per_sm, const int4* pairs, int* surv, ActiveList al, const StepParams* sp,
-                          const float* mlp_w)
+                          const float* mlp_w, int flow)
 {
     // sp (the loop's pass): the last block also runs the step-size proposal
     StepParams spv{};
@@ -1194,7 +1194,8 @@ void launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, const do
     const int per_sm = blocks_per_sm > 0 ? min(blocks_per_sm, occ) : occ;
     const int grid = max(1, min(cdiv(max_pairs, tile), num_sms * per_sm));
     void* args[] = {(void*)&geom, (void*)&pairs, (void*)&ctrl, (void*)&fp, (void*)&jkr_delta, (void*)&jkr_radius,
-                    (void*)&jbuf, (void*)&surv, (void*)&al, (void*)&spv, (void*)&mlp_w};
+                    (void*)&jbuf, (void*)&surv, (void*)&al, (void*)&spv, (void*)&mlp_w,
+                    (void*)&flow};
     cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(PS_T), args, 0, st);
     if (with_sum)
         k_pair_sum_rows<<<max(cdiv(cap_cells, 128), 1), 128, 0, st>>>(al.row_ptr, al.n_act, ctrl, jbuf, fcc, f32);
@@ -1341,6 +1342,38 @@ void launch_attempt_order(const Geom* geom, Ctrl* ctrl, const MechParams& P, int
     k_attempt_class<<<blocks, 256, 0, st>>>(geom, ctrl, P, flag);
     launch_scan(flag, &ctrl->n, pos, block_sums, cap_cells, st);
     k_attempt_order<<<blocks, 256, 0, st>>>(ctrl, flag, pos, order);
+}
+
+__device__ __forceinline__ void loop_begin(Ctrl* c, int todo)
+{
+    c->todo = todo;
+    c->hold = HOLD_NONE;
+    c->div_any = 0;
+    c->rounds = todo + 4;
+}
+__global__ void k_loop_begin(Ctrl* c, int todo) { loop_begin(c, todo); }
+__global__ void k_loop_begin_all(Ctrl* const* ctrls, int n, int todo)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) loop_begin(ctrls[k], todo);
+}
+__global__ void k_loop_round(Ctrl* c, unsigned long long cond_slow, unsigned long long cond_loop)
+{
+    const bool slow = c->hold != HOLD_NONE && c->todo > 0 && !c->halted;
+    const int left = c->todo - (slow ? 1 : 0);
+    c->rounds -= 1;
+    cudaGraphSetConditional((cudaGraphConditionalHandle)cond_slow, slow ? 1u : 0u);
+    cudaGraphSetConditional((cudaGraphConditionalHandle)cond_loop, left > 0 && !c->halted && c->rounds > 0 ? 1u : 0u);
+}
+
+void launch_loop_begin(Ctrl* ctrl, int todo, cudaStream_t st) { k_loop_begin<<<1, 1, 0, st>>>(ctrl, todo); }
+void launch_loop_begin_all(Ctrl* const* ctrls, int n, int todo, cudaStream_t st)
+{
+    k_loop_begin_all<<<cdiv(n, 128), 128, 0, st>>>(ctrls, n, todo);
+}
+void launch_loop_round(Ctrl* ctrl, unsigned long long cond_slow, unsigned long long cond_loop, cudaStream_t st)
+{
+    k_loop_round<<<1, 1, 0, st>>>(ctrl, cond_slow, cond_loop);
 }
 
 int attempt_blocks(int cap_cells) { return max(cdiv(cap_cells, AT_T), 1); }

@@ -13,6 +13,16 @@ const int MAX_STAGES = 7;
 // attempt copies its candidate state instead of re-running the step.
 enum CtrlMode { MODE_TRIAL = 0, MODE_RETRY = 1, MODE_FINAL = 2, MODE_COMMIT = 3 };
 
+// How a kernel of an iteration is launched.  FLOW_STEP: as one iteration of its own.  The loop
+// graph advances many: rounds of FLOW_FAST iterations, in which the kernels follow one another
+// without a conditional node and leave at once when there is nothing to do (no iteration
+// left) or the iteration needs more than them (Ctrl::hold), and after each round, only
+// then, one FLOW_SLOW iteration with everything.
+enum LoopFlow { FLOW_STEP = 0, FLOW_FAST = 1, FLOW_SLOW = 2, FLOW_BEGIN = 3 };
+// Why the fast iterations wait: the next iteration starts with divisions or the cell limit,
+// or the running one's first attempt failed its error test.
+enum LoopHold { HOLD_NONE = 0, HOLD_START = 1, HOLD_RETRY = 2 };
+
 // Step-size network: 32 features -> 64 -> 64 -> 1 (log dt ratio)
 const int MLP_IN = 32, MLP_H = 64;
 const int MLP_OFF_W1 = 0, MLP_OFF_B1 = MLP_OFF_W1 + MLP_H * MLP_IN, MLP_OFF_W2 = MLP_OFF_B1 + MLP_H;
@@ -111,7 +121,21 @@ struct Ctrl {
     // the list is stale by `drift`: the rule keeps mixed-precision trajectories bit for bit.
     double path;
     unsigned long long path_bits;
+    // the loop graph (LoopFlow): iterations still to take, and why the plain ones wait
+    int todo;
+    int hold;                           // LoopHold
+    int div_any;                        // a cell grew past Ldiv in the running attempt's step
+    int rounds;                         // rounds of the loop graph left (a bound)
 };
+
+// Nothing to do for a kernel of the loop graph?  `first`: it belongs to the part of the
+// iteration before a failed first attempt (already done when a slow iteration resumes one).
+__device__ __forceinline__ bool loop_idle(const Ctrl* c, int flow, bool first)
+{
+    if (flow == FLOW_STEP) return false;
+    if (c->todo <= 0) return true;
+    return flow == FLOW_FAST ? c->hold != HOLD_NONE : (first && c->hold == HOLD_RETRY);
+}
 
 struct Grid {
     double x0, y0, z0, edge, inv_edge;
@@ -140,6 +164,8 @@ struct StepParams {
     int mixed;                  // 1: mixed precision (3-D): cells in surface contact take the FP32
                                 // contact branch of the velocity solve
     int fric;                   // 1: cell-cell kinetic friction (3-D, FP64)
+    int div_on;                 // 1: cells may divide
+    double Ldiv;
     int stats_on;               // accumulate the network's features (learned or logging)
     double near_div_length;     // 0.9 Ldiv
     double4* stat_part;         // per-block (max |v_r|, sum |v_r|^2, sum growth, near-division count)
@@ -272,7 +298,7 @@ void launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, const do
                           const double* jkr_radius, Gen6* fcc, double4* jbuf, int mixed, int max_entries,
                           int cap_cells, int num_sms, cudaStream_t st, int with_sum, int dims, int tile,
                           int blocks_per_sm, const int4* pairs, int* surv, ActiveList al,
-                          const StepParams* sp = nullptr, const float* mlp_w = nullptr);
+                          const StepParams* sp = nullptr, const float* mlp_w = nullptr, int flow = FLOW_STEP);
 // the list of unordered pairs (i, j < i, lower entry k, partner entry rev[k]) after
 // k_csr_rev, cells in `order` (null: index order): counts -> scan -> fill; uses
 // `count` and `start` (cap_cells + 1) as scratch
@@ -304,6 +330,7 @@ struct AttemptArgs {
     unsigned long long cond;
     int use_cond;
     unsigned long long cond_run;
+    int flow;                   // LoopFlow
 };
 void launch_attempt(int kind, const AttemptArgs& a, int dims, cudaStream_t st);
 // one translation unit per stage count (abm_attempt.cuh)
@@ -361,7 +388,12 @@ struct DivideParams {
     double* feta;               // friction coefficient of each cell (daughters inherit it), or null
 };
 void launch_div_count(const Phys* phys, Ctrl* ctrl, const DivideParams& dp, int* flags,
-                      unsigned long long cond, int use_cond, cudaStream_t st);
+                      unsigned long long cond, int use_cond, cudaStream_t st, int flow = FLOW_STEP);
+// the loop graph: `todo` iterations ahead (of each of n contexts); then, once per round,
+// whether a slow iteration runs and whether another round follows
+void launch_loop_begin(Ctrl* ctrl, int todo, cudaStream_t st);
+void launch_loop_begin_all(Ctrl* const* ctrls, int n, int todo, cudaStream_t st);
+void launch_loop_round(Ctrl* ctrl, unsigned long long cond_slow, unsigned long long cond_loop, cudaStream_t st);
 void launch_div_body_pre(Ctrl* ctrl, const int* flags, const int* rank, int* mothers, int cap_cells,
                          cudaStream_t st);
 // room checks and the first try; use_cond: `cond` is set while a further try is needed

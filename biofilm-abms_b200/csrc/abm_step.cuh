@@ -186,7 +186,9 @@ __device__ __forceinline__ Gen6 sum_active_shares(const SHARE* row, int n)
 // Step-size controller, run once per attempt by the last block
 // (simulation.hpp:1690-1769; the final re-run is accepted unconditionally).
 // commit: the final step copies an accepted proposal (no RK evaluation of its own)
-static __device__ void controller_finish(Ctrl* c, const StepParams& sp, int kind, double E, bool commit = false)
+// longer: the step left a cell longer than Ldiv
+static __device__ void controller_finish(Ctrl* c, const StepParams& sp, int kind, double E, bool longer,
+                                         bool commit = false)
 {
     if (!commit) c->attempts += 1;
     if (kind == MODE_TRIAL)
@@ -252,6 +254,8 @@ static __device__ void controller_finish(Ctrl* c, const StepParams& sp, int kind
         c->hist_pos = (h + 1) % HIST;
         c->since_div = c->n_divide > 0 ? 0 : c->since_div + 1;
         c->cell_steps += c->n;
+        c->todo -= 1;
+        c->hold = (sp.div_on && (longer || (c->halt_n > 0 && c->n >= c->halt_n))) ? HOLD_START : HOLD_NONE;
         c->t += c->dt;
         c->iter += 1;
         c->iterations += 1;
