@@ -44,17 +44,11 @@ __global__ void __launch_bounds__(AT_T, (S <= 4 ? (V == 3 ? 3 : 6) : 1)) k_attem
             cudaGraphSetConditional((cudaGraphConditionalHandle)cond_run, 0u);
         return;
     }
-    if (KIND != 3 && !DRY && loop_idle(ctrl, flow, KIND == MODE_TRIAL))
+    if (KIND != 3 && !DRY && loop_idle(ctrl, flow))
     {
-        // a slow iteration that resumes after a failed first attempt goes on with the retries
-        if (flow == FLOW_SLOW && KIND == MODE_TRIAL && blockIdx.x == 0 && threadIdx.x == 0)
-        {
-            if (use_cond & 1)
-                cudaGraphSetConditional((cudaGraphConditionalHandle)cond,
-                                        (ctrl->todo > 0 && ctrl->mode == MODE_RETRY && ctrl->tries < sp.max_tries) ? 1u : 0u);
-            if (use_cond & 2)
-                cudaGraphSetConditional((cudaGraphConditionalHandle)cond_run, ctrl->todo > 0 ? 1u : 0u);
-        }
+        // nothing to resume: stop an enclosing WHILE node
+        if ((use_cond & 1) && blockIdx.x == 0 && threadIdx.x == 0)
+            cudaGraphSetConditional((cudaGraphConditionalHandle)cond, 0u);
         return;
     }
     const int n = ctrl->n;
@@ -493,9 +487,9 @@ __global__ void k_fr_check(Ctrl* ctrl, const int4* __restrict__ act, const int* 
 }
 
 template <int S>
-__global__ void k_fr_arm(Ctrl* ctrl, int flow, bool first)
+__global__ void k_fr_arm(Ctrl* ctrl, int flow)
 {
-    ctrl->fr_pending = ctrl->fr_ncand > 0 && !ctrl->halted && !loop_idle(ctrl, flow, first);
+    ctrl->fr_pending = ctrl->fr_ncand > 0 && !ctrl->halted && !loop_idle(ctrl, flow);
 }
 
 template <int KIND, bool NOISE, int DIM, int V>
@@ -546,7 +540,7 @@ void ABM_CAT(launch_attempt_, ABM_STAGES)(int kind, const AttemptArgs& a, int di
 void ABM_CAT(launch_friction_rounds_, ABM_STAGES)(int kind, const AttemptArgs& a, const int4* act, const int* fr_list,
                                                   int* fmask, double R, cudaStream_t st)
 {
-    k_fr_arm<ABM_STAGES><<<1, 1, 0, st>>>(a.ctrl, a.flow, kind == MODE_TRIAL);
+    k_fr_arm<ABM_STAGES><<<1, 1, 0, st>>>(a.ctrl, a.flow);
     for (int r = 1; r < ABM_STAGES; ++r)
     {
         launch_noise<3, 3>(kind, a, st);

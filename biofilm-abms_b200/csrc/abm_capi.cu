@@ -33,14 +33,19 @@ struct abm_ctx {
     // device state
     Geom* geom = nullptr; Vel* vel = nullptr; Phys* phys = nullptr; Gen6* fcc = nullptr;
     Geom* geom_c = nullptr; Vel* vel_c = nullptr; Gen6* gen_tmp = nullptr; Gen6* k0buf = nullptr;
-    Ctrl* ctrl = nullptr; Grid* grid = nullptr;
-    unsigned long long* bbox_acc = nullptr; unsigned int* bbox_counter = nullptr;
-    int *bin_count = nullptr, *bin_start = nullptr, *key = nullptr, *slot = nullptr, *sorted_cell = nullptr;
-    Geom* sorted_geom = nullptr;
+    Ctrl* ctrl = nullptr;
+    int* bbox = nullptr;
+    int2* part = nullptr;
+    int n_seen = 0;                  // cells when the host last looked
+    int n_ref = 0;                   // cells that the launches are shaped for
+    LaunchShape build;               // of the build launch
+    int *bin_count = nullptr, *bin_start = nullptr, *key = nullptr, *slot = nullptr, *sorted_cell = nullptr,
+        *sorted_key = nullptr;
+    float4 *sorted_pos = nullptr, *sorted_dir = nullptr;
     int *scratch = nullptr, *nbr_count = nullptr, *row_ptr = nullptr, *col = nullptr;
-    int *lower_end = nullptr, *rev = nullptr;
+    int* lower_end = nullptr;
     int4* pairs = nullptr;                                           // screened pair pass
-    int *pair_start = nullptr, *surv = nullptr;
+    int* surv = nullptr;
     int4* act = nullptr;                                             // active pairs (ActiveList)
     int* n_act = nullptr;
     unsigned char* keep_entry = nullptr;
@@ -56,7 +61,7 @@ struct abm_ctx {
     DivideParams dp;
     bool div_enabled = false;
     int cap_parents = 0;
-    int *div_flags = nullptr, *div_rank = nullptr, *mothers = nullptr, *div_check = nullptr, *div_sat = nullptr;
+    int *div_flags = nullptr, *mothers = nullptr, *div_check = nullptr, *div_sat = nullptr;
     int *div_ok = nullptr, *parents_dev = nullptr;
     Geom *d1 = nullptr, *d2 = nullptr;
     double *dlen = nullptr, *dgrowth = nullptr;
@@ -64,7 +69,7 @@ struct abm_ctx {
     float* mlp_w = nullptr;          // ABM_MLP_NPARAM FP32 master weights
     float* log_buf = nullptr;        // stepsize_log_capacity rows of MLP_LOG_COLS floats
     double4* stat_part = nullptr;    // per-block feature partials of the final attempt
-    int *order = nullptr, *order_flag = nullptr, *order_pos = nullptr;   // attempt order (3-D)
+    int* order = nullptr;            // attempt order (3-D)
     // frames: a ring of frame_slots snapshots of the cells (abm_set_frames)
     int frame_slots = 0;
     Geom* snap_geom = nullptr;
@@ -96,7 +101,7 @@ struct abm_ctx {
     // parameters
     ForceParams fp; StepParams sp; BuildParams bp;
     // graphs
-    cudaGraphExec_t g_iter = nullptr, g_rebuild = nullptr;
+    cudaGraphExec_t g_iter = nullptr;
     cudaGraphExec_t g_loop = nullptr;     // many Runge-Kutta iterations (append_loop)
     cudaGraphExec_t g_iter_k = nullptr;   // iter_k iterations in one graph (Verlet, post-step kernels)
     int iter_k = 1;
@@ -203,15 +208,12 @@ static void free_all(abm_ctx* c)
     if (c->g_iter) cudaGraphExecDestroy(c->g_iter);
     if (c->g_iter_k) cudaGraphExecDestroy(c->g_iter_k);
     if (c->g_loop) cudaGraphExecDestroy(c->g_loop);
-    if (c->g_rebuild) cudaGraphExecDestroy(c->g_rebuild);
-    void* ptrs[] = {c->geom, c->vel, c->phys, c->fcc, c->geom_c, c->vel_c, c->gen_tmp, c->k0buf, c->ctrl, c->grid,
-                    c->bbox_acc, c->bbox_counter, c->bin_count, c->bin_start, c->key, c->slot,
-                    c->sorted_cell, c->sorted_geom, c->scratch, c->nbr_count, c->row_ptr, c->col, c->lower_end, c->rev, c->pairs, c->pair_start, c->surv,
+    void* ptrs[] = {c->geom, c->vel, c->phys, c->fcc, c->geom_c, c->vel_c, c->gen_tmp, c->k0buf, c->ctrl, c->bbox, c->part, c->sorted_pos, c->sorted_dir, c->sorted_key,  c->bin_count, c->bin_start, c->key, c->slot,
+                    c->sorted_cell,  c->scratch, c->nbr_count, c->row_ptr, c->col, c->lower_end,  c->pairs,  c->surv,
                     c->act, c->n_act, c->keep_entry, c->gref, c->bar,c->jbuf,
-                    c->scan_sums, c->jkr_delta, c->jkr_radius, c->jkr_gam, c->jkr_rad2, c->staging, c->div_flags, c->div_rank,
+                    c->scan_sums, c->jkr_delta, c->jkr_radius, c->jkr_gam, c->jkr_rad2, c->staging, c->div_flags, 
                     c->mothers, c->div_check, c->div_sat, c->div_ok, c->parents_dev, c->d1, c->d2, c->dlen,
-                    c->dgrowth, c->mlp_w, c->log_buf, c->adhere, c->stat_part, c->order, c->order_flag,
-                    c->order_pos, c->snap_geom, c->snap_vel, c->snap_phys, c->frame_info, c->phys_c, c->keep,
+                    c->dgrowth, c->mlp_w, c->log_buf, c->adhere, c->stat_part, c->order,  c->snap_geom, c->snap_vel, c->snap_phys, c->frame_info, c->phys_c, c->keep,
                     c->keep_rank, c->feta, c->fbuf, c->fmask, c->fr_list, c->ystage, c->snap_feta, c->pbuf,
                     c->whalf};
     for (void* q : ptrs) if (q) cudaFree(q);
@@ -282,7 +284,6 @@ __global__ void k_set_clock(Ctrl* c, double t, double dt, int iter)
     c->t = t; c->dt = dt; c->iter = iter; c->mode = MODE_TRIAL; c->tries = 0; c->attempt = 0;
     c->err_bits = 0; c->blocks_done = 0;
 }
-__global__ void k_count_rebuild(Ctrl* c) { c->rebuilds += 1; }
 
 int abm_create(const abm_params* q, abm_ctx** out)
 {
@@ -336,21 +337,23 @@ int abm_create(const abm_params* q, abm_ctx** out)
     CK(cudaMalloc(&c->gen_tmp, cap * sizeof(Gen6)));
     CK(cudaMalloc(&c->k0buf, cap * sizeof(Gen6)));
     CK(cudaMalloc(&c->ctrl, sizeof(Ctrl)));
-    CK(cudaMalloc(&c->grid, sizeof(Grid)));
-    CK(cudaMalloc(&c->bbox_acc, 8 * sizeof(unsigned long long)));
-    CK(cudaMalloc(&c->bbox_counter, sizeof(unsigned int)));
+    const size_t max_blocks = std::max(build_shape(c->cap, c->num_sms).blocks, 16);
+    CK(cudaMalloc(&c->bbox, max_blocks * 8 * sizeof(int)));
+    CK(cudaMalloc(&c->part, max_blocks * sizeof(int2)));
     CK(cudaMalloc(&c->bin_count, (size_t)c->cap_bins * sizeof(int)));
-    CK(cudaMalloc(&c->bin_start, ((size_t)c->cap_bins + 1) * sizeof(int)));
+    CK(cudaMemset(c->bin_count, 0, (size_t)c->cap_bins * sizeof(int)));   // each build leaves it zero
+    CK(cudaMalloc(&c->bin_start, 2 * (size_t)c->cap_bins * sizeof(int)));   // one more per row of bins
     CK(cudaMalloc(&c->key, cap * sizeof(int)));
     CK(cudaMalloc(&c->slot, cap * sizeof(int)));
     CK(cudaMalloc(&c->sorted_cell, cap * sizeof(int)));
-    CK(cudaMalloc(&c->sorted_geom, cap * sizeof(Geom)));
+    CK(cudaMalloc(&c->sorted_key, cap * sizeof(int)));
+    CK(cudaMalloc(&c->sorted_pos, cap * sizeof(float4)));
+    CK(cudaMalloc(&c->sorted_dir, cap * sizeof(float4)));
     CK(cudaMalloc(&c->scratch, cap * c->cap_nbr * sizeof(int)));
     CK(cudaMalloc(&c->nbr_count, cap * sizeof(int)));
     CK(cudaMalloc(&c->row_ptr, (cap + 1) * sizeof(int)));
     CK(cudaMalloc(&c->col, cap * c->cap_nbr * sizeof(int)));
     CK(cudaMalloc(&c->lower_end, cap * sizeof(int)));
-    CK(cudaMalloc(&c->rev, cap * c->cap_nbr * sizeof(int)));
     CK(cudaMalloc(&c->pairs, cap * c->cap_nbr / 2 * sizeof(int4) + sizeof(int4)));
     CK(cudaMalloc(&c->surv, cap * c->cap_nbr / 2 * sizeof(int) + sizeof(int)));
     CK(cudaMalloc(&c->act, cap * c->cap_nbr / 2 * sizeof(int4) + sizeof(int4)));
@@ -359,14 +362,12 @@ int abm_create(const abm_params* q, abm_ctx** out)
     CK(cudaMalloc(&c->gref, cap * sizeof(Geom)));
     CK(cudaMalloc(&c->bar, sizeof(GridBar)));
     CK(cudaMemset(c->bar, 0, sizeof(GridBar)));
-    CK(cudaMalloc(&c->pair_start, (cap + 1) * sizeof(int)));
     CK(cudaMalloc(&c->jbuf, cap * c->cap_nbr * sizeof(double4)));
     CK(cudaMemset(c->lower_end, 0, cap * sizeof(int)));
     size_t ns = std::max(scan_block_sums_size((int)cap + 1), scan_block_sums_size(c->cap_bins + 1)) + 1;
     CK(cudaMalloc(&c->scan_sums, ns * sizeof(int)));
     CK(cudaMalloc(&c->staging, cap * STAGING_COLS * sizeof(double)));
     CK(cudaMalloc(&c->div_flags, cap * sizeof(int)));
-    CK(cudaMalloc(&c->div_rank, (cap + 1) * sizeof(int)));
     CK(cudaMalloc(&c->mothers, cap * sizeof(int)));
     CK(cudaMalloc(&c->div_check, cap * sizeof(int)));
     CK(cudaMalloc(&c->div_sat, cap * sizeof(int)));
@@ -383,9 +384,6 @@ int abm_create(const abm_params* q, abm_ctx** out)
     h.dt = p.max_stepsize;
     h.mode = MODE_TRIAL;
     CK(cudaMemcpy(c->ctrl, &h, sizeof(Ctrl), cudaMemcpyHostToDevice));
-    unsigned long long acc0[8] = {~0ull, ~0ull, ~0ull, 0ull, 0ull, 0ull, 0ull, 0ull};
-    CK(cudaMemcpy(c->bbox_acc, acc0, sizeof(acc0), cudaMemcpyHostToDevice));
-    CK(cudaMemset(c->bbox_counter, 0, sizeof(unsigned int)));
     // parameters of the kernels
     MechParams mp;
     mp.R = p.R; mp.Rcell = p.Rcell; mp.E0 = p.E0; mp.Ecell = p.Ecell; mp.sqrtR = std::sqrt(p.R);
@@ -514,8 +512,6 @@ int abm_create(const abm_params* q, abm_ctx** out)
     if (c->dims == 3)
     {
         CK(cudaMalloc(&c->order, (size_t)c->cap * sizeof(int)));
-        CK(cudaMalloc(&c->order_flag, ((size_t)c->cap + 1) * sizeof(int)));
-        CK(cudaMalloc(&c->order_pos, ((size_t)c->cap + 1) * sizeof(int)));
     }
     sp.order = c->order;
     return ABM_OK;
@@ -720,6 +716,20 @@ int abm_basal_dropped(abm_ctx* c, long long* dropped)
     return ABM_OK;
 }
 
+// The build launch and the pair pass are shaped for twice the cells that the host last knew
+// of (any number runs; a colony that has outgrown its shape only takes longer).  Called when
+// the host learns the number; a new shape drops the graphs, which hold the old one.
+static void shape_launches(abm_ctx* c)
+{
+    const int n = c->n_seen;
+    if (c->n_ref > 0 && n <= c->n_ref && 8LL * n >= c->n_ref) return;
+    const int ref = std::min(c->cap, std::max(2 * n, 256));
+    if (ref == c->n_ref) return;
+    c->n_ref = ref;
+    c->build = build_shape(ref, c->num_sms);
+    drop_iteration_graphs(c);
+}
+
 int abm_upload_cells(abm_ctx* c, const double* cm, int n, int ncols, int ld)
 {
     if (!c || !cm || n < 0 || ld < n) return fail(c, ABM_ERR_ARG, "bad cell array");
@@ -747,8 +757,9 @@ int abm_upload_cells(abm_ctx* c, const double* cm, int n, int ncols, int ld)
     k_set_n<<<1, 1, 0, c->st>>>(c->ctrl, n);
     CK(cudaGetLastError());
     if (c->n_host != n) c->nbrs_valid = false;
-    c->n_host = n;
+    c->n_host = c->n_seen = n;
     c->cells_loaded = true;
+    shape_launches(c);
     // division is possible when a cell already exceeds Ldiv or any cell can grow
     bool grows = (c->p.growth_mean != 0 || c->p.growth_std != 0) || switch_grows(c);
     const int col_growth = two_d ? 12 : 16, col_l = two_d ? 9 : 13;
@@ -776,7 +787,7 @@ int abm_download_cells(abm_ctx* c, double* cm, int ld)
     CK(cudaMemcpyAsync(&h, c->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     int n = h.n;
-    c->n_host = n;
+    c->n_host = c->n_seen = n;
     if (ld < n) return fail(c, ABM_ERR_ARG, "ld smaller than the cell count");
     if (n > 0)
     {
@@ -886,6 +897,7 @@ int abm_get_num_cells(abm_ctx* c, int* n)
     CK(cudaMemcpyAsync(&h, c->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     *n = h.n;
+    c->n_seen = h.n;
     return ABM_OK;
 }
 
@@ -925,7 +937,6 @@ int abm_set_parents(abm_ctx* c, const int* parents, int n)
         CK(cudaMalloc(&c->parents_dev, (size_t)c->cap_parents * sizeof(int)));
         // captured graphs hold the old buffer
         drop_iteration_graphs(c);
-        if (c->g_rebuild) { cudaGraphExecDestroy(c->g_rebuild); c->g_rebuild = nullptr; }
     }
     if (n > 0) CK(cudaMemcpyAsync(c->parents_dev, parents, (size_t)n * sizeof(int), cudaMemcpyHostToDevice, c->st));
     k_set_n_parents<<<1, 1, 0, c->st>>>(c->ctrl, n);
@@ -945,30 +956,31 @@ int abm_get_parents(abm_ctx* c, int* out, int cap, int* n)
     return ABM_OK;
 }
 
-// neighbor rebuild sequence (getCellNeighbors, mechanics.hpp:520-593)
-static void enqueue_rebuild(abm_ctx* c)
+// the neighbor set and the division (abm_build.cu)
+static void enqueue_build(abm_ctx* c, int what, int flow = FLOW_STEP)
 {
-    cudaStream_t st = c->st;
-    launch_bbox(c->geom, c->ctrl, c->grid, c->bbox_acc, c->bbox_counter, c->bp.prefilter, c->cap_bins, c->cap, st);
-    cudaMemsetAsync(c->bin_count, 0, (size_t)c->cap_bins * sizeof(int), st);
-    launch_bin_count(c->geom, c->ctrl, c->grid, c->bin_count, c->key, c->slot, c->cap, st);
-    launch_scan(c->bin_count, &c->grid->nbins, c->bin_start, c->scan_sums, c->cap_bins, st);
-    launch_bin_scatter(c->geom, c->ctrl, c->bin_start, c->key, c->slot, c->sorted_cell, c->sorted_geom, c->cap, st);
-    launch_pair_build(c->grid, c->bin_start, c->sorted_cell, c->sorted_geom, c->ctrl, c->bp, c->scratch,
-                      c->nbr_count, c->cap_bins, c->num_sms, st);
-    launch_scan(c->nbr_count, &c->ctrl->n, c->row_ptr, c->scan_sums, c->cap, st);
-    launch_csr_fill(c->ctrl, c->row_ptr, c->scratch, c->cap_nbr, c->col, c->ctrl, c->cap, st);
-    launch_csr_rev(c->ctrl, c->row_ptr, c->col, c->lower_end, c->rev, c->cap, st);
-    // pairs in the bin order of the sort just made (sorted_cell)
-    launch_pair_list(c->ctrl, c->row_ptr, c->lower_end, c->col, c->rev, c->nbr_count, c->pair_start, c->scan_sums,
-                     c->pairs, c->cap, st, c->sorted_cell);
-    if (c->dims == 2 && c->p.adhesion_mode != 0)
-        launch_adhere_flags(c->ctrl, c->row_ptr, c->col, c->geom, c->p.R, c->p.Rcell, c->adhere, c->cap, st);
-    if (c->order)
-        launch_attempt_order(c->geom, c->ctrl, c->sp.mp, c->order_flag, c->order_pos, c->scan_sums, c->order,
-                             c->cap, st);
-    k_count_rebuild<<<1, 1, 0, st>>>(c->ctrl);
+    BuildArgs a{};
+    a.geom = c->geom; a.vel = c->vel; a.phys = c->phys; a.ctrl = c->ctrl; a.bar = c->bar;
+    a.bbox = c->bbox; a.part = c->part; a.bin_count = c->bin_count; a.bin_start = c->bin_start;
+    a.key = c->key; a.slot = c->slot; a.sorted_cell = c->sorted_cell; a.sorted_key = c->sorted_key; a.sorted_pos = c->sorted_pos;
+    a.sorted_dir = c->sorted_dir;
+    a.cap_bins = c->cap_bins; a.cap_cells = c->cap;
+    a.bp = c->bp; a.mp = c->sp.mp;
+    a.scratch = c->scratch; a.count = c->nbr_count; a.row_ptr = c->row_ptr; a.col = c->col;
+    a.lower_end = c->lower_end; a.pairs = c->pairs; a.order = c->order;
+    a.adhere = c->dims == 2 && c->p.adhesion_mode != 0 ? c->adhere : nullptr;
+    a.dp = c->dp;
+    a.flags = c->div_flags; a.mothers = c->mothers; a.check = c->div_check; a.sat = c->div_sat; a.ok = c->div_ok;
+    a.d1 = c->d1; a.d2 = c->d2; a.dlen = c->dlen; a.dgrowth = c->dgrowth; a.parents = c->parents_dev;
+    launch_build(a, what, c->build, c->st, flow);
 }
+
+// getCellNeighbors (mechanics.hpp:520-593)
+static void enqueue_rebuild(abm_ctx* c) { enqueue_build(c, BUILD_NEIGHBORS); }
+
+// division and the neighbor rebuild the reference does after any division
+// (simulation.hpp:1654-1660)
+static void enqueue_growth(abm_ctx* c, int flow = FLOW_STEP) { enqueue_build(c, BUILD_GROWTH, flow); }
 
 // one iteration of the loop body without division: stage-invariant pair
 // forces, then the trial attempt, up to max_tries retries and the accepted
@@ -979,10 +991,10 @@ static void enqueue_rebuild(abm_ctx* c)
 // step-size features (and, learned, the proposed dt)
 static void enqueue_pair_force(abm_ctx* c, int with_gather, bool in_loop = false, int flow = FLOW_STEP)
 {
-    ActiveList al = {c->act, c->n_act, c->keep_entry, c->gref, c->row_ptr, c->bar};
+    ActiveList al = {c->act, c->n_act, c->keep_entry, c->gref, c->row_ptr, c->bar, 0};
     launch_pair_screened(c->geom, c->ctrl, c->fp, c->jkr_delta, c->jkr_radius, c->fcc, c->jbuf,
                          c->p.precision == ABM_PRECISION_MIXED, c->cap * c->cap_nbr, c->cap, c->num_sms, c->st,
-                         with_gather, c->dims, c->p.pair_tile, c->p.pair_blocks_per_sm, c->pairs, c->surv, al,
+                         with_gather, c->dims, c->p.pair_tile, c->p.pair_blocks_per_sm, c->pairs, c->surv, al, c->n_ref,
                          in_loop ? &c->sp : nullptr, c->mlp_w, flow);
 }
 
@@ -1068,47 +1080,6 @@ static int capture(abm_ctx* c, void (*fn)(abm_ctx*), cudaGraphExec_t* exec)
     return ABM_OK;
 }
 
-// division body (after the flag count): ranks, room checks on a fresh cell list,
-// up to ten tries, commit, then the neighbor rebuild the reference does after any
-// division (simulation.hpp:1654-1660)
-// the body up to the first try; use_cond: `cond` is set when further tries are needed
-static void enqueue_division_setup(abm_ctx* c, unsigned long long cond, int use_cond)
-{
-    cudaStream_t st = c->st;
-    launch_scan(c->div_flags, &c->ctrl->n, c->div_rank, c->scan_sums, c->cap, st);
-    launch_div_body_pre(c->ctrl, c->div_flags, c->div_rank, c->mothers, c->cap, st);
-    launch_bbox(c->geom, c->ctrl, c->grid, c->bbox_acc, c->bbox_counter, c->bp.prefilter, c->cap_bins, c->cap, st);
-    cudaMemsetAsync(c->bin_count, 0, (size_t)c->cap_bins * sizeof(int), st);
-    launch_bin_count(c->geom, c->ctrl, c->grid, c->bin_count, c->key, c->slot, c->cap, st);
-    launch_scan(c->bin_count, &c->grid->nbins, c->bin_start, c->scan_sums, c->cap_bins, st);
-    launch_bin_scatter(c->geom, c->ctrl, c->bin_start, c->key, c->slot, c->sorted_cell, c->sorted_geom, c->cap, st);
-    launch_div_first(c->geom, c->phys, c->ctrl, c->dp, c->grid, c->bin_start, c->sorted_cell, c->sorted_geom,
-                     c->div_flags, c->mothers, c->div_check, c->div_sat, c->d1, c->d2, c->dlen, c->dgrowth,
-                     c->div_ok, cond, use_cond, st);
-}
-
-static void enqueue_division_try(abm_ctx* c, int tr, unsigned long long cond, int use_cond)
-{
-    launch_div_try_round(c->geom, c->phys, c->ctrl, c->dp, c->grid, c->bin_start, c->sorted_cell, c->sorted_geom,
-                         c->div_flags, c->mothers, c->div_check, c->div_sat, c->d1, c->d2, c->dlen, c->dgrowth,
-                         c->div_ok, tr, cond, use_cond, c->st);
-}
-
-static void enqueue_division_commit(abm_ctx* c)
-{
-    launch_div_commit(c->geom, c->vel, c->phys, c->ctrl, c->dp, c->mothers, c->d1, c->d2, c->dlen, c->dgrowth,
-                      c->parents_dev, c->st);
-}
-
-// the whole body with the ten tries launched in a row (each exits at once once the
-// criterion holds for every dividing cell): the paths without conditional nodes
-static void enqueue_division_body(abm_ctx* c)
-{
-    enqueue_division_setup(c, 0, 0);
-    for (int tr = 1; tr < max_division_tries(); ++tr) enqueue_division_try(c, tr, 0, 0);
-    enqueue_division_commit(c);
-}
-
 // Capture fn into `graph` after `deps`; `deps` becomes the leaf set of the capture.
 static int capture_into(abm_ctx* c, cudaGraph_t graph, std::vector<cudaGraphNode_t>& deps,
                         const std::function<void()>& fn)
@@ -1143,25 +1114,6 @@ static int add_conditional(abm_ctx* c, cudaGraph_t graph, std::vector<cudaGraphN
     *body = np->conditional.phGraph_out[0];
     deps.assign(1, node);
     return ABM_OK;
-}
-
-// the body in a graph: the first try, then a WHILE node that runs further ones until the
-// distance criterion holds for every dividing cell or ten have run (growth.hpp:252), then
-// the commit and the neighbor rebuild
-static int capture_division_body(abm_ctx* c, cudaGraph_t body)
-{
-    std::vector<cudaGraphNode_t> bd;
-    cudaGraphConditionalHandle h_try = 0;
-    CK(cudaGraphConditionalHandleCreate(&h_try, body, 0, cudaGraphCondAssignDefault));
-    int rc = capture_into(c, body, bd, [&]() { enqueue_division_setup(c, h_try, 1); });
-    if (rc) return rc;
-    cudaGraph_t tries;
-    rc = add_conditional(c, body, bd, h_try, cudaGraphCondTypeWhile, &tries);
-    if (rc) return rc;
-    std::vector<cudaGraphNode_t> tb;
-    rc = capture_into(c, tries, tb, [&]() { enqueue_division_try(c, -1, h_try, 1); });
-    if (rc) return rc;
-    return capture_into(c, body, bd, [&]() { enqueue_division_commit(c); enqueue_rebuild(c); });
 }
 
 // After the accepted step (simulation.hpp:1831-2022): basal-only compaction and its
@@ -1242,30 +1194,25 @@ static int append_post_step(abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode
 
 // One loop iteration as a graph with conditional nodes, appended to G after `deps`
 // (empty: root nodes); `deps` becomes the iteration's leaf set:
-//   [division count] -> IF(n_divide > 0){division + rebuild}
-//   -> pair force -> [proposal] -> trial -> WHILE(retry requested){retry} -> final
-// With the learned controller a passing proposal closes the step in the trial, and
+//   [division and rebuild] -> pair force -> trial -> WHILE(retry requested){retry} -> final
+// With the learned and PI controllers a passing proposal closes the step in the trial, and
 // the rest runs only after a failed one:
 //   ... -> trial -> IF(proposal failed){retry x max_tries (each exits at once when
 //   no retry is pending) -> final}
+// flow FLOW_SLOW: only what follows a failed trial.
 static int append_iteration(abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode_t>& deps, int flow = FLOW_STEP)
 {
     // every handle must belong to a conditional node of this graph, or instantiation fails
-    cudaGraphConditionalHandle h_div = 0, h_retry = 0, h_run = 0;
+    cudaGraphConditionalHandle h_retry = 0, h_run = 0;
+    const bool slow = flow == FLOW_SLOW;
     const bool branch = c->sp.propose != 0;
     const bool retries = c->p.max_tries_update_stepsize > 0 && !branch;
     if (retries) CK(cudaGraphConditionalHandleCreate(&h_retry, G, 0, cudaGraphCondAssignDefault));
-    if (branch) CK(cudaGraphConditionalHandleCreate(&h_run, G, 0, cudaGraphCondAssignDefault));
+    if (branch && !slow) CK(cudaGraphConditionalHandleCreate(&h_run, G, 0, cudaGraphCondAssignDefault));
     int rc;
-    if (c->div_enabled)
+    if (c->div_enabled && !slow)
     {
-        CK(cudaGraphConditionalHandleCreate(&h_div, G, 0, cudaGraphCondAssignDefault));
-        rc = capture_into(c, G, deps, [&]() { launch_div_count(c->phys, c->ctrl, c->dp, c->div_flags, h_div, 1, c->st, flow); });
-        if (rc) return rc;
-        cudaGraph_t body;
-        rc = add_conditional(c, G, deps, h_div, cudaGraphCondTypeIf, &body);
-        if (rc) return rc;
-        rc = capture_division_body(c, body);
+        rc = capture_into(c, G, deps, [&]() { enqueue_growth(c); });
         if (rc) return rc;
     }
     if (c->verlet)
@@ -1284,11 +1231,14 @@ static int append_iteration(abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode
     trial.cond = h_retry;
     trial.use_cond = (retries ? 1 : 0) | (branch ? 2 : 0);
     trial.cond_run = h_run;
-    rc = capture_into(c, G, deps, [&]() {
-        enqueue_loop_pair_force(c, flow);
-        enqueue_attempt(c, MODE_TRIAL, trial);
-    });
-    if (rc) return rc;
+    if (!slow)
+    {
+        rc = capture_into(c, G, deps, [&]() {
+            enqueue_loop_pair_force(c, flow);
+            enqueue_attempt(c, MODE_TRIAL, trial);
+        });
+        if (rc) return rc;
+    }
     auto retry_attempt = [&](int use_cond) {
         AttemptArgs a = loop_attempt(c, flow);
         a.cond = h_retry;
@@ -1298,20 +1248,30 @@ static int append_iteration(abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode
     auto final_attempt = [&]() { enqueue_attempt(c, MODE_FINAL, loop_attempt(c, flow)); };
     if (branch)
     {
-        cudaGraph_t body;
-        rc = add_conditional(c, G, deps, h_run, cudaGraphCondTypeIf, &body);
-        if (rc) return rc;
-        std::vector<cudaGraphNode_t> bd;
-        rc = capture_into(c, body, bd, [&]() {
+        auto rest = [&]() {
             for (int r = 0; r < c->p.max_tries_update_stepsize; ++r) retry_attempt(0);
             final_attempt();
-        });
+        };
+        if (slow) rc = capture_into(c, G, deps, rest);
+        else
+        {
+            cudaGraph_t body;
+            rc = add_conditional(c, G, deps, h_run, cudaGraphCondTypeIf, &body);
+            if (rc) return rc;
+            std::vector<cudaGraphNode_t> bd;
+            rc = capture_into(c, body, bd, rest);
+        }
         if (rc) return rc;
     }
     else
     {
         if (retries)
         {
+            if (slow)
+            {
+                rc = capture_into(c, G, deps, [&]() { launch_retry_begin(c->ctrl, h_retry, c->st); });
+                if (rc) return rc;
+            }
             cudaGraph_t body;
             rc = add_conditional(c, G, deps, h_retry, cudaGraphCondTypeWhile, &body);
             if (rc) return rc;
@@ -1349,16 +1309,22 @@ static int instantiate_iterations(abm_ctx* c, int k, cudaGraphExec_t* exec)
 }
 
 // The loop graph, appended to G after `deps`: Ctrl::todo iterations.
-//   WHILE(iterations left){ LOOP_FAST x (pair pass -> trial [-> final])
-//                           -> IF(Ctrl::hold){one iteration with everything} }
+//   WHILE(iterations left){ LOOP_FAST x ([division] -> pair pass -> trial [-> final])
+//                           -> IF(Ctrl::hold){[division] or the rest of a failed first
+//                                             attempt's iteration} }
 // A conditional node costs 6-8 us between two kernels here (the kernels of a small colony take
-// 6 to 20), and an iteration of its own has two of them (divisions, retries), which most
-// iterations do not need.  In a fast iteration the kernels follow each other; a trial whose
-// error test asks for a retry, or a step that leaves a cell longer than Ldiv, sets
-// Ctrl::hold, the rest of the round's kernels leave at once (2 us each), and the slow
-// iteration after the round goes on from there.  64-cell colony 45 -> 28 us an iteration.
+// 6 to 20), and an iteration of its own needs one for its retries, which most iterations do
+// not use.  In a fast iteration the kernels follow each other; a trial whose error test asks
+// for a retry sets Ctrl::hold, the rest of the round's kernels leave at once (2 us each), and
+// the slow iteration after the round goes on from there.  The division launch leaves at once
+// unless the last step left a cell longer than Ldiv; it costs 3-4 us an iteration then, so
+// small colonies, which divide once in tens or hundreds of iterations, wait for the end of the
+// round instead (an event costs some 40 us more there: 64 cells 35 -> 31 us an iteration).
 // LOOP_FAST trades the round's own two nodes against those idle kernels.
 const int LOOP_FAST = 8;
+const int GROW_INLINE_CELLS = 1024;    // of LaunchShape's measure, twice the cells
+
+static bool grow_inline(const abm_ctx* c) { return c->div_enabled && c->n_ref > GROW_INLINE_CELLS; }
 
 static int append_loop(abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode_t>& deps)
 {
@@ -1373,6 +1339,7 @@ static int append_loop(abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode_t>& 
         const AttemptArgs a = loop_attempt(c, FLOW_FAST);
         for (int k = 0; k < LOOP_FAST; ++k)
         {
+            if (grow_inline(c)) enqueue_growth(c, FLOW_FAST);
             enqueue_loop_pair_force(c, FLOW_FAST);
             enqueue_attempt(c, MODE_TRIAL, a);
             // under the learned and PI controllers a passing trial closes the step
@@ -1386,6 +1353,11 @@ static int append_loop(abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode_t>& 
     rc = add_conditional(c, round, rd, h_slow, cudaGraphCondTypeIf, &slow);
     if (rc) return rc;
     std::vector<cudaGraphNode_t> sd;
+    if (c->div_enabled && !grow_inline(c))
+    {
+        rc = capture_into(c, slow, sd, [&]() { enqueue_growth(c, FLOW_SLOW); });
+        if (rc) return rc;
+    }
     return append_iteration(c, slow, sd, FLOW_SLOW);
 }
 
@@ -1410,8 +1382,7 @@ static bool has_loop(const abm_ctx* c) { return !c->verlet && !c->post_on; }
 // `step` iterations by the loop graph (no periodic rebuild among them)
 static int launch_loop(abm_ctx* c, int step)
 {
-    launch_loop_begin(c->ctrl, step, c->st);
-    if (c->div_enabled) launch_div_count(c->phys, c->ctrl, c->dp, c->div_flags, 0, 0, c->st, FLOW_BEGIN);
+    launch_loop_begin(c->ctrl, c->div_enabled, step, c->st);
     CK(cudaGraphLaunch(c->g_loop, c->st));
     return ABM_OK;
 }
@@ -1428,25 +1399,6 @@ static int build_iteration_graph(abm_ctx* c)
     if (rc) return rc;
     if (has_loop(c)) return ABM_OK;
     if (c->iter_k > 1) return instantiate_iterations(c, c->iter_k, &c->g_iter_k);
-    return ABM_OK;
-}
-
-// Division outside a graph: the flag count decides on the host whether the
-// body and the neighbor rebuild run.
-static int divide_now(abm_ctx* c, bool rebuild, int* n_divided)
-{
-    launch_div_count(c->phys, c->ctrl, c->dp, c->div_flags, 0, 0, c->st);
-    Ctrl h;
-    CK(cudaMemcpyAsync(&h, c->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    if (n_divided) *n_divided = h.n_divide;
-    if (h.n_divide > 0)
-    {
-        enqueue_division_body(c);
-        if (rebuild) enqueue_rebuild(c);
-        else c->nbrs_valid = false;
-        CK(cudaGetLastError());
-    }
     return ABM_OK;
 }
 
@@ -1527,11 +1479,7 @@ int abm_upload_neighbors(abm_ctx* c, const double* rows, int m, int ld)
     CK(cudaStreamSynchronize(c->st));
     h.n_dir = (int)cl.size();
     CK(cudaMemcpy(c->ctrl, &h, sizeof(Ctrl), cudaMemcpyHostToDevice));
-    launch_csr_rev(c->ctrl, c->row_ptr, c->col, c->lower_end, c->rev, c->cap, c->st);
-    launch_pair_list(c->ctrl, c->row_ptr, c->lower_end, c->col, c->rev, c->nbr_count, c->pair_start, c->scan_sums,
-                     c->pairs, c->cap, c->st);
-    if (c->dims == 2 && c->p.adhesion_mode != 0)
-        launch_adhere_flags(c->ctrl, c->row_ptr, c->col, c->geom, c->p.R, c->p.Rcell, c->adhere, c->cap, c->st);
+    enqueue_build(c, BUILD_RECORDS);
     CK(cudaGetLastError());
     c->nbrs_valid = true;
     return ABM_OK;
@@ -1812,11 +1760,13 @@ int abm_divide(abm_ctx* c, int* n_divided)
 {
     if (!c) return ABM_ERR_ARG;
     if (!c->cells_loaded) return fail(c, ABM_ERR_STATE, "no cells uploaded");
-    int rc = divide_now(c, false, n_divided);
-    if (rc) return rc;
-    rc = check_status(c);
+    enqueue_build(c, BUILD_DIVIDE);
+    CK(cudaGetLastError());
+    int rc = check_status(c);
     Ctrl h;
     CK(cudaMemcpy(&h, c->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost));
+    if (n_divided) *n_divided = h.n_divided;
+    if (h.n_divided > 0) c->nbrs_valid = false;
     c->n_host = h.n;
     return rc;
 }
@@ -1849,6 +1799,7 @@ int abm_get_stats(abm_ctx* c, abm_stats* s)
     s->t = h.t; s->dt = h.dt; s->last_max_error = h.last_max_error;
     s->n_cells = h.n; s->n_pairs = h.n_dir / 2;
     s->rejected = h.rejected; s->log_rows = h.log_rows; s->cell_steps = h.cell_steps;
+    c->n_seen = h.n;
     return check_status(c);
 }
 
@@ -1864,6 +1815,7 @@ int abm_iterate(abm_ctx* c, int n_iters, int n_cells_stop, abm_stats* stats)
         enqueue_rebuild(c);
         c->nbrs_valid = true;
     }
+    shape_launches(c);
     c->iter_k = 1;
     for (int k : {10, 5, 4, 2})
         if (c->p.iter_update_neighbors % k == 0) { c->iter_k = k; break; }
@@ -1884,7 +1836,6 @@ int abm_iterate(abm_ctx* c, int n_iters, int n_cells_stop, abm_stats* stats)
             }
         }
         if (c->graph_fallback && !c->g_iter) { rc = capture(c, enqueue_iteration, &c->g_iter); if (rc) return rc; }
-        if (!c->g_rebuild) { rc = capture(c, enqueue_rebuild, &c->g_rebuild); if (rc) return rc; }
     }
     for (int k = 0, next_check = 0; k < n_iters;)
     {
@@ -1934,7 +1885,7 @@ int abm_iterate(abm_ctx* c, int n_iters, int n_cells_stop, abm_stats* stats)
         }
         else
         {
-            if (c->div_enabled) { rc = divide_now(c, true, nullptr); if (rc) return rc; }
+            if (c->div_enabled) enqueue_growth(c);
             if (c->post_on)
             {
                 if (c->verlet) enqueue_verlet_step(c);
@@ -1954,10 +1905,7 @@ int abm_iterate(abm_ctx* c, int n_iters, int n_cells_stop, abm_stats* stats)
         k += step;
         // with the post-step kernels on, the periodic rebuild is part of the iteration
         if (!c->post_on && c->host_iter % c->p.iter_update_neighbors == 0)
-        {
-            if (c->p.use_graphs) CK(cudaGraphLaunch(c->g_rebuild, c->st));
-            else enqueue_rebuild(c);
-        }
+            enqueue_rebuild(c);
     }
     CK(cudaGetLastError());
     if (stats) return abm_get_stats(c, stats);
@@ -2132,7 +2080,8 @@ struct abm_batch {
     cudaStream_t st = nullptr;
     cudaGraphExec_t g_iter = nullptr, g_rebuild = nullptr;
     cudaGraphExec_t g_loop = nullptr;    // the loop graphs of all contexts, or null
-    Ctrl** ctrls = nullptr;              // their control records (device array)
+    Ctrl** ctrls = nullptr;              // their control records, and whether their cells may
+    int* divides = nullptr;              // divide (device arrays)
     int k_rebuild = 100;
     std::vector<cudaEvent_t> ev;
     cudaEvent_t done = nullptr;
@@ -2157,6 +2106,7 @@ void batch_free(abm_batch* b)
     if (b->g_iter) cudaGraphExecDestroy(b->g_iter);
     if (b->g_loop) cudaGraphExecDestroy(b->g_loop);
     if (b->ctrls) cudaFree(b->ctrls);
+    if (b->divides) cudaFree(b->divides);
     if (b->g_rebuild) cudaGraphExecDestroy(b->g_rebuild);
     for (cudaEvent_t e : b->ev) cudaEventDestroy(e);
     if (b->done) cudaEventDestroy(b->done);
@@ -2188,11 +2138,15 @@ int batch_iteration_graph(abm_batch* b)
 int batch_loop_graph(abm_batch* b)
 {
     std::vector<Ctrl*> ctrls;
+    std::vector<int> divides;
     for (abm_ctx* c : b->ctxs)
     {
         if (!has_loop(c)) return ABM_OK;
         ctrls.push_back(c->ctrl);
+        divides.push_back(c->div_enabled ? 1 : 0);
     }
+    BK(cudaMalloc(&b->divides, divides.size() * sizeof(int)));
+    BK(cudaMemcpy(b->divides, divides.data(), divides.size() * sizeof(int), cudaMemcpyHostToDevice));
     BK(cudaMalloc(&b->ctrls, ctrls.size() * sizeof(Ctrl*)));
     BK(cudaMemcpy(b->ctrls, ctrls.data(), ctrls.size() * sizeof(Ctrl*), cudaMemcpyHostToDevice));
     cudaGraph_t G = nullptr;
@@ -2201,11 +2155,7 @@ int batch_loop_graph(abm_batch* b)
     for (abm_ctx* c : b->ctxs)
     {
         std::vector<cudaGraphNode_t> deps;
-        if (c->div_enabled)
-            rc = capture_into(c, G, deps, [&]() {
-                launch_div_count(c->phys, c->ctrl, c->dp, c->div_flags, 0, 0, c->st, FLOW_BEGIN);
-            });
-        if (!rc) rc = append_loop(c, G, deps);
+        rc = append_loop(c, G, deps);
         if (rc) { rc = batch_fail(b, rc, "loop graph of a context: " + c->err); break; }
     }
     cudaError_t inst = cudaSuccess;
@@ -2295,7 +2245,7 @@ int abm_batch_iterate(abm_batch* b, int n_iters)
         int run = std::min(n_iters - it, b->k_rebuild - b->ctxs[0]->host_iter % b->k_rebuild);
         if (b->g_loop && run >= LOOP_FAST / 2)
         {
-            launch_loop_begin_all(b->ctrls, n, run, b->st);
+            launch_loop_begin_all(b->ctrls, b->divides, n, run, b->st);
             BK(cudaGraphLaunch(b->g_loop, b->st));
         }
         else

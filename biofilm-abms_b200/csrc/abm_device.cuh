@@ -299,6 +299,16 @@ __device__ __forceinline__ Dist dist_geom_mixed(const Geom& a, const Geom& b, in
     return o;
 }
 
+// x / b for a divisor b used many times, from its reciprocal r = 1.0 / b: with r correctly
+// rounded, q0 = x r and one correction by the exact remainder give the correctly rounded
+// quotient (Markstein, IBM J. Res. Dev. 34 (1990) 111, theorem 8; finite b != 0, no
+// underflow), so the result is the bits of x / b at three operations instead of a division.
+__device__ __forceinline__ double div_by(double x, double b, double r)
+{
+    const double q = __dmul_rn(x, r);
+    return __fma_rn(__fma_rn(-q, b, x), r, q);
+}
+
 // ---------------------------------------------------------------------------
 // Deterministic log, sin, cos for the division draws.  Two daughters of one
 // mother are placed exactly 2R apart end to end, where the JKR force jumps at
@@ -319,8 +329,10 @@ __device__ __forceinline__ double det_log(double x)
     if (m < 0.70710678118654752440) { m = __dmul_rn(m, 2.0); e = e - 1; }
     double f = __ddiv_rn(__dsub_rn(m, 1.0), __dadd_rn(m, 1.0));
     double f2 = __dmul_rn(f, f);
-    double p = __ddiv_rn(1.0, 29.0);
-    for (int k = 27; k >= 1; k -= 2) p = __dadd_rn(__dmul_rn(p, f2), __ddiv_rn(1.0, (double)k));
+    // the coefficients 1 / k are constants (a literal quotient is correctly rounded too)
+    double p = 1.0 / 29.0;
+#pragma unroll
+    for (int k = 27; k >= 1; k -= 2) p = __dadd_rn(__dmul_rn(p, f2), 1.0 / k);
     double ed = (double)e;
     return __dadd_rn(__dmul_rn(ed, LN2_HI), __dadd_rn(__dmul_rn(__dmul_rn(2.0, f), p), __dmul_rn(ed, LN2_LO)));
 }
@@ -332,11 +344,14 @@ __device__ __forceinline__ void det_sincos(double x, double& s, double& c)
     double k = rint(__dmul_rn(x, TWO_OVER_PI));
     double r = __dsub_rn(__dsub_rn(x, __dmul_rn(k, PIO2_HI)), __dmul_rn(k, PIO2_LO));
     double r2 = __dmul_rn(r, r);
+    // the quotients by constants through their reciprocals, corrected to the same bits
+    // (div_by): 22 divisions, 11 of them one after another, took most of a division's draws
     double ps = 1.0, pc = 1.0;
+#pragma unroll
     for (int n = 22; n >= 2; n -= 2)
     {
-        ps = __dsub_rn(1.0, __ddiv_rn(__dmul_rn(ps, r2), (double)((n + 1) * n)));
-        pc = __dsub_rn(1.0, __ddiv_rn(__dmul_rn(pc, r2), (double)(n * (n - 1))));
+        ps = __dsub_rn(1.0, div_by(__dmul_rn(ps, r2), (double)((n + 1) * n), 1.0 / ((n + 1) * n)));
+        pc = __dsub_rn(1.0, div_by(__dmul_rn(pc, r2), (double)(n * (n - 1)), 1.0 / (n * (n - 1))));
     }
     double sr = __dmul_rn(r, ps), cr = pc;
     int q = (int)((long long)k & 3);
@@ -494,16 +509,6 @@ __device__ __forceinline__ bool surface_contact(const MechParams& P, bool assume
 {
     if (!assume_2d) return (y[2] - h * y[5] < P.R) || (y[2] + h * y[5] < P.R);
     return y[2] < P.R;
-}
-
-// x / b for a divisor b used many times, from its reciprocal r = 1.0 / b: with r correctly
-// rounded, q0 = x r and one correction by the exact remainder give the correctly rounded
-// quotient (Markstein, IBM J. Res. Dev. 34 (1990) 111, theorem 8; finite b != 0, no
-// underflow), so the result is the bits of x / b at three operations instead of a division.
-__device__ __forceinline__ double div_by(double x, double b, double r)
-{
-    const double q = x * r;
-    return fma(fma(-q, b, x), r, q);
 }
 
 // What a cell's velocity needs at every stage of an attempt and that no stage changes: its

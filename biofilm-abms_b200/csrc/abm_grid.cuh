@@ -41,4 +41,14 @@ __device__ __forceinline__ bool grid_barrier(GridBar* bar, unsigned nb, Ctrl* ct
     return sh_ok != 0;
 }
 
+// Barrier over the blocks of one cluster, each calling it with all its threads.  The
+// hardware's release and acquire order global memory within the cluster; the fence keeps
+// the order at GPU scope as the grid barrier does.
+__device__ __forceinline__ void cluster_barrier()
+{
+    __threadfence();
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    __threadfence();
+}
+
 }   // namespace abm

@@ -1,10 +1,6 @@
 // CUDA kernels of the B200 mechanics step (sm_100a).
 //
-//   cell list      k_bbox -> k_bin_count -> scan -> k_bin_scatter        (uniform grid,
-//                  counting sort by bin)
-//   pair set       k_pair_build -> scan -> k_csr_fill -> k_csr_rev      (getCellNeighbors,
-//                  mechanics.hpp:520-593; CSR rows sorted by neighbor index), then the
-//                  pair records in bin order and the attempt order
+//   neighbor set, division   abm_build.cu
 //   pair force     k_pair_pass<MIXED, DIM>                              (cellCellInteractionForces,
 //                  mechanics.hpp:1209-1659; one record per unordered pair, screened
 //                  against an active list with a skin, both shares per pair; the last
@@ -20,20 +16,6 @@
 namespace abm {
 
 static inline int cdiv(long long a, long long b) { return (int)((a + b - 1) / b); }
-
-// ---------------------------------------------------------------------------
-// Order-preserving double <-> uint64 maps for atomic min/max
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ unsigned long long ord_enc(double x)
-{
-    unsigned long long u = (unsigned long long)__double_as_longlong(x);
-    return (u & 0x8000000000000000ull) ? ~u : (u | 0x8000000000000000ull);
-}
-__device__ __forceinline__ double ord_dec(unsigned long long u)
-{
-    u = (u & 0x8000000000000000ull) ? (u & 0x7fffffffffffffffull) : ~u;
-    return __longlong_as_double((long long)u);
-}
 
 // ---------------------------------------------------------------------------
 // Column-major cell arrays <-> device records
@@ -148,158 +130,6 @@ void launch_gen6_to_colmajor(const Gen6* g, int n, double* cm, cudaStream_t st)
 }
 
 // ---------------------------------------------------------------------------
-// Block reductions
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ double warp_min(double v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
-// ---------------------------------------------------------------------------
-// Cell list: bounding box -> grid (last block), counting sort by bin
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_bbox(const Geom* __restrict__ geom, Ctrl* ctrl, Grid* grid,
-                                              unsigned long long* acc, unsigned int* counter,
-                                              double edge, int cap_bins)
-{
-    __shared__ double sh[7][8];
-    __shared__ bool last;
-    const int n = ctrl->n;
-    double mn[3] = {1e300, 1e300, 1e300}, mx[3] = {-1e300, -1e300, -1e300}, mh = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    {
-        Geom g = load_geom(geom, i);
-        mn[0] = fmin(mn[0], g.rx); mn[1] = fmin(mn[1], g.ry); mn[2] = fmin(mn[2], g.rz);
-        mx[0] = fmax(mx[0], g.rx); mx[1] = fmax(mx[1], g.ry); mx[2] = fmax(mx[2], g.rz);
-        mh = fmax(mh, g.h);
-    }
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    double v[7] = {mn[0], mn[1], mn[2], mx[0], mx[1], mx[2], mh};
-    for (int k = 0; k < 3; ++k) v[k] = warp_min(v[k]);
-    for (int k = 3; k < 7; ++k) v[k] = warp_max(v[k]);
-    if (lane == 0) for (int k = 0; k < 7; ++k) sh[k][wid] = v[k];
-    __syncthreads();
-    if (threadIdx.x == 0)
-    {
-        for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-        {
-            for (int k = 0; k < 3; ++k) v[k] = fmin(v[k], sh[k][w]);
-            for (int k = 3; k < 7; ++k) v[k] = fmax(v[k], sh[k][w]);
-        }
-        for (int k = 0; k < 3; ++k) atomicMin(&acc[k], ord_enc(v[k]));
-        for (int k = 3; k < 7; ++k) atomicMax(&acc[k], ord_enc(v[k]));
-        __threadfence();
-        unsigned int done = atomicAdd(counter, 1u);
-        last = (done == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (last && threadIdx.x == 0)
-    {
-        __threadfence();
-        double lo[3], hi[3];
-        for (int k = 0; k < 3; ++k)
-        {
-            lo[k] = ord_dec(atomicAdd(&acc[k], 0ull));
-            hi[k] = ord_dec(atomicAdd(&acc[3 + k], 0ull));
-        }
-        double maxh = ord_dec(atomicAdd(&acc[6], 0ull));
-        if (n <= 0) { for (int k = 0; k < 3; ++k) { lo[k] = 0; hi[k] = 0; } maxh = 0; }
-        // fmin / fmax skip NaN coordinates; an axis without any finite one spans [0, 0], and
-        // an infinite extent, or one no grid of cap_bins bins can hold, is an overflow
-        bool bad = false;
-        for (int k = 0; k < 3; ++k)
-        {
-            if (!(lo[k] <= hi[k])) { lo[k] = 0; hi[k] = 0; }
-            if (!(hi[k] - lo[k] < 1e290)) bad = true;
-        }
-        double e = edge;
-        double nb[3] = {1.0, 1.0, 1.0};
-        for (int tries = 0; tries < 64 && !bad; ++tries)
-        {
-            for (int k = 0; k < 3; ++k) nb[k] = floor((hi[k] - lo[k]) / e) + 1;
-            if (nb[0] * nb[1] * nb[2] <= (double)cap_bins) break;
-            e *= 1.5;
-        }
-        if (bad || !(nb[0] * nb[1] * nb[2] <= (double)cap_bins))
-        {
-            // one bin: every later kernel stays in bounds, the pair build skips its work
-            // (the status is set) and the host reports the overflow
-            atomicOr(&ctrl->status, (int)ST_BIN_OVERFLOW);
-            for (int k = 0; k < 3; ++k) { nb[k] = 1.0; lo[k] = 0.0; }
-            e = edge;
-        }
-        Grid g;
-        g.x0 = lo[0]; g.y0 = lo[1]; g.z0 = lo[2]; g.edge = e; g.inv_edge = 1.0 / e;
-        g.nx = (int)nb[0]; g.ny = (int)nb[1]; g.nz = (int)nb[2];
-        g.nbins = g.nx * g.ny * g.nz;
-        g.max_half_l = maxh;
-        *grid = g;
-        // reset accumulators for the next rebuild
-        for (int k = 0; k < 3; ++k) { acc[k] = 0xffffffffffffffffull; acc[3 + k] = 0ull; }
-        acc[6] = 0ull;
-        *counter = 0u;
-    }
-}
-
-void launch_bbox(const Geom* geom, Ctrl* ctrl, Grid* grid, unsigned long long* acc,
-                 unsigned int* counter, double edge, int cap_bins, int cap_cells, cudaStream_t st)
-{
-    int blocks = min(cdiv(cap_cells, 256), 592);
-    k_bbox<<<max(blocks, 1), 256, 0, st>>>(geom, ctrl, grid, acc, counter, edge, cap_bins);
-}
-
-__device__ __forceinline__ int bin_coord(double x, double x0, double inv_edge, int nb)
-{
-    int b = (int)floor((x - x0) * inv_edge);
-    return b < 0 ? 0 : (b >= nb ? nb - 1 : b);
-}
-
-__global__ void k_bin_count(const Geom* __restrict__ geom, const Ctrl* ctrl, const Grid* grid,
-                            int* bin_count, int* key, int* slot)
-{
-    const int n = ctrl->n;
-    const Grid g = *grid;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    {
-        Geom c = load_geom(geom, i);
-        int bx = bin_coord(c.rx, g.x0, g.inv_edge, g.nx);
-        int by = bin_coord(c.ry, g.y0, g.inv_edge, g.ny);
-        int bz = bin_coord(c.rz, g.z0, g.inv_edge, g.nz);
-        int k = (bz * g.ny + by) * g.nx + bx;
-        if (k >= g.nbins) k = g.nbins - 1;
-        key[i] = k;
-        slot[i] = atomicAdd(&bin_count[k], 1);
-    }
-}
-
-void launch_bin_count(const Geom* geom, const Ctrl* ctrl, const Grid* grid, int* bin_count,
-                      int* key, int* slot, int cap_cells, cudaStream_t st)
-{
-    k_bin_count<<<max(cdiv(cap_cells, 256), 1), 256, 0, st>>>(geom, ctrl, grid, bin_count, key, slot);
-}
-
-__global__ void k_bin_scatter(const Geom* __restrict__ geom, const Ctrl* ctrl, const int* bin_start,
-                              const int* key, const int* slot, int* sorted_cell, Geom* sorted_geom)
-{
-    const int n = ctrl->n;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    {
-        int pos = bin_start[key[i]] + slot[i];
-        sorted_cell[pos] = i;
-        sorted_geom[pos] = load_geom(geom, i);
-    }
-}
-
-void launch_bin_scatter(const Geom* geom, const Ctrl* ctrl, const int* bin_start, const int* key,
-                        const int* slot, int* sorted_cell, Geom* sorted_geom, int cap_cells,
-                        cudaStream_t st)
-{
-    k_bin_scatter<<<max(cdiv(cap_cells, 256), 1), 256, 0, st>>>(geom, ctrl, bin_start, key, slot,
-                                                                 sorted_cell, sorted_geom);
-}
-
 // ---------------------------------------------------------------------------
 // Exclusive scan (three passes: block sums, one-block scan of the sums,
 // block scan + offset).  Up to 4096 * 4096 entries.
@@ -414,221 +244,7 @@ void launch_scan(const int* in, const int* len, int* out, int* block_sums, int c
     k_scan_final<<<nb, SCAN_T, 0, st>>>(in, len, block_sums, out, nb);
 }
 
-// ---------------------------------------------------------------------------
-// Pair build: one block per bin (grid-stride over bins), the bin's cells in
-// groups of up to PB_G.  The block's threads sweep the flattened (own cell,
-// candidate) products of the 27 surrounding bins with a cheap rejection test;
-// the survivors go to a per-warp queue and are evaluated 32 at a time, so the
-// exact FP64 distance runs on full warps instead of once per candidate for
-// whichever lane needs it.  A survivor is kept when it passes the reference's
-// two tests: centre distance < threshold + Ldiv + 2R and segment distance <
-// threshold (mechanics.hpp:548-577).  The segment distance is always evaluated
-// with the larger index as cell 1, as the reference's j < i loop does, so both
-// cells of a pair reach the same decision.  Rows are filled in any order
-// (shared-memory counters) and sorted by k_csr_fill.
-//
-// The rejection test is rigorous: every branch of dist_between_cells returns
-// points r1 + s n1, r2 + t n2 with |s| <= h1, |t| <= h2, so the computed |d|
-// is at least |r2 - r1| - h1 |n1| - h2 |n2| up to rounding (~1e-12 um at
-// these coordinates).  A candidate is dropped only when, in FP32 with a
-// 1e-4 um margin, |r2 - r1| > threshold + h1 max(1, |n1|^2) + h2 max(1, |n2|^2),
-// i.e. when its |d| is certainly >= threshold.
-// ---------------------------------------------------------------------------
-const int PB_T = 128, PB_G = 128, PB_WARPS = PB_T / 32, PB_SLICE = 1 << 20;
-
-struct PbShared {
-    double rx[PB_G], ry[PB_G], rz[PB_G];
-    float reach[PB_G];                  // h max(1, |n|^2)
-    int cnt[PB_G];
-    int q_own[PB_WARPS][64], q_pos[PB_WARPS][64];
-};
-
-// exact tests for one queued (own, candidate) product
-__device__ __forceinline__ void pb_exact(const Geom* __restrict__ sorted_geom, const int* __restrict__ sorted_cell,
-                                         int base, int own, int pos, const BuildParams& bp, PbShared& sh,
-                                         int* scratch)
-{
-    const Geom gm = sorted_geom[base + own], go = sorted_geom[pos];
-    const int cm = sorted_cell[base + own], o = sorted_cell[pos];
-    const Geom& gi = (cm > o) ? gm : go;
-    const Geom& gj = (cm > o) ? go : gm;
-    double cd = xnorm(xsub(x3(gi.rx, gi.ry, gi.rz), x3(gj.rx, gj.ry, gj.rz)));
-    if (!(cd < bp.prefilter)) return;
-    Dist d = dist_geom(gi, gj);
-    if (xnorm(x3(d.dx, d.dy, d.dz)) < bp.threshold)
-    {
-        const int slot = atomicAdd(&sh.cnt[own], 1);
-        if (slot < bp.cap_per_cell) scratch[(size_t)cm * bp.cap_per_cell + slot] = o;
-    }
-}
-
-__global__ void __launch_bounds__(PB_T) k_pair_build(const Grid* grid, const int* __restrict__ bin_start,
-                                                    const int* __restrict__ sorted_cell,
-                                                    const Geom* __restrict__ sorted_geom, const Ctrl* ctrl,
-                                                    BuildParams bp, int* scratch, int* count)
-{
-    __shared__ PbShared sh;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned lt = (1u << lane) - 1u;
-    const Grid g = *grid;
-    const int cap = bp.cap_per_cell;
-    const float thr = (float)bp.threshold + 1e-4f;
-    if (ctrl->status & ST_BIN_OVERFLOW)
-    {
-        // the cells do not fit a grid (k_bbox): an empty neighbor set, reported by the host
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < ctrl->n; i += gridDim.x * blockDim.x) count[i] = 0;
-        return;
-    }
-    for (int bin = blockIdx.x; bin < g.nbins; bin += gridDim.x)
-    {
-        const int s0 = bin_start[bin], s1 = bin_start[bin + 1];
-        if (s0 == s1) continue;
-        const int bx = bin % g.nx, by = (bin / g.nx) % g.ny, bz = bin / (g.nx * g.ny);
-        for (int base = s0; base < s1; base += PB_G)
-        {
-            const int G = min(PB_G, s1 - base);
-            __syncthreads();                                   // the previous group is done with sh
-            for (int q = threadIdx.x; q < G; q += PB_T)
-            {
-                const Geom x = sorted_geom[base + q];
-                sh.rx[q] = x.rx; sh.ry[q] = x.ry; sh.rz[q] = x.rz;
-                sh.reach[q] = segment_reach(x.h, x.nx, x.ny, x.nz);
-                sh.cnt[q] = 0;
-            }
-            __syncthreads();
-            int qn = 0;                                        // this warp's queue length (warp-uniform)
-            for (int dz = -1; dz <= 1; ++dz)
-            {
-                const int zz = bz + dz;
-                if (zz < 0 || zz >= g.nz) continue;
-                for (int dy = -1; dy <= 1; ++dy)
-                {
-                    const int yy = by + dy;
-                    if (yy < 0 || yy >= g.ny) continue;
-                    for (int dx = -1; dx <= 1; ++dx)
-                    {
-                        const int xx = bx + dx;
-                        if (xx < 0 || xx >= g.nx) continue;
-                        const int nbin = (zz * g.ny + yy) * g.nx + xx;
-                        if (nbin >= g.nbins) continue;
-                        const int nb0 = bin_start[nbin], nb1 = bin_start[nbin + 1];
-                        // candidates in slices of PB_SLICE so G * len stays far from INT_MAX
-                        for (int c0 = nb0; c0 < nb1; c0 += PB_SLICE)
-                        {
-                        const int total = G * min(PB_SLICE, nb1 - c0);
-                        // warps take consecutive 32-product slices; every lane of a
-                        // warp runs the same number of rounds.  Product idx is (own =
-                        // idx % G, candidate = idx / G); both advance by PB_T per round,
-                        // so they are stepped instead of divided.
-                        int q = (warp * 32 + lane) / G, r = (warp * 32 + lane) % G;
-                        const int dq = PB_T / G, dr = PB_T % G;
-                        for (int w0 = warp * 32; w0 < total; w0 += PB_T)
-                        {
-                            const int idx = w0 + lane;
-                            bool pass = false;
-                            int own = 0, pos = 0;
-                            const int own_r = r, cand_q = q;
-                            r += dr; q += dq;
-                            if (r >= G) { r -= G; q += 1; }
-                            if (idx < total)
-                            {
-                                own = own_r;
-                                pos = c0 + cand_q;
-                                if (pos != base + own)
-                                {
-                                    const Geom& c = sorted_geom[pos];
-                                    const double cx = __ldg(&c.rx), cy = __ldg(&c.ry), cz = __ldg(&c.rz);
-                                    const float fx = (float)(cx - sh.rx[own]);
-                                    const float fy = (float)(cy - sh.ry[own]);
-                                    const float fz = (float)(cz - sh.rz[own]);
-                                    const float L = thr + sh.reach[own]
-                                                    + segment_reach(__ldg(&c.h), __ldg(&c.nx), __ldg(&c.ny), __ldg(&c.nz));
-                                    pass = !(fx * fx + fy * fy + fz * fz > L * L);
-                                }
-                            }
-                            const unsigned m = __ballot_sync(0xffffffffu, pass);
-                            if (pass)
-                            {
-                                const int r = qn + __popc(m & lt);
-                                sh.q_own[warp][r] = own;
-                                sh.q_pos[warp][r] = pos;
-                            }
-                            qn += __popc(m);
-                            if (qn >= 32)
-                            {
-                                qn -= 32;
-                                __syncwarp();
-                                const int eo = sh.q_own[warp][qn + lane], ep = sh.q_pos[warp][qn + lane];
-                                __syncwarp();
-                                pb_exact(sorted_geom, sorted_cell, base, eo, ep, bp, sh, scratch);
-                            }
-                        }
-                        }
-                    }
-                }
-            }
-            __syncwarp();
-            if (lane < qn) pb_exact(sorted_geom, sorted_cell, base, sh.q_own[warp][lane], sh.q_pos[warp][lane], bp, sh,
-                                    scratch);
-            __syncthreads();                                   // every count of the group is final
-            for (int q = threadIdx.x; q < G; q += PB_T)
-            {
-                int cnt = sh.cnt[q];
-                if (cnt > cap) { atomicOr((int*)&ctrl->status, (int)ST_NBR_OVERFLOW); cnt = cap; }
-                count[sorted_cell[base + q]] = cnt;
-            }
-        }
-    }
-}
-
-void launch_pair_build(const Grid* grid, const int* bin_start, const int* sorted_cell,
-                       const Geom* sorted_geom, const Ctrl* ctrl, BuildParams bp, int* scratch,
-                       int* count, int cap_bins, int num_sms, cudaStream_t st)
-{
-    int blocks = min(cap_bins, num_sms * 16);
-    k_pair_build<<<max(blocks, 1), PB_T, 0, st>>>(grid, bin_start, sorted_cell, sorted_geom, ctrl, bp,
-                                                  scratch, count);
-}
-
-// CSR rows: copy each cell's list and sort it ascending (deterministic order for
-// the force reduction; the reference's table is i-major, j ascending).  One warp
-// per row: an entry's rank is the number of smaller entries in the row (entries
-// are distinct cell indices), counted with shuffles, and the entry lands at
-// row_ptr[i] + rank.
 const int CF_T = 256;
-
-__global__ void __launch_bounds__(CF_T) k_csr_fill(const Ctrl* ctrl, const int* __restrict__ row_ptr,
-                                                  const int* __restrict__ scratch, int cap, int* col, Ctrl* ctrl_w)
-{
-    const int n = ctrl->n;
-    const int lane = threadIdx.x & 31;
-    const int nwarps = gridDim.x * (CF_T / 32);
-    for (int i = (blockIdx.x * CF_T + threadIdx.x) >> 5; i < n; i += nwarps)
-    {
-        const int r0 = row_ptr[i], len = row_ptr[i + 1] - r0;
-        const int* src = scratch + (size_t)i * cap;
-        for (int a = 0; a < len; a += 32)
-        {
-            const int v = (a + lane < len) ? src[a + lane] : INT_MAX;
-            int rank = 0;
-            for (int b = 0; b < len; b += 32)
-            {
-                const int w = (b + lane < len) ? src[b + lane] : INT_MAX;
-#pragma unroll 8
-                for (int q = 0; q < 32; ++q) rank += (__shfl_sync(0xffffffffu, w, q) < v) ? 1 : 0;
-            }
-            if (a + lane < len) col[r0 + rank] = v;
-        }
-        if (i == n - 1 && lane == 0) ctrl_w->n_dir = r0 + len;
-    }
-    if (n == 0 && blockIdx.x == 0 && threadIdx.x == 0) ctrl_w->n_dir = 0;
-}
-
-void launch_csr_fill(const Ctrl* ctrl, const int* row_ptr, const int* scratch, int cap, int* col, Ctrl* ctrl_w,
-                     int cap_cells, cudaStream_t st)
-{
-    k_csr_fill<<<max(cdiv(cap_cells, CF_T / 32), 1), CF_T, 0, st>>>(ctrl, row_ptr, scratch, cap, col, ctrl_w);
-}
 
 // ---------------------------------------------------------------------------
 // Pair force: G lanes per cell walk its CSR row; each lane evaluates the
@@ -997,7 +613,7 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
                                                       const float* __restrict__ mlp_w, int flow)
 {
     __shared__ bool last;
-    if (ctrl->halted || loop_idle(ctrl, flow, true)) return;
+    if (ctrl->halted || loop_idle(ctrl, flow)) return;
     const bool split = PROPOSE && gridDim.x > 1;
     const bool proposer = split && blockIdx.x == gridDim.x - 1;
     const int work_blocks = split ? gridDim.x - 1 : gridDim.x;
@@ -1008,7 +624,10 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
     const int stride = work_blocks * blockDim.x;
     double ovl_max = 0.0;
     if (proposer)
+    {
+        if (al.cluster && refresh) cluster_barrier();
         mlp_propose_block(ctrl, sp, mlp_w);
+    }
     else if (refresh)
     {
         const int n_pairs = ctrl->n_dir >> 1, n = ctrl->n;
@@ -1032,7 +651,9 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
             pos = __shfl_sync(0xffffffffu, pos, 0);
             if (keep) surv[pos + __popc(mask & ((1u << lane) - 1u))] = p;
         }
-        if (!grid_barrier(al.bar, work_blocks, ctrl)) return;
+        // with a proposer, its block takes part in a cluster's barrier below
+        if (al.cluster) cluster_barrier();
+        else if (!grid_barrier(al.bar, work_blocks, ctrl)) return;
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
         {
             int cnt = 0;
@@ -1115,45 +736,51 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
     }
 }
 
-// The pair list visits cells in `order` (the cell list's bin order after a rebuild,
-// else index order): pairs of one region of space are screened together, so each
-// cell's record is fetched once and reused from the caches by its neighbours' pairs.
-
-__global__ void k_lower_counts(const Ctrl* ctrl, const int* __restrict__ row_ptr, const int* __restrict__ lower_end,
-                               const int* __restrict__ order, int* count)
+// A cluster of 16 blocks is more than the portable 8: allowed per kernel, and used only where
+// the device can place one.
+LaunchShape make_shape(const void* kernel, int block, long long threads, bool cluster, int num_sms)
 {
-    const int n = ctrl->n;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x)
+    const int MAX_CLUSTER = 16;
+    LaunchShape s;
+    const long long want = max((threads + block - 1) / block, 1LL);
+    if (cluster)
     {
-        const int i = order ? order[q] : q;
-        count[q] = lower_end[i] - row_ptr[i];
+        int size = 1;
+        while (size < MAX_CLUSTER && size < want) size *= 2;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = size; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        cfg.gridDim = dim3(size); cfg.blockDim = dim3(block); cfg.attrs = at; cfg.numAttrs = 1;
+        int fits = 0;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&fits, kernel, &cfg) == cudaSuccess && fits > 0)
+        {
+            s.blocks = size;
+            s.cluster = 1;
+            return s;
+        }
+        cudaGetLastError();
     }
+    int occ = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, block, 0);
+    s.blocks = (int)min(want, (long long)num_sms * max(occ, 1));
+    return s;
 }
 
-// a new pair list makes the active list stale (block 0 marks it)
-__global__ void k_pair_list_fill(Ctrl* ctrl, const int* __restrict__ row_ptr, const int* __restrict__ lower_end,
-                                 const int* __restrict__ col, const int* __restrict__ rev,
-                                 const int* __restrict__ order, const int* __restrict__ start, int4* pairs)
+void launch_shape(const void* kernel, const LaunchShape& shape, int block, void** args, cudaStream_t st)
 {
-    const int n = ctrl->n;
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->screen_valid = 0;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x)
+    if (!shape.cluster)
     {
-        const int i = order ? order[q] : q;
-        const int r0 = row_ptr[i], p0 = start[q];
-        for (int k = r0; k < lower_end[i]; ++k) pairs[p0 + (k - r0)] = make_int4(i, col[k], k, rev[k]);
+        cudaLaunchCooperativeKernel(kernel, dim3(shape.blocks), dim3(block), args, 0, st);
+        return;
     }
-}
-
-void launch_pair_list(const Ctrl* ctrl, const int* row_ptr, const int* lower_end, const int* col, const int* rev,
-                      int* count, int* start, int* block_sums, int4* pairs, int cap_cells, cudaStream_t st,
-                      const int* order)
-{
-    const int blocks = max(cdiv(cap_cells, 256), 1);
-    k_lower_counts<<<blocks, 256, 0, st>>>(ctrl, row_ptr, lower_end, order, count);
-    launch_scan(count, &ctrl->n, start, block_sums, cap_cells, st);
-    k_pair_list_fill<<<blocks, 256, 0, st>>>(const_cast<Ctrl*>(ctrl), row_ptr, lower_end, col, rev, order, start,
-                                             pairs);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = shape.blocks; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(shape.blocks); cfg.blockDim = dim3(block); cfg.stream = st; cfg.attrs = at; cfg.numAttrs = 1;
+    cudaLaunchKernelExC(&cfg, kernel, args);
 }
 
 // total dE/dq of each cell from its active shares (the API paths; the loop's first attempt
@@ -1170,65 +797,42 @@ __global__ void k_pair_sum_rows(const int* __restrict__ row_ptr, const int* __re
 void launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, const double* jkr_delta,
                           const double* jkr_radius, Gen6* fcc, double4* jbuf, int mixed, int max_entries,
                           int cap_cells, int num_sms, cudaStream_t st, int with_sum, int dims, int tile,
-                          int blocks_per_sm, const int4* pairs, int* surv, ActiveList al, const StepParams* sp,
+                          int blocks_per_sm, const int4* pairs, int* surv, ActiveList al, int cells,
+                          const StepParams* sp,
                           const float* mlp_w, int flow)
 {
     // sp (the loop's pass): the last block also runs the step-size proposal
     StepParams spv{};
     if (sp) spv = *sp;
     const int propose = (sp && sp->stats_on) ? 1 : 0;
-    // grid: at least `tile` pairs per block, at most the blocks that are resident at
-    // once (blocks_per_sm caps them per SM); the blocks stride over the pairs.  The launch
-    // is cooperative: the blocks of a refresh wait for one another.
-    tile = tile <= 0 ? 1024 : min(tile, PS_TILE_MAX);
-    const int max_pairs = max(max_entries / 2, 1);
     const bool f32 = mixed && dims != 2;
     const int p = propose ? 1 : 0;
     const void* const fn2[2] = {(const void*)k_pair_pass<false, 2, false>, (const void*)k_pair_pass<false, 2, true>};
     const void* const fn3m[2] = {(const void*)k_pair_pass<true, 3, false>, (const void*)k_pair_pass<true, 3, true>};
     const void* const fn3[2] = {(const void*)k_pair_pass<false, 3, false>, (const void*)k_pair_pass<false, 3, true>};
     const void* fn = dims == 2 ? fn2[p] : f32 ? fn3m[p] : fn3[p];
-    int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, fn, PS_T, 0);
-    occ = max(occ, 1);
-    const int per_sm = blocks_per_sm > 0 ? min(blocks_per_sm, occ) : occ;
-    const int grid = max(1, min(cdiv(max_pairs, tile), num_sms * per_sm));
+    // The blocks stride over the pairs; those of a refresh wait for one another, so the launch
+    // is one cluster for a small colony (the rule of the build launch), else a cooperative
+    // grid.  By default two threads per cell (1.5 to 2 active pairs a cell): blocks without work
+    // still join the barrier and take the room of a batch's other colonies.  With a tile set:
+    // at least that many pairs per block, at most the blocks resident at once (blocks_per_sm
+    // caps them per SM).
+    LaunchShape shape;
+    if (tile <= 0 && blocks_per_sm <= 0)
+        shape = make_shape(fn, PS_T, 2LL * cells + (p ? PS_T : 0), cells <= BUILD_CLUSTER_CELLS / 2, num_sms);
+    else
+    {
+        const int max_pairs = max(max_entries / 2, 1);
+        shape = make_shape(fn, PS_T, (long long)PS_T * cdiv(max_pairs, tile <= 0 ? 1024 : min(tile, PS_TILE_MAX)), false,
+                           num_sms);
+        if (blocks_per_sm > 0) shape.blocks = min(shape.blocks, num_sms * blocks_per_sm);
+    }
+    al.cluster = shape.cluster;
     void* args[] = {(void*)&geom, (void*)&pairs, (void*)&ctrl, (void*)&fp, (void*)&jkr_delta, (void*)&jkr_radius,
-                    (void*)&jbuf, (void*)&surv, (void*)&al, (void*)&spv, (void*)&mlp_w,
-                    (void*)&flow};
-    cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(PS_T), args, 0, st);
+                    (void*)&jbuf, (void*)&surv, (void*)&al, (void*)&spv, (void*)&mlp_w, (void*)&flow};
+    launch_shape(fn, shape, PS_T, args, st);
     if (with_sum)
         k_pair_sum_rows<<<max(cdiv(cap_cells, 128), 1), 128, 0, st>>>(al.row_ptr, al.n_act, ctrl, jbuf, fcc, f32);
-}
-
-// to_adhere (2D/include/simulation.hpp:242-258, one group in the adhesion map):
-// for each lower entry (i, j < i), dist of the (i, j) row > R + Rcell and < 2R
-__global__ void k_adhere_flags(const Ctrl* ctrl, const int* __restrict__ row_ptr, const int* __restrict__ col,
-                               const Geom* __restrict__ geom, double R, double Rcell, unsigned char* adhere)
-{
-    const int n = ctrl->n;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    {
-        const Geom gi = load_geom(geom, i);
-        for (int k = row_ptr[i]; k < row_ptr[i + 1]; ++k)
-        {
-            const int j = col[k];
-            unsigned char a = 0;
-            if (j < i)
-            {
-                Dist d = dist_geom(gi, load_geom(geom, j));
-                const double dist = xnorm(x3(d.dx, d.dy, d.dz));
-                a = (dist > R + Rcell && dist < 2 * R) ? 1 : 0;
-            }
-            adhere[k] = a;
-        }
-    }
-}
-
-void launch_adhere_flags(const Ctrl* ctrl, const int* row_ptr, const int* col, const Geom* geom, double R,
-                         double Rcell, unsigned char* adhere, int cap_cells, cudaStream_t st)
-{
-    k_adhere_flags<<<max(cdiv(cap_cells, 128), 1), 128, 0, st>>>(ctrl, row_ptr, col, geom, R, Rcell, adhere);
 }
 
 // the reference's 2-D dE/dq (cellCellRepulsiveForces + cellCellAdhesiveForces) from the
@@ -1307,69 +911,43 @@ void launch_frame_snapshot(const Geom* geom, const Vel* vel, const Phys* phys, C
                                              cap_cells, feta, snap_feta);
 }
 
-// Attempt order (3-D): the cells whose velocity takes the full surface solve
-// (area integrals, mechanics.hpp:2254-2309) first, then the others, each group in
-// index order, so that the warps of an attempt mostly run one of the three
-// branches of getVelocities (mechanics.hpp:2011-2347) instead of all of them.
-// Made at every neighbor rebuild from the cells of that moment; a cell that
-// changes branch before the next rebuild costs only divergence.  The order
-// changes no per-cell result.
-__global__ void k_attempt_class(const Geom* __restrict__ geom, const Ctrl* ctrl, MechParams P, int* flag)
-{
-    const int n = ctrl->n;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    {
-        const Geom g = load_geom(geom, i);
-        const bool a2 = g.nz < P.nz_threshold;
-        const bool contact = a2 ? (g.rz < P.R) : ((g.rz - g.h * g.nz < P.R) || (g.rz + g.h * g.nz < P.R));
-        flag[i] = (!P.no_surface && !a2 && contact) ? 1 : 0;
-    }
-}
-
-__global__ void k_attempt_order(Ctrl* ctrl, const int* __restrict__ flag, const int* __restrict__ pos, int* order)
-{
-    const int n = ctrl->n;
-    const int n_full = pos[n];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        order[flag[i] ? pos[i] : n_full + (i - pos[i])] = i;
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->n_order = n;
-}
-
-void launch_attempt_order(const Geom* geom, Ctrl* ctrl, const MechParams& P, int* flag, int* pos,
-                          int* block_sums, int* order, int cap_cells, cudaStream_t st)
-{
-    const int blocks = max(cdiv(cap_cells, 256), 1);
-    k_attempt_class<<<blocks, 256, 0, st>>>(geom, ctrl, P, flag);
-    launch_scan(flag, &ctrl->n, pos, block_sums, cap_cells, st);
-    k_attempt_order<<<blocks, 256, 0, st>>>(ctrl, flag, pos, order);
-}
-
-__device__ __forceinline__ void loop_begin(Ctrl* c, int todo)
+__device__ __forceinline__ void loop_begin(Ctrl* c, int divides, int todo)
 {
     c->todo = todo;
-    c->hold = HOLD_NONE;
+    c->hold = divides ? HOLD_START : HOLD_NONE;
     c->div_any = 0;
-    c->rounds = todo + 4;
+    c->rounds = 2 * todo + 4;
 }
-__global__ void k_loop_begin(Ctrl* c, int todo) { loop_begin(c, todo); }
-__global__ void k_loop_begin_all(Ctrl* const* ctrls, int n, int todo)
+__global__ void k_loop_begin(Ctrl* c, int divides, int todo) { loop_begin(c, divides, todo); }
+__global__ void k_loop_begin_all(Ctrl* const* ctrls, const int* divides, int n, int todo)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k < n) loop_begin(ctrls[k], todo);
+    if (k < n) loop_begin(ctrls[k], divides[k], todo);
 }
 __global__ void k_loop_round(Ctrl* c, unsigned long long cond_slow, unsigned long long cond_loop)
 {
     const bool slow = c->hold != HOLD_NONE && c->todo > 0 && !c->halted;
-    const int left = c->todo - (slow ? 1 : 0);
+    const int left = c->todo - (c->hold == HOLD_RETRY ? 1 : 0);
     c->rounds -= 1;
     cudaGraphSetConditional((cudaGraphConditionalHandle)cond_slow, slow ? 1u : 0u);
     cudaGraphSetConditional((cudaGraphConditionalHandle)cond_loop, left > 0 && !c->halted && c->rounds > 0 ? 1u : 0u);
 }
 
-void launch_loop_begin(Ctrl* ctrl, int todo, cudaStream_t st) { k_loop_begin<<<1, 1, 0, st>>>(ctrl, todo); }
-void launch_loop_begin_all(Ctrl* const* ctrls, int n, int todo, cudaStream_t st)
+void launch_loop_begin(Ctrl* ctrl, int divides, int todo, cudaStream_t st)
 {
-    k_loop_begin_all<<<cdiv(n, 128), 128, 0, st>>>(ctrls, n, todo);
+    k_loop_begin<<<1, 1, 0, st>>>(ctrl, divides, todo);
+}
+void launch_loop_begin_all(Ctrl* const* ctrls, const int* divides, int n, int todo, cudaStream_t st)
+{
+    k_loop_begin_all<<<cdiv(n, 128), 128, 0, st>>>(ctrls, divides, n, todo);
+}
+__global__ void k_retry_begin(const Ctrl* c, unsigned long long cond)
+{
+    cudaGraphSetConditional((cudaGraphConditionalHandle)cond, !loop_idle(c, FLOW_SLOW) && c->mode == MODE_RETRY ? 1u : 0u);
+}
+void launch_retry_begin(Ctrl* ctrl, unsigned long long cond, cudaStream_t st)
+{
+    k_retry_begin<<<1, 1, 0, st>>>(ctrl, cond);
 }
 void launch_loop_round(Ctrl* ctrl, unsigned long long cond_slow, unsigned long long cond_loop, cudaStream_t st)
 {

@@ -16,11 +16,12 @@ enum CtrlMode { MODE_TRIAL = 0, MODE_RETRY = 1, MODE_FINAL = 2, MODE_COMMIT = 3 
 // How a kernel of an iteration is launched.  FLOW_STEP: as one iteration of its own.  The loop
 // graph advances many: rounds of FLOW_FAST iterations, in which the kernels follow one another
 // without a conditional node and leave at once when there is nothing to do (no iteration
-// left) or the iteration needs more than them (Ctrl::hold), and after each round, only
-// then, one FLOW_SLOW iteration with everything.
-enum LoopFlow { FLOW_STEP = 0, FLOW_FAST = 1, FLOW_SLOW = 2, FLOW_BEGIN = 3 };
-// Why the fast iterations wait: the next iteration starts with divisions or the cell limit,
-// or the running one's first attempt failed its error test.
+// left, or Ctrl::hold), and after each round, only where Ctrl::hold asks for it, what the fast
+// iterations wait for: the FLOW_SLOW rest of an iteration whose first attempt failed, or a
+// division.
+enum LoopFlow { FLOW_STEP = 0, FLOW_FAST = 1, FLOW_SLOW = 2 };
+// Ctrl::hold: the next iteration has to start with the division launch (a cell has reached
+// the division length, or the colony its limit); or the running one waits for its retries.
 enum LoopHold { HOLD_NONE = 0, HOLD_START = 1, HOLD_RETRY = 2 };
 
 // Step-size network: 32 features -> 64 -> 64 -> 1 (log dt ratio)
@@ -42,6 +43,15 @@ enum StatusBits {
     ST_CELL_OVERFLOW = 8,  // division would exceed cap_cells
     ST_BARRIER = 16,       // a grid barrier's bounded wait ran out
 };
+
+// Blocks of a launch whose blocks wait for one another: one cluster, or a cooperative grid
+struct LaunchShape {
+    int blocks = 1;
+    int cluster = 0;
+};
+// `threads` threads of work in blocks of `block`
+LaunchShape make_shape(const void* kernel, int block, long long threads, bool cluster, int num_sms);
+void launch_shape(const void* kernel, const LaunchShape& shape, int block, void** args, cudaStream_t st);
 
 // Record of a barrier over the blocks of a cooperative launch (abm_grid.cuh)
 struct GridBar {
@@ -67,10 +77,10 @@ struct Ctrl {
     int n_divide;               // mothers in the pending division
     long long attempts, retries, iterations, rebuilds, divisions;
     unsigned long long eval_err_bits;   // scaled max error of the last API attempt
-    // division bookkeeping (growth.hpp:166-426)
-    int div_count;              // running count of flagged / satisfied cells
-    unsigned int div_blocks;    // last-block counter of the division kernels
-    int div_done, div_tries, last_div_tries;
+    int n_pairs;                // pair records made so far by a running build
+    int n_sorted;               // cells placed so far by its counting sort
+    int n_divided;              // mothers of the last division launch
+    int last_div_tries;
     int n_parents;              // length of the lineage vector
     long long div_events;       // iterations in which cells divided
     // step-size features (filled when StepParams::stats_on)
@@ -128,19 +138,19 @@ struct Ctrl {
     int rounds;                         // rounds of the loop graph left (a bound)
 };
 
-// Nothing to do for a kernel of the loop graph?  `first`: it belongs to the part of the
-// iteration before a failed first attempt (already done when a slow iteration resumes one).
-__device__ __forceinline__ bool loop_idle(const Ctrl* c, int flow, bool first)
+// Nothing to do for a kernel of the loop graph?
+__device__ __forceinline__ bool loop_idle(const Ctrl* c, int flow)
 {
-    if (flow == FLOW_STEP) return false;
-    if (c->todo <= 0) return true;
-    return flow == FLOW_FAST ? c->hold != HOLD_NONE : (first && c->hold == HOLD_RETRY);
+    return flow != FLOW_STEP && (c->todo <= 0 || c->hold != (flow == FLOW_FAST ? HOLD_NONE : HOLD_RETRY));
 }
 
 struct Grid {
     double x0, y0, z0, edge, inv_edge;
     int nx, ny, nz, nbins;
     double max_half_l;
+    double reach;               // no two neighbors' centres are farther apart
+    float max_reach;            // largest segment_reach
+    float margin;               // of the FP32 distance tests on sorted positions
 };
 
 struct StepParams {
@@ -227,6 +237,7 @@ struct ActiveList {
     Geom* gref;                 // the cells at the last refresh
     const int* row_ptr;
     GridBar* bar;
+    int cluster;                // the pass's blocks are one cluster
 };
 const int ACT_ADHERE = (int)0x80000000;
 
@@ -262,23 +273,7 @@ void launch_cells_to_colmajor_2d(const Geom* geom, const Vel* vel, const Phys* p
 // 2-D dE/dq (n x 4) from the pair sums (F, S): torques projected with the current n
 void launch_pair_dEdq_2d(const Geom* geom, const Gen6* fcc, const Ctrl* ctrl, double* cm, int cap_cells,
                          cudaStream_t st);
-// to_adhere of every CSR entry (2D/include/simulation.hpp:242-258)
-void launch_adhere_flags(const Ctrl* ctrl, const int* row_ptr, const int* col, const Geom* geom, double R,
-                         double Rcell, unsigned char* adhere, int cap_cells, cudaStream_t st);
 void launch_gen6_to_colmajor(const Gen6* g, int n, double* cm, cudaStream_t st);
-
-void launch_bbox(const Geom* geom, Ctrl* ctrl, Grid* grid, unsigned long long* scratch8,
-                 unsigned int* counter, double edge, int cap_bins, int cap_cells, cudaStream_t st);
-void launch_bin_count(const Geom* geom, const Ctrl* ctrl, const Grid* grid, int* bin_count,
-                      int* key, int* slot, int cap_cells, cudaStream_t st);
-void launch_bin_scatter(const Geom* geom, const Ctrl* ctrl, const int* bin_start, const int* key,
-                        const int* slot, int* sorted_cell, Geom* sorted_geom, int cap_cells,
-                        cudaStream_t st);
-void launch_pair_build(const Grid* grid, const int* bin_start, const int* sorted_cell,
-                       const Geom* sorted_geom, const Ctrl* ctrl, BuildParams bp, int* scratch,
-                       int* count, int cap_bins, int num_sms, cudaStream_t st);
-void launch_csr_fill(const Ctrl* ctrl, const int* row_ptr, const int* scratch, int cap_per_cell,
-                     int* col, Ctrl* ctrl_w, int cap_cells, cudaStream_t st);
 
 // exclusive scan of len (device int) entries; out has len + 1 entries, out[len] = total
 void launch_scan(const int* in, const int* len, int* out, int* block_sums, int cap, cudaStream_t st);
@@ -293,19 +288,13 @@ void launch_pair_force(const Geom* geom, const int* row_ptr, const int* lower_en
 void launch_csr_rev(const Ctrl* ctrl, const int* row_ptr, const int* col, int* lower_end, int* rev,
                     int cap_cells, cudaStream_t st);
 // pass over the active pairs (both shares into jbuf), refreshing the active list when it is
-// stale; with_sum also writes each cell's total into fcc.
+// stale; with_sum also writes each cell's total into fcc.  cells: about how many there are
+// (the launch's shape; more only take longer).
 void launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, const double* jkr_delta,
                           const double* jkr_radius, Gen6* fcc, double4* jbuf, int mixed, int max_entries,
                           int cap_cells, int num_sms, cudaStream_t st, int with_sum, int dims, int tile,
-                          int blocks_per_sm, const int4* pairs, int* surv, ActiveList al,
+                          int blocks_per_sm, const int4* pairs, int* surv, ActiveList al, int cells,
                           const StepParams* sp = nullptr, const float* mlp_w = nullptr, int flow = FLOW_STEP);
-// the list of unordered pairs (i, j < i, lower entry k, partner entry rev[k]) after
-// k_csr_rev, cells in `order` (null: index order): counts -> scan -> fill; uses
-// `count` and `start` (cap_cells + 1) as scratch
-void launch_pair_list(const Ctrl* ctrl, const int* row_ptr, const int* lower_end, const int* col, const int* rev,
-                      int* count, int* start, int* block_sums, int4* pairs, int cap_cells, cudaStream_t st,
-                      const int* order = nullptr);
-
 // kind: MODE_TRIAL / MODE_RETRY / MODE_FINAL for the loop, 3 = evaluation for the API
 // (writes candidates and errors without touching the controller)
 // cond / use_cond: WHILE-node handle that the trial and retry attempts set to 1
@@ -339,7 +328,6 @@ void launch_attempt_4(int kind, const AttemptArgs& a, int dims, cudaStream_t st)
 void launch_attempt_6(int kind, const AttemptArgs& a, int dims, cudaStream_t st);
 void launch_attempt_7(int kind, const AttemptArgs& a, int dims, cudaStream_t st);
 // accepted proposal of the learned controller: candidate -> state (no-op otherwise)
-// the attempt order of the cells (3-D): full surface solve first (made at every rebuild)
 // one frame of the ring: the state after the accepted step that marked it
 struct FrameInfo {
     double t;
@@ -349,8 +337,6 @@ struct FrameInfo {
 void launch_frame_snapshot(const Geom* geom, const Vel* vel, const Phys* phys, Ctrl* ctrl, Geom* snap_geom,
                            Vel* snap_vel, Phys* snap_phys, FrameInfo* info, int slots, int cap_cells,
                            cudaStream_t st, const double* feta = nullptr, double* snap_feta = nullptr);
-void launch_attempt_order(const Geom* geom, Ctrl* ctrl, const MechParams& P, int* flag, int* pos,
-                          int* block_sums, int* order, int cap_cells, cudaStream_t st);
 void launch_velocities(const Geom* geom, const Vel* vel, const Phys* phys, const Gen6* fcc,
                        const Ctrl* ctrl, const StepParams& sp, Gen6* v_out, int cap_cells,
                        cudaStream_t st, int dims = 3);
@@ -372,7 +358,7 @@ void launch_mlp_train(float* master, float* m1, float* m2, float* G, const float
 const int AT_T = 128;           // threads of an attempt block, one cell each
 int attempt_blocks(int cap_cells);
 
-// division (growth.hpp:66-426), abm_divide.cu
+// division (growth.hpp:66-426), abm_divide.cuh
 struct DivideParams {
     double R, Rcell, Ldiv;
     double growth_mean, growth_std, daughter_length_std, angle_xy_bound, angle_z_bound;
@@ -387,29 +373,50 @@ struct DivideParams {
     double rates[4];
     double* feta;               // friction coefficient of each cell (daughters inherit it), or null
 };
-void launch_div_count(const Phys* phys, Ctrl* ctrl, const DivideParams& dp, int* flags,
-                      unsigned long long cond, int use_cond, cudaStream_t st, int flow = FLOW_STEP);
+// Neighbor set and division (abm_build.cu): one cooperative launch
+struct BuildArgs {
+    Geom* geom;
+    Vel* vel;
+    Phys* phys;
+    Ctrl* ctrl;
+    GridBar* bar;
+    int cluster;                            // the blocks are one cluster (else a cooperative grid)
+    // cell list
+    int* bbox;                              // 8 per block
+    int2* part;                             // per-block partial sums of the scans
+    int *bin_count, *bin_start, *key, *slot, *sorted_cell, *sorted_key;
+    float4 *sorted_pos, *sorted_dir;        // (r, reach) from the box's corner; (n, h)
+    int cap_bins, cap_cells;
+    // neighbor set
+    BuildParams bp;
+    MechParams mp;
+    int *scratch, *count, *row_ptr, *col, *lower_end;
+    int4* pairs;
+    int* order;                             // attempt order (3-D), or null
+    unsigned char* adhere;                  // to_adhere of every CSR entry (2-D adhesion), or null
+    // division
+    DivideParams dp;
+    int *flags, *mothers, *check, *sat, *ok;
+    Geom *d1, *d2;
+    double *dlen, *dgrowth;
+    int* parents;
+};
+enum BuildWhat { BUILD_NEIGHBORS, BUILD_GROWTH, BUILD_DIVIDE, BUILD_RECORDS };
+const int BUILD_CLUSTER_CELLS = 8192;
+LaunchShape build_shape(int cells, int num_sms);
+void launch_build(const BuildArgs& args, int what, const LaunchShape& shape, cudaStream_t st, int flow = FLOW_STEP);
+
 // the loop graph: `todo` iterations ahead (of each of n contexts); then, once per round,
 // whether a slow iteration runs and whether another round follows
-void launch_loop_begin(Ctrl* ctrl, int todo, cudaStream_t st);
-void launch_loop_begin_all(Ctrl* const* ctrls, int n, int todo, cudaStream_t st);
+// (divides: the first iteration starts with a look for mothers and the cell limit)
+void launch_loop_begin(Ctrl* ctrl, int divides, int todo, cudaStream_t st);
+void launch_loop_begin_all(Ctrl* const* ctrls, const int* divides, int n, int todo, cudaStream_t st);
+// a slow iteration starts: its first retry is pending (a handle's default value holds for
+// the first pass through its graph only)
+void launch_retry_begin(Ctrl* ctrl, unsigned long long cond, cudaStream_t st);
 void launch_loop_round(Ctrl* ctrl, unsigned long long cond_slow, unsigned long long cond_loop, cudaStream_t st);
 void launch_div_body_pre(Ctrl* ctrl, const int* flags, const int* rank, int* mothers, int cap_cells,
                          cudaStream_t st);
-// room checks and the first try; use_cond: `cond` is set while a further try is needed
-void launch_div_first(const Geom* geom, const Phys* phys, Ctrl* ctrl, const DivideParams& dp, const Grid* grid,
-                      const int* bin_start, const int* sorted_cell, const Geom* sorted_geom, const int* flags,
-                      const int* mothers, int* check, int* sat, Geom* d1, Geom* d2, double* dlen, double* dgrowth,
-                      int* ok, unsigned long long cond, int use_cond, cudaStream_t st);
-void launch_div_try_round(const Geom* geom, const Phys* phys, Ctrl* ctrl, const DivideParams& dp, const Grid* grid,
-                          const int* bin_start, const int* sorted_cell, const Geom* sorted_geom, const int* flags,
-                          const int* mothers, const int* check, int* sat, Geom* d1, Geom* d2, double* dlen,
-                          double* dgrowth, int* ok, int tr, unsigned long long cond, int use_cond, cudaStream_t st);
-int max_division_tries();
-void launch_div_commit(Geom* geom, Vel* vel, Phys* phys, Ctrl* ctrl, const DivideParams& dp, const int* mothers,
-                       const Geom* d1, const Geom* d2, const double* dlen, const double* dgrowth, int* parents,
-                       cudaStream_t st);
-
 // Phenotype switching between two groups and what it drives, after each accepted step
 // (abm_switch.cu): Markov switching (switch.hpp:45-95), the attribute and gamma ramps
 // (simulation.hpp:1872-1957), local viscosity (simulation.hpp:1958-2020) and basal-only
