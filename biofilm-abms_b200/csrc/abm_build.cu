@@ -332,27 +332,6 @@ __device__ __forceinline__ void exact_pair(const BuildArgs& a, int p, int q)
     }
 }
 
-// Can two segments be nearer than `limit`?  may_touch in FP32: the gap between their
-// projections on the direction of the FP32 closest points bounds their distance from below
-// for any direction; a = (n, h) of each, w from the first centre to the second.  limit holds
-// a margin for the rounding (1e-5 of the lengths that enter, some 20 FP32 roundings).
-__device__ __forceinline__ bool near_f(const float4& a, const float4& b, float wx, float wy, float wz, float limit)
-{
-    const float B = a.x * b.x + a.y * b.y + a.z * b.z;
-    const float D = a.x * wx + a.y * wy + a.z * wz, E = b.x * wx + b.y * wy + b.z * wz;
-    const float den = 1.f - B * B;
-    float s = den > 1e-6f ? __fdividef(D - B * E, den) : 0.f;
-    s = fminf(fmaxf(s, -a.w), a.w);
-    const float t = fminf(fmaxf(B * s - E, -b.w), b.w);
-    s = fminf(fmaxf(B * t + D, -a.w), a.w);
-    const float dx = wx + t * b.x - s * a.x, dy = wy + t * b.y - s * a.y, dz = wz + t * b.z - s * a.z;
-    const float d2 = dx * dx + dy * dy + dz * dz;
-    if (!(d2 > 1e-6f)) return true;
-    const float gap = (dx * wx + dy * wy + dz * wz) - a.w * fabsf(dx * a.x + dy * a.y + dz * a.z)
-                      - b.w * fabsf(dx * b.x + dy * b.y + dz * b.z);
-    return !(gap > limit * sqrtf(d2));
-}
-
 // A cell's row `r` of the half neighborhood: its own row first, then the rows after it
 __device__ __forceinline__ void half_row(int r, int rings, int& dy, int& dz)
 {

@@ -991,7 +991,7 @@ static void enqueue_growth(abm_ctx* c, int flow = FLOW_STEP) { enqueue_build(c, 
 // step-size features (and, learned, the proposed dt)
 static void enqueue_pair_force(abm_ctx* c, int with_gather, bool in_loop = false, int flow = FLOW_STEP)
 {
-    ActiveList al = {c->act, c->n_act, c->keep_entry, c->gref, c->row_ptr, c->bar, 0};
+    ActiveList al = {c->act, c->n_act, c->keep_entry, c->gref, c->row_ptr, c->bar, 0, nullptr};
     launch_pair_screened(c->geom, c->ctrl, c->fp, c->jkr_delta, c->jkr_radius, c->fcc, c->jbuf,
                          c->p.precision == ABM_PRECISION_MIXED, c->cap * c->cap_nbr, c->cap, c->num_sms, c->st,
                          with_gather, c->dims, c->p.pair_tile, c->p.pair_blocks_per_sm, c->pairs, c->surv, al, c->n_ref,
@@ -1033,12 +1033,22 @@ static void enqueue_attempt(abm_ctx* c, int kind, const AttemptArgs& a)
     launch_attempt(kind, a, c->dims, c->st);
 }
 
-// one velocity-Verlet step (integration mode 0) at the context's dt, growth included
+// one velocity-Verlet step (integration mode 0) at the context's dt, growth included: pair
+// shares and cells at the current state, then at the drifted one
 static void enqueue_verlet_step(abm_ctx* c)
 {
-    launch_verlet_step(c->geom, c->vel, c->phys, c->geom_c, c->vel_c, c->whalf, c->ctrl, c->sp, c->fp,
-                       c->jkr_delta, c->jkr_radius, c->pairs, c->row_ptr, c->lower_end, c->jbuf, c->pbuf, c->rho,
-                       c->cap, c->cap * c->cap_nbr / 2, c->st);
+    const VerletArgs a = {c->geom, c->vel, c->geom_c, c->vel_c, c->phys, c->whalf, c->row_ptr, c->n_act, c->jbuf,
+                          c->pbuf, c->gref, c->rho};
+    const ActiveList al = {c->act, c->n_act, c->keep_entry, c->gref, c->row_ptr, c->bar, 0, c->pbuf};
+    for (int phase = 0; phase < 2; ++phase)
+    {
+        ForceParams fp = c->fp;
+        fp.vel = phase == 0 ? c->vel : c->vel_c;
+        launch_pair_screened(phase == 0 ? c->geom : c->geom_c, c->ctrl, fp, c->jkr_delta, c->jkr_radius, c->fcc, c->jbuf,
+                             0, c->cap * c->cap_nbr, c->cap, c->num_sms, c->st, 0, c->dims, c->p.pair_tile,
+                             c->p.pair_blocks_per_sm, c->pairs, c->surv, al, c->n_ref);
+        launch_verlet_cells(phase, a, c->ctrl, c->sp, c->cap, c->st);
+    }
 }
 
 static void enqueue_attempts(abm_ctx* c)

@@ -72,6 +72,27 @@ __device__ __forceinline__ bool may_touch(const Geom& a, const Geom& b, double l
     return !(gap > (limit + 1e-9) * dn);
 }
 
+// Can two segments be nearer than `limit`?  may_touch in FP32: the gap between their
+// projections on the direction of the FP32 closest points bounds their distance from below
+// for any direction; a = (n, h) of each, w from the first centre to the second.  limit holds
+// a margin for the rounding (1e-5 of the lengths that enter, some 20 FP32 roundings).
+__device__ __forceinline__ bool near_f(const float4& a, const float4& b, float wx, float wy, float wz, float limit)
+{
+    const float B = a.x * b.x + a.y * b.y + a.z * b.z;
+    const float D = a.x * wx + a.y * wy + a.z * wz, E = b.x * wx + b.y * wy + b.z * wz;
+    const float den = 1.f - B * B;
+    float s = den > 1e-6f ? __fdividef(D - B * E, den) : 0.f;
+    s = fminf(fmaxf(s, -a.w), a.w);
+    const float t = fminf(fmaxf(B * s - E, -b.w), b.w);
+    s = fminf(fmaxf(B * t + D, -a.w), a.w);
+    const float dx = wx + t * b.x - s * a.x, dy = wy + t * b.y - s * a.y, dz = wz + t * b.z - s * a.z;
+    const float d2 = dx * dx + dy * dy + dz * dz;
+    if (!(d2 > 1e-6f)) return true;
+    const float gap = (dx * wx + dy * wy + dz * wz) - a.w * fabsf(dx * a.x + dy * a.y + dz * a.z)
+                      - b.w * fabsf(dx * b.x + dy * b.y + dz * b.z);
+    return !(gap > limit * sqrtf(d2));
+}
+
 // How far a segment reaches from its centre, in FP32: every computed distance vector joins
 // points r1 + s n1 and r2 + t n2 with |s| <= h1, |t| <= h2, so |d| >= |r2 - r1| less both
 // reaches, up to rounding.
@@ -405,58 +426,6 @@ __device__ __forceinline__ double std_normal(double u, double v)
     return __dmul_rn(__dsqrt_rn(__dmul_rn(-2.0, det_log(u))), c);
 }
 
-// ---------------------------------------------------------------------------
-// Surface integrals (integrals.hpp) with the overlap powers taken from one
-// square root per end: p^{k/2} = p^{floor(k/2)} (sqrt p)^{k mod 2}.
-// ---------------------------------------------------------------------------
-struct EndPow {               // end overlaps phi(-h) (p) and phi(+h) (q) and their roots
-    double p, q, sp, sq;
-};
-
-// p^(e/2) for e = 1..7 (e = 2 (gamma + 1))
-__device__ __forceinline__ double half_pow(double x, double sx, int e)
-{
-    double r = (e & 1) ? sx : 1.0;
-    for (int k = 0; k < (e >> 1); ++k) r *= x;
-    return r;
-}
-__device__ __forceinline__ double epw(const EndPow& w, int e, bool second)
-{
-    return second ? half_pow(w.q, w.sq, e) : half_pow(w.p, w.sp, e);
-}
-
-// integrals.hpp:116-140 (integral1) with gamma + 1 = e / 2; the division by
-// nz (gamma + 1) is a multiplication by inz = 1 / nz and the constant 2 / e
-__device__ __forceinline__ double integral1(const EndPow& w, double inz, double h, int e, double ss)
-{
-    const double ig1 = 2.0 / e;
-    if (ss > h) return (epw(w, e, false) - epw(w, e, true)) * inz * ig1;
-    else if (ss > -h) return epw(w, e, false) * inz * ig1;
-    return 0.0;
-}
-
-// integrals.hpp:159-184 (integral2) with gamma + 1 = e / 2
-__device__ __forceinline__ double integral2(const EndPow& w, double inz, double h, int e, double ss)
-{
-    double term1 = integral1(w, inz, h, e + 2, ss);
-    double term2 = 0.0;
-    if (ss > h) term2 = -h * (epw(w, e, false) + epw(w, e, true));
-    else if (ss > -h) term2 = -h * epw(w, e, false);
-    return (term1 + term2) * inz * (2.0 / e);
-}
-
-// The end overlaps that integral1/2 and areaIntegrals read (integrals.hpp:56-60,
-// 431-441): both ends when ss > h, the lower end when -h < ss <= h.
-__device__ __forceinline__ EndPow end_pows(double rz, double nz, double R, double h, double ss)
-{
-    EndPow w;
-    w.p = 0.0; w.q = 0.0;
-    if (ss > h) { w.p = R - rz - (-h) * nz; w.q = R - rz - h * nz; }
-    else if (ss > -h) { w.p = R - rz - (-h) * nz; }
-    w.sp = sqrt(w.p); w.sq = sqrt(w.q);
-    return w;
-}
-
 struct MechParams {
     double R, Rcell, E0, Ecell;
     double sqrtR;
@@ -477,31 +446,6 @@ __device__ __forceinline__ void surface_dEdq_flat(const MechParams& P, double rz
         rep2 = -(2 * P.E0) * ph * l;
         adh2 = sigma0 * (P.sqrtR / 2) * l / sqrt(ph);
     }
-}
-
-// integrals.hpp:400-463 (areaIntegrals)
-__device__ __forceinline__ void area_integrals(const MechParams& P, double nz, double h, double ss,
-                                               const EndPow& w, double& A1, double& A2, double& A3)
-{
-    const double R = P.R;
-    double int4 = (ss > h) ? 2 * h : ((ss > -h) ? ss + h : 0.0);
-    double int5 = (-h < ss && ss <= h) ? (ss * ss - h * h) / 2.0 : 0.0;
-    double int6 = (ss > h) ? 2 * h * h * h / 3.0 : ((ss > -h) ? (ss * ss * ss + h * h * h) / 3.0 : 0.0);
-    const double inz = 1.0 / nz;
-    double int1a = integral1(w, inz, h, 3, ss);
-    double int1b = integral1(w, inz, h, 5, ss);
-    double int1c = integral1(w, inz, h, 7, ss);
-    double onz = 1 - nz * nz;
-    double piRnz2 = M_PI * R * nz * nz;
-    A1 = P.sqrtR * onz * int1a + piRnz2 * int4;
-    const double p3 = epw(w, 3, false), q3 = epw(w, 3, true);
-    double term2 = -h * (p3 + q3);
-    double int2a = (int1b + term2) * inz * (1.0 / 1.5);
-    A2 = P.sqrtR * onz * int2a + piRnz2 * int5;
-    term2 = -h * (epw(w, 5, false) + epw(w, 5, true));
-    double int2b = (int1c + term2) * inz * (1.0 / 2.5);
-    double int3 = (2 * int2b + h * h * (p3 - q3)) * inz * (1.0 / 1.5);
-    A3 = P.sqrtR * onz * int3 + piRnz2 * int6;
 }
 
 // Does a cell touch the surface (mechanics.hpp:2080-2090)?

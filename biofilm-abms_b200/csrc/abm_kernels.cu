@@ -5,7 +5,6 @@
 //                  mechanics.hpp:1209-1659; one record per unordered pair, screened
 //                  against an active list with a skin, both shares per pair; the last
 //                  block makes the step-size proposal of the learned controller)
-//                  k_pair_force<G> serves the no-alloc entry point (G lanes per cell)
 //   RK attempt     abm_attempt.cuh
 #include <cstdio>
 #include "abm_grid.cuh"
@@ -244,51 +243,6 @@ void launch_scan(const int* in, const int* len, int* out, int* block_sums, int c
     k_scan_final<<<nb, SCAN_T, 0, st>>>(in, len, block_sums, out, nb);
 }
 
-const int CF_T = 256;
-
-// ---------------------------------------------------------------------------
-// Pair force: G lanes per cell walk its CSR row; each lane evaluates the
-// distance (larger index as cell 1) and the Hertz / JKR + hard-core magnitude
-// of mechanics.hpp:1390-1659 (or :1209-1350 without adhesion), accumulates the
-// cell's share of dE/dq, and the G partial sums are combined by xor shuffles.
-// ---------------------------------------------------------------------------
-// FP32 variant: segment distance (FP64 near-parallel branch kept), overlap,
-// Hertz / JKR magnitude and direction in single precision
-__device__ __forceinline__ PairOut pair_force_fp32(const Geom& gi, const Geom& gj, const ForceParams& fp,
-                                                   const double* td, const double* tr, int rounding)
-{
-    PairOut out;
-    out.touch = false;
-    Dist d = dist_geom_mixed(gi, gj, rounding);
-    // the overlap from the FP64 distance vector, then the force law in FP32
-    const double distd = sqrt((d.dx * d.dx + d.dy * d.dy) + d.dz * d.dz);
-    const double overlap_d = 2 * fp.R - distd;
-    if (!(overlap_d > 0)) return out;
-    float dx = (float)d.dx, dy = (float)d.dy, dz = (float)d.dz;
-    const float dist = (float)distd;
-    const float R = (float)fp.R, max_overlap = (float)fp.max_overlap;
-    float overlap = (float)overlap_d;
-    float inv = 1.f / dist;
-    float m;
-    const double gamma = fp.adhesion ? fmin(gi.gamma, gj.gamma) : 0.0;
-    if (fp.adhesion && gamma > 0)
-    {
-        // the JKR magnitude term1 - term2 cancels near the force balance, where most
-        // adhering contacts sit: it keeps FP64 (table lookup included)
-        m = (float)(fp.jkr_ng ? jkr_magnitude_variable(distd, gamma, fp, td) : jkr_magnitude(distd, gamma, fp, td, tr));
-    }
-    else if (overlap <= max_overlap) m = (float)fp.pf0 * overlap * sqrtf(overlap);
-    else
-    {
-        m = (float)fp.pf2;
-        if (!fp.adhesion) { float e = overlap - max_overlap; m += (float)fp.pf1 * e * sqrtf(e); }
-    }
-    if (fp.adhesion && overlap > max_overlap) { float e = overlap - max_overlap; m += (float)fp.pf1 * e * sqrtf(e); }
-    out.vx = (double)(m * dx * inv); out.vy = (double)(m * dy * inv); out.vz = (double)(m * dz * inv);
-    out.s = d.s; out.t = d.t; out.ovl = overlap; out.touch = true;
-    return out;
-}
-
 // 2-D pair (2D/include/mechanics.hpp:448-547 and :572-670 with
 // 2D/include/adhesion.hpp:403-448).  Returns p = cell i's translational dE/dq of the
 // pair (Hertz v_ij minus strength * the JKR vector); i's torque share is s p and
@@ -317,158 +271,6 @@ __device__ __forceinline__ PairOut pair_force_2d(const Geom& gi, const Geom& gj,
     out.vx = px; out.vy = py; out.vz = 0.0;
     out.s = d.s; out.t = d.t; out.ovl = overlap; out.touch = true;
     return out;
-}
-
-const int PF_T = 256, JKR_MAX = 512;
-
-// Pass 1: G lanes per cell i walk the lower part of its sorted CSR row (j < i),
-// evaluate each unordered pair once, keep i's share and write j's share
-// (v, t) into the slot of i in row j (rev[k]).
-template <int G, bool MIXED, int DIM>
-__global__ void __launch_bounds__(PF_T) k_pair_force(const Geom* __restrict__ geom, const int* __restrict__ row_ptr,
-                                                    const int* __restrict__ lower_end, const int* __restrict__ col,
-                                                    const int* __restrict__ rev, Ctrl* ctrl, ForceParams fp,
-                                                    const double* __restrict__ jkr_delta,
-                                                    const double* __restrict__ jkr_radius, Gen6* fcc,
-                                                    double4* __restrict__ jbuf)
-{
-    __shared__ double td[JKR_MAX], tr[JKR_MAX];
-    if (ctrl->halted) return;
-    for (int k = threadIdx.x; k < fp.jkr_n; k += blockDim.x) { td[k] = jkr_delta[k]; tr[k] = jkr_radius[k]; }
-    __syncthreads();
-    const int n = ctrl->n;
-    const int lane = threadIdx.x & (G - 1);
-    const unsigned gmask = (G == 32) ? 0xffffffffu
-                                     : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
-    const int groups_per_grid = gridDim.x * (blockDim.x / G);
-    double ovl_max = 0.0;
-    for (int cell = (blockIdx.x * blockDim.x + threadIdx.x) / G; cell < n; cell += groups_per_grid)
-    {
-        const Geom gc = load_geom(geom, cell);
-        double acc[6] = {0, 0, 0, 0, 0, 0};
-        const int r0 = row_ptr[cell], r1 = lower_end[cell];
-        for (int k = r0 + lane; k < r1; k += G)
-        {
-            const int o = col[k];
-            const Geom go = load_geom(geom, o);
-            PairOut p;
-            if (DIM == 2) p = pair_force_2d(gc, go, fp, fp.adhere[k] != 0);
-            else p = MIXED ? pair_force_fp32(gc, go, fp, td, tr, ROUND_ROW) : pair_force_fp64(gc, go, fp, td, tr);
-            double4 js = make_double4(0.0, 0.0, 0.0, 0.0);
-            if (p.touch)
-            {
-                acc[0] += p.vx; acc[1] += p.vy; acc[2] += p.vz;
-                acc[3] += p.s * p.vx; acc[4] += p.s * p.vy; acc[5] += p.s * p.vz;
-                js = make_double4(p.vx, p.vy, p.vz, p.t);
-                ovl_max = fmax(ovl_max, p.ovl);
-            }
-            jbuf[rev[k]] = js;
-        }
-#pragma unroll
-        for (int off = G / 2; off > 0; off >>= 1)
-#pragma unroll
-            for (int c = 0; c < 6; ++c) acc[c] += __shfl_xor_sync(gmask, acc[c], off, G);
-        if (lane == 0)
-        {
-            Gen6 out;
-            for (int c = 0; c < 6; ++c) out.f[c] = acc[c];
-            fcc[cell] = out;
-        }
-    }
-    if (fp.stats)
-    {
-        ovl_max = warp_max(ovl_max);
-        if ((threadIdx.x & 31) == 0 && ovl_max > 0)
-            atomicMax(&ctrl->st_ovl_bits[ctrl->iter & 1], (unsigned long long)__double_as_longlong(ovl_max));
-    }
-}
-
-// Pass 2: each cell j adds the shares its higher-index neighbors left in the
-// upper part of its row: (-v, -t v).
-template <int G>
-__global__ void __launch_bounds__(PF_T) k_pair_gather(const int* __restrict__ row_ptr, const int* __restrict__ lower_end,
-                                                     const Ctrl* ctrl, const double4* __restrict__ jbuf, Gen6* fcc)
-{
-    const int n = ctrl->n;
-    const int lane = threadIdx.x & (G - 1);
-    const unsigned gmask = (G == 32) ? 0xffffffffu
-                                     : (((1u << G) - 1u) << ((threadIdx.x & 31) & ~(G - 1)));
-    const int groups_per_grid = gridDim.x * (blockDim.x / G);
-    for (int cell = (blockIdx.x * blockDim.x + threadIdx.x) / G; cell < n; cell += groups_per_grid)
-    {
-        double acc[6] = {0, 0, 0, 0, 0, 0};
-        for (int k = lower_end[cell] + lane; k < row_ptr[cell + 1]; k += G)
-        {
-            double4 js = jbuf[k];
-            acc[0] -= js.x; acc[1] -= js.y; acc[2] -= js.z;
-            acc[3] -= js.w * js.x; acc[4] -= js.w * js.y; acc[5] -= js.w * js.z;
-        }
-#pragma unroll
-        for (int off = G / 2; off > 0; off >>= 1)
-#pragma unroll
-            for (int c = 0; c < 6; ++c) acc[c] += __shfl_xor_sync(gmask, acc[c], off, G);
-        if (lane == 0)
-        {
-            Gen6 f = fcc[cell];
-            for (int c = 0; c < 6; ++c) f.f[c] += acc[c];
-            fcc[cell] = f;
-        }
-    }
-}
-
-void launch_pair_force(const Geom* geom, const int* row_ptr, const int* lower_end, const int* col, const int* rev,
-                       Ctrl* ctrl, ForceParams fp, const double* jkr_delta, const double* jkr_radius,
-                       Gen6* fcc, double4* jbuf, int lanes, int mixed, int cap_cells, cudaStream_t st,
-                       int with_gather, int dims)
-{
-    int blocks = max(cdiv((long long)cap_cells * lanes, PF_T), 1);
-#define PF_CASE(G) \
-    if (lanes == G) { \
-        if (dims == 2) k_pair_force<G, false, 2><<<blocks, PF_T, 0, st>>>(geom, row_ptr, lower_end, col, rev, ctrl, fp, jkr_delta, jkr_radius, fcc, jbuf); \
-        else if (mixed) k_pair_force<G, true, 3><<<blocks, PF_T, 0, st>>>(geom, row_ptr, lower_end, col, rev, ctrl, fp, jkr_delta, jkr_radius, fcc, jbuf); \
-        else k_pair_force<G, false, 3><<<blocks, PF_T, 0, st>>>(geom, row_ptr, lower_end, col, rev, ctrl, fp, jkr_delta, jkr_radius, fcc, jbuf); \
-        if (with_gather) k_pair_gather<G><<<blocks, PF_T, 0, st>>>(row_ptr, lower_end, ctrl, jbuf, fcc); \
-        return; }
-    PF_CASE(4) PF_CASE(8) PF_CASE(16) PF_CASE(32)
-#undef PF_CASE
-}
-
-// Reverse slots and the end of the lower part of each sorted CSR row: for an
-// entry (i, j) with j < i, rev = position of i in row j.
-// Reverse indices and the lower part of each row, one warp per row: lower_end[i]
-// is the first entry with j >= i (rows are sorted), and every lower entry (i, j)
-// finds the position of i in row j by binary search.
-__global__ void __launch_bounds__(CF_T) k_csr_rev(const Ctrl* ctrl, const int* __restrict__ row_ptr,
-                                                 const int* __restrict__ col, int* lower_end, int* rev)
-{
-    const int n = ctrl->n;
-    const int lane = threadIdx.x & 31;
-    const int nwarps = gridDim.x * (CF_T / 32);
-    for (int i = (blockIdx.x * CF_T + threadIdx.x) >> 5; i < n; i += nwarps)
-    {
-        const int r0 = row_ptr[i], r1 = row_ptr[i + 1];
-        int lower = 0;
-        for (int k0 = r0; k0 < r1; k0 += 32)
-        {
-            const int k = k0 + lane;
-            const int j = k < r1 ? col[k] : INT_MAX;
-            const bool lo = j < i;
-            lower += __popc(__ballot_sync(0xffffffffu, lo));
-            if (lo)
-            {
-                int a = row_ptr[j], b = row_ptr[j + 1];
-                while (a < b) { const int mid = (a + b) >> 1; if (col[mid] < i) a = mid + 1; else b = mid; }
-                rev[k] = a;
-            }
-        }
-        if (lane == 0) lower_end[i] = r0 + lower;
-    }
-}
-
-void launch_csr_rev(const Ctrl* ctrl, const int* row_ptr, const int* col, int* lower_end, int* rev,
-                    int cap_cells, cudaStream_t st)
-{
-    k_csr_rev<<<max(cdiv(cap_cells, CF_T / 32), 1), CF_T, 0, st>>>(ctrl, row_ptr, col, lower_end, rev);
 }
 
 // ---------------------------------------------------------------------------
@@ -595,6 +397,50 @@ __device__ __forceinline__ void pair_shares(const Geom& gi, const Geom& gj, cons
     }
 }
 
+// The velocity-Verlet share of one active pair: the pair force v with the body coordinate
+// (jbuf) and its JKR part (pbuf, mechanics.hpp:1209-1659 and adhesion.hpp:282-526 with
+// include_constraint), friction (mechanics.hpp:1031-1175) from the state's own velocities
+// and contact points; the partner's with the minus sign.
+__device__ __forceinline__ void verlet_shares(const Geom& gi, const Geom& gj, const int4& pr, const ForceParams& fp,
+                                              const double* __restrict__ td, const double* __restrict__ tr,
+                                              double4* __restrict__ jbuf, double4* __restrict__ pbuf)
+{
+    const PairOut p = pair_force_fp64(gi, gj, fp, td, tr);
+    double4 own = make_double4(0.0, 0.0, 0.0, 0.0), part = own;
+    double t = 0.0;
+    if (p.touch)
+    {
+        own = make_double4(p.vx, p.vy, p.vz, p.s);
+        t = p.t;
+        const double ux = p.dx / p.dist, uy = p.dy / p.dist, uz = p.dz / p.dist;
+        part = make_double4(p.mj * ux, p.mj * uy, p.mj * uz, 0.0);
+        if (fp.fric)
+        {
+            const X3 dv = x3(p.dx, p.dy, p.dz);
+            const Vel ui = fp.vel[pr.x], uj = fp.vel[pr.y];
+            const double eta = fmin(fp.feta[pr.x], fp.feta[pr.y]);
+            double rv[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                rv[c] = (ui.v[c] + p.s * ui.v[3 + c]) - (uj.v[c] + p.t * uj.v[3 + c]);
+            bool flat = false;
+            if (fp.surface && fabs(__ddiv_rn(p.dz, p.dist)) < 1e-3)
+            {
+                const double lim = 1.01 * fp.R;
+                flat = __dadd_rn(gi.rz, __dmul_rn(p.s, gi.nz)) < lim &&
+                       __dadd_rn(gj.rz, __dmul_rn(p.t, gj.nz)) < lim;
+            }
+            double f[3];
+            friction_force(dv, p.dist, flat, rv, eta, fp, f);
+            own.x -= f[0]; own.y -= f[1]; own.z -= f[2];
+        }
+    }
+    jbuf[pr.z] = own;
+    jbuf[pr.w] = make_double4(-own.x, -own.y, -own.z, t);
+    pbuf[pr.z] = part;
+    pbuf[pr.w] = make_double4(-part.x, -part.y, -part.z, 0.0);
+}
+
 // With PROPOSE the pass also makes the iteration's step-size proposal
 // (mlp_propose_block). Its features read the previous iteration's overlap maximum
 // (st_ovl_bits of the other parity, which no block of this pass writes), so the
@@ -605,7 +451,7 @@ __device__ __forceinline__ void pair_shares(const Geom& gi, const Geom& gj, cons
 // template parameter so that the passes without it carry none of its code, and the
 // bound of two resident blocks per SM (at most 128 registers) holds the pair loop's
 // occupancy whatever the proposal adds.
-template <bool MIXED, int DIM, bool PROPOSE>
+template <bool MIXED, int DIM, bool PROPOSE, bool VERLET = false>
 __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ geom, const int4* __restrict__ pairs,
                                                       Ctrl* ctrl, ForceParams fp, const double* __restrict__ td,
                                                       const double* __restrict__ tr, double4* __restrict__ jbuf,
@@ -676,8 +522,11 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
             const bool adhere = DIM == 2 && fp.adhere[pr.z] != 0;
             al.act[q] = make_int4(rec.x, adhere ? rec.y | ACT_ADHERE : rec.y, rec.z, rec.w);
             bool cand = false;
-            pair_shares<MIXED, DIM>(load_geom(geom, rec.x), load_geom(geom, rec.y), rec, adhere, fp, td, tr, jbuf,
-                                    ovl_max, cand, rounding);
+            if constexpr (VERLET)
+                verlet_shares(load_geom(geom, rec.x), load_geom(geom, rec.y), rec, fp, td, tr, jbuf, al.pbuf);
+            else
+                pair_shares<MIXED, DIM>(load_geom(geom, rec.x), load_geom(geom, rec.y), rec, adhere, fp, td, tr, jbuf,
+                                        ovl_max, cand, rounding);
             if (cand) fp.fr_list[atomicAdd(&ctrl->fr_ncand_next, 1)] = q;
         }
     }
@@ -690,8 +539,11 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
             const bool adhere = DIM == 2 && rec.y < 0;
             if (DIM == 2) rec.y &= ~ACT_ADHERE;
             bool cand = false;
-            pair_shares<MIXED, DIM>(load_geom(geom, rec.x), load_geom(geom, rec.y), rec, adhere, fp, td, tr, jbuf,
-                                    ovl_max, cand, rounding);
+            if constexpr (VERLET)
+                verlet_shares(load_geom(geom, rec.x), load_geom(geom, rec.y), rec, fp, td, tr, jbuf, al.pbuf);
+            else
+                pair_shares<MIXED, DIM>(load_geom(geom, rec.x), load_geom(geom, rec.y), rec, adhere, fp, td, tr, jbuf,
+                                        ovl_max, cand, rounding);
             if (cand) fp.fr_list[atomicAdd(&ctrl->fr_ncand_next, 1)] = q;
         }
     }
@@ -720,7 +572,7 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
             ctrl->drift = 0.0;
         }
         if (MIXED && rounding == ROUND_STALE) ctrl->path = 0.0;
-        if (fp.fric)
+        if (fp.fric && !VERLET)
         {
             // the candidates of this pass; no stage has a changed decision yet
             ctrl->fr_ncand = atomicAdd(&ctrl->fr_ncand_next, 0);
@@ -810,7 +662,7 @@ void launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, const do
     const void* const fn2[2] = {(const void*)k_pair_pass<false, 2, false>, (const void*)k_pair_pass<false, 2, true>};
     const void* const fn3m[2] = {(const void*)k_pair_pass<true, 3, false>, (const void*)k_pair_pass<true, 3, true>};
     const void* const fn3[2] = {(const void*)k_pair_pass<false, 3, false>, (const void*)k_pair_pass<false, 3, true>};
-    const void* fn = dims == 2 ? fn2[p] : f32 ? fn3m[p] : fn3[p];
+    const void* fn = al.pbuf ? (const void*)k_pair_pass<false, 3, false, true> : dims == 2 ? fn2[p] : f32 ? fn3m[p] : fn3[p];
     // The blocks stride over the pairs; those of a refresh wait for one another, so the launch
     // is one cluster for a small colony (the rule of the build launch), else a cooperative
     // grid.  By default two threads per cell (1.5 to 2 active pairs a cell): blocks without work

@@ -238,6 +238,7 @@ struct ActiveList {
     const int* row_ptr;
     GridBar* bar;
     int cluster;                // the pass's blocks are one cluster
+    double4* pbuf;              // velocity Verlet: the JKR part of each share (else null)
 };
 const int ACT_ADHERE = (int)0x80000000;
 
@@ -279,14 +280,6 @@ void launch_gen6_to_colmajor(const Gen6* g, int n, double* cm, cudaStream_t st);
 void launch_scan(const int* in, const int* len, int* out, int* block_sums, int cap, cudaStream_t st);
 size_t scan_block_sums_size(int cap);
 
-// two passes: each unordered pair once from the row of its larger index, then the
-// partner's share gathered from the reverse slots (jbuf, one double4 per CSR entry)
-void launch_pair_force(const Geom* geom, const int* row_ptr, const int* lower_end, const int* col, const int* rev,
-                       Ctrl* ctrl, ForceParams fp, const double* jkr_delta, const double* jkr_radius,
-                       Gen6* fcc, double4* jbuf, int lanes, int mixed, int cap_cells, cudaStream_t st,
-                       int with_gather = 1, int dims = 3);
-void launch_csr_rev(const Ctrl* ctrl, const int* row_ptr, const int* col, int* lower_end, int* rev,
-                    int cap_cells, cudaStream_t st);
 // pass over the active pairs (both shares into jbuf), refreshing the active list when it is
 // stale; with_sum also writes each cell's total into fcc.  cells: about how many there are
 // (the launch's shape; more only take longer).
@@ -454,11 +447,25 @@ void launch_basal_compact(Geom* geom, Vel* vel, Phys* phys, Geom* geom_tmp, Vel*
                           double* feta = nullptr, double* feta_tmp = nullptr);
 void launch_periodic_rebuild_cond(const Ctrl* ctrl, int every, unsigned long long cond, cudaStream_t st);
 
-// velocity Verlet (abm_verlet.cu): one step of integration mode 0 at ctrl->dt, growth included
-void launch_verlet_step(Geom* geom, Vel* vel, Phys* phys, Geom* geom_c, Vel* vel_c, double4* whalf, Ctrl* ctrl,
-                        const StepParams& sp, const ForceParams& fp, const double* td, const double* tr,
-                        const int4* pairs, const int* row_ptr, const int* lower_end, double4* jbuf, double4* pbuf,
-                        double rho, int cap_cells, int cap_pairs, cudaStream_t st);
+// velocity Verlet (abm_verlet.cu): the cells' part of one step of integration mode 0 at
+// ctrl->dt; phase 0 after the pair pass at the current state (half kick, drift to geom_c /
+// vel_c), phase 1 after the pass at the drifted state (kick, growth, bookkeeping)
+struct VerletArgs {
+    Geom* geom;
+    Vel* vel;
+    Geom* geom_c;
+    Vel* vel_c;
+    Phys* phys;
+    double4* whalf;          // half-step angular velocity of each cell
+    const int* row_ptr;
+    const int* n_act;
+    const double4* jbuf;
+    const double4* pbuf;
+    const Geom* gref;        // the cells at the last refresh of the active pairs
+    double rho;              // cell density M0 / (pi ((4/3) R^3 + R^2 L0))
+};
+void launch_verlet_cells(int phase, const VerletArgs& a, Ctrl* ctrl, const StepParams& sp, int cap_cells,
+                         cudaStream_t st);
 
 // friction: before an attempt, trial passes that run the stages of the cells with
 // candidate contacts and checks that recompute the candidates' planar decisions from

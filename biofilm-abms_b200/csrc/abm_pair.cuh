@@ -108,6 +108,43 @@ __device__ __forceinline__ PairOut pair_force_fp64(const Geom& gi, const Geom& g
     return out;
 }
 
+// FP32 variant: segment distance (FP64 near-parallel branch kept), overlap,
+// Hertz / JKR magnitude and direction in single precision
+__device__ __forceinline__ PairOut pair_force_fp32(const Geom& gi, const Geom& gj, const ForceParams& fp,
+                                                   const double* td, const double* tr, int rounding)
+{
+    PairOut out;
+    out.touch = false;
+    Dist d = dist_geom_mixed(gi, gj, rounding);
+    // the overlap from the FP64 distance vector, then the force law in FP32
+    const double distd = sqrt((d.dx * d.dx + d.dy * d.dy) + d.dz * d.dz);
+    const double overlap_d = 2 * fp.R - distd;
+    if (!(overlap_d > 0)) return out;
+    float dx = (float)d.dx, dy = (float)d.dy, dz = (float)d.dz;
+    const float dist = (float)distd;
+    const float R = (float)fp.R, max_overlap = (float)fp.max_overlap;
+    float overlap = (float)overlap_d;
+    float inv = 1.f / dist;
+    float m;
+    const double gamma = fp.adhesion ? fmin(gi.gamma, gj.gamma) : 0.0;
+    if (fp.adhesion && gamma > 0)
+    {
+        // the JKR magnitude term1 - term2 cancels near the force balance, where most
+        // adhering contacts sit: it keeps FP64 (table lookup included)
+        m = (float)(fp.jkr_ng ? jkr_magnitude_variable(distd, gamma, fp, td) : jkr_magnitude(distd, gamma, fp, td, tr));
+    }
+    else if (overlap <= max_overlap) m = (float)fp.pf0 * overlap * sqrtf(overlap);
+    else
+    {
+        m = (float)fp.pf2;
+        if (!fp.adhesion) { float e = overlap - max_overlap; m += (float)fp.pf1 * e * sqrtf(e); }
+    }
+    if (fp.adhesion && overlap > max_overlap) { float e = overlap - max_overlap; m += (float)fp.pf1 * e * sqrtf(e); }
+    out.vx = (double)(m * dx * inv); out.vy = (double)(m * dy * inv); out.vz = (double)(m * dz * inv);
+    out.s = d.s; out.t = d.t; out.ovl = overlap; out.touch = true;
+    return out;
+}
+
 // mechanics.hpp:1031-1175 (cellCellFrictionForces, include_constraint = false) for one
 // touching pair (i, j), i = pr.x the larger index, from the pair's distance record: the
 // friction force on cell i is -eta sqrt(Req overlap) times the tangential part of the

@@ -1,13 +1,11 @@
-// Velocity-Verlet step of the 3-D model (integration mode 0; kmnam/biofilm-ABMs,
-// ABM-3d/ABM-3d-cpp/include: stepVelocityVerlet, mechanics.hpp:2668-2996, called from
-// simulation.hpp:1786-1798 with the cell density of simulation.hpp:1279-1290):
-//
-//   k_verlet_pairs  (y0)       the pair forces in their include_constraint form
-//   k_verlet_cells  phase 0    forces -> accelerations, half kick, drift of both cell ends
-//                              with the half-step velocity and angular velocity -> geom_c
-//   k_verlet_pairs  (drifted)  the same at the drifted state (updateNeighborDistances)
-//   k_verlet_cells  phase 1    forces -> second half kick, dn = omega x n, growth
-//   k_verlet_accept            the clock and the loop's counters
+// Velocity Verlet (integration mode 0: stepVelocityVerlet, mechanics.hpp:2668-2996) with the
+// include_constraint force forms.
+//   k_pair_pass<..., VERLET>   the pair shares at the current state, over the active pairs
+//   k_verlet_cells<0>  forces -> accelerations, half kick, drift of both cell ends
+//   k_pair_pass<..., VERLET>   the same at the drifted state (updateNeighborDistances)
+//   k_verlet_cells<1>  forces -> accelerations, second half kick, growth; its last block
+//                      closes the step
+// Both cell passes report how far the cells have moved since the active pairs were listed.
 //
 // The include_constraint forms (mechanics.hpp:1298-1311, 1554-1566, 1608-1617,
 // adhesion.hpp:355-366, mechanics.hpp:718-755, 845-886, 1152-1161): the orientation rows of
@@ -19,80 +17,16 @@
 // plus the noise, minus the ambient viscosity eta0 l^3 (dr, l^6 (n x dn) / 12)
 // (mechanics.hpp:1784-1820), minus the cell-surface friction (mechanics.hpp:1821-1917),
 // capped row by row at cell_surface_coulomb_coeff times the constrained surface repulsion.
-#include "abm_kernels.cuh"
-#include "abm_pair.cuh"
+//
+// A cell's serial FP64 chain bounds the cell passes, as it does the Runge-Kutta attempts
+// (16 us each for 5,000 cells); the row sums run over the active shares only, cells clear of
+// the surface leave its integrals out, and the contact cases are one formula
+// (velocity_tilted).
+#include "abm_step.cuh"
 
 namespace abm {
 
-const int VV_T = 256;
-
-static inline int cdiv_v(int a, int b) { return (a + b - 1) / b; }
-
-// include_constraint form of one pair's shares at the given state (geom, vel): (v, s)
-// into both entries as the Runge-Kutta pass writes them, and the JKR part of v into pbuf
-__global__ void k_verlet_pairs(const Geom* __restrict__ geom, const Vel* __restrict__ vel,
-                               const int4* __restrict__ pairs, const Ctrl* ctrl, ForceParams fp,
-                               const double* __restrict__ td, const double* __restrict__ tr, double4* jbuf,
-                               double4* pbuf)
-{
-    if (ctrl->halted) return;
-    const int n_pairs = ctrl->n_dir >> 1;
-    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n_pairs; q += gridDim.x * blockDim.x)
-    {
-        const int4 pr = pairs[q];
-        const Geom gi = load_geom(geom, pr.x), gj = load_geom(geom, pr.y);
-        const PairOut p = pair_force_fp64(gi, gj, fp, td, tr);
-        double4 own = make_double4(0.0, 0.0, 0.0, 0.0), other = own, part = own;
-        if (p.touch)
-        {
-            own = make_double4(p.vx, p.vy, p.vz, p.s);
-            other = make_double4(p.vx, p.vy, p.vz, p.t);
-            const double ux = p.dx / p.dist, uy = p.dy / p.dist, uz = p.dz / p.dist;
-            part = make_double4(p.mj * ux, p.mj * uy, p.mj * uz, 0.0);
-            if (fp.fric)
-            {
-                // mechanics.hpp:1031-1175 at this state: the stored velocities of the state
-                // and the planar decision of its contact points
-                const X3 dv = x3(p.dx, p.dy, p.dz);
-                const Vel ui = vel[pr.x], uj = vel[pr.y];
-                const double eta = fmin(fp.feta[pr.x], fp.feta[pr.y]);
-                double rv[3];
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-                    rv[c] = (ui.v[c] + p.s * ui.v[3 + c]) - (uj.v[c] + p.t * uj.v[3 + c]);
-                bool flat = false;
-                if (fp.surface && fabs(__ddiv_rn(p.dz, p.dist)) < 1e-3)
-                {
-                    const double lim = 1.01 * fp.R;
-                    flat = __dadd_rn(gi.rz, __dmul_rn(p.s, gi.nz)) < lim &&
-                           __dadd_rn(gj.rz, __dmul_rn(p.t, gj.nz)) < lim;
-                }
-                double f[3];
-                friction_force(dv, p.dist, flat, rv, eta, fp, f);
-                own.x -= f[0]; own.y -= f[1]; own.z -= f[2];
-                other.x -= f[0]; other.y -= f[1]; other.z -= f[2];
-            }
-        }
-        jbuf[pr.z] = own;
-        jbuf[pr.w] = other;
-        pbuf[pr.z] = part;
-        pbuf[pr.w] = part;
-    }
-}
-
-struct VerletArgs {
-    const Geom* g_in;        // the state the forces are evaluated at
-    const Vel* v_in;
-    Geom* g_out;             // phase 0: the drifted state; phase 1: the new state
-    Vel* v_out;
-    Phys* phys;
-    double4* whalf;          // half-step angular velocity of each cell
-    const int* row_ptr;
-    const int* lower_end;
-    const double4* jbuf;
-    const double4* pbuf;
-    double rho;              // cell density M0 / (pi ((4/3) R^3 + R^2 L0))
-};
+const int VV_T = 128;
 
 __device__ __forceinline__ void cross3(const double a[3], const double b[3], double o[3])
 {
@@ -109,14 +43,21 @@ __device__ __forceinline__ void verlet_force(const StepParams& sp, const VerletA
     const double n[3] = {g.nx, g.ny, g.nz};
     // the pair sums in CSR order, then the constrained orientation rows
     double F[3] = {0, 0, 0}, Tc[3] = {0, 0, 0}, Tp[3] = {0, 0, 0};
-    const int le = a.lower_end[i], r1 = a.row_ptr[i + 1];
-    for (int e = a.row_ptr[i]; e < r1; ++e)
+    const int r0 = a.row_ptr[i], na = a.n_act[i];
+    for (int k = 0; k < na; k += 2)
     {
-        const double4 js = a.jbuf[e], pp = a.pbuf[e];
-        const double sg = e < le ? 1.0 : -1.0, w = sg * js.w;
-        F[0] += sg * js.x; F[1] += sg * js.y; F[2] += sg * js.z;
-        Tc[0] += w * (js.x - pp.x); Tc[1] += w * (js.y - pp.y); Tc[2] += w * (js.z - pp.z);
-        Tp[0] += w * pp.x; Tp[1] += w * pp.y; Tp[2] += w * pp.z;
+        double4 js[2], pp[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) if (k + q < na) { js[q] = a.jbuf[r0 + k + q]; pp[q] = a.pbuf[r0 + k + q]; }
+#pragma unroll
+        for (int q = 0; q < 2; ++q)
+            if (k + q < na)
+            {
+                const double w = js[q].w;
+                F[0] += js[q].x; F[1] += js[q].y; F[2] += js[q].z;
+                Tc[0] += w * (js[q].x - pp[q].x); Tc[1] += w * (js[q].y - pp[q].y); Tc[2] += w * (js[q].z - pp[q].z);
+                Tp[0] += w * pp[q].x; Tp[1] += w * pp[q].y; Tp[2] += w * pp[q].z;
+            }
     }
     double dE[6];
     double tcr[3];
@@ -126,36 +67,54 @@ __device__ __forceinline__ void verlet_force(const StepParams& sp, const VerletA
     dE[3] = tcr[0] + (Tp[0] - np * n[0]);
     dE[4] = tcr[1] + (Tp[1] - np * n[1]);
     dE[5] = tcr[2] + (Tp[2] - np * n[2]);
-    // cell-surface repulsion and adhesion, include_constraint (mechanics.hpp:673-910)
+    // cell-surface repulsion and adhesion, include_constraint (mechanics.hpp:673-910), and the
+    // area integrals of the friction (integrals.hpp:400-463)
     double rep[6] = {0, 0, 0, 0, 0, 0}, adh[6] = {0, 0, 0, 0, 0, 0};
+    double A1 = 0.0, A2 = 0.0, A3 = 0.0;
     const bool a2 = g.nz < P.nz_threshold;
     const double l = ph.l, h = g.h, R = P.R;
-    double ss = 0.0;
-    EndPow w;
-    w.p = w.q = w.sp = w.sq = 0.0;
-    if (!P.no_surface)
+    // the test of cell_velocity_fp64: a cell whose lower end is clear of the surface
+    const bool clear = P.no_surface || (!a2 && g.rz - h * fabs(g.nz) > R + 1e-6 * (1.0 + fabs(g.rz)));
+    if (!clear)
     {
         if (a2) surface_dEdq_flat(P, g.rz, l, ph.sigma0, rep[2], adh[2]);
         else
         {
-            ss = (R - g.rz) / g.nz;
-            w = end_pows(g.rz, g.nz, R, h, ss);
-            const double nz = g.nz, nz2 = nz * nz, inz = 1.0 / nz;
+            const double nz = g.nz, nz2 = nz * nz, onz = 1.0 - nz2;
+            const double Rmrz = R - g.rz, inz = 1.0 / nz, ss = Rmrz / nz;
+            const bool both = ss > h, any = ss > -h, partial = fabs(ss) < h;
+            const double p = any ? Rmrz + h * nz : 0.0, q = both ? Rmrz - h * nz : 0.0;
+            const double P1 = sqrt(p), Q1 = sqrt(q);
+            const double P3 = P1 * p, Q3 = Q1 * q, P4 = p * p, Q4 = q * q;
+            const double P5 = P3 * p, Q5 = Q3 * q, P6 = P4 * p, Q6 = Q4 * q, P7 = P5 * p, Q7 = Q5 * q;
+            const double D1 = (P1 - Q1) * inz * 2.0;
+            const double D3 = (P3 - Q3) * inz * (2.0 / 3.0);
+            const double D4 = (P4 - Q4) * inz * 0.5;
+            const double D5 = (P5 - Q5) * inz * (2.0 / 5.0);
+            const double D6 = (P6 - Q6) * inz * (2.0 / 6.0);
+            const double D7 = (P7 - Q7) * inz * (2.0 / 7.0);
+            const double M1 = (D3 - h * (P1 + Q1)) * inz * 2.0;
+            const double M3 = (D5 - h * (P3 + Q3)) * inz * (2.0 / 3.0);
+            const double M4 = (D6 - h * (P4 + Q4)) * inz * 0.5;
+            const double M5 = (D7 - h * (P5 + Q5)) * inz * (2.0 / 5.0);
             const double pf0 = 2 * P.E0;
-            rep[2] = -pf0 * ((1.0 - nz2) * integral1(w, inz, h, 4, ss) + P.sqrtR * nz2 * integral1(w, inz, h, 3, ss));
+            rep[2] = -pf0 * (onz * D4 + P.sqrtR * nz2 * D3);
             const double cx = g.ny, cy = -g.nx;
-            const double W = (1.0 - nz2) * integral2(w, inz, h, 4, ss) + P.sqrtR * nz2 * integral2(w, inz, h, 3, ss);
+            const double W = onz * M4 + P.sqrtR * nz2 * M3;
             rep[3] = -pf0 * cx * W;
             rep[4] = -pf0 * cy * W;
             const double a0 = P.sqrtR / 2, a1 = 2 * M_PI * R;
-            const bool partial = fabs(ss) < h;
-            const double term2 = partial ? (a1 / 2) * nz : 0.0;
-            adh[2] = (a0 * (1 - nz2) * integral1(w, inz, h, 1, ss) + term2) * ph.sigma0;
-            const double i2 = integral2(w, inz, h, 1, ss);
-            const double w1 = partial ? (a1 / 2) * ss * nz * cx : 0.0;
-            const double w2 = partial ? (a1 / 2) * ss * nz * cy : 0.0;
-            adh[3] = (a0 * (1 - nz2) * i2 * cx - w1) * ph.sigma0;
-            adh[4] = (a0 * (1 - nz2) * i2 * cy - w2) * ph.sigma0;
+            adh[2] = (a0 * onz * D1 + (partial ? (a1 / 2) * nz : 0.0)) * ph.sigma0;
+            const double w1 = partial ? (a1 / 2) * ss * nz : 0.0;
+            adh[3] = (a0 * onz * M1 - w1) * cx * ph.sigma0;
+            adh[4] = (a0 * onz * M1 - w1) * cy * ph.sigma0;
+            const double i4 = both ? 2 * h : (any ? ss + h : 0.0);
+            const double i5 = (any && !both) ? (ss * ss - h * h) / 2.0 : 0.0;
+            const double i6 = both ? 2 * h * h * h / 3.0 : (any ? (ss * ss * ss + h * h * h) / 3.0 : 0.0);
+            const double piRnz2 = M_PI * R * nz2;
+            A1 = P.sqrtR * onz * D3 + piRnz2 * i4;
+            A2 = P.sqrtR * onz * M3 + piRnz2 * i5;
+            A3 = P.sqrtR * onz * ((2 * M5 + h * h * (P3 - Q3)) * inz * (2.0 / 3.0)) + piRnz2 * i6;
         }
     }
 #pragma unroll
@@ -177,41 +136,39 @@ __device__ __forceinline__ void verlet_force(const StepParams& sp, const VerletA
     const double dn[3] = {u.v[3], u.v[4], u.v[5]};
     double om[3];
     cross3(n, dn, om);
-    const double li = pow(l, 3.0);
-    const double A = ph.eta0 * li, B = ph.eta0 * li * li * li;
+    const double li = l * l * l;
+    const double A = ph.eta0 * li, B = ph.eta0 * li * li * li * (1.0 / 12);
     f[0] -= A * u.v[0]; f[1] -= A * u.v[1]; f[2] -= A * u.v[2];
-    f[3] -= B * om[0] / 12; f[4] -= B * om[1] / 12; f[5] -= B * om[2] / 12;
-    if (!P.no_surface)
+    f[3] -= B * om[0]; f[4] -= B * om[1]; f[5] -= B * om[2];
+    if (!clear)
     {
         // cell-surface friction (mechanics.hpp:1821-1917)
         double csf[6] = {0, 0, 0, 0, 0, 0};
         const double q[3] = {u.v[0], u.v[1], 0.0};
         const double m[3] = {om[1] * n[2] - om[2] * n[1], om[2] * n[0] - om[0] * n[2], 0.0};
-        const double eta = ph.eta1;
+        const double eta = ph.eta1 * P.invR;
         if (a2)
         {
             const double phz = R - g.rz;
             if (phz > 0)
             {
-                const double area = sqrt(R) * sqrt(phz) * l;
-                csf[0] = eta * q[0] * area / R;
-                csf[1] = eta * q[1] * area / R;
+                const double area = P.sqrtR * sqrt(phz) * l;
+                csf[0] = eta * q[0] * area;
+                csf[1] = eta * q[1] * area;
                 const double cz = n[0] * m[1] - n[1] * m[0];
-                csf[5] = eta * cz * area * (l * l) / (12 * R);
+                csf[5] = eta * cz * area * (l * l) * (1.0 / 12);
             }
         }
         else
         {
-            double A1, A2, A3;
-            area_integrals(P, g.nz, h, ss, w, A1, A2, A3);
-            csf[0] = eta * (q[0] * A1 + m[0] * A2) / R;
-            csf[1] = eta * (q[1] * A1 + m[1] * A2) / R;
+            csf[0] = eta * (q[0] * A1 + m[0] * A2);
+            csf[1] = eta * (q[1] * A1 + m[1] * A2);
             double c1[3], c2[3];
             cross3(n, q, c1);
             cross3(n, m, c2);
-            csf[3] = eta * (c1[0] * A2 + c2[0] * A3) / R;
-            csf[4] = eta * (c1[1] * A2 + c2[1] * A3) / R;
-            csf[5] = eta * (c1[2] * A2 + c2[2] * A3) / R;
+            csf[3] = eta * (c1[0] * A2 + c2[0] * A3);
+            csf[4] = eta * (c1[1] * A2 + c2[1] * A3);
+            csf[5] = eta * (c1[2] * A2 + c2[2] * A3);
         }
         if (P.coulomb > 0)
         {
@@ -219,7 +176,10 @@ __device__ __forceinline__ void verlet_force(const StepParams& sp, const VerletA
             for (int c = 0; c < 6; ++c) { sf += csf[c] * csf[c]; sr += rep[c] * rep[c]; }
             const double fn = sqrt(sf), max_norm = P.coulomb * sqrt(sr);
             if (fn > max_norm)
-                for (int c = 0; c < 6; ++c) csf[c] *= (max_norm / fn);
+            {
+                const double scale = max_norm / fn;
+                for (int c = 0; c < 6; ++c) csf[c] *= scale;
+            }
         }
 #pragma unroll
         for (int c = 0; c < 6; ++c) f[c] -= csf[c];
@@ -231,19 +191,20 @@ __device__ __forceinline__ void verlet_force(const StepParams& sp, const VerletA
 __device__ __forceinline__ void verlet_accel(const double f[6], const double n[3], double length, double rho,
                                              double R, double lin[3], double ang[3])
 {
-    const double volume = M_PI * ((4. / 3.) * pow(R, 3.0) + R * R * length);
+    const double volume = M_PI * ((4. / 3.) * (R * R * R) + R * R * length);
     const double mass = rho * volume;
     const double diam = 2 * R, d2 = diam * diam, d3 = d2 * diam, d4 = d3 * diam;
     const double l2 = length * length, l3 = l2 * length;
     const double mom_par = d4 * (length / 32 + diam / 60) * (rho * M_PI);
     const double mom_perp = d2 * (4 * d3 + 15 * length * d2 + 20 * l2 * diam + 10 * l3) / 480 * (rho * M_PI);
+    const double im = 1.0 / mass, ipar = 1.0 / mom_par, iperp = 1.0 / mom_perp;
     const double tq[3] = {f[3], f[4], f[5]};
     const double tn = (tq[0] * n[0] + tq[1] * n[1]) + tq[2] * n[2];
     for (int c = 0; c < 3; ++c)
     {
-        lin[c] = f[c] / mass;
+        lin[c] = f[c] * im;
         const double tpar = tn * n[c], tperp = tq[c] - tpar;
-        ang[c] = tpar / mom_par + tperp / mom_perp;
+        ang[c] = tpar * ipar + tperp * iperp;
     }
 }
 
@@ -254,18 +215,53 @@ __device__ __forceinline__ void normalize3(double n[3])
     if (n[2] < 0) { n[0] = -n[0]; n[1] = -n[1]; n[2] = -n[2]; }
 }
 
-template <int PHASE>
-__global__ void k_verlet_cells(Ctrl* ctrl, StepParams sp, VerletArgs a)
+// the accepted step's bookkeeping (the accepted branch of the controller, with the
+// reference's zero error for a Verlet step, simulation.hpp:1786-1798)
+__device__ __forceinline__ void verlet_accept(Ctrl* c)
 {
+    c->attempts += 1;
+    c->last_max_error = 0.0;
+    const int h = c->hist_pos;
+    c->hist_dt[h] = c->dt;
+    c->hist_err[h] = 0.0;
+    c->hist_acc[h] = 1;
+    c->hist_pos = (h + 1) % HIST;
+    c->since_div = c->n_divide > 0 ? 0 : c->since_div + 1;
+    c->cell_steps += c->n;
+    c->t += c->dt;
+    c->iter += 1;
+    c->iterations += 1;
+    if (c->dt_write > 0)
+    {
+        const double t_old_factor = fmod(c->t - c->dt + 1e-12, c->dt_write);
+        const double t_new_factor = fmod(c->t + 1e-12, c->dt_write);
+        if (t_old_factor > t_new_factor) c->frame_due = 1;
+    }
+}
+
+template <int PHASE>
+__global__ void __launch_bounds__(VV_T) k_verlet_cells(Ctrl* ctrl, StepParams sp, VerletArgs a)
+{
+    __shared__ double sh_drift[VV_T / 32];
+    __shared__ bool last;
     if (ctrl->halted) return;
     const int n = ctrl->n;
+    // the grid covers the capacity; blocks past the cells leave at once and are not counted
+    const int blocks = max((n + VV_T - 1) / VV_T, 1);
+    if (blockIdx.x >= blocks) return;
+    const Geom* g_in = PHASE == 0 ? a.geom : a.geom_c;
+    const Vel* v_in = PHASE == 0 ? a.vel : a.vel_c;
+    Geom* g_out = PHASE == 0 ? a.geom_c : a.geom;
+    Vel* v_out = PHASE == 0 ? a.vel_c : a.vel;
+    double drift = 0.0;
     const double dt = ctrl->dt, hdt = 0.5 * dt;
     const int iter = ctrl->iter;
     const double R = sp.mp.R;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    const int i = blockIdx.x * VV_T + threadIdx.x;
+    if (i < n)
     {
-        const Geom g = a.g_in[i];
-        const Vel u = a.v_in[i];
+        const Geom g = g_in[i];
+        const Vel u = v_in[i];
         const Phys ph = a.phys[i];
         double f[6];
         verlet_force(sp, a, i, g, u, ph, iter, f);
@@ -323,51 +319,40 @@ __global__ void k_verlet_cells(Ctrl* ctrl, StepParams sp, VerletArgs a)
                   isfinite(nn[2])))
                 atomicOr(&ctrl->status, (int)ST_NAN);
         }
-        a.g_out[i] = go;
-        a.v_out[i] = vo;
+        g_out[i] = go;
+        v_out[i] = vo;
+        const Geom r = a.gref[i];
+        const double ax = go.rx - r.rx, ay = go.ry - r.ry, az = go.rz - r.rz;
+        const double bx = go.nx - r.nx, by = go.ny - r.ny, bz = go.nz - r.nz;
+        drift = sqrt(ax * ax + ay * ay + az * az) + go.h * sqrt(bx * bx + by * by + bz * bz) + fabs(go.h - r.h);
+        // a state that is no number keeps every pair in the list
+        if (!isfinite(drift)) drift = 1e300;
     }
-}
-
-// the accepted step's bookkeeping (the accepted branch of the controller, with the
-// reference's zero error for a Verlet step, simulation.hpp:1786-1798)
-__global__ void k_verlet_accept(Ctrl* c)
-{
-    if (c->halted) return;
-    c->attempts += 1;
-    c->last_max_error = 0.0;
-    const int h = c->hist_pos;
-    c->hist_dt[h] = c->dt;
-    c->hist_err[h] = 0.0;
-    c->hist_acc[h] = 1;
-    c->hist_pos = (h + 1) % HIST;
-    c->since_div = c->n_divide > 0 ? 0 : c->since_div + 1;
-    c->cell_steps += c->n;
-    c->t += c->dt;
-    c->iter += 1;
-    c->iterations += 1;
-    if (c->dt_write > 0)
+    drift = warp_max(drift);
+    if ((threadIdx.x & 31) == 0) sh_drift[threadIdx.x >> 5] = drift;
+    __syncthreads();
+    if (threadIdx.x == 0)
     {
-        const double t_old_factor = fmod(c->t - c->dt + 1e-12, c->dt_write);
-        const double t_new_factor = fmod(c->t + 1e-12, c->dt_write);
-        if (t_old_factor > t_new_factor) c->frame_due = 1;
+        for (int w = 1; w < VV_T / 32; ++w) drift = fmax(drift, sh_drift[w]);
+        if (drift > 0) atomicMax(&ctrl->drift_bits, (unsigned long long)__double_as_longlong(drift));
+        __threadfence();
+        last = atomicAdd(&ctrl->blocks_done, 1u) == blocks - 1;
     }
-    c->screen_valid = 0;
+    if (threadIdx.x == 0 && last)
+    {
+        __threadfence();
+        ctrl->drift = __longlong_as_double((long long)atomicExch(&ctrl->drift_bits, 0ull));
+        ctrl->blocks_done = 0u;
+        if (PHASE == 1) verlet_accept(ctrl);
+    }
 }
 
-void launch_verlet_step(Geom* geom, Vel* vel, Phys* phys, Geom* geom_c, Vel* vel_c, double4* whalf, Ctrl* ctrl,
-                        const StepParams& sp, const ForceParams& fp, const double* td, const double* tr,
-                        const int4* pairs, const int* row_ptr, const int* lower_end, double4* jbuf, double4* pbuf,
-                        double rho, int cap_cells, int cap_pairs, cudaStream_t st)
+void launch_verlet_cells(int phase, const VerletArgs& a, Ctrl* ctrl, const StepParams& sp, int cap_cells,
+                         cudaStream_t st)
 {
-    const int pb = max(min(cdiv_v(cap_pairs, VV_T), 148 * 16), 1);
-    const int cb = max(min(cdiv_v(cap_cells, VV_T), 148 * 8), 1);
-    VerletArgs a0 = {geom, vel, geom_c, vel_c, phys, whalf, row_ptr, lower_end, jbuf, pbuf, rho};
-    VerletArgs a1 = {geom_c, vel_c, geom, vel, phys, whalf, row_ptr, lower_end, jbuf, pbuf, rho};
-    k_verlet_pairs<<<pb, VV_T, 0, st>>>(geom, vel, pairs, ctrl, fp, td, tr, jbuf, pbuf);
-    k_verlet_cells<0><<<cb, VV_T, 0, st>>>(ctrl, sp, a0);
-    k_verlet_pairs<<<pb, VV_T, 0, st>>>(geom_c, vel_c, pairs, ctrl, fp, td, tr, jbuf, pbuf);
-    k_verlet_cells<1><<<cb, VV_T, 0, st>>>(ctrl, sp, a1);
-    k_verlet_accept<<<1, 1, 0, st>>>(ctrl);
+    const int blocks = max((cap_cells + VV_T - 1) / VV_T, 1);
+    if (phase == 0) k_verlet_cells<0><<<blocks, VV_T, 0, st>>>(ctrl, sp, a);
+    else k_verlet_cells<1><<<blocks, VV_T, 0, st>>>(ctrl, sp, a);
 }
 
 }   // namespace abm

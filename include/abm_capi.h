@@ -91,7 +91,7 @@ typedef struct abm_params {
     int precision;               /* ABM_PRECISION_FP64 or ABM_PRECISION_MIXED */
     int cap_cells;               /* device capacity in cells (>= the largest population) */
     int cap_neighbors_per_cell;  /* directed neighbor slots per cell (0 = default: 192 in 3-D, 64 in 2-D) */
-    int pair_lanes;              /* lanes per cell of the no-alloc entry point's pair kernel: 4, 8, 16 or 32 (0 = 8) */
+    int pair_lanes;              /* lanes per row of the no-alloc entry point's sums: 4, 8, 16 or 32 (0 = 8) */
     int use_graphs;              /* 1 = capture the iteration in a CUDA graph */
     /* step-size control (no reference counterpart beyond ABM_CONTROLLER_REFERENCE) */
     int controller;              /* ABM_CONTROLLER_REFERENCE, ABM_CONTROLLER_LEARNED or ABM_CONTROLLER_PI */
@@ -352,7 +352,7 @@ const char* abm_mlp_last_error(void);
  * ready when the stream reaches that point.  3-D model only (dims 0 or 3);
  * adhesion_mode 0 or 1; precision ABM_PRECISION_FP64 or ABM_PRECISION_MIXED.
  *
- * Scratch lives in one fixed __device__ array of about 21 MB that every GPU
+ * Scratch lives in one fixed __device__ array of about 24 MB that every GPU
  * loading this library holds until the process exits.  Limits per call:
  * n <= ABM_NOALLOC_MAX_CELLS, n_entries <= ABM_NOALLOC_MAX_ENTRIES; larger
  * inputs return ABM_ERR_CAPACITY.  The first call on a device looks up the
