@@ -34,6 +34,11 @@ __global__ void __launch_bounds__(AT_T, (S <= 4 ? (V == 3 ? 3 : 6) : 1)) k_attem
     __shared__ double sh_max[AT_T / 32], sh_drift[AT_T / 32], sh_path[AT_T / 32];
     __shared__ double4 sh_stat[AT_T / 32];
     __shared__ bool last;
+    __shared__ Ctrl sc;                 // the last block's copy of the control record
+    // the cell of this thread by the attempt order, read beside the control record (the order
+    // has an entry for every cell of the capacity)
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int ordered = (KIND != 3 && sp.order && t < sp.order_cap) ? sp.order[t] : t;
     if (DRY && (!ctrl->fr_pending || (KIND != 3 && ctrl->halted))) return;
     if (KIND != 3 && ctrl->halted)
     {
@@ -91,7 +96,6 @@ __global__ void __launch_bounds__(AT_T, (S <= 4 ? (V == 3 ? 3 : 6) : 1)) k_attem
     else { dt = eval_dt; attempt = eval_attempt; }
     // the step was closed by a proposal that passed the error test
     if (KIND == MODE_FINAL && mode == MODE_COMMIT) return;
-    const bool commit = false;
     // a proposal (learned or PI) advances the state in place; the attempts after a failed
     // proposal start from the copy of y0 it kept
     const bool in_place = !DRY && (KIND == MODE_TRIAL) && sp.propose;
@@ -103,7 +107,7 @@ __global__ void __launch_bounds__(AT_T, (S <= 4 ? (V == 3 ? 3 : 6) : 1)) k_attem
     // the first attempt of an iteration sums the cell's pair shares (pg.fused); under
     // the reference controller the trial writes the total back for the rest, under the
     // proposing ones every attempt sums them
-    const bool do_gather = pg.fused && !commit &&
+    const bool do_gather = pg.fused &&
                            (KIND == MODE_TRIAL || (KIND == MODE_FINAL && !trial_ran) || sp.propose);
     double local_max = 0.0;
     bool bad = false, longer = false;
@@ -115,10 +119,9 @@ __global__ void __launch_bounds__(AT_T, (S <= 4 ? (V == 3 ? 3 : 6) : 1)) k_attem
     // one cell per thread: the grid covers the capacity (attempt_blocks); thread t takes
     // the t-th cell of the attempt order (cells appended after the order was made, in
     // index order).  The body is a do-while(false) block so that `continue` leaves it.
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) do
     {
-        const int i = t < n_order ? sp.order[t] : t;
+        const int i = t < n_order ? ordered : t;
         if (DRY)
         {
             // only cells with a candidate contact have stage states to report
@@ -357,11 +360,19 @@ __global__ void __launch_bounds__(AT_T, (S <= 4 ? (V == 3 ? 3 : 6) : 1)) k_attem
         }
     }
     __syncthreads();
-    if ((KIND == MODE_FINAL || in_place) && sp.stats_on && last)
+    if (KIND == 3 || !last) return;
+    // The last block works on a copy of the control record, fetched and put back by all its
+    // threads at once: one field after another, each a trip to L2 behind the store before it,
+    // the controller took longer than some cells' velocities.
+    __threadfence();
+    static_assert(sizeof(Ctrl) % 8 == 0, "the control record is copied in 8-byte words");
+    for (int w = threadIdx.x; w < (int)(sizeof(Ctrl) / 8); w += AT_T)
+        reinterpret_cast<unsigned long long*>(&sc)[w] = __ldcg(reinterpret_cast<const unsigned long long*>(ctrl) + w);
+    __syncthreads();
+    if ((KIND == MODE_FINAL || in_place) && sp.stats_on)
     {
         // step-size features of the accepted step (a failed proposal's are replaced
         // by the final attempt's): every block's partial, in block order
-        __threadfence();
         double4 a = make_double4(0.0, 0.0, 0.0, 0.0);
         for (int b = threadIdx.x; b < blocks; b += AT_T)
         {
@@ -388,46 +399,47 @@ __global__ void __launch_bounds__(AT_T, (S <= 4 ? (V == 3 ? 3 : 6) : 1)) k_attem
                 const double4 b = sh_stat[w];
                 t.x = fmax(t.x, b.x); t.y += b.y; t.z += b.z; t.w += b.w;
             }
-            ctrl->st_vmax_bits = (unsigned long long)__double_as_longlong(t.x);
-            ctrl->st_v2_fx = (unsigned long long)llrint(ldexp(t.y, STAT_V2_SHIFT));
-            ctrl->st_g_fx = (unsigned long long)llrint(ldexp(fmax(t.z, 0.0), STAT_G_SHIFT));
-            ctrl->st_near_div = (unsigned long long)t.w;
+            sc.st_vmax_bits = (unsigned long long)__double_as_longlong(t.x);
+            sc.st_v2_fx = (unsigned long long)llrint(ldexp(t.y, STAT_V2_SHIFT));
+            sc.st_g_fx = (unsigned long long)llrint(ldexp(fmax(t.z, 0.0), STAT_G_SHIFT));
+            sc.st_near_div = (unsigned long long)t.w;
         }
     }
-    if (KIND != 3 && last && threadIdx.x == 0)
+    if (threadIdx.x == 0)
     {
-        __threadfence();
-        double E = __longlong_as_double((long long)atomicAdd(&ctrl->err_bits, 0ull));
-        E = fmax(E, sp.min_error);
-        if (commit) E = ctrl->last_trial_error;
+        const double E = fmax(__longlong_as_double((long long)sc.err_bits), sp.min_error);
         // motion of the new state, counted once the step is accepted
-        const double dm = __longlong_as_double((long long)atomicAdd(&ctrl->drift_bits, 0ull));
-        const double pm = F32 ? __longlong_as_double((long long)atomicAdd(&ctrl->path_bits, 0ull)) : 0.0;
-        if (KIND == MODE_FINAL) { ctrl->drift = dm; ctrl->path += pm; }
-        ctrl->drift_bits = 0ull;
-        ctrl->path_bits = 0ull;
-        ctrl->err_bits = 0ull;
-        ctrl->blocks_done = 0u;
-        const bool grown = atomicExch(&ctrl->div_any, 0) != 0;
-        controller_finish(ctrl, sp, KIND, E, grown, commit);
-        if (in_place && ctrl->mode == MODE_COMMIT)
+        const double dm = __longlong_as_double((long long)sc.drift_bits);
+        const double pm = F32 ? __longlong_as_double((long long)sc.path_bits) : 0.0;
+        if (KIND == MODE_FINAL) { sc.drift = dm; sc.path += pm; }
+        const bool grown = sc.div_any != 0;
+        sc.drift_bits = 0ull;
+        sc.path_bits = 0ull;
+        sc.err_bits = 0ull;
+        sc.blocks_done = 0u;
+        sc.div_any = 0;
+        controller_finish(&sc, sp, KIND, E, grown);
+        if (in_place && sc.mode == MODE_COMMIT)
         {
             // the proposal passed: its state is in place; close the step and leave
             // MODE_COMMIT so that this iteration's final attempt exits at once
-            ctrl->drift = dm;
-            ctrl->path += pm;
-            controller_finish(ctrl, sp, MODE_FINAL, E, grown, true);
-            ctrl->mode = MODE_COMMIT;
+            sc.drift = dm;
+            sc.path += pm;
+            controller_finish(&sc, sp, MODE_FINAL, E, grown, true);
+            sc.mode = MODE_COMMIT;
         }
-        else if (flow == FLOW_FAST && KIND == MODE_TRIAL && (sp.propose || ctrl->mode == MODE_RETRY))
-            ctrl->hold = HOLD_RETRY;       // the slow iteration goes on from here
+        else if (flow == FLOW_FAST && KIND == MODE_TRIAL && (sp.propose || sc.mode == MODE_RETRY))
+            sc.hold = HOLD_RETRY;          // the slow iteration goes on from here
         // another retry?  (bounded: the controller schedules at most max_tries of them)
         if ((use_cond & 1) && (KIND == MODE_TRIAL || KIND == MODE_RETRY))
             cudaGraphSetConditional((cudaGraphConditionalHandle)cond,
-                                    (ctrl->mode == MODE_RETRY && ctrl->tries < sp.max_tries) ? 1u : 0u);
+                                    (sc.mode == MODE_RETRY && sc.tries < sp.max_tries) ? 1u : 0u);
         if ((use_cond & 2) && KIND == MODE_TRIAL)
-            cudaGraphSetConditional((cudaGraphConditionalHandle)cond_run, ctrl->mode != MODE_COMMIT ? 1u : 0u);
+            cudaGraphSetConditional((cudaGraphConditionalHandle)cond_run, sc.mode != MODE_COMMIT ? 1u : 0u);
     }
+    __syncthreads();
+    for (int w = threadIdx.x; w < (int)(sizeof(Ctrl) / 8); w += AT_T)
+        reinterpret_cast<unsigned long long*>(ctrl)[w] = reinterpret_cast<const unsigned long long*>(&sc)[w];
 }
 
 // Friction decision check over the candidate pairs of the last pair pass: the planar

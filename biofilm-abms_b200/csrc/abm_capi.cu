@@ -514,6 +514,7 @@ int abm_create(const abm_params* q, abm_ctx** out)
         CK(cudaMalloc(&c->order, (size_t)c->cap * sizeof(int)));
     }
     sp.order = c->order;
+    sp.order_cap = c->order ? c->cap : 0;
     return ABM_OK;
 }
 

@@ -553,6 +553,9 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
         if (lane == 0 && ovl_max > 0)
             atomicMax(&ctrl->st_ovl_bits[ctrl->iter & 1], (unsigned long long)__double_as_longlong(ovl_max));
     }
+    // the pass leaves nothing to close?  (a count over the blocks would only cost its trips)
+    const bool restart = MIXED && rounding == ROUND_STALE;
+    if (!refresh && !restart && !(fp.fric && !VERLET) && !(PROPOSE && !split)) return;
     __syncthreads();
     if (threadIdx.x == 0)
     {
@@ -571,7 +574,7 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
             ctrl->screen_valid = 1;
             ctrl->drift = 0.0;
         }
-        if (MIXED && rounding == ROUND_STALE) ctrl->path = 0.0;
+        if (restart) ctrl->path = 0.0;
         if (fp.fric && !VERLET)
         {
             // the candidates of this pass; no stage has a changed decision yet

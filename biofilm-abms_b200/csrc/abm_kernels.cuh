@@ -182,6 +182,7 @@ struct StepParams {
     float* log_buf;             // MLP_LOG_COLS floats per row, log_cap rows (ring)
     int log_cap;
     const int* order;           // attempt order of the first ctrl->n_order cells (3-D), or null
+    int order_cap;              // its entries
 };
 
 struct ForceParams {
