@@ -15,16 +15,20 @@ namespace abm {
 // that read y0 back from that copy.
 // use_cond bit 0: `cond` is the retry WHILE node's handle; bit 1: `cond_run` is the
 // handle of the IF node around the final attempt (0 after a committed proposal).
-// Launch bounds: six blocks per SM (85 registers) for the 2- and 4-stage tableaux, the
-// fastest measured for the 100k-cell step (three for their friction trial pass, which
-// would spill at six); no bound for the 6- and 7-stage ones, which spill below ~130.
+// B: blocks per SM that the launch bounds ask for.  2- and 4-stage FP64: four (128
+// registers), but six (85, some spilled) where all blocks fit the chip at once with six and
+// not with four (75,777 to 113,664 cells): HE21 / BS32 steps at 5,000, 60,000, 90,000 and
+// 140,000 cells took 28.1 / 34.8, 39.4 / 45.5, 57.2 / 62.5, 76.8 / 86.0 us with four and
+// 29.4 / 36.8, 42.5 / 49.5, 51.5 / 62.7, 83.5 / 104 us with six.  Mixed precision and friction:
+// six; the friction trial pass, which would spill, three.  6 and 7 stages: no bound (they
+// spill below ~130 registers).
 // V: 0 FP64; 1 mixed precision; 2 FP64 with cell-cell friction, whose candidate contacts
 // add, at each stage whose planar decision differs from the one at y0, the recorded change
 // of their shares; 3 the friction trial pass, which runs only the stages of the cells with
 // candidate contacts and records their stage states (z, n_z) for the decision check, with
 // no other effect.
-template <int S, int KIND, bool NOISE, int DIM, int V>
-__global__ void __launch_bounds__(AT_T, (S <= 4 ? (V == 3 ? 3 : 6) : 1)) k_attempt(Geom* geom, Vel* vel, Phys* phys, const Gen6* fcc,
+template <int S, int KIND, bool NOISE, int DIM, int V, int B>
+__global__ void __launch_bounds__(AT_T, B) k_attempt(Geom* geom, Vel* vel, Phys* phys, const Gen6* fcc,
                                                  Ctrl* ctrl, StepParams sp, Geom* geom_c, Vel* vel_c,
                                                  Gen6* err_out, Gen6* k0buf, double eval_dt, int eval_attempt,
                                                  unsigned long long cond, int use_cond, PairGather pg,
@@ -504,12 +508,25 @@ __global__ void k_fr_arm(Ctrl* ctrl, int flow)
     ctrl->fr_pending = ctrl->fr_ncand > 0 && !ctrl->halted && !loop_idle(ctrl, flow);
 }
 
+template <int KIND, bool NOISE, int DIM, int V, int B>
+static void launch_bound(const AttemptArgs& a, cudaStream_t st)
+{
+    k_attempt<ABM_STAGES, KIND, NOISE, DIM, V, B><<<attempt_blocks(a.cap_cells), AT_T, 0, st>>>(
+        a.geom, a.vel, a.phys, a.fcc, a.ctrl, *a.sp, a.geom_c, a.vel_c, a.err_out, a.k0buf, a.eval_dt, a.eval_attempt,
+        a.cond, a.use_cond, a.pg, a.cond_run, a.flow);
+}
+
 template <int KIND, bool NOISE, int DIM, int V>
 static void launch_one(const AttemptArgs& a, cudaStream_t st)
 {
-    k_attempt<ABM_STAGES, KIND, NOISE, DIM, V><<<attempt_blocks(a.cap_cells), AT_T, 0, st>>>(
-        a.geom, a.vel, a.phys, a.fcc, a.ctrl, *a.sp, a.geom_c, a.vel_c, a.err_out, a.k0buf, a.eval_dt, a.eval_attempt,
-        a.cond, a.use_cond, a.pg, a.cond_run, a.flow);
+    if constexpr (ABM_STAGES > 4) launch_bound<KIND, NOISE, DIM, V, 1>(a, st);
+    else if constexpr (V != 0) launch_bound<KIND, NOISE, DIM, V, (V == 3 ? 3 : 6)>(a, st);
+    else
+    {
+        const int blocks = attempt_blocks(a.cells);
+        if (blocks > 4 * a.num_sms && blocks <= 6 * a.num_sms) launch_bound<KIND, NOISE, DIM, V, 6>(a, st);
+        else launch_bound<KIND, NOISE, DIM, V, 4>(a, st);
+    }
 }
 
 template <bool NOISE, int DIM, int V>

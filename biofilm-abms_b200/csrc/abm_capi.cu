@@ -1020,6 +1020,7 @@ static AttemptArgs loop_attempt(abm_ctx* c, int flow = FLOW_STEP)
     c->sp.Ldiv = c->p.Ldiv;
     a.geom = c->geom; a.vel = c->vel; a.phys = c->phys; a.fcc = c->fcc; a.ctrl = c->ctrl; a.sp = &c->sp;
     a.geom_c = c->geom_c; a.vel_c = c->vel_c; a.k0buf = c->k0buf; a.cap_cells = c->cap;
+    a.cells = c->n_seen; a.num_sms = c->num_sms;
     a.pg = {sum_in_attempt(c) ? (f32 ? 3 : 2) : 0, c->row_ptr, c->n_act, c->jbuf, c->fcc, c->gref,
             c->fbuf, c->fmask, c->ystage, c->cap};
     return a;

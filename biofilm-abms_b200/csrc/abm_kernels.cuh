@@ -304,6 +304,7 @@ struct AttemptArgs {
     Vel* vel_c;
     Gen6* k0buf;
     int cap_cells;
+    int cells, num_sms;         // cells there are, as far as the host knows (the kernel's shape)
     PairGather pg;
     // the API's evaluation
     Gen6* err_out;
