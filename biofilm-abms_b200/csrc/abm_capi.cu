@@ -16,6 +16,7 @@
 #include <algorithm>
 #include <functional>
 #include "abm_kernels.cuh"
+#include "abm_host.hpp"
 #include "../../include/abm_capi.h"
 
 using namespace abm;
@@ -290,6 +291,7 @@ int abm_create(const abm_params* q, abm_ctx** out)
     if (!q || !out) return ABM_ERR_ARG;
     *out = nullptr;
     abm_ctx* c = new abm_ctx();
+    host_copy_retain();
     c->p = *q;
     abm_params& p = c->p;
     int ndev = 0;
@@ -524,6 +526,7 @@ int abm_destroy(abm_ctx* c)
     if (c->st) cudaStreamSynchronize(c->st);
     free_all(c);
     delete c;
+    host_copy_release();
     return ABM_OK;
 }
 
@@ -796,8 +799,8 @@ int abm_download_cells(abm_ctx* c, double* cm, int ld)
         else launch_cells_to_colmajor(c->geom, c->vel, c->phys, n, c->ncols, n, c->has_gamma, c->staging, c->st);
         int rc = stage_eta_column(c, c->feta, n);
         if (rc) return rc;
-        CK(cudaMemcpy2DAsync(cm, (size_t)ld * sizeof(double), c->staging, (size_t)n * sizeof(double),
-                             (size_t)n * sizeof(double), c->ncols, cudaMemcpyDeviceToHost, c->st));
+        CK(copy_to_host(c->dev, cm, (size_t)ld * sizeof(double), c->staging, (size_t)n * sizeof(double),
+                        (size_t)n * sizeof(double), c->ncols, c->st));
     }
     CK(cudaStreamSynchronize(c->st));
     return ABM_OK;
@@ -884,8 +887,8 @@ int abm_download_frame(abm_ctx* c, int index, double* cm, int ld, int* n, double
             rc = stage_eta_column(c, c->snap_feta + off, f.n);
             if (rc) return rc;
         }
-        CK(cudaMemcpy2DAsync(cm, (size_t)ld * sizeof(double), c->staging, (size_t)f.n * sizeof(double),
-                             (size_t)f.n * sizeof(double), c->ncols, cudaMemcpyDeviceToHost, c->st));
+        CK(copy_to_host(c->dev, cm, (size_t)ld * sizeof(double), c->staging, (size_t)f.n * sizeof(double),
+                        (size_t)f.n * sizeof(double), c->ncols, c->st));
     }
     CK(cudaStreamSynchronize(c->st));
     return ABM_OK;
@@ -1457,8 +1460,8 @@ int abm_download_neighbors(abm_ctx* c, double* rows, int ld, int cap, int* m)
     CK(cudaMallocAsync(&d_rows, (size_t)std::max(mm, 1) * ncol * sizeof(double), c->st));
     launch_table_rows(c->ctrl, c->row_ptr, c->col, c->key, c->geom, d_rows, std::max(mm, 1), c->cap, c->st, c->dims);
     if (mm > 0)
-        CK(cudaMemcpy2DAsync(rows, (size_t)ld * sizeof(double), d_rows, (size_t)mm * sizeof(double),
-                             (size_t)mm * sizeof(double), ncol, cudaMemcpyDeviceToHost, c->st));
+        CK(copy_to_host(c->dev, rows, (size_t)ld * sizeof(double), d_rows, (size_t)mm * sizeof(double),
+                        (size_t)mm * sizeof(double), ncol, c->st));
     CK(cudaFreeAsync(d_rows, c->st));
     CK(cudaStreamSynchronize(c->st));
     return ABM_OK;
@@ -1673,7 +1676,8 @@ static int download_gen6(abm_ctx* c, const Gen6* src, double* out)
                                cudaMemcpyDeviceToHost, c->st));
     }
     else
-        CK(cudaMemcpyAsync(out, c->staging, (size_t)n * 6 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+        CK(copy_to_host(c->dev, out, (size_t)n * 6 * sizeof(double), c->staging, (size_t)n * 6 * sizeof(double),
+                        (size_t)n * 6 * sizeof(double), 1, c->st));
     CK(cudaStreamSynchronize(c->st));
     return ABM_OK;
 }
@@ -1739,7 +1743,8 @@ int abm_rk_attempt(abm_ctx* c, double dt, int attempt, double* cells_out, double
         else launch_cells_to_colmajor(c->geom_c, c->vel_c, c->phys, n, c->ncols, n, c->has_gamma, c->staging, c->st);
         rc = stage_eta_column(c, c->feta, n);
         if (rc) return rc;
-        CK(cudaMemcpyAsync(cells_out, c->staging, (size_t)n * c->ncols * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+        const size_t bytes = (size_t)n * c->ncols * sizeof(double);
+        CK(copy_to_host(c->dev, cells_out, bytes, c->staging, bytes, bytes, 1, c->st));
     }
     if (errors_out)
     {
