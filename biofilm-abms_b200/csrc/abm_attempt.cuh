@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(AT_T, B) k_attempt(Geom* geom, Vel* vel, Phys*
                 for (int j = 0; j < st; ++j) m += k[j][c] * sp.A[st][j];
                 y[c] = y0[c] + m * dt;
             }
-            normalize_n<F32>(y);
+            normalize_n(y);
             if constexpr (DIM == 2) velocity_2d(y, drag, cc, nz2, k[st]);
             else if constexpr (FRIC)
             {
@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(AT_T, B) k_attempt(Geom* geom, Vel* vel, Phys*
             double y1[6];
 #pragma unroll
             for (int c = 0; c < 6; ++c) y1[c] = y0[c] + d1[c];
-            normalize_n<F32>(y1);
+            normalize_n(y1);
             Geom go = g;
             go.rx = y1[0]; go.ry = y1[1]; go.rz = y1[2]; go.nx = y1[3]; go.ny = y1[4]; go.nz = y1[5];
             Vel vo;

@@ -22,32 +22,23 @@ __device__ __forceinline__ double warp_max(double v)
     return v;
 }
 
-// The orientation of a stage state, normalised, with n_z >= 0.  FP64: one division and its
-// exact corrections (div_by) in place of three divisions, the same bits.  Mixed precision
-// keeps the divisions: the compiler contracts the FP32 sums of velocity_contact_f32 (a b + c d
-// into one of its two fused forms) by the shape of the code around them, and with div_by in
-// that code a last FP32 bit changed in one contact cell of three; the learned controller
-// rounds its features to BF16, so such a bit can change the steps of a whole run.  The free
-// branch keeps its divisions (velocity_free_or_flat) for the same reason.
-template <bool F32>
+// The orientation of a stage state, normalised, with n_z >= 0: one division and its exact
+// corrections (div_by) in place of three divisions, the same bits
 __device__ __forceinline__ void normalize_n(double y[6])
 {
-    const double nrm = sqrt((y[3] * y[3] + y[4] * y[4]) + y[5] * y[5]);
-    if (F32)
-    {
-        y[3] /= nrm; y[4] /= nrm; y[5] /= nrm;
-    }
-    else
-    {
-        const double inv = 1.0 / nrm;
-        y[3] = div_by(y[3], nrm, inv); y[4] = div_by(y[4], nrm, inv); y[5] = div_by(y[5], nrm, inv);
-    }
+    const double nrm = sqrt((y[3] * y[3] + y[4] * y[4]) + y[5] * y[5]), inv = 1.0 / nrm;
+    y[3] = div_by(y[3], nrm, inv); y[4] = div_by(y[4], nrm, inv); y[5] = div_by(y[5], nrm, inv);
     if (y[5] < 0) { y[3] = -y[3]; y[4] = -y[4]; y[5] = -y[5]; }
 }
 
 // Mixed precision: a cell in surface contact (and not lying on the substrate) takes the
 // FP32 contact branch (velocity_contact_f32); the others keep the FP64 branches (i) and
-// (ii), whose surface forces are zero off the surface and the horizontal shortcut on it
+// (ii), whose surface forces are zero off the surface and the horizontal shortcut on it.
+// The free branch keeps its divisions (velocity_free_or_flat): the compiler contracts the
+// FP32 sums of velocity_contact_f32 (a b + c d into one of its two fused forms) by the shape
+// of the code around them, and with div_by there a last FP32 bit changed in one contact cell
+// of three; the learned controller rounds its features to BF16, so such a bit can change the
+// steps of a whole run.
 __device__ __forceinline__ void cell_velocity_f32(const MechParams& P, bool a2, const double y[6], double l, double h,
                                                   double eta0, double eta1, double sigma0, const CellDrag& d,
                                                   const Vel* __restrict__ drp, const double f0[6], double v[6])
