@@ -450,11 +450,11 @@ def launches(variant, t, max_tries=3):
     # its retries (WHILE node) and the final attempt.  Learned controller: the pair
     # pass also makes the proposal; the trial closes a passing step, and only a failed
     # proposal runs the IF node's max_tries retry launches and the final attempt.
-    # 18 kernels per neighbor rebuild.
+    # One kernel per neighbor rebuild.
     learned = VARIANTS[variant]["controller"] == 1
     if learned:
-        return t["iterations"] * 2 + t["rejected"] * (max_tries + 1) + 18 * t["rebuilds"]
-    return t["iterations"] * 3 + t["retries"] + 18 * t["rebuilds"]
+        return t["iterations"] * 2 + t["rejected"] * (max_tries + 1) + t["rebuilds"]
+    return t["iterations"] * 3 + t["retries"] + t["rebuilds"]
 
 
 def relerr(a, b):
