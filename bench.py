@@ -445,16 +445,20 @@ def roofline(kernels, rebuild_ms):
             "rebuild_ms_per_rebuild": rebuild_ms}
 
 
-def launches(variant, t, max_tries=3):
+KERNELS_PER_REBUILD = 1
+
+
+def launches(variant, t, max_tries=3, per_rebuild=18):
     # per iteration: the pair pass, then the attempts.  Reference controller: the trial,
     # its retries (WHILE node) and the final attempt.  Learned controller: the pair
     # pass also makes the proposal; the trial closes a passing step, and only a failed
     # proposal runs the IF node's max_tries retry launches and the final attempt.
-    # One kernel per neighbor rebuild.
+    # per_rebuild kernels per neighbor rebuild: KERNELS_PER_REBUILD of this build (the default is
+    # the chain of kernels that it replaces).
     learned = VARIANTS[variant]["controller"] == 1
     if learned:
-        return t["iterations"] * 2 + t["rejected"] * (max_tries + 1) + t["rebuilds"]
-    return t["iterations"] * 3 + t["retries"] + t["rebuilds"]
+        return t["iterations"] * 2 + t["rejected"] * (max_tries + 1) + per_rebuild * t["rebuilds"]
+    return t["iterations"] * 3 + t["retries"] + per_rebuild * t["rebuilds"]
 
 
 def relerr(a, b):
@@ -648,7 +652,7 @@ def run_b200(args):
                                           "rebuild_charge_ms": h["rebuild_charge_ms"],
                                           "simulated_h_in_timed_region": h["t_sim_h"],
                                           "stepsize_network": weights_note if head == "chosen" else None}),
-            "e2e": h["e2e"], "gpu_launches": launches(head, h),
+            "e2e": h["e2e"], "gpu_launches": launches(head, h, per_rebuild=KERNELS_PER_REBUILD),
             "roofline": roof,
             "clocks": {k: h["clocks"][k] for k in ("sm_mhz", "sm_max_mhz", "reasons")}}
     if other:

@@ -255,7 +255,7 @@ enum MixedRounding {
     ROUND_LIST,     // a pass over the active pairs
     ROUND_STALE,    // such a pass after a stale list (see Ctrl::path): the projections of w
                     // start from the y product
-    ROUND_ROW,      // the row walk of k_pair_force: h1 n1 rounded before it enters w
+    ROUND_ROW,      // the row walk of the no-alloc forces: h1 n1 rounded before it enters w
 };
 __device__ __forceinline__ Dist dist_geom_mixed(const Geom& a, const Geom& b, int rounding)
 {

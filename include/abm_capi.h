@@ -292,8 +292,8 @@ int abm_set_cell_limit(abm_ctx* ctx, int n_max);
 /* ---------------------------------------------------------------------------
  * Batches (no reference counterpart: the reference runs replicates as separate jobs).
  * A batch advances independent contexts (replicate biofilms of any sizes, each with
- * its own clock, step size and controller) by one CUDA graph launch per iteration:
- * every context's iteration graph is a branch of one graph, so a context's results
+ * its own clock, step size and controller) by one CUDA graph launch up to the next joint
+ * rebuild: every context's loop is a branch of one graph, so a context's results
  * are bit-identical to advancing it alone.  Contexts must share a device and
  * iter_update_neighbors.  Batch calls report errors through abm_batch_last_error().
  * ------------------------------------------------------------------------- */
