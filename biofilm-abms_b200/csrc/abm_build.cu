@@ -232,6 +232,7 @@ __device__ bool cell_list(const BuildArgs& a, int n, int nb, BuildShared& sh, bo
             if (bad) atomicOr(&a.ctrl->status, (int)ST_BIN_OVERFLOW);
             a.ctrl->n_pairs = 0;
             a.ctrl->n_sorted = 0;
+            a.ctrl->no_table = bad;
         }
     }
     for (int i = gt; i < n; i += gs)
@@ -499,6 +500,9 @@ __device__ __forceinline__ int group_sum(int v)
 // ascending (the deterministic order of the force sums; the reference's table is i-major,
 // j ascending): an entry's rank is the number of smaller entries of its row.  Barriers: 1
 // between, 1 at the end.
+// When a cell has more neighbors than a row holds, every row is left empty, as where no grid
+// holds the cells: rows cut off one by one would hold entries without their partners' entries,
+// and neither the number of pair records nor the slots of their shares would be right.
 __device__ bool make_rows(const BuildArgs& a, int n, int nb, BuildShared& sh, bool bad, int& n_dir)
 {
     const int chunk = (n + nb - 1) / nb;
@@ -515,18 +519,24 @@ __device__ bool make_rows(const BuildArgs& a, int n, int nb, BuildShared& sh, bo
             a.count[i] = m | (f ? FLAG_BIT : 0);
             s.x += m; s.y += f;
         }
-        if (over) atomicOr(&a.ctrl->status, (int)ST_NBR_OVERFLOW);
+        if (over)
+        {
+            atomicOr(&a.ctrl->status, (int)ST_NBR_OVERFLOW);
+            a.ctrl->no_table = 1;
+        }
         block_scan(s, sh, total);
         if (threadIdx.x == 0) a.part[blockIdx.x] = total;
     }
     if (!build_barrier(a, nb)) return false;
     int2 off, all;
     chunk_offset(a.part, nb, sh, off, all);
+    const bool empty = __ldcg(&a.ctrl->no_table) != 0;
+    if (empty) off.x = all.x = 0;
     for (int i0 = c0; i0 < c1; i0 += BD_T)
     {
         const int i = i0 + threadIdx.x;
         const int v = i < c1 ? a.count[i] : 0;
-        const int2 mine = make_int2(v & ~FLAG_BIT, (v & FLAG_BIT) ? 1 : 0);
+        const int2 mine = make_int2(empty ? 0 : v & ~FLAG_BIT, (v & FLAG_BIT) ? 1 : 0);
         const int2 ex = block_scan(mine, sh, total);
         if (i < c1)
         {
@@ -544,7 +554,7 @@ __device__ bool make_rows(const BuildArgs& a, int n, int nb, BuildShared& sh, bo
     {
         const bool valid = i0 + group < c1;
         const int i = valid ? i0 + group : c0;
-        const int r0 = a.row_ptr[i], len = valid ? a.count[i] & ~FLAG_BIT : 0;
+        const int r0 = a.row_ptr[i], len = valid && !empty ? a.count[i] & ~FLAG_BIT : 0;
         const int* src = a.scratch + (size_t)i * a.bp.cap_per_cell;
         // warp-uniform rounds, so that the shuffles cover all lanes
         int longest = len;
@@ -748,7 +758,7 @@ __global__ void __launch_bounds__(BD_T, 1) k_build(const __grid_constant__ Build
     if (what == BUILD_RECORDS)
     {
         lower_ends(a, n, nb);
-        if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->n_pairs = 0;
+        if (blockIdx.x == 0 && threadIdx.x == 0) { ctrl->n_pairs = 0; ctrl->no_table = 0; }
         if (!build_barrier(a, nb)) return;
         pair_records(a, n, nb, false);
         if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->screen_valid = 0;

@@ -542,6 +542,7 @@ static int check_status(abm_ctx* c)
     Ctrl h;
     CK(cudaMemcpyAsync(&h, c->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
+    if (h.no_table) c->nbrs_valid = false;
     if (h.status & ST_NAN) return fail(c, ABM_ERR_NAN, "NaN/Inf in the RK error norm or velocities");
     if (h.status & ST_NBR_OVERFLOW) return fail(c, ABM_ERR_CAPACITY, "neighbors per cell exceed cap_neighbors_per_cell");
     if (h.status & ST_BIN_OVERFLOW) return fail(c, ABM_ERR_CAPACITY, "cell-list grid exceeds the bin capacity");

@@ -79,6 +79,7 @@ struct Ctrl {
     unsigned long long eval_err_bits;   // scaled max error of the last API attempt
     int n_pairs;                // pair records made so far by a running build
     int n_sorted;               // cells placed so far by its counting sort
+    int no_table;               // the last build found no neighbor set (an overflow): it is empty
     int n_divided;              // mothers of the last division launch
     int last_div_tries;
     int n_parents;              // length of the lineage vector
