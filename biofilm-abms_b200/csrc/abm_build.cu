@@ -625,6 +625,9 @@ __device__ __forceinline__ void pair_records(const BuildArgs& a, int n, int nb, 
             const int j = a.col[r0 + e];
             int x = a.row_ptr[j], y = a.row_ptr[j + 1];
             while (x < y) { const int mid = (x + y) >> 1; if (a.col[mid] < i) x = mid + 1; else y = mid; }
+            // a pair that the caller's rows list more than once: each of its entries with another
+            // one of the partner's
+            for (int q = e; q > 0 && a.col[r0 + q - 1] == j; --q) ++x;
             a.pairs[pos + e] = make_int4(i, j, r0 + e, x);
             if (a.adhere)
             {
