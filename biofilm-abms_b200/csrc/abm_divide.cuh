@@ -37,7 +37,9 @@ __device__ __forceinline__ bool old_cells_within(const BuildArgs& a, const Geom&
     const double reach = limit + q.h + g.max_half_l;
     const float lim = (float)limit + g.margin + segment_reach(q.h, q.nx, q.ny, q.nz);
     const float qx = (float)(q.rx - g.x0), qy = (float)(q.ry - g.y0), qz = (float)(q.rz - g.z0);
-    const int rings = max(1, (int)ceil(reach * g.inv_edge));
+    // no more rings than the grid has bins, whatever the longest cell's length: the sums below
+    // stay in range
+    const int rings = max(1, (int)fmin(ceil(reach * g.inv_edge), (double)max(g.nx, max(g.ny, g.nz))));
     const int bx = min(max((int)floor((q.rx - g.x0) * g.inv_edge), 0), g.nx - 1);
     const int by = min(max((int)floor((q.ry - g.y0) * g.inv_edge), 0), g.ny - 1);
     const int bz = min(max((int)floor((q.rz - g.z0) * g.inv_edge), 0), g.nz - 1);
