@@ -170,7 +170,8 @@ __device__ __forceinline__ Grid make_grid(const Box& b, const BuildArgs& a, bool
     Grid g;
     // the pair test is |r_j - r_i| < prefilter and |d| < threshold, |d| >= |r_j - r_i| less
     // both reaches
-    g.reach = fmin(a.bp.prefilter, a.bp.threshold + 2 * reach + 1e-3);
+    // (a prefilter that no pair passes still needs bins of some size)
+    g.reach = fmax(fmin(a.bp.prefilter, a.bp.threshold + 2 * reach + 1e-3), 1e-3);
     double e = 0.5 * g.reach * (1 + 1e-6);
     double nb[3] = {1.0, 1.0, 1.0};
     for (int tries = 0; tries < 68 && !bad; ++tries)
