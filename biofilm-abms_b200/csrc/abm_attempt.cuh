@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(AT_T, B) k_attempt(Geom* geom, Vel* vel, Phys*
             cudaGraphSetConditional((cudaGraphConditionalHandle)cond_run, 0u);
         return;
     }
+    if (KIND == 3 && (ctrl->halted & HALT_LOST)) return;
     if (KIND != 3 && !DRY && loop_idle(ctrl, flow))
     {
         // nothing to resume: stop an enclosing WHILE node

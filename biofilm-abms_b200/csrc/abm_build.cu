@@ -671,7 +671,7 @@ __device__ bool divide_cells(const BuildArgs& a, int& n, int nb, BuildShared& sh
     if (blockIdx.x == 0 && threadIdx.x == 0)
     {
         // every block has read them
-        ctrl->halted = 0;
+        atomicAnd(&ctrl->halted, ~(int)HALT_CELLS);
         ctrl->hold = HOLD_NONE;
         ctrl->n_divided = 0;
     }
@@ -754,6 +754,7 @@ __global__ void __launch_bounds__(BD_T, 1) k_build(const __grid_constant__ Build
 {
     __shared__ BuildShared sh;
     Ctrl* ctrl = a.ctrl;
+    if (ctrl->halted & HALT_LOST) return;
     if (flow != FLOW_STEP && (ctrl->todo <= 0 || ctrl->hold != HOLD_START)) return;
     int n = ctrl->n;
     const int nb = gridDim.x;
@@ -780,7 +781,7 @@ __global__ void __launch_bounds__(BD_T, 1) k_build(const __grid_constant__ Build
         // terminate() at the top of the loop: no division and no step once n reaches the limit
         if (ctrl->halt_n > 0 && n >= ctrl->halt_n)
         {
-            if (blockIdx.x == 0 && threadIdx.x == 0) { ctrl->halted = 1; ctrl->n_divided = 0; }
+            if (blockIdx.x == 0 && threadIdx.x == 0) { atomicOr(&ctrl->halted, (int)HALT_CELLS); ctrl->n_divided = 0; }
             return;
         }
         int divided;

@@ -277,9 +277,9 @@ static void fill_tableau(StepParams& sp, int mode, bool& ok)
     sp.inv_q1 = 1.0 / (q + 1);
 }
 
-__global__ void k_set_n(Ctrl* c, int n) { c->n = n; c->halted = 0; c->screen_valid = 0; c->n_order = 0; }
+__global__ void k_set_n(Ctrl* c, int n) { c->n = n; c->halted &= HALT_LOST; c->screen_valid = 0; c->n_order = 0; }
 __global__ void k_screen_stale(Ctrl* c) { c->screen_valid = 0; }
-__global__ void k_set_halt(Ctrl* c, int n_max) { c->halt_n = n_max; c->halted = 0; }
+__global__ void k_set_halt(Ctrl* c, int n_max) { c->halt_n = n_max; c->halted &= HALT_LOST; }
 __global__ void k_set_clock(Ctrl* c, double t, double dt, int iter)
 {
     c->t = t; c->dt = dt; c->iter = iter; c->mode = MODE_TRIAL; c->tries = 0; c->attempt = 0;
@@ -1459,6 +1459,7 @@ int abm_download_neighbors(abm_ctx* c, double* rows, int ld, int cap, int* m)
     Ctrl h;
     CK(cudaMemcpyAsync(&h, c->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
+    if (h.halted & HALT_LOST) return check_status(c);
     int mm = h.n_dir / 2;
     if (m) *m = mm;
     if (!rows) return ABM_OK;
@@ -1992,7 +1993,10 @@ static int row_entries(abm_ctx* c, std::vector<int>& entries)
     const int n = c->n_host;
     std::vector<int> rp(n + 1), cl;
     CK(cudaMemcpyAsync(rp.data(), c->row_ptr, (n + 1) * sizeof(int), cudaMemcpyDeviceToHost, c->st));
+    Ctrl h;
+    CK(cudaMemcpyAsync(&h, c->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
+    if (h.halted & HALT_LOST) return check_status(c);
     cl.resize(rp[n]);
     if (rp[n] > 0) CK(cudaMemcpy(cl.data(), c->col, rp[n] * sizeof(int), cudaMemcpyDeviceToHost));
     entries.clear();

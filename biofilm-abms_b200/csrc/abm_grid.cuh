@@ -5,7 +5,8 @@
 namespace abm {
 
 // Polls before a barrier gives up (about a second): a launch whose blocks cannot all
-// arrive ends with ST_BARRIER instead of spinning on.
+// arrive ends with ST_BARRIER instead of spinning on.  The record then holds arrivals of a
+// launch that has ended, so no later launch may wait on it (HALT_LOST).
 const unsigned GRID_BAR_POLLS = 1u << 21;
 
 // Barrier over `nb` blocks, each of which calls it with all its threads (sense reversal:
@@ -33,7 +34,12 @@ __device__ __forceinline__ bool grid_barrier(GridBar* bar, unsigned nb, Ctrl* ct
             do {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(&bar->gen) : "memory");
             } while (now == gen && ++polls < GRID_BAR_POLLS);
-            if (now == gen) { ok = 0; atomicOr(&ctrl->status, (int)ST_BARRIER); }
+            if (now == gen)
+            {
+                ok = 0;
+                atomicOr(&ctrl->status, (int)ST_BARRIER);
+                atomicOr(&ctrl->halted, (int)HALT_LOST);
+            }
         }
         sh_ok = ok;
     }

@@ -639,11 +639,18 @@ void launch_shape(const void* kernel, const LaunchShape& shape, int block, void*
 }
 
 // total dE/dq of each cell from its active shares (the API paths; the loop's first attempt
-// does the same sum itself)
+// does the same sum itself); no number where the pass before it lost its blocks (HALT_LOST)
 __global__ void k_pair_sum_rows(const int* __restrict__ row_ptr, const int* __restrict__ n_act, const Ctrl* ctrl,
                                 const double4* __restrict__ jbuf, Gen6* fcc, int f32)
 {
     const int n = ctrl->n;
+    if (ctrl->halted & HALT_LOST)
+    {
+        const double nan = __longlong_as_double(0x7ff8000000000000ll);
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+            for (int c = 0; c < 6; ++c) fcc[i].f[c] = nan;
+        return;
+    }
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         fcc[i] = f32 ? sum_active_shares(reinterpret_cast<const float4*>(jbuf) + row_ptr[i], n_act[i])
                      : sum_active_shares(jbuf + row_ptr[i], n_act[i]);

@@ -24,6 +24,11 @@ enum LoopFlow { FLOW_STEP = 0, FLOW_FAST = 1, FLOW_SLOW = 2 };
 // the division length, or the colony its limit); or the running one waits for its retries.
 enum LoopHold { HOLD_NONE = 0, HOLD_START = 1, HOLD_RETRY = 2 };
 
+// Ctrl::halted: the population has reached its limit; or a wait among a launch's blocks has run
+// out, after which the barrier record, the bin counts and the neighbor set are not to be used:
+// every kernel that would leaves at once, and the status stays ST_BARRIER.
+enum HaltBits { HALT_CELLS = 1, HALT_LOST = 2 };
+
 // Step-size network: 32 features -> 64 -> 64 -> 1 (log dt ratio)
 const int MLP_IN = 32, MLP_H = 64;
 const int MLP_OFF_W1 = 0, MLP_OFF_B1 = MLP_OFF_W1 + MLP_H * MLP_IN, MLP_OFF_W2 = MLP_OFF_B1 + MLP_H;
@@ -102,7 +107,7 @@ struct Ctrl {
     // cell-count stop on the device (terminate(), simulation.hpp:1600-1615): decided at the
     // start of each iteration by the division count; a halted context skips its iterations
     int halt_n;                         // 0 = no limit
-    int halted;
+    int halted;                         // HaltBits
     long long cell_steps;               // sum of the population over accepted steps
     // screened pair pass: the active list (pairs that passed the bound test with the
     // skin at the last refresh) and the motion since then
