@@ -11,7 +11,7 @@
 #include <atomic>
 #include <cstring>
 #include <mutex>
-#include <system_error>
+#include <exception>
 #include <thread>
 #include <vector>
 #include <cuda_runtime.h>
@@ -132,9 +132,10 @@ cudaError_t copy_to_host(int dev, void* dst, size_t dpitch, const void* src, siz
         };
         std::vector<std::thread> threads;
         threads.reserve(workers);
-        // a thread that cannot be started leaves its pieces to the others
+        // a thread that cannot be started (no thread, or no memory for one) leaves its pieces to
+        // the others; the ones that run are joined in any case
         try { for (int k = 1; k < workers; ++k) threads.emplace_back(work, k); }
-        catch (const std::system_error&) {}
+        catch (const std::exception&) {}
         work(0);
         for (std::thread& t : threads) t.join();
         return (cudaError_t)failed.load();
