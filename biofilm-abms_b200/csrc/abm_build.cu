@@ -809,12 +809,12 @@ LaunchShape build_shape(int cells, int num_sms)
     return make_shape((const void*)k_build, BD_T, (long long)cells * BD_SEARCH, cells <= BUILD_CLUSTER_CELLS, num_sms);
 }
 
-void launch_build(const BuildArgs& args, int what, const LaunchShape& shape, cudaStream_t st, int flow)
+cudaError_t launch_build(const BuildArgs& args, int what, const LaunchShape& shape, cudaStream_t st, int flow)
 {
     BuildArgs a = args;
     a.cluster = shape.cluster;
     void* p[] = {(void*)&a, (void*)&what, (void*)&flow};
-    launch_shape((const void*)k_build, shape, BD_T, p, st);
+    return launch_shape((const void*)k_build, shape, BD_T, p, st);
 }
 
 }   // namespace abm

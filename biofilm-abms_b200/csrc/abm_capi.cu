@@ -108,6 +108,7 @@ struct abm_ctx {
     int iter_k = 1;
     bool graph_fallback = false;     // conditional nodes could not be built
     std::string graph_note;
+    cudaError_t refused = cudaSuccess;   // by a launch since a capture began
 };
 
 static const int STAGING_COLS = 32;
@@ -961,6 +962,14 @@ int abm_get_parents(abm_ctx* c, int* out, int cap, int* n)
     return ABM_OK;
 }
 
+// A launch whose blocks wait for one another may be refused (its blocks do not all fit).  The
+// call that made it reports that by cudaGetLastError; a capture has to know at once, since its
+// graph would be kept without the kernel.
+static void note_launch(abm_ctx* c, cudaError_t e)
+{
+    if (c->refused == cudaSuccess) c->refused = e;
+}
+
 // the neighbor set and the division (abm_build.cu)
 static void enqueue_build(abm_ctx* c, int what, int flow = FLOW_STEP)
 {
@@ -977,7 +986,7 @@ static void enqueue_build(abm_ctx* c, int what, int flow = FLOW_STEP)
     a.dp = c->dp;
     a.flags = c->div_flags; a.mothers = c->mothers; a.check = c->div_check; a.sat = c->div_sat; a.ok = c->div_ok;
     a.d1 = c->d1; a.d2 = c->d2; a.dlen = c->dlen; a.dgrowth = c->dgrowth; a.parents = c->parents_dev;
-    launch_build(a, what, c->build, c->st, flow);
+    note_launch(c, launch_build(a, what, c->build, c->st, flow));
 }
 
 // getCellNeighbors (mechanics.hpp:520-593)
@@ -997,10 +1006,10 @@ static void enqueue_growth(abm_ctx* c, int flow = FLOW_STEP) { enqueue_build(c, 
 static void enqueue_pair_force(abm_ctx* c, int with_gather, bool in_loop = false, int flow = FLOW_STEP)
 {
     ActiveList al = {c->act, c->n_act, c->keep_entry, c->gref, c->row_ptr, c->bar, 0, nullptr};
-    launch_pair_screened(c->geom, c->ctrl, c->fp, c->jkr_delta, c->jkr_radius, c->fcc, c->jbuf,
-                         c->p.precision == ABM_PRECISION_MIXED, c->cap * c->cap_nbr, c->cap, c->num_sms, c->st,
-                         with_gather, c->dims, c->p.pair_tile, c->p.pair_blocks_per_sm, c->pairs, c->surv, al, c->n_ref,
-                         in_loop ? &c->sp : nullptr, c->mlp_w, flow);
+    note_launch(c, launch_pair_screened(c->geom, c->ctrl, c->fp, c->jkr_delta, c->jkr_radius, c->fcc, c->jbuf,
+                                        c->p.precision == ABM_PRECISION_MIXED, c->cap * c->cap_nbr, c->cap, c->num_sms,
+                                        c->st, with_gather, c->dims, c->p.pair_tile, c->p.pair_blocks_per_sm, c->pairs,
+                                        c->surv, al, c->n_ref, in_loop ? &c->sp : nullptr, c->mlp_w, flow));
 }
 
 // pair_sum 1 (default): the first attempt sums each cell's shares itself; 2: a
@@ -1050,9 +1059,10 @@ static void enqueue_verlet_step(abm_ctx* c)
     {
         ForceParams fp = c->fp;
         fp.vel = phase == 0 ? c->vel : c->vel_c;
-        launch_pair_screened(phase == 0 ? c->geom : c->geom_c, c->ctrl, fp, c->jkr_delta, c->jkr_radius, c->fcc, c->jbuf,
-                             0, c->cap * c->cap_nbr, c->cap, c->num_sms, c->st, 0, c->dims, c->p.pair_tile,
-                             c->p.pair_blocks_per_sm, c->pairs, c->surv, al, c->n_ref);
+        note_launch(c, launch_pair_screened(phase == 0 ? c->geom : c->geom_c, c->ctrl, fp, c->jkr_delta, c->jkr_radius,
+                                            c->fcc, c->jbuf, 0, c->cap * c->cap_nbr, c->cap, c->num_sms, c->st, 0,
+                                            c->dims, c->p.pair_tile, c->p.pair_blocks_per_sm, c->pairs, c->surv, al,
+                                            c->n_ref));
         launch_verlet_cells(phase, a, c->ctrl, c->sp, c->cap, c->st);
     }
 }
@@ -1087,10 +1097,12 @@ static void enqueue_iteration(abm_ctx* c)
 static int capture(abm_ctx* c, void (*fn)(abm_ctx*), cudaGraphExec_t* exec)
 {
     cudaGraph_t g;
+    c->refused = cudaSuccess;
     CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
     fn(c);
     CK(cudaStreamEndCapture(c->st, &g));
-    cudaError_t inst_plain = cudaGraphInstantiate(exec, g, 0);
+    cudaError_t inst_plain = c->refused;
+    if (inst_plain == cudaSuccess) inst_plain = cudaGraphInstantiate(exec, g, 0);
     cudaGraphDestroy(g);
     CK(inst_plain);
     return ABM_OK;
@@ -1102,6 +1114,7 @@ static int capture_into(abm_ctx* c, cudaGraph_t graph, std::vector<cudaGraphNode
 {
     CK(cudaStreamBeginCaptureToGraph(c->st, graph, deps.empty() ? nullptr : deps.data(), nullptr, deps.size(),
                                      cudaStreamCaptureModeThreadLocal));
+    c->refused = cudaSuccess;
     fn();
     cudaStreamCaptureStatus status;
     const cudaGraphNode_t* leaves = nullptr;
@@ -1109,6 +1122,7 @@ static int capture_into(abm_ctx* c, cudaGraph_t graph, std::vector<cudaGraphNode
     cudaError_t info = cudaStreamGetCaptureInfo(c->st, &status, nullptr, nullptr, &leaves, &nleaves);
     std::vector<cudaGraphNode_t> next(leaves, leaves + (info == cudaSuccess ? nleaves : 0));
     CK(cudaStreamEndCapture(c->st, nullptr));
+    CK(c->refused);
     CK(info);
     deps = next;
     return ABM_OK;

@@ -623,19 +623,15 @@ LaunchShape make_shape(const void* kernel, int block, long long threads, bool cl
     return s;
 }
 
-void launch_shape(const void* kernel, const LaunchShape& shape, int block, void** args, cudaStream_t st)
+cudaError_t launch_shape(const void* kernel, const LaunchShape& shape, int block, void** args, cudaStream_t st)
 {
-    if (!shape.cluster)
-    {
-        cudaLaunchCooperativeKernel(kernel, dim3(shape.blocks), dim3(block), args, 0, st);
-        return;
-    }
+    if (!shape.cluster) return cudaLaunchCooperativeKernel(kernel, dim3(shape.blocks), dim3(block), args, 0, st);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = shape.blocks; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.gridDim = dim3(shape.blocks); cfg.blockDim = dim3(block); cfg.stream = st; cfg.attrs = at; cfg.numAttrs = 1;
-    cudaLaunchKernelExC(&cfg, kernel, args);
+    return cudaLaunchKernelExC(&cfg, kernel, args);
 }
 
 // total dE/dq of each cell from its active shares (the API paths; the loop's first attempt
@@ -656,7 +652,7 @@ __global__ void k_pair_sum_rows(const int* __restrict__ row_ptr, const int* __re
                      : sum_active_shares(jbuf + row_ptr[i], n_act[i]);
 }
 
-void launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, const double* jkr_delta,
+cudaError_t launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, const double* jkr_delta,
                           const double* jkr_radius, Gen6* fcc, double4* jbuf, int mixed, int max_entries,
                           int cap_cells, int num_sms, cudaStream_t st, int with_sum, int dims, int tile,
                           int blocks_per_sm, const int4* pairs, int* surv, ActiveList al, int cells,
@@ -692,9 +688,10 @@ void launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, const do
     al.cluster = shape.cluster;
     void* args[] = {(void*)&geom, (void*)&pairs, (void*)&ctrl, (void*)&fp, (void*)&jkr_delta, (void*)&jkr_radius,
                     (void*)&jbuf, (void*)&surv, (void*)&al, (void*)&spv, (void*)&mlp_w, (void*)&flow};
-    launch_shape(fn, shape, PS_T, args, st);
+    const cudaError_t e = launch_shape(fn, shape, PS_T, args, st);
     if (with_sum)
         k_pair_sum_rows<<<max(cdiv(cap_cells, 128), 1), 128, 0, st>>>(al.row_ptr, al.n_act, ctrl, jbuf, fcc, f32);
+    return e;
 }
 
 // the reference's 2-D dE/dq (cellCellRepulsiveForces + cellCellAdhesiveForces) from the

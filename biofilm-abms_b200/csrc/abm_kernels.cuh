@@ -56,7 +56,8 @@ struct LaunchShape {
 };
 // `threads` threads of work in blocks of `block`
 LaunchShape make_shape(const void* kernel, int block, long long threads, bool cluster, int num_sms);
-void launch_shape(const void* kernel, const LaunchShape& shape, int block, void** args, cudaStream_t st);
+// the runtime's answer: a launch that it refuses did not happen
+cudaError_t launch_shape(const void* kernel, const LaunchShape& shape, int block, void** args, cudaStream_t st);
 
 // Record of a barrier over the blocks of a cooperative launch (abm_grid.cuh)
 struct GridBar {
@@ -290,7 +291,7 @@ size_t scan_block_sums_size(int cap);
 // pass over the active pairs (both shares into jbuf), refreshing the active list when it is
 // stale; with_sum also writes each cell's total into fcc.  cells: about how many there are
 // (the launch's shape; more only take longer).
-void launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, const double* jkr_delta,
+cudaError_t launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, const double* jkr_delta,
                           const double* jkr_radius, Gen6* fcc, double4* jbuf, int mixed, int max_entries,
                           int cap_cells, int num_sms, cudaStream_t st, int with_sum, int dims, int tile,
                           int blocks_per_sm, const int4* pairs, int* surv, ActiveList al, int cells,
@@ -405,7 +406,7 @@ struct BuildArgs {
 enum BuildWhat { BUILD_NEIGHBORS, BUILD_GROWTH, BUILD_DIVIDE, BUILD_RECORDS };
 const int BUILD_CLUSTER_CELLS = 8192;
 LaunchShape build_shape(int cells, int num_sms);
-void launch_build(const BuildArgs& args, int what, const LaunchShape& shape, cudaStream_t st, int flow = FLOW_STEP);
+cudaError_t launch_build(const BuildArgs& args, int what, const LaunchShape& shape, cudaStream_t st, int flow = FLOW_STEP);
 
 // the loop graph: `todo` iterations ahead (of each of n contexts); then, once per round,
 // whether a slow iteration runs and whether another round follows
