@@ -736,7 +736,7 @@ __device__ bool divide_cells(const BuildArgs& a, int& n, int nb, BuildShared& sh
         ctrl->div_events += 1;
         ctrl->last_div_tries = tries;
         ctrl->n_divided = nd;
-        ctrl->screen_valid = 0;            // new cells: the active pair list is stale
+        ctrl->screen_valid = ctrl->path_valid = 0;     // new cells: the active pair list is stale
     }
     n += nd;
     divided = nd;
@@ -766,7 +766,7 @@ __global__ void __launch_bounds__(BD_T, 1) k_build(const __grid_constant__ Build
         if (blockIdx.x == 0 && threadIdx.x == 0) { ctrl->n_pairs = 0; ctrl->no_table = 0; }
         if (!build_barrier(a, nb)) return;
         pair_records(a, n, nb, false);
-        if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->screen_valid = 0;
+        if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->screen_valid = ctrl->path_valid = 0;
         return;
     }
     if (what == BUILD_NEIGHBORS)
@@ -797,7 +797,7 @@ __global__ void __launch_bounds__(BD_T, 1) k_build(const __grid_constant__ Build
     {
         ctrl->n_dir = n_dir;
         if (a.order) ctrl->n_order = n;
-        ctrl->screen_valid = 0;            // a new pair list makes the active list stale
+        ctrl->screen_valid = ctrl->path_valid = 0;     // a new pair list makes the active list stale
         ctrl->rebuilds += 1;
     }
 }

@@ -278,8 +278,8 @@ static void fill_tableau(StepParams& sp, int mode, bool& ok)
     sp.inv_q1 = 1.0 / (q + 1);
 }
 
-__global__ void k_set_n(Ctrl* c, int n) { c->n = n; c->halted &= HALT_LOST; c->screen_valid = 0; c->n_order = 0; }
-__global__ void k_screen_stale(Ctrl* c) { c->screen_valid = 0; }
+__global__ void k_set_n(Ctrl* c, int n) { c->n = n; c->halted &= HALT_LOST; c->screen_valid = c->path_valid = 0; c->n_order = 0; }
+__global__ void k_screen_stale(Ctrl* c) { c->screen_valid = c->path_valid = 0; }
 __global__ void k_set_halt(Ctrl* c, int n_max) { c->halt_n = n_max; c->halted &= HALT_LOST; }
 __global__ void k_set_clock(Ctrl* c, double t, double dt, int iter)
 {
@@ -1538,9 +1538,14 @@ int abm_upload_neighbors(abm_ctx* c, const double* rows, int m, int ld)
 // parameters (and network weights), loaded from a checkpoint written at an
 // iteration boundary, continues bit for bit where the uninterrupted run continues.
 //
-// File: "ABMCKP01", six int32 (dims, ncols, n, pairs m, lineage length, 0), the
-// CkState block, cells (ncols x n doubles, column-major), pair cell indices (m int32
-// i, then m int32 j, each pair once as the neighbor table lists it), lineage (int32).
+// Mixed precision has one more thing to keep: the motion sum that decides how a pass rounds
+// (Ctrl::path).
+//
+// File: "ABMCKP01", six int32 (dims, ncols, n, pairs m, lineage length, mixed), the
+// CkState block, with mixed = 1 the CkMixed block, cells (ncols x n doubles, column-major),
+// pair cell indices (m int32 i, then m int32 j, each pair once as the neighbor table lists
+// it), lineage (int32).  mixed = 0: an FP64 context's file, or one of mixed precision that was
+// written without the block; such a run resumes with its next pass rounded as after a rebuild.
 // Host byte order.
 struct CkState {
     double t, dt, dt_try, factor, last_max_error, last_trial_error, dt_prev;
@@ -1551,6 +1556,10 @@ struct CkState {
     unsigned long long st_vmax_bits, st_ovl_bits[2], st_v2_fx, st_g_fx, st_near_div;
 };
 static_assert(sizeof(CkState) % 8 == 0, "checkpoint state block is made of 8-byte fields");
+struct CkMixed {
+    double path;
+    long long path_valid;
+};
 static const char CK_MAGIC[8] = {'A', 'B', 'M', 'C', 'K', 'P', '0', '1'};
 
 static void ck_from_ctrl(const Ctrl& h, CkState& s)
@@ -1611,11 +1620,13 @@ int abm_save_checkpoint(abm_ctx* c, const char* path)
     CkState s;
     std::memset(&s, 0, sizeof(s));
     ck_from_ctrl(h, s);
-    const int hdr[6] = {c->dims, ncols, n, m, n_par, 0};
+    const int mixed = c->sp.mixed;
+    const CkMixed x = {h.path, h.path_valid};
+    const int hdr[6] = {c->dims, ncols, n, m, n_par, mixed};
     FILE* f = std::fopen(path, "wb");
     if (!f) return fail(c, ABM_ERR_ARG, std::string("cannot open ") + path + " for writing");
     bool ok = std::fwrite(CK_MAGIC, 1, 8, f) == 8 && std::fwrite(hdr, sizeof(int), 6, f) == 6 &&
-              std::fwrite(&s, sizeof(s), 1, f) == 1;
+              std::fwrite(&s, sizeof(s), 1, f) == 1 && (!mixed || std::fwrite(&x, sizeof(x), 1, f) == 1);
     if (ok && n > 0) ok = std::fwrite(cells.data(), sizeof(double), (size_t)n * ncols, f) == (size_t)n * ncols;
     if (ok && m > 0) ok = std::fwrite(pairs.data(), sizeof(int), pairs.size(), f) == pairs.size();
     if (ok && n_par > 0) ok = std::fwrite(parents.data(), sizeof(int), parents.size(), f) == parents.size();
@@ -1632,8 +1643,10 @@ int abm_load_checkpoint(abm_ctx* c, const char* path)
     char magic[8];
     int hdr[6];
     CkState s;
+    CkMixed x = {0.0, 0};
     bool ok = std::fread(magic, 1, 8, f) == 8 && std::memcmp(magic, CK_MAGIC, 8) == 0 &&
-              std::fread(hdr, sizeof(int), 6, f) == 6 && std::fread(&s, sizeof(s), 1, f) == 1;
+              std::fread(hdr, sizeof(int), 6, f) == 6 && std::fread(&s, sizeof(s), 1, f) == 1 &&
+              (hdr[5] == 0 || (hdr[5] == 1 && std::fread(&x, sizeof(x), 1, f) == 1));
     const int dims = ok ? hdr[0] : 0, ncols = ok ? hdr[1] : 0, n = ok ? hdr[2] : -1, m = ok ? hdr[3] : -1,
               n_par = ok ? hdr[4] : -1;
     if (!ok || n < 0 || m < 0 || n_par < 0 || ncols <= 0 || ncols > STAGING_COLS)
@@ -1659,7 +1672,7 @@ int abm_load_checkpoint(abm_ctx* c, const char* path)
     if (ok) ok = std::fgetc(f) == EOF;                // nothing after the lineage
     std::fclose(f);
     if (!ok) return fail(c, ABM_ERR_ARG, std::string("truncated or oversized checkpoint: ") + path);
-    if (!(s.dt > 0) || s.iter < 0 || s.iter > INT_MAX || s.hist_pos < 0 || s.hist_pos >= HIST)
+    if (!(s.dt > 0) || s.iter < 0 || s.iter > INT_MAX || s.hist_pos < 0 || s.hist_pos >= HIST || !(x.path >= 0))
         return fail(c, ABM_ERR_ARG, "the checkpoint's clock or controller history is out of range");
     // the checks abm_upload_neighbors makes, before anything reaches the context, so
     // that a rejected file leaves it as it was
@@ -1683,6 +1696,8 @@ int abm_load_checkpoint(abm_ctx* c, const char* path)
     CK(cudaMemcpyAsync(&h, c->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     ck_to_ctrl(s, h);
+    h.path = x.path;
+    h.path_valid = x.path_valid != 0;
     CK(cudaMemcpy(c->ctrl, &h, sizeof(Ctrl), cudaMemcpyHostToDevice));
     return ABM_OK;
 }

@@ -463,9 +463,9 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
     const bool split = PROPOSE && gridDim.x > 1;
     const bool proposer = split && blockIdx.x == gridDim.x - 1;
     const int work_blocks = split ? gridDim.x - 1 : gridDim.x;
-    auto stale = [&](double moved) { return !ctrl->screen_valid || !(2.0 * moved * (1.0 + 1e-6) + 1e-9 < fp.skin); };
-    const bool refresh = stale(ctrl->drift);
-    const int rounding = MIXED && stale(ctrl->path) ? ROUND_STALE : ROUND_LIST;
+    auto stale = [&](int valid, double moved) { return !valid || !(2.0 * moved * (1.0 + 1e-6) + 1e-9 < fp.skin); };
+    const bool refresh = stale(ctrl->screen_valid, ctrl->drift);
+    const int rounding = MIXED && stale(ctrl->path_valid, ctrl->path) ? ROUND_STALE : ROUND_LIST;
     const int lane = threadIdx.x & 31;
     const int stride = work_blocks * blockDim.x;
     double ovl_max = 0.0;
@@ -574,7 +574,7 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
             ctrl->screen_valid = 1;
             ctrl->drift = 0.0;
         }
-        if (restart) ctrl->path = 0.0;
+        if (restart) { ctrl->path = 0.0; ctrl->path_valid = 1; }
         if (fp.fric && !VERLET)
         {
             // the candidates of this pass; no stage has a changed decision yet

@@ -136,8 +136,11 @@ struct Ctrl {
     // mixed precision: the sum over the accepted steps of the largest motion in each.  A pass
     // whose list would be stale by this sum takes ROUND_STALE (dist_geom_mixed), whether or not
     // the list is stale by `drift`: the rule keeps mixed-precision trajectories bit for bit.
+    // A loaded checkpoint brings the sum and path_valid back, so that the first pass after it
+    // rounds as the uninterrupted run's does, although its list has to be made anew.
     double path;
     unsigned long long path_bits;
+    int path_valid;                     // as screen_valid, but for a loaded checkpoint
     // the loop graph (LoopFlow): iterations still to take, and why the plain ones wait
     int todo;
     int hold;                           // LoopHold

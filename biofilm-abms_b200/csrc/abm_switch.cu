@@ -208,7 +208,7 @@ __global__ void k_basal_commit(Ctrl* ctrl)
     if (m >= ctrl->n) return;
     ctrl->basal_dropped += ctrl->n - m;
     ctrl->n = m;
-    ctrl->screen_valid = 0;          // the active pair list names the old rows
+    ctrl->screen_valid = ctrl->path_valid = 0;     // the active pair list names the old rows
     ctrl->n_order = 0;
 }
 
