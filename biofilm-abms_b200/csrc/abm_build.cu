@@ -803,10 +803,11 @@ __global__ void __launch_bounds__(BD_T, 1) k_build(const __grid_constant__ Build
 }
 
 // The blocks of a launch for about `cells` cells (more only take longer): one cluster of up to
-// 16 for a small colony, else a cooperative grid of up to two per SM, 4 threads a cell.
-LaunchShape build_shape(int cells, int num_sms)
+// 16 for a small colony, else a cooperative grid of up to two per SM, BD_SEARCH threads a cell.
+LaunchShape build_shape(int cells, int num_sms, int share)
 {
-    return make_shape((const void*)k_build, BD_T, (long long)cells * BD_SEARCH, cells <= BUILD_CLUSTER_CELLS, num_sms);
+    return make_shape((const void*)k_build, BD_T, (long long)cells * BD_SEARCH, cells <= BUILD_CLUSTER_CELLS, num_sms,
+                      share);
 }
 
 cudaError_t launch_build(const BuildArgs& args, int what, const LaunchShape& shape, cudaStream_t st, int flow)

@@ -39,6 +39,7 @@ struct abm_ctx {
     int2* part = nullptr;
     int n_seen = 0;                  // cells when the host last looked
     int n_ref = 0;                   // cells that the launches are shaped for
+    int share = 1;                   // and the contexts that they share the device with (a batch)
     LaunchShape build;               // of the build launch
     int *bin_count = nullptr, *bin_start = nullptr, *key = nullptr, *slot = nullptr, *sorted_cell = nullptr,
         *sorted_key = nullptr;
@@ -732,7 +733,7 @@ static void shape_launches(abm_ctx* c)
     const int ref = std::min(c->cap, std::max(2 * n, 256));
     if (ref == c->n_ref) return;
     c->n_ref = ref;
-    c->build = build_shape(ref, c->num_sms);
+    c->build = build_shape(ref, c->num_sms, c->share);
     drop_iteration_graphs(c);
 }
 
@@ -1009,7 +1010,7 @@ static void enqueue_pair_force(abm_ctx* c, int with_gather, bool in_loop = false
     note_launch(c, launch_pair_screened(c->geom, c->ctrl, c->fp, c->jkr_delta, c->jkr_radius, c->fcc, c->jbuf,
                                         c->p.precision == ABM_PRECISION_MIXED, c->cap * c->cap_nbr, c->cap, c->num_sms,
                                         c->st, with_gather, c->dims, c->p.pair_tile, c->p.pair_blocks_per_sm, c->pairs,
-                                        c->surv, al, c->n_ref, in_loop ? &c->sp : nullptr, c->mlp_w, flow));
+                                        c->surv, al, c->n_ref, c->share, in_loop ? &c->sp : nullptr, c->mlp_w, flow));
 }
 
 // pair_sum 1 (default): the first attempt sums each cell's shares itself; 2: a
@@ -1062,7 +1063,7 @@ static void enqueue_verlet_step(abm_ctx* c)
         note_launch(c, launch_pair_screened(phase == 0 ? c->geom : c->geom_c, c->ctrl, fp, c->jkr_delta, c->jkr_radius,
                                             c->fcc, c->jbuf, 0, c->cap * c->cap_nbr, c->cap, c->num_sms, c->st, 0,
                                             c->dims, c->p.pair_tile, c->p.pair_blocks_per_sm, c->pairs, c->surv, al,
-                                            c->n_ref));
+                                            c->n_ref, c->share));
         launch_verlet_cells(phase, a, c->ctrl, c->sp, c->cap, c->st);
     }
 }
@@ -2174,6 +2175,16 @@ void batch_free(abm_batch* b)
     if (b->st) cudaStreamDestroy(b->st);
 }
 
+// the shapes of the launches that a batch captures: each context's share of the device
+void set_share(abm_batch* b, int share)
+{
+    for (abm_ctx* c : b->ctxs)
+    {
+        c->share = share;
+        c->build = build_shape(c->n_ref, c->num_sms, share);
+    }
+}
+
 // one graph: every context's next iteration as an independent branch
 int batch_iteration_graph(abm_batch* b)
 {
@@ -2261,6 +2272,7 @@ int abm_batch_create(abm_ctx* const* ctxs, int n, abm_batch** out)
     }
     int rc = ABM_OK;
     cudaGraph_t GR = nullptr;
+    set_share(b, n);
     do {
         if (cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming) != cudaSuccess)
@@ -2285,6 +2297,7 @@ int abm_batch_create(abm_ctx* const* ctxs, int n, abm_batch** out)
         if (!rc && !b->g_loop) rc = batch_iteration_graph(b);
     } while (0);
     if (GR) cudaGraphDestroy(GR);
+    set_share(b, 1);
     if (rc) { batch_free(b); delete b; return rc; }
     *out = b;
     return ABM_OK;
@@ -2314,7 +2327,13 @@ int abm_batch_iterate(abm_batch* b, int n_iters)
         else
         {
             run = 1;
-            if (!b->g_iter) { int rc = batch_iteration_graph(b); if (rc) return rc; }
+            if (!b->g_iter)
+            {
+                set_share(b, n);
+                const int rc = batch_iteration_graph(b);
+                set_share(b, 1);
+                if (rc) return rc;
+            }
             BK(cudaGraphLaunch(b->g_iter, b->st));
         }
         it += run;

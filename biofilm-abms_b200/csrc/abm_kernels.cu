@@ -593,7 +593,7 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
 
 // A cluster of 16 blocks is more than the portable 8: allowed per kernel, and used only where
 // the device can place one.
-LaunchShape make_shape(const void* kernel, int block, long long threads, bool cluster, int num_sms)
+LaunchShape make_shape(const void* kernel, int block, long long threads, bool cluster, int num_sms, int share)
 {
     const int MAX_CLUSTER = 16;
     LaunchShape s;
@@ -619,7 +619,8 @@ LaunchShape make_shape(const void* kernel, int block, long long threads, bool cl
     }
     int occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, block, 0);
-    s.blocks = (int)min(want, (long long)num_sms * max(occ, 1));
+    // a share of the chip, but no less than the largest cluster
+    s.blocks = (int)min(want, (long long)max(num_sms * max(occ, 1) / max(share, 1), min(MAX_CLUSTER, num_sms)));
     return s;
 }
 
@@ -653,11 +654,10 @@ __global__ void k_pair_sum_rows(const int* __restrict__ row_ptr, const int* __re
 }
 
 cudaError_t launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, const double* jkr_delta,
-                          const double* jkr_radius, Gen6* fcc, double4* jbuf, int mixed, int max_entries,
-                          int cap_cells, int num_sms, cudaStream_t st, int with_sum, int dims, int tile,
-                          int blocks_per_sm, const int4* pairs, int* surv, ActiveList al, int cells,
-                          const StepParams* sp,
-                          const float* mlp_w, int flow)
+                                 const double* jkr_radius, Gen6* fcc, double4* jbuf, int mixed, int max_entries,
+                                 int cap_cells, int num_sms, cudaStream_t st, int with_sum, int dims, int tile,
+                                 int blocks_per_sm, const int4* pairs, int* surv, ActiveList al, int cells, int share,
+                                 const StepParams* sp, const float* mlp_w, int flow)
 {
     // sp (the loop's pass): the last block also runs the step-size proposal
     StepParams spv{};
@@ -677,12 +677,13 @@ cudaError_t launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, c
     // caps them per SM).
     LaunchShape shape;
     if (tile <= 0 && blocks_per_sm <= 0)
-        shape = make_shape(fn, PS_T, 2LL * cells + (p ? PS_T : 0), cells <= BUILD_CLUSTER_CELLS / 2, num_sms);
+        shape = make_shape(fn, PS_T, 2LL * cells + (p ? PS_T : 0), cells <= BUILD_CLUSTER_CELLS / 2, num_sms,
+                           share);
     else
     {
         const int max_pairs = max(max_entries / 2, 1);
         shape = make_shape(fn, PS_T, (long long)PS_T * cdiv(max_pairs, tile <= 0 ? 1024 : min(tile, PS_TILE_MAX)), false,
-                           num_sms);
+                           num_sms, share);
         if (blocks_per_sm > 0) shape.blocks = min(shape.blocks, num_sms * blocks_per_sm);
     }
     al.cluster = shape.cluster;

@@ -54,8 +54,12 @@ struct LaunchShape {
     int blocks = 1;
     int cluster = 0;
 };
-// `threads` threads of work in blocks of `block`
-LaunchShape make_shape(const void* kernel, int block, long long threads, bool cluster, int num_sms);
+// `threads` threads of work in blocks of `block`.  share: the contexts that run side by side in
+// a batch.  A cooperative grid starts when all its blocks have room, so one that fills the chip
+// waits for every other context's work and holds up theirs: a batch of 24 growing colonies of
+// 20,000 cells took 2.8 ms an iteration with whole-chip grids (2.6 as the chain of plain kernels
+// before them) and takes 0.97 with a 24th of the chip each; 8 of them at rest 108 and 56 us.
+LaunchShape make_shape(const void* kernel, int block, long long threads, bool cluster, int num_sms, int share);
 // the runtime's answer: a launch that it refuses did not happen
 cudaError_t launch_shape(const void* kernel, const LaunchShape& shape, int block, void** args, cudaStream_t st);
 
@@ -293,12 +297,12 @@ size_t scan_block_sums_size(int cap);
 
 // pass over the active pairs (both shares into jbuf), refreshing the active list when it is
 // stale; with_sum also writes each cell's total into fcc.  cells: about how many there are
-// (the launch's shape; more only take longer).
+// (the launch's shape; more only take longer); share: as for make_shape.
 cudaError_t launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, const double* jkr_delta,
-                          const double* jkr_radius, Gen6* fcc, double4* jbuf, int mixed, int max_entries,
-                          int cap_cells, int num_sms, cudaStream_t st, int with_sum, int dims, int tile,
-                          int blocks_per_sm, const int4* pairs, int* surv, ActiveList al, int cells,
-                          const StepParams* sp = nullptr, const float* mlp_w = nullptr, int flow = FLOW_STEP);
+                                 const double* jkr_radius, Gen6* fcc, double4* jbuf, int mixed, int max_entries,
+                                 int cap_cells, int num_sms, cudaStream_t st, int with_sum, int dims, int tile,
+                                 int blocks_per_sm, const int4* pairs, int* surv, ActiveList al, int cells, int share,
+                                 const StepParams* sp = nullptr, const float* mlp_w = nullptr, int flow = FLOW_STEP);
 // kind: MODE_TRIAL / MODE_RETRY / MODE_FINAL for the loop, 3 = evaluation for the API
 // (writes candidates and errors without touching the controller)
 // cond / use_cond: WHILE-node handle that the trial and retry attempts set to 1
@@ -408,7 +412,7 @@ struct BuildArgs {
 };
 enum BuildWhat { BUILD_NEIGHBORS, BUILD_GROWTH, BUILD_DIVIDE, BUILD_RECORDS };
 const int BUILD_CLUSTER_CELLS = 8192;
-LaunchShape build_shape(int cells, int num_sms);
+LaunchShape build_shape(int cells, int num_sms, int share = 1);
 cudaError_t launch_build(const BuildArgs& args, int what, const LaunchShape& shape, cudaStream_t st, int flow = FLOW_STEP);
 
 // the loop graph: `todo` iterations ahead (of each of n contexts); then, once per round,

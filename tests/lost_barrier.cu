@@ -90,7 +90,7 @@ int main()
     al.act = marked<int4>(n * cap_nbr / 2 + 1); al.n_act = marked<int>(n); al.keep = marked<unsigned char>(n * cap_nbr);
     al.gref = marked<Geom>(n); al.row_ptr = a.row_ptr; al.bar = bar;
     launch_pair_screened(geom, ctrl, fp, nullptr, nullptr, fcc, jbuf, 0, n * cap_nbr, n, 148, 0, 1, 3, 0, 0, a.pairs,
-                         marked<int>(n * cap_nbr / 2 + 1), al, n);
+                         marked<int>(n * cap_nbr / 2 + 1), al, n, 1);
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
     EXPECT(untouched(a.bin_count, bins) && untouched(a.bin_start, 2 * bins) && untouched(a.row_ptr, n + 1));
