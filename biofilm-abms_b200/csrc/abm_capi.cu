@@ -21,6 +21,64 @@
 
 using namespace abm;
 
+// How many cells each of one or several contexts holds, as far as the host knows.  Where they
+// divide, the host has the counts copied out after some iterations and reads what has arrived,
+// without a wait unless it is LOOK_AHEAD looks ahead of the device.
+const int LOOK_EVERY = 64;              // iterations, at least, from one look to the next
+const int LOOK_AHEAD = 8;
+const int LOOK_RUN = 256;               // iterations, at most, of one launch where cells divide
+struct CountLooks {
+    std::vector<int> n = {0};
+    int* arrived = nullptr;             // pinned: LOOK_AHEAD rings of the counts
+    cudaEvent_t ev[LOOK_AHEAD] = {};
+    long long taken = 0, read = 0;
+    int since = 0;                      // iterations since the last look
+    bool off = false;                   // no pinned memory for them
+
+    // the host has the count by itself: the looks under way are older
+    void seen(int cells) { n[0] = cells; read = taken; }
+    // copy the counts, `from` in device memory, out behind the work on `st`
+    cudaError_t take(const int* from, cudaStream_t st)
+    {
+        cudaError_t e = cudaSuccess;
+        const size_t m = n.size();
+        since = 0;
+        if (!arrived && !off)
+        {
+            off = cudaMallocHost(&arrived, LOOK_AHEAD * m * sizeof(int)) != cudaSuccess;
+            if (off) arrived = nullptr;
+            for (cudaEvent_t& v : ev) off = off || cudaEventCreateWithFlags(&v, cudaEventDisableTiming) != cudaSuccess;
+            if (off) { free(); cudaGetLastError(); }
+        }
+        if (off) return e;
+        if (taken - read == LOOK_AHEAD && (e = read_arrived()) != cudaSuccess) return e;
+        const int slot = (int)(taken % LOOK_AHEAD);
+        if ((e = cudaMemcpyAsync(arrived + slot * m, from, m * sizeof(int), cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+            (e = cudaEventRecord(ev[slot], st)) != cudaSuccess)
+            return e;
+        taken += 1;
+        return e;
+    }
+    cudaError_t read_arrived()
+    {
+        const size_t m = n.size();
+        for (; read < taken; ++read)
+        {
+            const int slot = (int)(read % LOOK_AHEAD);
+            const cudaError_t e = taken - read == LOOK_AHEAD ? cudaEventSynchronize(ev[slot]) : cudaEventQuery(ev[slot]);
+            if (e == cudaErrorNotReady) { cudaGetLastError(); break; }
+            if (e != cudaSuccess) return e;
+            n.assign(arrived + slot * m, arrived + (slot + 1) * m);
+        }
+        return cudaSuccess;
+    }
+    void free()
+    {
+        for (cudaEvent_t& v : ev) if (v) { cudaEventDestroy(v); v = nullptr; }
+        if (arrived) { cudaFreeHost(arrived); arrived = nullptr; }
+    }
+};
+
 struct abm_ctx {
     abm_params p;
     std::string err;
@@ -37,7 +95,7 @@ struct abm_ctx {
     Ctrl* ctrl = nullptr;
     int* bbox = nullptr;
     int2* part = nullptr;
-    int n_seen = 0;                  // cells when the host last looked
+    CountLooks looks;                // how many cells there are, as far as the host knows
     int n_ref = 0;                   // cells that the launches are shaped for
     int share = 1;                   // and the contexts that they share the device with (a batch)
     LaunchShape build;               // of the build launch
@@ -220,6 +278,7 @@ static void free_all(abm_ctx* c)
                     c->keep_rank, c->feta, c->fbuf, c->fmask, c->fr_list, c->ystage, c->snap_feta, c->pbuf,
                     c->whalf};
     for (void* q : ptrs) if (q) cudaFree(q);
+    c->looks.free();
     if (c->st) cudaStreamDestroy(c->st);
 }
 
@@ -724,15 +783,18 @@ int abm_basal_dropped(abm_ctx* c, long long* dropped)
 }
 
 // The build launch and the pair pass are shaped for twice the cells that the host last knew
-// of (any number runs; a colony that has outgrown its shape only takes longer).  Called when
-// the host learns the number; a new shape drops the graphs, which hold the old one.
+// of.  Any number runs, but a colony that has outgrown its shape takes longer: one grown from 32
+// to 3,800 cells in one call 0.73 s with its first shape, 0.47 when the shape follows.  Called
+// where the host may have learnt the number; a new shape drops the graphs, which hold the old
+// one (once in a doubling).
 static void shape_launches(abm_ctx* c)
 {
-    const int n = c->n_seen;
+    const int n = c->looks.n[0];
     if (c->n_ref > 0 && n <= c->n_ref && 8LL * n >= c->n_ref) return;
-    const int ref = std::min(c->cap, std::max(2 * n, 256));
+    const int ref = (int)std::min<long long>(c->cap, std::max(2LL * n, 256LL));
     if (ref == c->n_ref) return;
     c->n_ref = ref;
+    if (c->g_iter || c->g_iter_k || c->g_loop) cudaStreamSynchronize(c->st);     // they may be running
     c->build = build_shape(ref, c->num_sms, c->share);
     drop_iteration_graphs(c);
 }
@@ -764,7 +826,8 @@ int abm_upload_cells(abm_ctx* c, const double* cm, int n, int ncols, int ld)
     k_set_n<<<1, 1, 0, c->st>>>(c->ctrl, n);
     CK(cudaGetLastError());
     if (c->n_host != n) c->nbrs_valid = false;
-    c->n_host = c->n_seen = n;
+    c->n_host = n;
+    c->looks.seen(n);
     c->cells_loaded = true;
     shape_launches(c);
     // division is possible when a cell already exceeds Ldiv or any cell can grow
@@ -794,7 +857,8 @@ int abm_download_cells(abm_ctx* c, double* cm, int ld)
     CK(cudaMemcpyAsync(&h, c->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     int n = h.n;
-    c->n_host = c->n_seen = n;
+    c->n_host = n;
+    c->looks.seen(n);
     if (ld < n) return fail(c, ABM_ERR_ARG, "ld smaller than the cell count");
     if (n > 0)
     {
@@ -904,7 +968,7 @@ int abm_get_num_cells(abm_ctx* c, int* n)
     CK(cudaMemcpyAsync(&h, c->ctrl, sizeof(Ctrl), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
     *n = h.n;
-    c->n_seen = h.n;
+    c->looks.seen(h.n);
     return ABM_OK;
 }
 
@@ -1034,7 +1098,7 @@ static AttemptArgs loop_attempt(abm_ctx* c, int flow = FLOW_STEP)
     c->sp.Ldiv = c->p.Ldiv;
     a.geom = c->geom; a.vel = c->vel; a.phys = c->phys; a.fcc = c->fcc; a.ctrl = c->ctrl; a.sp = &c->sp;
     a.geom_c = c->geom_c; a.vel_c = c->vel_c; a.k0buf = c->k0buf; a.cap_cells = c->cap;
-    a.cells = c->n_seen; a.num_sms = c->num_sms;
+    a.cells = c->looks.n[0]; a.num_sms = c->num_sms;
     a.pg = {sum_in_attempt(c) ? (f32 ? 3 : 2) : 0, c->row_ptr, c->n_act, c->jbuf, c->fcc, c->gref,
             c->fbuf, c->fmask, c->ystage, c->cap};
     return a;
@@ -1442,6 +1506,9 @@ static int build_iteration_graph(abm_ctx* c)
     return ABM_OK;
 }
 
+// can the colony outgrow the shape of its launches?
+static bool may_outgrow(const abm_ctx* c) { return c->div_enabled && c->n_ref < c->cap; }
+
 static int ready_for_forces(abm_ctx* c)
 {
     if (!c->cells_loaded) return fail(c, ABM_ERR_STATE, "no cells uploaded");
@@ -1453,6 +1520,7 @@ int abm_build_neighbors(abm_ctx* c, int* m)
 {
     if (!c) return ABM_ERR_ARG;
     if (!c->cells_loaded) return fail(c, ABM_ERR_STATE, "no cells uploaded");
+    shape_launches(c);
     enqueue_rebuild(c);
     CK(cudaGetLastError());
     c->nbrs_valid = true;
@@ -1818,6 +1886,7 @@ int abm_divide(abm_ctx* c, int* n_divided)
 {
     if (!c) return ABM_ERR_ARG;
     if (!c->cells_loaded) return fail(c, ABM_ERR_STATE, "no cells uploaded");
+    shape_launches(c);
     enqueue_build(c, BUILD_DIVIDE);
     CK(cudaGetLastError());
     int rc = check_status(c);
@@ -1826,6 +1895,7 @@ int abm_divide(abm_ctx* c, int* n_divided)
     if (n_divided) *n_divided = h.n_divided;
     if (h.n_divided > 0) c->nbrs_valid = false;
     c->n_host = h.n;
+    c->looks.seen(h.n);
     return rc;
 }
 
@@ -1857,8 +1927,30 @@ int abm_get_stats(abm_ctx* c, abm_stats* s)
     s->t = h.t; s->dt = h.dt; s->last_max_error = h.last_max_error;
     s->n_cells = h.n; s->n_pairs = h.n_dir / 2;
     s->rejected = h.rejected; s->log_rows = h.log_rows; s->cell_steps = h.cell_steps;
-    c->n_seen = h.n;
+    c->looks.seen(h.n);
     return check_status(c);
+}
+
+// the graph that the next `n_iters` iterations run by, made if there is none
+static int ready_graphs(abm_ctx* c, int n_iters)
+{
+    int rc = ABM_OK;
+    const bool loop = has_loop(c) && n_iters >= LOOP_FAST / 2;
+    if (!(loop ? c->g_loop : c->g_iter) && !c->graph_fallback)
+    {
+        rc = loop ? build_loop_graph(c) : build_iteration_graph(c);
+        if (rc)
+        {
+            // conditional nodes unavailable: keep the error for abm_graph_info and fall back to
+            // a straight-line graph (retries exit early) with division decided on the host
+            c->graph_note = c->err;
+            c->graph_fallback = true;
+            cudaGetLastError();
+            drop_iteration_graphs(c);
+        }
+    }
+    if (c->graph_fallback && !c->g_iter) return capture(c, enqueue_iteration, &c->g_iter);
+    return ABM_OK;
 }
 
 int abm_iterate(abm_ctx* c, int n_iters, int n_cells_stop, abm_stats* stats)
@@ -1868,33 +1960,17 @@ int abm_iterate(abm_ctx* c, int n_iters, int n_cells_stop, abm_stats* stats)
     if (rc) return rc;
     if (c->sp.network && !c->mlp_loaded)
         return fail(c, ABM_ERR_STATE, "the learned controller needs weights (abm_stepsize_set_weights)");
+    if (may_outgrow(c)) CK(c->looks.read_arrived());
+    shape_launches(c);
     if (!c->nbrs_valid)
     {
         enqueue_rebuild(c);
         c->nbrs_valid = true;
     }
-    shape_launches(c);
     c->iter_k = 1;
     for (int k : {10, 5, 4, 2})
         if (c->p.iter_update_neighbors % k == 0) { c->iter_k = k; break; }
-    if (c->p.use_graphs)
-    {
-        const bool loop = has_loop(c) && n_iters >= LOOP_FAST / 2;
-        if (!(loop ? c->g_loop : c->g_iter) && !c->graph_fallback)
-        {
-            rc = loop ? build_loop_graph(c) : build_iteration_graph(c);
-            if (rc)
-            {
-                // conditional nodes unavailable: keep the error for abm_graph_info and fall back to
-                // a straight-line graph (retries exit early) with division decided on the host
-                c->graph_note = c->err;
-                c->graph_fallback = true;
-                cudaGetLastError();
-                drop_iteration_graphs(c);
-            }
-        }
-        if (c->graph_fallback && !c->g_iter) { rc = capture(c, enqueue_iteration, &c->g_iter); if (rc) return rc; }
-    }
+    if (c->p.use_graphs && (rc = ready_graphs(c, n_iters))) return rc;
     for (int k = 0, next_check = 0; k < n_iters;)
     {
         if (n_cells_stop > 0 && c->div_enabled && k >= next_check)
@@ -1904,6 +1980,14 @@ int abm_iterate(abm_ctx* c, int n_iters, int n_cells_stop, abm_stats* stats)
             CK(cudaStreamSynchronize(c->st));
             if (h.n >= n_cells_stop) break;
             next_check = k + 16;
+            c->looks.seen(h.n);
+        }
+        if (may_outgrow(c))
+        {
+            if (c->looks.since >= LOOK_EVERY) CK(c->looks.take(&c->ctrl->n, c->st));
+            CK(c->looks.read_arrived());
+            shape_launches(c);
+            if (c->p.use_graphs && (rc = ready_graphs(c, n_iters))) return rc;
         }
         int step = 1;
         if (c->p.use_graphs && !c->graph_fallback)
@@ -1924,6 +2008,7 @@ int abm_iterate(abm_ctx* c, int n_iters, int n_cells_stop, abm_stats* stats)
                 }
                 run = std::min(run, kk - k);
             }
+            if (may_outgrow(c) && run >= LOOK_RUN + LOOP_FAST) run = LOOK_RUN;
             if (has_loop(c) && run >= LOOP_FAST / 2 && c->g_loop)
             {
                 rc = launch_loop(c, run);
@@ -1961,6 +2046,7 @@ int abm_iterate(abm_ctx* c, int n_iters, int n_cells_stop, abm_stats* stats)
             else enqueue_iteration(c);
         }
         c->host_iter += step;
+        c->looks.since += step;
         k += step;
         // with the post-step kernels on, the periodic rebuild is part of the iteration
         if (!c->post_on && c->host_iter % c->p.iter_update_neighbors == 0)
@@ -2142,8 +2228,11 @@ struct abm_batch {
     cudaStream_t st = nullptr;
     cudaGraphExec_t g_iter = nullptr, g_rebuild = nullptr;
     cudaGraphExec_t g_loop = nullptr;    // the loop graphs of all contexts, or null
-    Ctrl** ctrls = nullptr;              // their control records, and whether their cells may
-    int* divides = nullptr;              // divide (device arrays)
+    Ctrl** ctrls = nullptr;              // their control records, whether their cells may divide,
+    int *divides = nullptr, *counts = nullptr;       // and a copy of their counts (device arrays)
+    CountLooks looks;
+    std::vector<int> refs;               // cells that the graphs' launches are shaped for
+    bool follow = true;                  // make the graphs anew where a colony outgrows its shape
     int k_rebuild = 100;
     std::vector<cudaEvent_t> ev;
     cudaEvent_t done = nullptr;
@@ -2169,6 +2258,8 @@ void batch_free(abm_batch* b)
     if (b->g_loop) cudaGraphExecDestroy(b->g_loop);
     if (b->ctrls) cudaFree(b->ctrls);
     if (b->divides) cudaFree(b->divides);
+    if (b->counts) cudaFree(b->counts);
+    b->looks.free();
     if (b->g_rebuild) cudaGraphExecDestroy(b->g_rebuild);
     for (cudaEvent_t e : b->ev) cudaEventDestroy(e);
     if (b->done) cudaEventDestroy(b->done);
@@ -2185,56 +2276,124 @@ void set_share(abm_batch* b, int share)
     }
 }
 
-// one graph: every context's next iteration as an independent branch
-int batch_iteration_graph(abm_batch* b)
+// one graph of every context's branch
+template <class APPEND>
+int batch_graph(abm_batch* b, const char* what, cudaGraphExec_t* exec, APPEND append)
 {
     cudaGraph_t G = nullptr;
     BK(cudaGraphCreate(&G, 0));
     int rc = ABM_OK;
+    set_share(b, (int)b->ctxs.size());
     for (abm_ctx* c : b->ctxs)
     {
         std::vector<cudaGraphNode_t> deps;
-        rc = append_iteration(c, G, deps);
-        if (rc) { rc = batch_fail(b, rc, "iteration graph of a context: " + c->err); break; }
+        rc = append(c, G, deps);
+        if (rc) { rc = batch_fail(b, rc, std::string(what) + " graph of a context: " + c->err); break; }
     }
+    set_share(b, 1);
+    cudaGraphExec_t made = nullptr;
     cudaError_t inst = cudaSuccess;
-    if (!rc) inst = cudaGraphInstantiate(&b->g_iter, G, 0);
+    if (!rc) inst = cudaGraphInstantiate(&made, G, 0);
     cudaGraphDestroy(G);
     if (rc) return rc;
     BK(inst);
+    if (*exec) cudaGraphExecDestroy(*exec);
+    *exec = made;
     return ABM_OK;
 }
 
-// one graph: every context's loop as an independent branch, each at its own pace up to the
-// joint rebuild
+// every context's next iteration
+int batch_iteration_graph(abm_batch* b)
+{
+    return batch_graph(b, "iteration", &b->g_iter, [](abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode_t>& deps) {
+        return append_iteration(c, G, deps);
+    });
+}
+
+// every context's loop, each at its own pace up to the joint rebuild
 int batch_loop_graph(abm_batch* b)
+{
+    for (abm_ctx* c : b->ctxs) if (!has_loop(c)) return ABM_OK;
+    return batch_graph(b, "loop", &b->g_loop, [](abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode_t>& deps) {
+        return append_loop(c, G, deps);
+    });
+}
+
+int batch_rebuild_graph(abm_batch* b)
+{
+    return batch_graph(b, "rebuild", &b->g_rebuild, [](abm_ctx* c, cudaGraph_t G, std::vector<cudaGraphNode_t>& deps) {
+        return capture_into(c, G, deps, [&]() { enqueue_rebuild(c); });
+    });
+}
+
+int batch_graphs(abm_batch* b)
+{
+    int rc = batch_rebuild_graph(b);
+    if (!rc) rc = batch_loop_graph(b);
+    if (!rc && (!b->g_loop || b->g_iter)) rc = batch_iteration_graph(b);
+    b->refs.clear();
+    for (const abm_ctx* c : b->ctxs) b->refs.push_back(c->n_ref);
+    return rc;
+}
+
+int batch_arrays(abm_batch* b)
 {
     std::vector<Ctrl*> ctrls;
     std::vector<int> divides;
     for (abm_ctx* c : b->ctxs)
     {
-        if (!has_loop(c)) return ABM_OK;
         ctrls.push_back(c->ctrl);
         divides.push_back(c->div_enabled ? 1 : 0);
     }
+    b->looks.n.assign(b->ctxs.size(), 0);
+    BK(cudaMalloc(&b->counts, divides.size() * sizeof(int)));
     BK(cudaMalloc(&b->divides, divides.size() * sizeof(int)));
     BK(cudaMemcpy(b->divides, divides.data(), divides.size() * sizeof(int), cudaMemcpyHostToDevice));
     BK(cudaMalloc(&b->ctrls, ctrls.size() * sizeof(Ctrl*)));
     BK(cudaMemcpy(b->ctrls, ctrls.data(), ctrls.size() * sizeof(Ctrl*), cudaMemcpyHostToDevice));
-    cudaGraph_t G = nullptr;
-    BK(cudaGraphCreate(&G, 0));
-    int rc = ABM_OK;
-    for (abm_ctx* c : b->ctxs)
+    return ABM_OK;
+}
+
+__global__ void k_counts(Ctrl* const* ctrls, int n, int* out)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < n) out[k] = ctrls[k]->n;
+}
+
+// Look at the counts, and where a context has outgrown the shape of its launches, shape those of
+// all contexts that have grown for their present sizes and make the graphs anew (a doubling of
+// the batch costs one such stop).  Graphs that cannot be made leave the old ones, which run any
+// number of cells.
+int batch_follow(abm_batch* b)
+{
+    bool any = false, grown = false;
+    const int n = (int)b->ctxs.size();
+    auto may_grow = [&](int k) { return b->ctxs[k]->div_enabled && b->refs[k] < b->ctxs[k]->cap; };
+    for (int k = 0; k < n; ++k) any = any || may_grow(k);
+    if (!any || !b->follow) return ABM_OK;
+    if (b->looks.since >= LOOK_EVERY)
     {
-        std::vector<cudaGraphNode_t> deps;
-        rc = append_loop(c, G, deps);
-        if (rc) { rc = batch_fail(b, rc, "loop graph of a context: " + c->err); break; }
+        k_counts<<<(n + 127) / 128, 128, 0, b->st>>>(b->ctrls, n, b->counts);
+        BK(b->looks.take(b->counts, b->st));
     }
-    cudaError_t inst = cudaSuccess;
-    if (!rc) inst = cudaGraphInstantiate(&b->g_loop, G, 0);
-    cudaGraphDestroy(G);
-    if (rc) return rc;
-    BK(inst);
+    const long long had = b->looks.read;
+    BK(b->looks.read_arrived());
+    if (b->looks.read == had) return ABM_OK;
+    for (int k = 0; k < n; ++k)
+    {
+        b->ctxs[k]->looks.seen(b->looks.n[k]);
+        grown = grown || (may_grow(k) && b->looks.n[k] > b->refs[k]);
+    }
+    if (!grown) return ABM_OK;
+    BK(cudaStreamSynchronize(b->st));
+    for (int k = 0; k < n; ++k)
+    {
+        abm_ctx* c = b->ctxs[k];
+        if (2LL * b->looks.n[k] > b->refs[k]) c->n_ref = 0;     // shaped anew, not only once outgrown
+        shape_launches(c);
+    }
+    b->follow = batch_graphs(b) == ABM_OK;
+    if (!b->follow) { b->err.clear(); g_batch_err.clear(); cudaGetLastError(); }
     return ABM_OK;
 }
 }   // namespace
@@ -2268,11 +2427,14 @@ int abm_batch_create(abm_ctx* const* ctxs, int n, abm_batch** out)
         { delete b; return batch_fail(nullptr, ABM_ERR_STATE, "JKR table not set"); }
         if (c->host_iter % b->k_rebuild != ctxs[0]->host_iter % b->k_rebuild)
         { delete b; return batch_fail(nullptr, ABM_ERR_STATE, "contexts must be in phase of the rebuild cadence"); }
+        // the graphs are made for the sizes of this moment
+        int now = 0;
+        const int rc = abm_get_num_cells(c, &now);
+        if (rc) { const std::string why = c->err; delete b; return batch_fail(nullptr, rc, why); }
+        shape_launches(c);
         if (!c->nbrs_valid) { enqueue_rebuild(c); c->nbrs_valid = true; }
     }
     int rc = ABM_OK;
-    cudaGraph_t GR = nullptr;
-    set_share(b, n);
     do {
         if (cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming) != cudaSuccess)
@@ -2282,22 +2444,9 @@ int abm_batch_create(abm_ctx* const* ctxs, int n, abm_batch** out)
             if (cudaEventCreateWithFlags(&b->ev[k], cudaEventDisableTiming) != cudaSuccess)
                 rc = batch_fail(b, ABM_ERR_CUDA, "event creation failed");
         if (rc) break;
-        if (cudaGraphCreate(&GR, 0) != cudaSuccess)
-        { rc = batch_fail(b, ABM_ERR_CUDA, "graph creation failed"); break; }
-        for (abm_ctx* c : b->ctxs)
-        {
-            std::vector<cudaGraphNode_t> rdeps;
-            rc = capture_into(c, GR, rdeps, [&]() { enqueue_rebuild(c); });
-            if (rc) { rc = batch_fail(b, rc, "rebuild graph of a context: " + c->err); break; }
-        }
-        if (rc) break;
-        if (cudaGraphInstantiate(&b->g_rebuild, GR, 0) != cudaSuccess)
-        { rc = batch_fail(b, ABM_ERR_CUDA, "graph instantiation failed"); break; }
-        rc = batch_loop_graph(b);
-        if (!rc && !b->g_loop) rc = batch_iteration_graph(b);
+        rc = batch_arrays(b);
+        if (!rc) rc = batch_graphs(b);
     } while (0);
-    if (GR) cudaGraphDestroy(GR);
-    set_share(b, 1);
     if (rc) { batch_free(b); delete b; return rc; }
     *out = b;
     return ABM_OK;
@@ -2318,7 +2467,10 @@ int abm_batch_iterate(abm_batch* b, int n_iters)
     }
     for (int it = 0; it < n_iters;)
     {
+        int rc = batch_follow(b);
+        if (rc) return rc;
         int run = std::min(n_iters - it, b->k_rebuild - b->ctxs[0]->host_iter % b->k_rebuild);
+        if (run >= LOOK_RUN + LOOP_FAST) run = LOOK_RUN;
         if (b->g_loop && run >= LOOP_FAST / 2)
         {
             launch_loop_begin_all(b->ctrls, b->divides, n, run, b->st);
@@ -2327,16 +2479,11 @@ int abm_batch_iterate(abm_batch* b, int n_iters)
         else
         {
             run = 1;
-            if (!b->g_iter)
-            {
-                set_share(b, n);
-                const int rc = batch_iteration_graph(b);
-                set_share(b, 1);
-                if (rc) return rc;
-            }
+            if (!b->g_iter) { int rc = batch_iteration_graph(b); if (rc) return rc; }
             BK(cudaGraphLaunch(b->g_iter, b->st));
         }
         it += run;
+        b->looks.since += run;
         bool rebuild = false;
         for (abm_ctx* c : b->ctxs)
         {

@@ -267,7 +267,9 @@ int abm_last_division_tries(abm_ctx* ctx, int* tries);
  * controller -> grow -> refresh distances -> t, iter -> rebuild every
  * iter_update_neighbors.  Stops early when n_cells_stop > 0 and the population
  * reaches it.  Runs asynchronously on the context stream; stats (optional)
- * forces a synchronisation. */
+ * forces a synchronisation.  Where cells divide, the host follows their number to
+ * shape the launches and stays at most some hundreds of iterations ahead of the
+ * device. */
 int abm_iterate(abm_ctx* ctx, int n_iters, int n_cells_stop, abm_stats* stats);
 int abm_get_stats(abm_ctx* ctx, abm_stats* stats);
 /* "conditional" when the iteration graph uses IF/WHILE nodes, otherwise why it could not

@@ -1,0 +1,106 @@
+"""Colonies that grow far beyond the size at which the host last shaped their launches, in one
+long call and in a batch: the same states, bit for bit, as by short calls, and the speed of a
+context made at the present size."""
+import time
+
+import numpy as np
+import pytest
+
+import abm_b200
+from abm_b200 import replicates, workloads
+
+pytestmark = pytest.mark.gpu
+FOUNDERS, STEPS = 32, 8000              # 32 -> 3,800 cells
+
+
+def context(seed, cells=None, **kw):
+    p = dict(replicates.CONFIG0, growth_mean=10.0, growth_std=0.1, max_error_allowed=1e-6, cap_cells=16064, rng_seed=seed)
+    p.update(kw)
+    sim = abm_b200.Simulation(**p)
+    if cells is None:
+        cells = np.asfortranarray(np.tile(workloads.founder_2d(), (FOUNDERS, 1)))
+        cells[:, 0] = np.arange(FOUNDERS)
+        cells[:, 1] += 60.0 * (np.arange(FOUNDERS) % 6)
+        cells[:, 2] += 60.0 * (np.arange(FOUNDERS) // 6)
+        cells[:, 12] = 10.0
+    sim.upload_cells(cells)
+    sim.set_parents(-np.ones(len(cells), dtype=np.int32))
+    sim.set_clock(0.0, 1e-4, 0)
+    sim.get_cell_neighbors()
+    return sim
+
+
+def timed(work, wait):
+    t = time.perf_counter()
+    work()
+    wait()
+    return time.perf_counter() - t
+
+
+def same(a, b):
+    assert a.stats() == b.stats() and a.clock() == b.clock()
+    assert np.array_equal(a.parents(), b.parents())
+    assert np.array_equal(a.download_cells(), b.download_cells())
+
+
+# 0.73 s when the shape stayed that of 32 cells, 0.47 by short calls
+def test_one_long_call():
+    context(5).iterate(100)                                  # what the first call pays
+    one, many, silent = context(1), context(1), context(1)
+    t_one = timed(lambda: one.iterate(STEPS), one.synchronize)
+
+    def short():
+        for _ in range(STEPS // 50):
+            many.iterate(50)
+
+    def no_stats():
+        for _ in range(STEPS // 50):
+            silent.iterate(50, stats=False)
+
+    t_many = timed(short, many.synchronize)
+    t_silent = timed(no_stats, silent.synchronize)
+    print("one call %.3f s, short calls %.3f s, without statistics %.3f s" % (t_one, t_many, t_silent))
+    assert one.stats()["n_cells"] > 64 * FOUNDERS
+    same(one, many)
+    same(one, silent)
+    assert max(t_one, t_silent) < 1.25 * t_many
+    for s in (one, many, silent):
+        s.close()
+
+
+# a rebuild interval longer than a stretch of the loop that the host looks at, not a multiple of it
+def test_long_rebuild_interval():
+    kw = dict(iter_update_neighbors=610, growth_mean=10.0)
+    one, many = context(3, **kw), context(3, **kw)
+    one.iterate(2007)
+    for k in [7] + 40 * [50]:
+        many.iterate(k)
+    same(one, many)
+    assert one.stats()["n_cells"] > FOUNDERS
+    one.close()
+    many.close()
+
+
+# the last stretch 2.2 times as long as in a new batch when the shapes stayed those of 32 cells
+def test_batch_of_founders():
+    sims = [context(10 + k) for k in range(8)]
+    alone = context(13)
+    batch = abm_b200.Batch(sims)
+    batch.iterate(STEPS - 500)
+    batch.synchronize()
+    fresh = [context(10 + k, s.download_cells()) for k, s in enumerate(sims)]
+    for f, s in zip(fresh, sims):
+        f.set_clock(s.clock()[0], s.clock()[1], s.clock()[2])
+    new = abm_b200.Batch(fresh)
+    t_new = timed(lambda: new.iterate(500), new.synchronize)
+    t_old = timed(lambda: batch.iterate(500), batch.synchronize)
+    n_new, n_old = fresh[3].stats()["n_cells"], sims[3].stats()["n_cells"]
+    print("grown batch %.3f s, new batch %.3f s (%d, %d cells)" % (t_old, t_new, n_old, n_new))
+    alone.iterate(STEPS)
+    same(alone, sims[3])
+    assert n_old > 64 * FOUNDERS
+    assert t_old < 1.4 * t_new
+    batch.close()
+    new.close()
+    for s in sims + fresh + [alone]:
+        s.close()
