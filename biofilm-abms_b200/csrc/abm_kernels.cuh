@@ -89,7 +89,6 @@ struct Ctrl {
     unsigned long long eval_err_bits;   // scaled max error of the last API attempt
     int n_pairs;                // pair records made so far by a running build
     int n_sorted;               // cells placed so far by its counting sort
-    int no_table;               // the last build found no neighbor set (an overflow): it is empty
     int n_divided;              // mothers of the last division launch
     int last_div_tries;
     int n_parents;              // length of the lineage vector
@@ -144,12 +143,13 @@ struct Ctrl {
     // rounds as the uninterrupted run's does, although its list has to be made anew.
     double path;
     unsigned long long path_bits;
-    int path_valid;                     // as screen_valid, but for a loaded checkpoint
     // the loop graph (LoopFlow): iterations still to take, and why the plain ones wait
     int todo;
     int hold;                           // LoopHold
     int div_any;                        // a cell grew past Ldiv in the running attempt's step
     int rounds;                         // rounds of the loop graph left (a bound)
+    int no_table;                       // the last build found no neighbor set (an overflow): it is empty
+    int path_valid;                     // as screen_valid, but that a loaded checkpoint keeps it (see path)
 };
 
 // Nothing to do for a kernel of the loop graph?
