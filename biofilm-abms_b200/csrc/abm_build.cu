@@ -529,15 +529,20 @@ __device__ bool make_rows(const BuildArgs& a, int n, int nb, BuildShared& sh, bo
         if (threadIdx.x == 0) a.part[blockIdx.x] = total;
     }
     if (!build_barrier(a, nb)) return false;
+    const int no_table = __ldcg(&a.ctrl->no_table);        // under way beside the offsets' loads
     int2 off, all;
     chunk_offset(a.part, nb, sh, off, all);
-    const bool empty = __ldcg(&a.ctrl->no_table) != 0;
-    if (empty) off.x = all.x = 0;
+    if (no_table)
+    {
+        off.x = all.x = 0;
+        for (int i = c0 + threadIdx.x; i < c1; i += BD_T) a.count[i] &= FLAG_BIT;
+        __syncthreads();
+    }
     for (int i0 = c0; i0 < c1; i0 += BD_T)
     {
         const int i = i0 + threadIdx.x;
         const int v = i < c1 ? a.count[i] : 0;
-        const int2 mine = make_int2(empty ? 0 : v & ~FLAG_BIT, (v & FLAG_BIT) ? 1 : 0);
+        const int2 mine = make_int2(v & ~FLAG_BIT, (v & FLAG_BIT) ? 1 : 0);
         const int2 ex = block_scan(mine, sh, total);
         if (i < c1)
         {
@@ -555,7 +560,7 @@ __device__ bool make_rows(const BuildArgs& a, int n, int nb, BuildShared& sh, bo
     {
         const bool valid = i0 + group < c1;
         const int i = valid ? i0 + group : c0;
-        const int r0 = a.row_ptr[i], len = valid && !empty ? a.count[i] & ~FLAG_BIT : 0;
+        const int r0 = a.row_ptr[i], len = valid ? a.count[i] & ~FLAG_BIT : 0;
         const int* src = a.scratch + (size_t)i * a.bp.cap_per_cell;
         // warp-uniform rounds, so that the shuffles cover all lanes
         int longest = len;
@@ -628,7 +633,8 @@ __device__ __forceinline__ void pair_records(const BuildArgs& a, int n, int nb, 
             while (x < y) { const int mid = (x + y) >> 1; if (a.col[mid] < i) x = mid + 1; else y = mid; }
             // a pair that the caller's rows list more than once: each of its entries with another
             // one of the partner's
-            for (int q = e; q > 0 && a.col[r0 + q - 1] == j; --q) ++x;
+            if (!sorted)
+                for (int q = e; q > 0 && a.col[r0 + q - 1] == j; --q) ++x;
             a.pairs[pos + e] = make_int4(i, j, r0 + e, x);
             if (a.adhere)
             {
