@@ -677,7 +677,7 @@ cudaError_t launch_pair_screened(const Geom* geom, Ctrl* ctrl, ForceParams fp, c
     // caps them per SM).
     LaunchShape shape;
     if (tile <= 0 && blocks_per_sm <= 0)
-        shape = make_shape(fn, PS_T, 2LL * cells + (p ? PS_T : 0), cells <= BUILD_CLUSTER_CELLS / 2, num_sms,
+        shape = make_shape(fn, PS_T, 2LL * cells + (p ? PS_T : 0), cells <= PAIR_CLUSTER_CELLS, num_sms,
                            share);
     else
     {

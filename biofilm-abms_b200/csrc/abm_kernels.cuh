@@ -54,8 +54,8 @@ struct LaunchShape {
     int blocks = 1;
     int cluster = 0;
 };
-// `threads` threads of work in blocks of `block`.  share: the contexts that run side by side in
-// a batch.  A cooperative grid starts when all its blocks have room, so one that fills the chip
+// `threads` threads of work in blocks of `block`, on a `share`-th of the chip (the contexts of a
+// batch run side by side).  A cooperative grid starts when all its blocks have room, so one that fills the chip
 // waits for every other context's work and holds up theirs: a batch of 24 growing colonies of
 // 20,000 cells took 2.8 ms an iteration with whole-chip grids (2.6 as the chain of plain kernels
 // before them) and takes 0.97 with a 24th of the chip each; 8 of them at rest 108 and 56 us.
@@ -411,7 +411,8 @@ struct BuildArgs {
     int* parents;
 };
 enum BuildWhat { BUILD_NEIGHBORS, BUILD_GROWTH, BUILD_DIVIDE, BUILD_RECORDS };
-const int BUILD_CLUSTER_CELLS = 8192;
+const int BUILD_CLUSTER_CELLS = 8192;       // launches shaped for more are cooperative grids
+const int PAIR_CLUSTER_CELLS = BUILD_CLUSTER_CELLS / 2;
 LaunchShape build_shape(int cells, int num_sms, int share = 1);
 cudaError_t launch_build(const BuildArgs& args, int what, const LaunchShape& shape, cudaStream_t st, int flow = FLOW_STEP);
 
