@@ -88,6 +88,7 @@ struct abm_ctx {
     int ncols = 0, has_gamma = 0;
     int n_host = 0;
     bool cells_loaded = false, nbrs_valid = false;
+    bool limited = false;            // a cell limit is set
     int host_iter = 0;
     // device state
     Geom* geom = nullptr; Vel* vel = nullptr; Phys* phys = nullptr; Gen6* fcc = nullptr;
@@ -1506,6 +1507,17 @@ static int build_iteration_graph(abm_ctx* c)
     return ABM_OK;
 }
 
+// A colony that has reached its cell limit stands still: every kernel of a step leaves at once.
+// A call that evaluates its present state (forces, velocities, one attempt) runs the same
+// kernels, so while it does the halt is put aside.
+__global__ void k_halt_aside(Ctrl* c) { c->waiting = c->halted & HALT_CELLS; c->halted &= ~HALT_CELLS; }
+__global__ void k_halt_back(Ctrl* c) { c->halted |= c->waiting; c->waiting = 0; }
+struct Evaluation {
+    abm_ctx* c;
+    explicit Evaluation(abm_ctx* ctx) : c(ctx) { if (c->limited) k_halt_aside<<<1, 1, 0, c->st>>>(c->ctrl); }
+    ~Evaluation() { if (c->limited) k_halt_back<<<1, 1, 0, c->st>>>(c->ctrl); }
+};
+
 // can the colony outgrow the shape of its launches?
 static bool may_outgrow(const abm_ctx* c) { return c->div_enabled && c->n_ref < c->cap; }
 
@@ -1797,7 +1809,7 @@ int abm_cell_cell_forces(abm_ctx* c, double* out)
     int rc = ready_for_forces(c);
     if (rc) return rc;
     if (!c->nbrs_valid) return fail(c, ABM_ERR_STATE, "neighbors not built");
-    enqueue_pair_force(c, 1);
+    { Evaluation e(c); enqueue_pair_force(c, 1); }
     CK(cudaGetLastError());
     if (c->dims == 2)
     {
@@ -1818,7 +1830,7 @@ int abm_get_velocities(abm_ctx* c, double* out)
     int rc = ready_for_forces(c);
     if (rc) return rc;
     if (!c->nbrs_valid) return fail(c, ABM_ERR_STATE, "neighbors not built");
-    enqueue_pair_force(c, 1);
+    { Evaluation e(c); enqueue_pair_force(c, 1); }
     launch_velocities(c->geom, c->vel, c->phys, c->fcc, c->ctrl, c->sp, c->gen_tmp, c->cap, c->st, c->dims);
     CK(cudaGetLastError());
     rc = download_gen6(c, c->gen_tmp, out);
@@ -1836,14 +1848,13 @@ int abm_rk_attempt(abm_ctx* c, double dt, int attempt, double* cells_out, double
     int rc = ready_for_forces(c);
     if (rc) return rc;
     if (!c->nbrs_valid) return fail(c, ABM_ERR_STATE, "neighbors not built");
-    enqueue_pair_force(c, 1);
     k_clear_eval<<<1, 1, 0, c->st>>>(c->ctrl);
     AttemptArgs a = loop_attempt(c);
     a.pg.fused = 0;
     a.err_out = c->gen_tmp;
     a.eval_dt = dt;
     a.eval_attempt = attempt;
-    enqueue_attempt(c, 3, a);
+    { Evaluation e(c); enqueue_pair_force(c, 1); enqueue_attempt(c, 3, a); }
     CK(cudaGetLastError());
     const int n = c->n_host;
     if (cells_out && n > 0)
@@ -2162,6 +2173,7 @@ int abm_set_cell_limit(abm_ctx* c, int n_max)
     if (!c || n_max < 0) return ABM_ERR_ARG;
     k_set_halt<<<1, 1, 0, c->st>>>(c->ctrl, n_max);
     CK(cudaGetLastError());
+    c->limited = n_max > 0;
     return ABM_OK;
 }
 

@@ -150,6 +150,7 @@ struct Ctrl {
     int rounds;                         // rounds of the loop graph left (a bound)
     int no_table;                       // the last build found no neighbor set (an overflow): it is empty
     int path_valid;                     // as screen_valid, but that a loaded checkpoint keeps it (see path)
+    int waiting;                        // HALT_CELLS, while a call evaluates a colony at its limit
 };
 
 // Nothing to do for a kernel of the loop graph?
