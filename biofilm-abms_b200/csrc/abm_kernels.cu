@@ -463,7 +463,7 @@ __global__ void __launch_bounds__(PS_T, 2) k_pair_pass(const Geom* __restrict__ 
     const bool split = PROPOSE && gridDim.x > 1;
     const bool proposer = split && blockIdx.x == gridDim.x - 1;
     const int work_blocks = split ? gridDim.x - 1 : gridDim.x;
-    auto stale = [&](int valid, double moved) { return !valid || !(2.0 * moved * (1.0 + 1e-6) + 1e-9 < fp.skin); };
+    auto stale = [&](const int& valid, const double& moved) { return !valid || !(2.0 * moved * (1.0 + 1e-6) + 1e-9 < fp.skin); };
     const bool refresh = stale(ctrl->screen_valid, ctrl->drift);
     const int rounding = MIXED && stale(ctrl->path_valid, ctrl->path) ? ROUND_STALE : ROUND_LIST;
     const int lane = threadIdx.x & 31;
