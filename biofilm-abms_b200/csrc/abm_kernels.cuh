@@ -84,7 +84,7 @@ struct Ctrl {
     int status;                 // StatusBits
     int n;                      // cells
     int n_dir;                  // directed neighbor entries (2 x pairs)
-    int n_divide;               // mothers in the pending division
+    int no_table;               // the last build found no neighbor set (an overflow): it is empty
     long long attempts, retries, iterations, rebuilds, divisions;
     unsigned long long eval_err_bits;   // scaled max error of the last API attempt
     int n_pairs;                // pair records made so far by a running build
@@ -100,7 +100,7 @@ struct Ctrl {
     unsigned long long st_v2_fx;        // sum |v_r|^2 * 2^STAT_V2_SHIFT
     unsigned long long st_g_fx;         // sum of growth rates * 2^STAT_G_SHIFT
     unsigned long long st_near_div;     // cells with l > 0.9 Ldiv
-    int since_div;                      // iterations since cells last divided
+    int since_div;                      // accepted steps so far (feature 31, abm_propose.cuh)
     double hist_dt[HIST], hist_err[HIST];   // accepted dt and its scaled error, newest at hist_pos - 1
     int hist_acc[HIST];                 // 1 if that iteration's first attempt passed the error test
     int hist_pos;
@@ -148,7 +148,6 @@ struct Ctrl {
     int hold;                           // LoopHold
     int div_any;                        // a cell grew past Ldiv in the running attempt's step
     int rounds;                         // rounds of the loop graph left (a bound)
-    int no_table;                       // the last build found no neighbor set (an overflow): it is empty
     int path_valid;                     // as screen_valid, but that a loaded checkpoint keeps it (see path)
     int waiting;                        // HALT_CELLS, while a call evaluates a colony at its limit
 };
@@ -337,7 +336,6 @@ void launch_attempt_2(int kind, const AttemptArgs& a, int dims, cudaStream_t st)
 void launch_attempt_4(int kind, const AttemptArgs& a, int dims, cudaStream_t st);
 void launch_attempt_6(int kind, const AttemptArgs& a, int dims, cudaStream_t st);
 void launch_attempt_7(int kind, const AttemptArgs& a, int dims, cudaStream_t st);
-// accepted proposal of the learned controller: candidate -> state (no-op otherwise)
 // one frame of the ring: the state after the accepted step that marked it
 struct FrameInfo {
     double t;
@@ -364,7 +362,6 @@ void launch_mlp_grad(const float* master, const float* X, const float* T, int n,
                      cudaStream_t st);
 void launch_mlp_train(float* master, float* m1, float* m2, float* G, const float* X, const float* T, int n,
                       int epochs, float lr, unsigned seed, float* loss_out, cudaStream_t st);
-// features of the running iteration -> log row; with sp.network also the dt of the first attempt
 const int AT_T = 128;           // threads of an attempt block, one cell each
 int attempt_blocks(int cap_cells);
 
@@ -426,8 +423,6 @@ void launch_loop_begin_all(Ctrl* const* ctrls, const int* divides, int n, int to
 // the first pass through its graph only)
 void launch_retry_begin(Ctrl* ctrl, unsigned long long cond, cudaStream_t st);
 void launch_loop_round(Ctrl* ctrl, unsigned long long cond_slow, unsigned long long cond_loop, cudaStream_t st);
-void launch_div_body_pre(Ctrl* ctrl, const int* flags, const int* rank, int* mothers, int cap_cells,
-                         cudaStream_t st);
 // Phenotype switching between two groups and what it drives, after each accepted step
 // (abm_switch.cu): Markov switching (switch.hpp:45-95), the attribute and gamma ramps
 // (simulation.hpp:1872-1957), local viscosity (simulation.hpp:1958-2020) and basal-only

@@ -34,8 +34,9 @@ __device__ __forceinline__ void mma_bf16(float c[4], uint32_t a0, uint32_t a1, u
 //   20..27  1 if that step's first attempt passed the error test
 //   28      mean growth rate (1/h)
 //   29      fraction of cells longer than 0.9 Ldiv
-//   30      log10(1 + cells dividing this iteration)
-//   31      ln(1 + iterations since the last division) / 5
+//   30      0 (the place of the cells dividing in the iteration, which was 0 in every row the
+//           weights were trained on: the count was cleared before it was read)
+//   31      ln(1 + accepted steps so far) / 5 (for the same reason divisions do not restart it)
 // Before any history exists the slots repeat the current dt with error 1, passed.
 //
 // The proposal is ln(dt / dt_prev) = clamp(b + y, ln 0.2, ln 10) with y the network
@@ -128,7 +129,7 @@ static __device__ __forceinline__ void mlp_propose_block(Ctrl* ctrl, const StepP
         feat[29] = (float)(near * inv_n);
         break;
     }
-    case 6: feat[30] = (float)log10(1.0 + (double)ctrl->n_divide); break;
+    case 6: feat[30] = 0.f; break;
     case 7: feat[31] = (float)(log1p((double)ctrl->since_div) / 5.0); break;
     default: break;
     }

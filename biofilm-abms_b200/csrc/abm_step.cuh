@@ -243,7 +243,7 @@ static __device__ void controller_finish(Ctrl* c, const StepParams& sp, int kind
         c->hist_err[h] = E;
         c->hist_acc[h] = c->first_passed;
         c->hist_pos = (h + 1) % HIST;
-        c->since_div = c->n_divide > 0 ? 0 : c->since_div + 1;
+        c->since_div += 1;
         c->cell_steps += c->n;
         c->todo -= 1;
         c->hold = (sp.div_on && (longer || (c->halt_n > 0 && c->n >= c->halt_n))) ? HOLD_START : HOLD_NONE;

@@ -226,7 +226,7 @@ __device__ __forceinline__ void verlet_accept(Ctrl* c)
     c->hist_err[h] = 0.0;
     c->hist_acc[h] = 1;
     c->hist_pos = (h + 1) % HIST;
-    c->since_div = c->n_divide > 0 ? 0 : c->since_div + 1;
+    c->since_div += 1;
     c->cell_steps += c->n;
     c->t += c->dt;
     c->iter += 1;
