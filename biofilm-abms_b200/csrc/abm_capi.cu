@@ -1,11 +1,12 @@
 // C ABI of the B200 mechanics step (declared in include/abm_capi.h).
 //
 // A context owns the device state (cell records, CSR neighbor set, cell-list
-// buffers, controller state), one CUDA stream and two CUDA graphs: one loop
-// iteration (pair force -> trial attempt -> retries -> final attempt with
-// growth) and one neighbor rebuild (bbox -> counting sort -> pair build ->
-// CSR).  All sizes that change during a run (cell count, pair count, bin
-// count) live in device memory, so the graphs are captured once and replayed.
+// buffers, controller state), one CUDA stream and its CUDA graphs: the loop graph,
+// which takes many iterations per launch (append_loop), and graphs of one or a few
+// iterations for short calls, velocity Verlet and the post-step kernels.  The neighbor
+// build and the division are one plain launch (k_build).  All sizes that change during
+// a run (cell count, pair count, bin count) live in device memory; a graph is made
+// anew only when a colony has outgrown the shape of its launches (shape_launches).
 #include <cfloat>
 #include <climits>
 #include <cmath>
@@ -1478,7 +1479,9 @@ static int build_loop_graph(abm_ctx* c)
 static bool has_loop(const abm_ctx* c) { return !c->verlet && !c->post_on; }
 
 // A Verlet run that stops at a cell count looks at it after every 16 single steps, so that it
-// ends on the same step whatever graphs there are.
+// ends on the same step whatever graphs there are.  max_tries_update_stepsize has no other
+// meaning for a Verlet step, which is never retried: with 0 the run goes by graphs of ten steps
+// and looks between those, and callers of either kind may rely on the step where it ends.
 static bool verlet_one_by_one(const abm_ctx* c, int n_cells_stop)
 {
     return c->verlet && c->p.max_tries_update_stepsize > 0 && n_cells_stop > 0 && c->div_enabled;
@@ -2348,24 +2351,26 @@ int batch_graphs(abm_batch* b)
     int rc = batch_rebuild_graph(b);
     if (!rc) rc = batch_loop_graph(b);
     if (!rc && (!b->g_loop || b->g_iter)) rc = batch_iteration_graph(b);
+    if (rc) return rc;
+    // what the graphs were made for
+    std::vector<int> divides;
     b->refs.clear();
-    for (const abm_ctx* c : b->ctxs) b->refs.push_back(c->n_ref);
-    return rc;
+    for (const abm_ctx* c : b->ctxs)
+    {
+        b->refs.push_back(c->n_ref);
+        divides.push_back(c->div_enabled ? 1 : 0);
+    }
+    BK(cudaMemcpy(b->divides, divides.data(), divides.size() * sizeof(int), cudaMemcpyHostToDevice));
+    return ABM_OK;
 }
 
 int batch_arrays(abm_batch* b)
 {
     std::vector<Ctrl*> ctrls;
-    std::vector<int> divides;
-    for (abm_ctx* c : b->ctxs)
-    {
-        ctrls.push_back(c->ctrl);
-        divides.push_back(c->div_enabled ? 1 : 0);
-    }
-    b->looks.n.assign(b->ctxs.size(), 0);
-    BK(cudaMalloc(&b->counts, divides.size() * sizeof(int)));
-    BK(cudaMalloc(&b->divides, divides.size() * sizeof(int)));
-    BK(cudaMemcpy(b->divides, divides.data(), divides.size() * sizeof(int), cudaMemcpyHostToDevice));
+    for (abm_ctx* c : b->ctxs) ctrls.push_back(c->ctrl);
+    b->looks.n.assign(ctrls.size(), 0);
+    BK(cudaMalloc(&b->counts, ctrls.size() * sizeof(int)));
+    BK(cudaMalloc(&b->divides, ctrls.size() * sizeof(int)));
     BK(cudaMalloc(&b->ctrls, ctrls.size() * sizeof(Ctrl*)));
     BK(cudaMemcpy(b->ctrls, ctrls.data(), ctrls.size() * sizeof(Ctrl*), cudaMemcpyHostToDevice));
     return ABM_OK;
@@ -2433,6 +2438,7 @@ int abm_batch_create(abm_ctx* const* ctxs, int n, abm_batch** out)
         if (!c || !c->cells_loaded) { delete b; return batch_fail(nullptr, ABM_ERR_STATE, "every context needs cells"); }
         if (c->post_on)
         { delete b; return batch_fail(nullptr, ABM_ERR_STATE, "switching and basal-only contexts run through abm_iterate"); }
+        // (those with max_tries_update_stepsize = 0 are taken, as verlet_one_by_one tells them apart)
         if (c->verlet && c->p.max_tries_update_stepsize > 0)
         { delete b; return batch_fail(nullptr, ABM_ERR_CUDA, "velocity-Verlet contexts run through abm_iterate"); }
         if (c->dev != dev) { delete b; return batch_fail(nullptr, ABM_ERR_ARG, "contexts on different devices"); }
