@@ -705,8 +705,8 @@ def run_replicates(args):
     """Batched 2-D replicates: args.replicates colonies with log-uniform target sizes in
     [500, 50000], each grown from one founder cell with its own seed (or, with
     --replicate-start near-target, from a seeded colony at 90 % of its target), with
-    config-0 growth and division (BS32, tol 1e-8) until its target; one graph launch per
-    iteration advances all of them.  The screened pair pass's shape per size decade
+    config-0 growth and division (BS32, tol 1e-8) until its target; one graph launch up
+    to the next joint rebuild advances all of them.  The screened pair pass's shape per size decade
     comes from the autotuner.  W + K iterations are run; the line reports the K timed
     ones, whatever sizes the colonies have reached by then."""
     import torch

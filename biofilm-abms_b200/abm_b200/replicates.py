@@ -3,8 +3,8 @@ advanced together, each with its own seed, clock and adaptive step).
 
 The 2-D driver (ABM-2d/ABM-2d-cpp/include/simulation.hpp:163-237) runs one colony
 per job; here every replicate is a context of its own and a Batch advances all of
-them with one CUDA graph launch per iteration.  The screened pair pass's tile and
-grid shape are picked per replicate-size decade by the autotuner
+them with one CUDA graph launch up to their next joint neighbor rebuild.  The screened
+pair pass's tile and grid shape are picked per replicate-size decade by the autotuner
 (abm_autotune_pair_tile).
 """
 import numpy as np

@@ -250,7 +250,7 @@ __device__ __forceinline__ float dot3f(float a0, float b0, float a1, float b1, f
 // and sums are written with their roundings, so that the result does not depend on where the
 // function is inlined: the learned controller rounds its features to BF16, and a last FP32
 // bit can change the steps it takes.  There are three roundings, equally accurate, one for
-// each kind of pass, as the compiler once contracted them there:
+// each kind of pass; one for all would change the last bits of mixed-precision runs:
 enum MixedRounding {
     ROUND_LIST,     // a pass over the active pairs
     ROUND_STALE,    // such a pass after a stale list (see Ctrl::path): the projections of w
