@@ -25,8 +25,8 @@ using namespace abm;
 // How many cells each of one or several contexts holds, as far as the host knows.  Where they
 // divide, the host has the counts copied out after some iterations and reads what has arrived,
 // without a wait unless it is LOOK_AHEAD looks ahead of the device.
-const int LOOK_EVERY = 64;              // iterations, at least, from one look to the next
-const int LOOK_AHEAD = 8;
+const int LOOK_EVERY = 200;             // iterations, at least, from one look to the next (some 5 us each)
+const int LOOK_AHEAD = 4;
 const int LOOK_RUN = 256;               // iterations, at most, of one launch where cells divide
 struct CountLooks {
     std::vector<int> n = {0};
