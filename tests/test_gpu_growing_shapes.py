@@ -43,29 +43,35 @@ def same(a, b):
     assert np.array_equal(a.download_cells(), b.download_cells())
 
 
-# 0.73 s when the shape stayed that of 32 cells, 0.47 by short calls
+# 0.66 s, and 0.72 without statistics, when the shape stayed that of 32 cells; 0.44 by short calls.
+# The better of two runs of each.
 def test_one_long_call():
     context(5).iterate(100)                                  # what the first call pays
-    one, many, silent = context(1), context(1), context(1)
-    t_one = timed(lambda: one.iterate(STEPS), one.synchronize)
 
-    def short():
+    def one(sim):
+        sim.iterate(STEPS)
+
+    def short(sim):
         for _ in range(STEPS // 50):
-            many.iterate(50)
+            sim.iterate(50)
 
-    def no_stats():
+    def silent(sim):
         for _ in range(STEPS // 50):
-            silent.iterate(50, stats=False)
+            sim.iterate(50, stats=False)
 
-    t_many = timed(short, many.synchronize)
-    t_silent = timed(no_stats, silent.synchronize)
-    print("one call %.3f s, short calls %.3f s, without statistics %.3f s" % (t_one, t_many, t_silent))
-    assert one.stats()["n_cells"] > 64 * FOUNDERS
-    same(one, many)
-    same(one, silent)
-    assert max(t_one, t_silent) < 1.25 * t_many
-    for s in (one, many, silent):
-        s.close()
+    best, sims = {}, []
+    for work in (one, short, silent, one, short, silent):
+        sim = context(1)
+        t = timed(lambda: work(sim), sim.synchronize)
+        best[work] = min(t, best.get(work, t))
+        sims.append(sim)
+    print("one call %.3f s, short calls %.3f s, without statistics %.3f s" % (best[one], best[short], best[silent]))
+    assert sims[0].stats()["n_cells"] > 64 * FOUNDERS
+    for other in sims[1:]:
+        same(sims[0], other)
+    assert max(best[one], best[silent]) < 1.3 * best[short]
+    for sim in sims:
+        sim.close()
 
 
 # a rebuild interval longer than a stretch of the loop that the host looks at, not a multiple of it
@@ -81,7 +87,8 @@ def test_long_rebuild_interval():
     many.close()
 
 
-# the last stretch 2.2 times as long as in a new batch when the shapes stayed those of 32 cells
+# the last stretch 2.4 times as long as in a new batch when the shapes stayed those of 32 cells;
+# 1.1 now, more where the graphs are made anew within it
 def test_batch_of_founders():
     sims = [context(10 + k) for k in range(8)]
     alone = context(13)
@@ -99,7 +106,7 @@ def test_batch_of_founders():
     alone.iterate(STEPS)
     same(alone, sims[3])
     assert n_old > 64 * FOUNDERS
-    assert t_old < 1.4 * t_new
+    assert t_old < 1.7 * t_new
     batch.close()
     new.close()
     for s in sims + fresh + [alone]:
