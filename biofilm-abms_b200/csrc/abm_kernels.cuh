@@ -55,10 +55,11 @@ struct LaunchShape {
     int cluster = 0;
 };
 // `threads` threads of work in blocks of `block`, on a `share`-th of the chip (the contexts of a
-// batch run side by side).  A cooperative grid starts when all its blocks have room, so one that fills the chip
-// waits for every other context's work and holds up theirs: a batch of 24 growing colonies of
-// 20,000 cells took 2.8 ms an iteration with whole-chip grids (2.6 as the chain of plain kernels
-// before them) and takes 0.97 with a 24th of the chip each; 8 of them at rest 108 and 56 us.
+// batch run side by side).  A cooperative grid starts when all its blocks have room, so one that
+// fills the chip waits for every other context's work and holds up theirs: a batch of 24 growing
+// colonies of 20,000 cells took 2.8 ms an iteration with whole-chip grids (2.6 as the chain of
+// plain kernels before them) and takes 0.97 with a 24th of the chip each; 8 of them at rest 108
+// and 56 us.
 LaunchShape make_shape(const void* kernel, int block, long long threads, bool cluster, int num_sms, int share);
 // the runtime's answer: a launch that it refuses did not happen
 cudaError_t launch_shape(const void* kernel, const LaunchShape& shape, int block, void** args, cudaStream_t st);
